@@ -126,7 +126,7 @@ int check_stage1(const ft_decode_args* a) {
 // Can the warp-MMA kernel take these arguments?  Returns a reason or NULL.
 const char* mma_obstacle(const ft_decode_args* a) {
   if (a->dtype == FT_F32) return "fp32 inputs";
-  if (a->head_dim != 64 && a->head_dim != 128) return "head_dim not 64 or 128";
+  if (a->head_dim != 64 && a->head_dim != 128 && a->head_dim != 256) return "head_dim not 64, 128 or 256";
   if (!aligned16(a->q) || !aligned16(a->k_buffer) || !aligned16(a->v_buffer)) return "q/k/v not 16-byte aligned";
   if (a->q_stride0 % 8 || a->q_stride1 % 8 || a->k_stride0 % 8 || a->k_stride1 % 8 || a->v_stride0 % 8 ||
       a->v_stride1 % 8)
@@ -150,8 +150,10 @@ int pick_path(const ft_decode_args* a) {
   if (a->path == FT_PATH_MMA || a->path == FT_PATH_TCGEN05 || a->path == FT_PATH_MMA_WIDE || a->path == FT_PATH_STREAM ||
       a->path == FT_PATH_PERSIST) {
     if (why != nullptr) return fail(FT_ERR_UNSUPPORTED, "tensor-core path unavailable: %s", why);
-    if ((a->path == FT_PATH_TCGEN05 || a->path == FT_PATH_PERSIST) && a->head_dim != 128)
-      return fail(FT_ERR_UNSUPPORTED, "the tcgen05 kernels need head_dim 128, got %d", a->head_dim);
+    if (a->path == FT_PATH_PERSIST && a->head_dim != 128)
+      return fail(FT_ERR_UNSUPPORTED, "the persistent kernel needs head_dim 128, got %d", a->head_dim);
+    if (a->path != FT_PATH_TCGEN05 && a->head_dim == 256)
+      return fail(FT_ERR_UNSUPPORTED, "head_dim 256 has the tcgen05 kernel only");
     return a->path;
   }
   if (a->path != FT_PATH_AUTO) return fail(FT_ERR_INVALID_ARGUMENT, "unknown path %d", a->path);
@@ -356,10 +358,10 @@ ft::TcParams tc_params(const ft::Stage1Params& p, const ft_decode_args* a) {
                              a->k_stride1, 1, 64) &&
                tensor_map_3d(&tp.v_map, a->v_buffer, a->dtype, d, a->kv_rows, a->num_kv_heads, a->v_stride0,
                              a->v_stride1, 1, 64);
-  // Q by TMA (tcgen05 kernel, head_dim 128): one box per request covering its G heads (at most 8 per box), or one
+  // Q by TMA (tcgen05 kernel): one box per request covering its G heads (at most 8 per box), or one
   // box for a whole tile of consecutive requests, when G is a power of two up to 128
   const int g = p.group;
-  if (tp.has_tma && d == 128 && g >= 1 && g <= 128 && (g & (g - 1)) == 0) {
+  if (tp.has_tma && g >= 1 && g <= 128 && (g & (g - 1)) == 0) {
     const int box_heads = g < 8 ? g : 8;
     if (tensor_map_3d(&tp.q_map, a->q, a->dtype, d, a->batch, a->num_qo_heads, a->q_stride0, a->q_stride1, box_heads, 1) &&
         tensor_map_3d(&tp.q_map_tile, a->q, a->dtype, d, a->batch, a->num_qo_heads, a->q_stride0, a->q_stride1, g, 128 / g))
@@ -368,14 +370,14 @@ ft::TcParams tc_params(const ft::Stage1Params& p, const ft_decode_args* a) {
   return tp;
 }
 
-template <typename T>
+template <typename T, int D>
 int launch_tc(const ft::TcParams& p, int hkv, cudaStream_t st) {
-  using C = ft::TcCfg;
+  using C = ft::TcCfg<D>;
   if (dry_run("stage1_tc_kernel")) return FT_OK;
   static OncePerDevice once;
-  FT_CUDA_OK(raise_smem_limit(once, ft::stage1_tc_kernel<T>, C::SMEM_BYTES));
+  FT_CUDA_OK(raise_smem_limit(once, ft::stage1_tc_kernel<T, D>, C::SMEM_BYTES));
   const unsigned grid = (unsigned)p.p.node_count * (unsigned)hkv;
-  FT_CUDA_OK(launch_early(ft::stage1_tc_kernel<T>, grid, C::THREADS, C::SMEM_BYTES, st, p));
+  FT_CUDA_OK(launch_early(ft::stage1_tc_kernel<T, D>, grid, C::THREADS, C::SMEM_BYTES, st, p));
   count_launch();
   return FT_OK;
 }
@@ -412,16 +414,16 @@ int launch_persist(ft::TcParams p, int hkv, cudaStream_t st) {
   return FT_OK;
 }
 
-template <typename T>
+template <typename T, int D>
 int launch_fused(ft::TcParams p, int hkv, cudaStream_t st) {
-  constexpr int smem_a = ft::TcCfg::SMEM_BYTES > ft::StreamCfg<128>::SMEM_BYTES ? ft::TcCfg::SMEM_BYTES
-                                                                                : ft::StreamCfg<128>::SMEM_BYTES;
-  constexpr int smem = smem_a > ft::NarrowCfg<128, 2>::SMEM_BYTES ? smem_a : ft::NarrowCfg<128, 2>::SMEM_BYTES;
+  constexpr int smem_a = ft::TcCfg<D>::SMEM_BYTES > ft::StreamCfg<D>::SMEM_BYTES ? ft::TcCfg<D>::SMEM_BYTES
+                                                                                    : ft::StreamCfg<D>::SMEM_BYTES;
+  constexpr int smem = smem_a > ft::NarrowCfg<D, 2>::SMEM_BYTES ? smem_a : ft::NarrowCfg<D, 2>::SMEM_BYTES;
   static_assert(smem <= 115712, "two CTAs must fit in one SM's shared memory");
   if (dry_run("stage1_fused_kernel")) return FT_OK;
   static OncePerDevice once;
   int dev = 0;
-  FT_CUDA_OK(raise_smem_limit(once, ft::stage1_fused_kernel<T>, smem, &dev));
+  FT_CUDA_OK(raise_smem_limit(once, ft::stage1_fused_kernel<T, D>, smem, &dev));
   // Few-row tasks: a full set of persistent workers when each would get several tasks and the many-row CTAs
   // do not fill the device more than once (the task pipeline then hides the per-task start-up; the workers
   // take the slots the many-row CTAs leave and, as those finish, theirs too); one CTA per task otherwise (the
@@ -439,29 +441,29 @@ int launch_fused(ft::TcParams p, int hkv, cudaStream_t st) {
   if (wide + few_ctas > 0x7fffffffLL) return fail(FT_ERR_TOO_LARGE, "vnodes x kv heads exceeds the grid limit");
   p.p.workers = (int)workers;
   p.p.lead_wide = (int)lead;
-  FT_CUDA_OK(launch_early(ft::stage1_fused_kernel<T>, (unsigned)(wide + few_ctas), ft::TcCfg::THREADS, smem, st, p));
+  FT_CUDA_OK(launch_early(ft::stage1_fused_kernel<T, D>, (unsigned)(wide + few_ctas), ft::TcCfg<D>::THREADS, smem, st, p));
   count_launch();
   return FT_OK;
 }
 
-// path: AUTO (<= 16 rows: persistent workers or narrow; above: tcgen05 when head_dim is 128, else wide),
+// path: AUTO (<= 16 rows: persistent workers or narrow; above: tcgen05; head_dim 256 has the tcgen05 kernel only),
 // STREAM (like AUTO, always the persistent workers), MMA (narrow / wide), MMA_WIDE (wide for everything),
 // TCGEN05 (tcgen05 for everything)
 template <typename T, int D>
 int launch_tensor(const ft::Stage1Params& p, const ft_decode_args* a, int hkv, cudaStream_t st, int max_rows, int path) {
-  if constexpr (D == 128) {
-    if (path == FT_PATH_TCGEN05 || ((path == FT_PATH_AUTO || path == FT_PATH_STREAM) && max_rows > 16))
-      return launch_tc<T>(tc_params(p, a), hkv, st);
+  if (D == 256 || path == FT_PATH_TCGEN05 || ((path == FT_PATH_AUTO || path == FT_PATH_STREAM) && max_rows > 16))
+    return launch_tc<T, D>(tc_params(p, a), hkv, st);
+  if constexpr (D != 256) {
+    if (max_rows <= 16) {
+      // few-row tasks only: persistent workers when there are several tasks per CTA slot, else one CTA per task
+      int dev = 0;
+      FT_CUDA_OK(cudaGetDevice(&dev));
+      const bool many = (int64_t)p.node_count * hkv >= 8LL * sm_count(dev);
+      if (path == FT_PATH_STREAM || (path == FT_PATH_AUTO && many)) return launch_stream<T, D>(tc_params(p, a), hkv, st);
+    }
+    if (path != FT_PATH_MMA_WIDE && max_rows <= 16) return launch_narrow<T, D>(p, hkv, st);
+    return launch_mma<T, D>(p, hkv, st);
   }
-  if (max_rows <= 16) {
-    // few-row tasks only: persistent workers when there are several tasks per CTA slot, else one CTA per task
-    int dev = 0;
-    FT_CUDA_OK(cudaGetDevice(&dev));
-    const bool many = (int64_t)p.node_count * hkv >= 8LL * sm_count(dev);
-    if (path == FT_PATH_STREAM || (path == FT_PATH_AUTO && many)) return launch_stream<T, D>(tc_params(p, a), hkv, st);
-  }
-  if (path != FT_PATH_MMA_WIDE && max_rows <= 16) return launch_narrow<T, D>(p, hkv, st);
-  return launch_mma<T, D>(p, hkv, st);
 }
 
 // fp32 storage at head_dim 64 / 128 with 16-byte aligned rows: the tiled CUDA-core kernel
@@ -504,11 +506,18 @@ int launch_stage1_range(const ft_decode_args* a, int path, int offset, int count
   cudaStream_t st = static_cast<cudaStream_t>(a->stream);
   const int hkv = a->num_kv_heads;
   if (path != FT_PATH_GENERIC) {
-    if (a->dtype == FT_F16)
-      return a->head_dim == 128 ? launch_tensor<__half, 128>(p, a, hkv, st, max_rows, path)
-                                : launch_tensor<__half, 64>(p, a, hkv, st, max_rows, path);
-    return a->head_dim == 128 ? launch_tensor<__nv_bfloat16, 128>(p, a, hkv, st, max_rows, path)
-                              : launch_tensor<__nv_bfloat16, 64>(p, a, hkv, st, max_rows, path);
+    const bool f16 = a->dtype == FT_F16;
+    switch (a->head_dim) {
+      case 64:
+        return f16 ? launch_tensor<__half, 64>(p, a, hkv, st, max_rows, path)
+                   : launch_tensor<__nv_bfloat16, 64>(p, a, hkv, st, max_rows, path);
+      case 128:
+        return f16 ? launch_tensor<__half, 128>(p, a, hkv, st, max_rows, path)
+                   : launch_tensor<__nv_bfloat16, 128>(p, a, hkv, st, max_rows, path);
+      default:
+        return f16 ? launch_tensor<__half, 256>(p, a, hkv, st, max_rows, path)
+                   : launch_tensor<__nv_bfloat16, 256>(p, a, hkv, st, max_rows, path);
+    }
   }
   // fp32 storage: the tiled kernel when the caller named no path (FT_PATH_GENERIC stays the scalar kernel) and the
   // phase's request tile bounds its rows
@@ -602,7 +611,7 @@ int ft_stage1(const ft_decode_args* a) {
   const int64_t r1 = a->phase_q_tile_sizes[1] > 0 ? (int64_t)a->phase_q_tile_sizes[1] * group : 1 << 30;
   const int rows0 = (int)(r0 < (1 << 30) ? r0 : (1 << 30)), rows1 = (int)(r1 < (1 << 30) ? r1 : (1 << 30));
   const bool same_kernel = path == FT_PATH_GENERIC || path == FT_PATH_MMA_WIDE || path == FT_PATH_TCGEN05 ||
-                           ((rows0 > 16) == (rows1 > 16));
+                           a->head_dim == 256 || ((rows0 > 16) == (rows1 > 16));
   // the persistent kernel takes every task of the launch, whatever its row count
   if (path == FT_PATH_PERSIST && a->device_phase_info != nullptr) {
     ft::Stage1Params p = stage1_params(a);  // node_offset / node_count come from the device array
@@ -626,16 +635,19 @@ int ft_stage1(const ft_decode_args* a) {
     }
     return FT_OK;
   }
-  // head_dim 128, many-row phase followed directly by the few-row phase: one grid with both kernel bodies
-  if (path == FT_PATH_AUTO && a->head_dim == 128 && n0 > 0 && n1 > 0 && o1 == o0 + n0 && rows0 > 16 && rows1 <= 16) {
+  // head_dim 64 / 128, many-row phase followed directly by the few-row phase: one grid with both kernel bodies
+  if (path == FT_PATH_AUTO && a->head_dim <= 128 && n0 > 0 && n1 > 0 && o1 == o0 + n0 && rows0 > 16 && rows1 <= 16) {
     ft::Stage1Params p = stage1_params(a);
     p.node_offset = o0;
     p.node_count = n0 + n1;
     p.node_split = n0;
     cudaStream_t st = static_cast<cudaStream_t>(a->stream);
     const ft::TcParams tp = tc_params(p, a);
-    return a->dtype == FT_F16 ? launch_fused<__half>(tp, a->num_kv_heads, st)
-                              : launch_fused<__nv_bfloat16>(tp, a->num_kv_heads, st);
+    if (a->head_dim == 64)
+      return a->dtype == FT_F16 ? launch_fused<__half, 64>(tp, a->num_kv_heads, st)
+                                : launch_fused<__nv_bfloat16, 64>(tp, a->num_kv_heads, st);
+    return a->dtype == FT_F16 ? launch_fused<__half, 128>(tp, a->num_kv_heads, st)
+                              : launch_fused<__nv_bfloat16, 128>(tp, a->num_kv_heads, st);
   }
   // Adjacent phases that want the same kernel go out as one grid.
   if (n0 > 0 && n1 > 0 && o1 == o0 + n0 && same_kernel)

@@ -111,9 +111,10 @@ int build_plan(const int32_t* parent, const int32_t* seqlen, int32_t n_nodes, co
     if (m.num_sms <= 0 || m.ctas_per_sm <= 0 || !(m.waves > 0) || m.tile_tokens <= 0 || m.rows_per_cta <= 0 ||
         m.min_chunk <= 0 || m.nominal_split <= 0 || !(m.ridge_flop_per_byte > 0) || m.elem_bytes <= 0)
       return FT_ERR_INVALID_ARGUMENT;
-  } else if (head_dim == 128) {
+  } else if (head_dim == 64 || head_dim == 128 || head_dim == 256) {
     m.rows_per_cta = 128;  // the tcgen05 stage-1 kernel holds 128 query rows per CTA
-    m.ridge_flop_per_byte = 4 * m.ridge_flop_per_byte;
+    m.ridge_flop_per_byte = (head_dim == 64 ? 2 : 4) * m.ridge_flop_per_byte;
+    if (head_dim == 256) m.ctas_per_sm = 1;
   }
   ft_plan* plan = new (std::nothrow) ft_plan();
   if (plan == nullptr) return FT_ERR_TOO_LARGE;

@@ -73,35 +73,45 @@
 
 namespace ft {
 
+// D: head_dim, 64, 128 or 256.  An operand row is NB = D / 64 blocks of 128 bytes, one after the other as [rows][128 B];
+// shared memory and tensor memory hold two CTAs per SM at head_dim 64 and 128, one at 256 (O alone is 256 columns).
+// Measured per decode step against the kernels that took these head sizes before: 64 requests on a 4096-token prefix,
+// 16/8 heads of 256 15 741 -> 58.5 us (scalar kernel before; every row re-read K and V); 512 leaves under 1,4,16 nodes,
+// 32/8 heads of 64 101 -> 69.6 us (mma.sync, 51.5 us of it, and a second launch for the leaves before).
+template <int D_>
 struct TcCfg {
   static constexpr int THREADS = 256;
   static constexpr int ROWS = 128;    // query rows per pass (UMMA M)
   static constexpr int TILE = 64;     // tokens per tile (UMMA N of S, K of P.V)
-  static constexpr int D = 128;
-  static constexpr int Q_OFF = 0;                     // 2 blocks x [128 rows][128 B]
-  static constexpr int NSK = 3;                       // K ring: one stage more than V, K being needed a softmax earlier
-  static constexpr int K_OFF = 32768;                 // NSK buffers x (2 blocks x [64 tok][128 B])
-  static constexpr int V_OFF = K_OFF + NSK * 16384;   // 2 buffers, same shape
+  static constexpr int D = D_;
+  static constexpr int NB = D / 64;
+  static constexpr int TILE_BYTES = NB * 8192;        // one K or V tile: NB blocks x [64 tok][128 B]
+  static constexpr int Q_OFF = 0;                     // NB blocks x [128 rows][128 B]
+  static constexpr int NSK = D == 256 ? 2 : 3;        // K ring: one stage more than V, K being needed a softmax earlier
+  static constexpr int K_OFF = NB * 16384;
+  static constexpr int V_OFF = K_OFF + NSK * TILE_BYTES;   // 2 buffers
   static constexpr int IDX_SLOTS = 3;
-  static constexpr int IDX_OFF = V_OFF + 2 * 16384;   // IDX_SLOTS x 64 row ids
+  static constexpr int IDX_OFF = V_OFF + 2 * TILE_BYTES;   // IDX_SLOTS x 64 row ids
   static constexpr int BAR_OFF = IDX_OFF + IDX_SLOTS * 64 * 4;
   static constexpr int NBARS = 18;
   static constexpr int ABORT_OFF = BAR_OFF + NBARS * 8;
   static constexpr int TMEM_SLOT_OFF = ABORT_OFF + 4;
   static constexpr int SMEM_BYTES = TMEM_SLOT_OFF + 4;
-  static constexpr int TMEM_COLS = 256;
+  static constexpr int TMEM_COLS = D == 256 ? 512 : 256;
   static constexpr int S_COL = 0, O_COL = 128;        // S is double-buffered: columns [0,64) and [64,128)
   static constexpr int WAIT_LIMIT = 1 << 16;          // probes of mbarrier.try_wait before a wait gives up
   // barrier indices
   static constexpr int K_FULL = 0, K_EMPTY = 3, V_FULL = 6, V_EMPTY = 8, S_FULL = 10, P_FULL = 12, PV_DONE = 14,
                        Q_FULL = 16;
-  static constexpr int OUT_STRIDE = 528;              // bytes between staged output rows (512 + 16: conflict-free 16-byte stores)
+  static constexpr int OUT_STRIDE = D * 4 + 16;       // bytes between staged output rows (+ 16: conflict-free 16-byte stores)
   static constexpr int REGS_SOFTMAX = 184, REGS_OTHER = 72;
   static constexpr int REGS_WORKER = 232;             // few-row workers of the fused kernel: four warps, the other four leave
+  static constexpr int CPR = D / 8, RPI = 32 / CPR;   // gathers: 16-byte chunks per row, rows per warp instruction
+  static_assert(D == 256 || SMEM_BYTES <= 115712, "two CTAs must fit in one SM's shared memory");
+  static_assert(SMEM_BYTES <= 232448, "one CTA must fit in one SM's shared memory");
+  static_assert(128 * OUT_STRIDE <= IDX_OFF, "the staged output rows reuse the Q, K and V buffers");
+  static_assert((REGS_SOFTMAX + REGS_OTHER) * 128 <= 2 * 128 * 128, "register trade must balance");
 };
-static_assert(TcCfg::SMEM_BYTES <= 115712, "two CTAs must fit in one SM's shared memory");
-static_assert(128 * TcCfg::OUT_STRIDE <= TcCfg::IDX_OFF, "the staged output rows reuse the Q, K and V buffers");
-static_assert((TcCfg::REGS_SOFTMAX + TcCfg::REGS_OTHER) * 128 <= 2 * 128 * 128, "register trade must balance");
 
 template <int N>
 __device__ __forceinline__ void reg_grow() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(N)); }
@@ -209,7 +219,7 @@ __device__ __forceinline__ float exp2_fma(float x) {
 // Bounded wait for the phase of `bar` with the given parity.  Gives up after WAIT_LIMIT probes or as soon as
 // another role has raised the CTA's abort flag; the caller then raises the flag itself and unwinds.
 __device__ __forceinline__ bool tc_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-  for (int it = 0; it < TcCfg::WAIT_LIMIT; ++it) {
+  for (int it = 0; it < TcCfg<128>::WAIT_LIMIT; ++it) {
     uint32_t ok;
     asm volatile(
         "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
@@ -226,14 +236,15 @@ __device__ __forceinline__ bool tc_wait(uint32_t bar, uint32_t parity, volatile 
 // zero-fill invalid rows themselves, so the loop has no branch.  Kept out of line: tiles of consecutive rows - every
 // tile of the benchmark shapes - never come here, and their loaders' code stays as small as it was.
 // ids in shared memory (K loader); returns true when a row id inside the chunk was out of range
-template <typename T>
+template <typename T, int D>
 __device__ __noinline__ bool tc_gather_tile_smem(uint32_t buf, const T* base, int64_t stride, const int* ids, int t, int id_lim,
                                                  uint32_t row_lim, int lane) {
-  const int c = lane & 15;
+  using C = TcCfg<D>;
+  const int c = lane % C::CPR;
   bool bad = false;
 #pragma unroll 4
-  for (int i = 0; i < 32; ++i) {
-    const int r = (lane >> 4) + 2 * i, pos = t * TcCfg::TILE + r;
+  for (int i = 0; i < C::TILE / C::RPI; ++i) {
+    const int r = lane / C::CPR + C::RPI * i, pos = t * C::TILE + r;
     const uint32_t row = pos < id_lim ? (uint32_t)ids[r] : 0xffffffffu;
     const bool ok = row < row_lim;  // padding (0xffffffff), negative and too-large ids all fail this test
     bad |= !ok && pos < id_lim;
@@ -242,16 +253,17 @@ __device__ __noinline__ bool tc_gather_tile_smem(uint32_t buf, const T* base, in
   return bad;
 }
 // ids in registers, two per lane: row r is slot r >> 5 of lane r & 31 (V loader)
-template <typename T>
+template <typename T, int D>
 __device__ __noinline__ bool tc_gather_tile_regs(uint32_t buf, const T* base, int64_t stride, int id0, int id1, int t, int id_lim,
                                                  uint32_t row_lim, int lane) {
-  const int c = lane & 15;
+  using C = TcCfg<D>;
+  const int c = lane % C::CPR;
   bool bad = false;
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
 #pragma unroll 4
-    for (int i = 0; i < 16; ++i) {
-      const int r = (lane >> 4) + 2 * i + 32 * h, pos = t * TcCfg::TILE + r;
+    for (int i = 0; i < 32 / C::RPI; ++i) {
+      const int r = lane / C::CPR + C::RPI * i + 32 * h, pos = t * C::TILE + r;
       const int id = __shfl_sync(0xffffffffu, h == 0 ? id0 : id1, r & 31);
       const uint32_t row = pos < id_lim ? (uint32_t)id : 0xffffffffu;
       const bool ok = row < row_lim;
@@ -262,9 +274,9 @@ __device__ __noinline__ bool tc_gather_tile_regs(uint32_t buf, const T* base, in
   return bad;
 }
 
-template <typename T>
+template <typename T, int D>
 __device__ __forceinline__ void tc_body(const TcParams& tp, uint8_t* smem, const int vn, const int kvh) {
-  using C = TcCfg;
+  using C = TcCfg<D>;
   const Stage1Params& p = tp.p;
   const uint32_t sm = smem_u32(smem);
   const uint32_t q_sm = sm + C::Q_OFF, idx_sm = sm + C::IDX_OFF, bars = sm + C::BAR_OFF;
@@ -344,8 +356,8 @@ __device__ __forceinline__ void tc_body(const TcParams& tp, uint8_t* smem, const
   const int32_t* ids_of_chunk = kv_ids_base(p, kv_off);
   if (rows > 0 && id_lim < kv_len && tid == 0) flag_error(FT_DEV_BAD_KV_INDEX);
   const uint32_t row_lim = (uint32_t)(p.kv_rows < 0x7fffffffLL ? p.kv_rows : 0x7fffffffLL);
-  auto k_buf = [&](int t) { return sm + C::K_OFF + (t % C::NSK) * 16384; };
-  auto v_buf = [&](int t) { return sm + C::V_OFF + (t & 1) * 16384; };
+  auto k_buf = [&](int t) { return sm + C::K_OFF + (t % C::NSK) * C::TILE_BYTES; };
+  auto v_buf = [&](int t) { return sm + C::V_OFF + (t & 1) * C::TILE_BYTES; };
 
   // Tiles are numbered g = 0, 1, 2, ... across passes; tile g uses V / S buffer g & 1 for the (g >> 1)-th time and K
   // buffer g % NSK for the (g / NSK)-th time, which gives every wait its barrier phase without per-barrier counters.
@@ -477,7 +489,7 @@ __device__ __forceinline__ void tc_body(const TcParams& tp, uint8_t* smem, const
             }
             tc_fence_after();
 #pragma unroll
-            for (int cb = 0; cb < 4; ++cb) {  // this warp's rows of O in tensor memory
+            for (int cb = 0; cb < D / 32; ++cb) {  // this warp's rows of O in tensor memory
               float o[32];
               tmem_ld32(t_lane + C::O_COL + cb * 32, o);
 #pragma unroll
@@ -515,7 +527,7 @@ __device__ __forceinline__ void tc_body(const TcParams& tp, uint8_t* smem, const
           // stage the normalised row in shared memory (every operand buffer is idle by now)
           const uint32_t out_row = sm + (uint32_t)tid * C::OUT_STRIDE;
 #pragma unroll
-          for (int cb = 0; cb < 4; ++cb) {
+          for (int cb = 0; cb < D / 32; ++cb) {
             float o[32];
             if (ntiles > 0) {
               tmem_ld32(t_lane + C::O_COL + cb * 32, o);  // warp-collective: every lane of the warp takes part
@@ -532,18 +544,24 @@ __device__ __forceinline__ void tc_body(const TcParams& tp, uint8_t* smem, const
           if (tid == 0) FT_TL_MARK(8);
           if (store)
             p.mid_lse[part * p.ml_s0 + head] = l_run > 0.f ? (m_used + log2f(l_run)) * 0.6931471805599453f : -INFINITY;
-          // each warp staged its own 32 rows: write them out one row per instruction (32 lanes x 16 bytes)
+          // each warp staged its own 32 rows: write them out in full-row pieces of 512 bytes (32 lanes x 16 bytes; two
+          // rows at a time at head_dim 64, two pieces per row at 256)
           __syncwarp();
           float* my_dst = store ? p.mid_o + part * p.mo_s0 + (int64_t)head * p.mo_s1 : nullptr;
-          const uint32_t warp_rows = sm + (uint32_t)(warp * 32) * C::OUT_STRIDE + lane * 16;
+          constexpr int LPR = D >= 128 ? 32 : D / 4, RPS = 32 / LPR;  // lanes per row, rows per store instruction
+          const uint32_t warp_rows = sm + (uint32_t)(warp * 32 + lane / LPR) * C::OUT_STRIDE + (lane % LPR) * 16;
 #pragma unroll 16
-          for (int i = 0; i < 32; ++i) {
-            float* dst = reinterpret_cast<float*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(my_dst), i));
-            float4 x;
-            asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];\n"
-                         : "=f"(x.x), "=f"(x.y), "=f"(x.z), "=f"(x.w)
-                         : "r"(warp_rows + i * C::OUT_STRIDE));
-            if (dst != nullptr) reinterpret_cast<float4*>(dst)[lane] = x;
+          for (int i = 0; i < 32 / RPS; ++i) {
+            float* dst = reinterpret_cast<float*>(
+                __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(my_dst), i * RPS + lane / LPR));
+#pragma unroll
+            for (int h = 0; h < (D + 127) / 128; ++h) {
+              float4 x;
+              asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];\n"
+                           : "=f"(x.x), "=f"(x.y), "=f"(x.z), "=f"(x.w)
+                           : "r"(warp_rows + i * RPS * C::OUT_STRIDE + h * 512));
+              if (dst != nullptr) reinterpret_cast<float4*>(dst)[lane % LPR + 32 * h] = x;
+            }
           }
           if (tid == 0) FT_TL_MARK(9);
         }
@@ -556,7 +574,7 @@ __device__ __forceinline__ void tc_body(const TcParams& tp, uint8_t* smem, const
       if (warp >= 6) {
         // ================================================================ Q gather (64 threads)
         // request ids of this pass's slots -> the (still unused) V buffers, then the rows themselves
-        const int qt = tid - 192, ld_c = qt & 15, ld_r = qt >> 4;
+        const int qt = tid - 192, ld_c = qt % C::CPR, ld_r = qt / C::CPR;
         const int row_end = min(rows, row0 + C::ROWS);
         const int first_slot = row0 / G, nslots = (row_end - 1) / G - first_slot + 1;  // <= 128
         for (int i = qt; i < nslots; i += 64) {
@@ -583,9 +601,10 @@ __device__ __forceinline__ void tc_body(const TcParams& tp, uint8_t* smem, const
         }
         if (in_order) {
           if (qt == 0) {
-            mbar_arrive_expect_tx(bar(C::Q_FULL), 32768);  // full boxes: rows past the task's requests are dead rows
-            tma_load_3d(q_sm, &tp.q_map_tile, 0, kvh * G, req_of[0], bar(C::Q_FULL));
-            tma_load_3d(q_sm + 16384, &tp.q_map_tile, 64, kvh * G, req_of[0], bar(C::Q_FULL));
+            mbar_arrive_expect_tx(bar(C::Q_FULL), C::NB * 16384);  // full boxes: rows past the task's requests are dead rows
+#pragma unroll
+            for (int h = 0; h < C::NB; ++h)
+              tma_load_3d(q_sm + h * 16384, &tp.q_map_tile, 64 * h, kvh * G, req_of[0], bar(C::Q_FULL));
           } else {
             mbar_arrive(bar(C::Q_FULL));
           }
@@ -597,7 +616,7 @@ __device__ __forceinline__ void tc_body(const TcParams& tp, uint8_t* smem, const
           for (int i = qt; i < nslots; i += 64) {
             const int req = req_of[i];
             if (req >= 0 && req < p.batch)
-              bytes += (uint32_t)G * 256u;
+              bytes += (uint32_t)G * (2u * D);
             else if ((int64_t)q_off + first_slot + i >= 0 && (int64_t)q_off + first_slot + i < p.num_partial_rows)
               flag_error(FT_DEV_BAD_Q_INDEX);
           }
@@ -608,15 +627,16 @@ __device__ __forceinline__ void tc_body(const TcParams& tp, uint8_t* smem, const
               for (int sub = 0; sub < G; sub += br) {
                 const int r = i * G + sub;
                 const uint32_t dst = q_sm + (uint32_t)((r >> 3) * 1024 + (r & 7) * 128);
-                tma_load_3d(dst, &tp.q_map, 0, kvh * G + sub, req, bar(C::Q_FULL));
-                tma_load_3d(dst + 16384, &tp.q_map, 64, kvh * G + sub, req, bar(C::Q_FULL));
+#pragma unroll
+                for (int h = 0; h < C::NB; ++h)
+                  tma_load_3d(dst + h * 16384, &tp.q_map, 64 * h, kvh * G + sub, req, bar(C::Q_FULL));
               }
             }
           }
         } else {
 #pragma unroll 4
-          for (int ps = 0; ps < 32; ++ps) {
-            const int r = ps * 4 + ld_r;
+          for (int ps = 0; ps < C::ROWS * C::CPR / 64; ++ps) {
+            const int r = ps * (64 / C::CPR) + ld_r;
             const int prow = row0 + r;
             int64_t src = -1;
             if (prow < rows) {
@@ -668,14 +688,14 @@ __device__ __forceinline__ void tc_body(const TcParams& tp, uint8_t* smem, const
 #endif
             if (dense) {
               if (lane == 0) {
-                mbar_arrive_expect_tx(full, 16384);
-                tma_load_3d(buf, &tp.v_map, 0, kvh, first_row, full);
-                tma_load_3d(buf + 8192, &tp.v_map, 64, kvh, first_row, full);
+                mbar_arrive_expect_tx(full, C::TILE_BYTES);
+#pragma unroll
+                for (int h = 0; h < C::NB; ++h) tma_load_3d(buf + h * 8192, &tp.v_map, 64 * h, kvh, first_row, full);
               } else {
                 mbar_arrive(full);
               }
             } else {
-              const bool bad = tc_gather_tile_regs<T>(buf, vbase, p.v_s0, cur[0], cur[1], t, id_lim, row_lim, lane);
+              const bool bad = tc_gather_tile_regs<T, D>(buf, vbase, p.v_s0, cur[0], cur[1], t, id_lim, row_lim, lane);
               if (bad) flag_error(FT_DEV_BAD_KV_INDEX);
               mbar_arrive_on_cp_async(full);
             }
@@ -702,16 +722,16 @@ __device__ __forceinline__ void tc_body(const TcParams& tp, uint8_t* smem, const
                              bool dense, int first_row) {
           if (dense) {
             if (lane == 0) {
-              mbar_arrive_expect_tx(full, 16384);
-              tma_load_3d(buf, map, 0, kvh, first_row, full);
-              tma_load_3d(buf + 8192, map, 64, kvh, first_row, full);
+              mbar_arrive_expect_tx(full, C::TILE_BYTES);
+#pragma unroll
+              for (int h = 0; h < C::NB; ++h) tma_load_3d(buf + h * 8192, map, 64 * h, kvh, first_row, full);
             } else {
               mbar_arrive(full);
             }
             return;
           }
           const int* ids = ring + (t % C::IDX_SLOTS) * C::TILE;
-          const bool bad = tc_gather_tile_smem<T>(buf, base, stride, ids, t, id_lim, row_lim, lane);
+          const bool bad = tc_gather_tile_smem<T, D>(buf, base, stride, ids, t, id_lim, row_lim, lane);
           if (bad) flag_error(FT_DEV_BAD_KV_INDEX);
           mbar_arrive_on_cp_async(full);
         };
@@ -755,9 +775,9 @@ __device__ __forceinline__ void tc_body(const TcParams& tp, uint8_t* smem, const
         // ================================================================ MMA issue
         if (lane == 0) {
           const uint32_t idesc_s = tc_idesc<T>(128, C::TILE, false);
-          const uint32_t idesc_o = tc_idesc<T>(128, 64, true);  // P.V in two 64-column halves: the shape of S
+          const uint32_t idesc_o = tc_idesc<T>(128, 64, true);  // P.V in 64-column pieces: the shape of S
           const uint64_t q_desc = tc_desc(q_sm, 16, 1024);
-          auto issue_pv = [&](int t) {  // O += P_t V_t : per half of O, 4 k-steps of 16 tokens, A = P_t in tensor memory
+          auto issue_pv = [&](int t) {  // O += P_t V_t : per 64 columns of O, 4 k-steps of 16 tokens, A = P_t in tensor memory
             const int g = g0 + t, b = g & 1;
             const uint32_t use = (uint32_t)(g >> 1) & 1u;
             if (!tc_wait(bar(C::P_FULL + b), use, abort_flag)) return false;
@@ -769,7 +789,7 @@ __device__ __forceinline__ void tc_body(const TcParams& tp, uint8_t* smem, const
             tc_fence_after();
             const uint32_t p_tmem = tmem + C::S_COL + b * C::TILE;
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
+            for (int h = 0; h < C::NB; ++h) {
               const uint64_t v_desc = tc_desc(v_buf(g) + h * 8192, 8192, 1024);
 #pragma unroll
               for (int ks = 0; ks < 4; ++ks)
@@ -798,7 +818,7 @@ __device__ __forceinline__ void tc_body(const TcParams& tp, uint8_t* smem, const
             tc_fence_after();
             const uint64_t k_desc = tc_desc(k_buf(g), 16, 1024);
 #pragma unroll
-            for (int ks = 0; ks < 8; ++ks) {  // 8 k-steps of 16 along head_dim: +32 B inside a block, +1 block after 4
+            for (int ks = 0; ks < D / 16; ++ks) {  // k-steps of 16 along head_dim: +32 B inside a block, +1 block after 4
               const uint64_t a = q_desc + (uint64_t)((ks >> 2) * (16384 >> 4) + (ks & 3) * 2);
               const uint64_t bb = k_desc + (uint64_t)((ks >> 2) * (8192 >> 4) + (ks & 3) * 2);
               tc_mma(tmem + C::S_COL + b * C::TILE, a, bb, idesc_s, ks > 0);
@@ -827,18 +847,20 @@ __device__ __forceinline__ void tc_body(const TcParams& tp, uint8_t* smem, const
   }
 }
 
-template <typename T>
-__global__ void __launch_bounds__(TcCfg::THREADS, 2) stage1_tc_kernel(const __grid_constant__ TcParams tp) {
+// The bound of two CTAs per SM holds the compiler to 128 registers per thread at head_dim 256 too, where shared memory
+// leaves room for one: the register trade above counts on exactly that.
+template <typename T, int D>
+__global__ void __launch_bounds__(TcCfg<D>::THREADS, 2) stage1_tc_kernel(const __grid_constant__ TcParams tp) {
   allow_dependent_launch();
   extern __shared__ __align__(1024) uint8_t smem[];
   int vn, kvh;
   task_of_block(tp.p, blockIdx.x, vn, kvh);
   FT_TL_BEGIN();
-  tc_body<T>(tp, smem, vn, kvh);
+  tc_body<T, D>(tp, smem, vn, kvh);
   FT_TL_END(1);
 }
 
-// Both task families in one grid (head_dim 128): the tensor-bound many-row CTAs (tcgen05 body, one task each)
+// Both task families in one grid (head_dim 64 and 128): the tensor-bound many-row CTAs (tcgen05 body, one task each)
 // and the memory-bound few-row CTAs (swapped-operand body) share the SMs instead of running back to back.
 // Block order, which is the order the hardware starts them in:
 //   [0, lead)                 many-row tasks 0 .. lead-1
@@ -846,8 +868,8 @@ __global__ void __launch_bounds__(TcCfg::THREADS, 2) stage1_tc_kernel(const __gr
 //                             (p.workers > 0), or one CTA per few-row task (p.workers == 0)
 //   the rest                  the remaining many-row tasks
 // `lead` leaves room for the few-row CTAs to start at once beside the first many-row CTAs.
-template <typename T>
-__global__ void __launch_bounds__(TcCfg::THREADS, 2) stage1_fused_kernel(const __grid_constant__ TcParams tp) {
+template <typename T, int D>
+__global__ void __launch_bounds__(TcCfg<D>::THREADS, 2) stage1_fused_kernel(const __grid_constant__ TcParams tp) {
   allow_dependent_launch();
   extern __shared__ __align__(1024) uint8_t smem[];
   const Stage1Params& p = tp.p;
@@ -858,7 +880,7 @@ __global__ void __launch_bounds__(TcCfg::THREADS, 2) stage1_fused_kernel(const _
   FT_TL_BEGIN();
   if (b < p.lead_wide || b >= p.lead_wide + few_ctas) {
     const int task = b < p.lead_wide ? b : b - few_ctas;
-    tc_body<T>(tp, smem, p.node_offset + task / H, task % H);
+    tc_body<T, D>(tp, smem, p.node_offset + task / H, task % H);
     FT_TL_END(1);
   } else {
     // This CTA will not allocate tensor memory.  Saying so at once matters: the SM admits no second CTA of a
@@ -868,14 +890,14 @@ __global__ void __launch_bounds__(TcCfg::THREADS, 2) stage1_fused_kernel(const _
       reg_shrink<24>();
       return;
     }
-    reg_grow<TcCfg::REGS_WORKER>();
+    reg_grow<TcCfg<D>::REGS_WORKER>();
     wait_for_prior_grid();  // nothing of the preceding kernel's is read or overwritten before this
     const int w = b - p.lead_wide;
     if (p.workers > 0) {
-      stream_worker<T, 128>(tp, smem, wide_tasks, few_tasks, w, p.workers);
+      stream_worker<T, D>(tp, smem, wide_tasks, few_tasks, w, p.workers);
     } else {
       const int task = wide_tasks + w;
-      narrow_dispatch<T, 128>(p, smem, p.node_offset + task / H, task % H);
+      narrow_dispatch<T, D>(p, smem, p.node_offset + task / H, task % H);
     }
     FT_TL_END(2);
   }

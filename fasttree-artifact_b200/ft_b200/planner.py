@@ -714,9 +714,11 @@ def b200_tables_native_direct(tree, node_base, node_offset, extra, batch_size, n
 def b200_model_for(params, head_dim, model=None):
     explicit = model or getattr(params, "b200_model", None)
     m = explicit or B200Model()
-    if explicit is None and head_dim == 128:
-        # the tcgen05 stage-1 kernel holds 128 query rows per CTA (head_dim 128 only)
-        m = replace(m, rows_per_cta=128, ridge_flop_per_byte=4 * m.ridge_flop_per_byte)
+    if explicit is None and (head_dim == 128 or (head_dim in (64, 256) and getattr(params, "kv_elem_bytes", 2) == 2)):
+        # the tcgen05 stage-1 kernel holds 128 query rows per CTA; at head_dim 64 its softmax, which sets the tile's
+        # time, covers half the flops, and at 256 one CTA fills an SM
+        m = replace(m, rows_per_cta=128, ridge_flop_per_byte=(2 if head_dim == 64 else 4) * m.ridge_flop_per_byte,
+                    ctas_per_sm=1 if head_dim == 256 else m.ctas_per_sm)
     if explicit is None and getattr(params, "kv_elem_bytes", 2) == 4:
         # fp32 storage runs on the CUDA-core kernel: 32-token tiles, one warp per scheduler, so a chunk costs
         # several microseconds per tile and a small problem is better cut down to single tiles

@@ -35,7 +35,7 @@ enum ft_path {
   FT_PATH_GENERIC = 1, /* scalar fp32 kernel: any dtype, head_dim <= 256 */
   FT_PATH_MMA = 2,     /* mma.sync tensor-core kernels, 16-bit types, head_dim 64/128: per phase the
                           narrow (swapped-operand) kernel for <= 16 query rows per task, else the wide one */
-  FT_PATH_TCGEN05 = 3, /* tcgen05/TMEM kernel for 128-row tasks, 16-bit types, head_dim 128 */
+  FT_PATH_TCGEN05 = 3, /* tcgen05/TMEM kernel for 128-row tasks, 16-bit types, head_dim 64/128/256 */
   FT_PATH_MMA_WIDE = 4, /* the wide mma.sync kernel for every task (ablation / cross-check) */
   FT_PATH_STREAM = 5,   /* like AUTO, but few-row phases run the persistent kernel that pipelines across tasks */
   FT_PATH_PERSIST = 6   /* one persistent tcgen05 kernel (a CTA per SM) for every task: 16-bit types, head_dim 128 */
@@ -272,13 +272,13 @@ typedef struct ft_plan ft_plan;
 
 typedef struct ft_b200_model { /* machine constants of the cost model; NULL in ft_plan_b200_build = defaults */
   int32_t num_sms;             /* 148 */
-  int32_t ctas_per_sm;         /* 2 */
+  int32_t ctas_per_sm;         /* 2 (1 at head_dim 256) */
   double waves;                /* rounds of resident CTAs to aim for: 1.0 */
   int32_t tile_tokens;         /* KV tile of the stage-1 kernels: 64 */
-  int32_t rows_per_cta;        /* query rows one CTA holds: 64 (128 at head_dim 128) */
+  int32_t rows_per_cta;        /* query rows one CTA holds: 64 (128 at head_dim 64, 128 and 256) */
   int32_t min_chunk;           /* never cut a node's KV finer than this many tokens: 128 */
   int32_t nominal_split;       /* chunk length assumed while deciding the edges: 512 */
-  double ridge_flop_per_byte;  /* flops that cost as much time as one streamed byte: 90 (360 at head_dim 128) */
+  double ridge_flop_per_byte;  /* flops that cost as much time as one streamed byte: 90 (180 at head_dim 64, 360 at 128, 256) */
   int32_t task_overhead_bytes; /* fixed cost of one more CTA in streamed-byte equivalents: 16384 */
   int32_t elem_bytes;          /* 2 */
   int32_t group_member_tokens; /* nodes up to this long, with few enough requests for the few-row kernels, may be
