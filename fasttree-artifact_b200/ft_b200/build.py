@@ -1,4 +1,4 @@
-"""Builds libfasttree_b200.so (sm_100a) in-tree with nvcc.
+"""Builds libfasttree_b200.so (sm_100a) and the Python call module ft_call.so in-tree, with nvcc and g++.
 
 Usage:  python fasttree-artifact_b200/ft_b200/build.py [--force] [--verbose]
 """
@@ -14,6 +14,10 @@ INCLUDE = os.path.join(ROOT, "include")
 LIB_PATH = os.path.join(PKG_DIR, "libfasttree_b200.so")
 
 SOURCES = ["ft_api.cu", "ft_planner.cu"]
+
+CALL_PATH = os.path.join(PKG_DIR, "ft_call.so")     # Python extension: checks, argument block and call of a decode step
+CALL_SOURCE = os.path.join(CSRC, "ft_call.cpp")
+CALL_STAMP = CALL_PATH + ".srchash"
 
 
 def _nvcc():
@@ -49,6 +53,52 @@ def _stale():
         return fh.read().strip() != _source_digest()
 
 
+def _call_digest():
+    """What the call module was built from: its source, the C ABI's header, and the torch and Python it links to."""
+    import hashlib
+    import torch
+    h = hashlib.sha256(f"{torch.__version__} {sys.version}".encode())
+    for path in (CALL_SOURCE, os.path.join(INCLUDE, "fasttree_b200.h")):
+        with open(path, "rb") as fh:
+            h.update(fh.read())
+    return h.hexdigest()
+
+
+def call_module_stale():
+    if not os.path.exists(CALL_PATH) or not os.path.exists(CALL_STAMP):
+        return True
+    with open(CALL_STAMP) as fh:
+        return fh.read().strip() != _call_digest()
+
+
+def build_call_module(force=False, verbose=False):
+    """Compile ft_call.cpp into a Python extension module against the installed torch."""
+    if not force and not call_module_stale():
+        return CALL_PATH
+    import sysconfig
+    import torch
+    torch_dir = os.path.dirname(torch.__file__)
+    cxx = shutil.which("g++") or shutil.which("c++")
+    if cxx is None:
+        raise RuntimeError("g++ not found; the call module cannot be built")
+    cuda_home = os.path.dirname(os.path.dirname(_nvcc()))
+    cmd = [cxx, "-shared", "-fPIC", "-O2", "-std=c++17", "-fvisibility=hidden",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           "-I", INCLUDE, "-I", os.path.join(torch_dir, "include"),
+           "-I", os.path.join(torch_dir, "include", "torch", "csrc", "api", "include"),
+           "-I", os.path.join(cuda_home, "include"), "-I", sysconfig.get_paths()["include"],
+           CALL_SOURCE, "-o", CALL_PATH, "-L", os.path.join(torch_dir, "lib"),
+           "-ltorch_python", "-ltorch_cpu", "-lc10_cuda", "-lc10"]
+    res = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    if verbose or res.returncode != 0:
+        print(res.stdout)
+    if res.returncode != 0:
+        raise RuntimeError("g++ failed:\n" + res.stdout)
+    with open(CALL_STAMP, "w") as fh:
+        fh.write(_call_digest() + "\n")
+    return CALL_PATH
+
+
 def build_library(force=False, verbose=False):
     """Compile every CUDA source for sm_100a into one shared library."""
     if not force and not _stale():
@@ -74,3 +124,4 @@ def build_library(force=False, verbose=False):
 
 if __name__ == "__main__":
     print(build_library(force="--force" in sys.argv, verbose="--verbose" in sys.argv))
+    print(build_call_module(force="--force" in sys.argv, verbose="--verbose" in sys.argv))

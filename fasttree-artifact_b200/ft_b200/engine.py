@@ -13,10 +13,9 @@ import torch
 
 from . import lib as _lib
 
-_DTYPES = {torch.float16: _lib.FT_F16, torch.bfloat16: _lib.FT_BF16, torch.float32: _lib.FT_F32}
-
+# What is remembered about a plan: per vnode_to_q_entries table (by tensor object, weakly) whether it carries row ranges
+# (:func:`split_q_entries`).  id(tensor) -> (weak reference to it, (version, data_ptr, numel), rows or -1)
 _ARG_CACHE = {}
-_ARG_CACHE_MAX = 256
 
 
 def _require_cuda(name, t):
@@ -35,16 +34,7 @@ def _table(name, t):
     return t
 
 
-def _pair(name, x):
-    x = list(x)
-    if len(x) != 2:
-        raise ValueError(f"{name} must have two entries (one per phase)")
-    return int(x[0]), int(x[1])
-
-
 ROW_RANGE_MAGIC = 0x46545252          # "FTRR": trailer of a vnode_to_q_entries table that carries row ranges
-
-_RANGE_CACHE = {}     # id(tensor) -> (weak reference to it, (version, data_ptr, numel), rows or -1)
 
 
 def _version_of(t):
@@ -85,17 +75,18 @@ def split_q_entries(vnode_to_q_entries):
     must not fall inside a CUDA graph capture."""
     t = vnode_to_q_entries
     n = t.numel()
-    if n < 5 or (n - 2) % 3 != 0:
-        return n, None
     state = (_version_of(t), t.data_ptr(), n)
     ident = id(t)
-    known = _RANGE_CACHE.get(ident)
+    known = _ARG_CACHE.get(ident)
     if known is not None and known[0]() is t and known[1] == state:
         hit = known[2]
     else:
-        magic, rows = t.view(-1)[-2:].tolist()
-        hit = rows if (magic == ROW_RANGE_MAGIC and 3 * rows + 2 == n) else -1
-        _RANGE_CACHE[ident] = (weakref.ref(t, lambda _r, k=ident: _RANGE_CACHE.pop(k, None)), state, hit)
+        hit = -1
+        if n >= 5 and (n - 2) % 3 == 0:
+            magic, rows = t.view(-1)[-2:].tolist()
+            if magic == ROW_RANGE_MAGIC and 3 * rows + 2 == n:
+                hit = rows
+        _ARG_CACHE[ident] = (weakref.ref(t, lambda _r, k=ident: _ARG_CACHE.pop(k, None)), state, hit)
     if hit < 0:
         return n, None
     return hit, t.view(-1)[hit:3 * hit].view(hit, 2)
@@ -105,13 +96,25 @@ def row_ranges_of(vnode_to_q_entries):
     return split_q_entries(vnode_to_q_entries)[1]
 
 
-def build_args(q, k_buffer, v_buffer, o, vnode_to_kv_entries, vnode_to_kv_offs, vnode_to_kv_lens,
-               vnode_to_q_entries, vnode_to_q_offs, vnode_to_q_lens, req_to_vnode_entries,
-               req_to_vnode_offs, req_to_vnode_lens, mid_o, mid_lse, phase_node_nums, phase_node_offsets,
-               phase_q_tile_sizes, phase_kv_tile_sizes, sm_scale, logit_cap=-1, path="auto", o_lse=None,
-               stream=None, row_ranges="detect", phase_info=None, kv_entries_aux=None):
-    """Validate the tensors and fill a :class:`DecodeArgs` struct.  ``kv_entries_aux``: an
-    int32 CUDA tensor, the second row-id table that vnodes with bit 30 of their
+def _resolve(args, path, row_ranges):
+    """``(path code, row-range tensor or None, partial rows or -1)`` of a call's arguments."""
+    code = _lib.PATHS.get(path)
+    if code is None:
+        raise ValueError(f"path must be one of {sorted(_lib.PATHS)}")
+    if isinstance(row_ranges, str):
+        if row_ranges != "detect":
+            raise ValueError("row_ranges must be 'detect', None or an int32 tensor")
+        _table("vnode_to_q_entries", args[7])
+        rows, ranges = split_q_entries(args[7])
+        return code, ranges, rows
+    return code, row_ranges, -1
+
+
+def build_args(*args, path="auto", o_lse=None, stream=None, row_ranges="detect", phase_info=None, kv_entries_aux=None,
+               logit_cap=-1):
+    """A filled :class:`DecodeArgs` struct; raises ``ValueError`` where a tensor does not fit.  Positional arguments
+    are those of the reference's ``fasttree_decode`` up to and including ``sm_scale`` (and ``logit_cap``).
+    ``kv_entries_aux``: an int32 CUDA tensor, the second row-id table that vnodes with bit 30 of their
     ``vnode_to_kv_offs`` value set read (grouped private tails of the serving path).  ``phase_info``: an
     int32 CUDA tensor ``[n0, n1, o0, o1]`` that stage 1 reads on the device in
     place of ``phase_node_nums`` / ``phase_node_offsets`` (the launch then does not
@@ -119,181 +122,36 @@ def build_args(q, k_buffer, v_buffer, o, vnode_to_kv_entries, vnode_to_kv_offs, 
     ``"detect"`` looks for ranges packed into ``vnode_to_q_entries`` (see
     :func:`pack_row_ranges`), ``None`` says the plan has none (no look-up, no
     device read), a tensor gives the table explicitly."""
-    for name, t in (("q", q), ("k_buffer", k_buffer), ("v_buffer", v_buffer), ("o", o),
-                    ("mid_o", mid_o), ("mid_lse", mid_lse)):
-        _require_cuda(name, t)
-    if q.dim() != 3 or o.dim() != 3 or k_buffer.dim() != 3 or v_buffer.dim() != 3:
-        raise ValueError("q, o must be [batch, heads, head_dim] and k/v buffers [rows, kv_heads, head_dim]")
-    if q.dtype not in _DTYPES:
-        raise ValueError(f"unsupported dtype {q.dtype}")
-    if not (k_buffer.dtype == v_buffer.dtype == o.dtype == q.dtype):
-        raise ValueError("q, k_buffer, v_buffer and o must share one dtype")
-    if q.shape[-1] != k_buffer.shape[-1] or q.shape[-1] != v_buffer.shape[-1]:
-        raise ValueError("head_dim of q, k_buffer and v_buffer differ")          # reference: assert Lq == Lk
-    if o.shape != q.shape:
-        raise ValueError("o must have the shape of q")
-    for name, t in (("q", q), ("k_buffer", k_buffer), ("v_buffer", v_buffer), ("o", o), ("mid_o", mid_o)):
-        if t.stride(-1) != 1:
-            raise ValueError(f"{name}: the head_dim axis must be contiguous")
-    if mid_o.dtype != torch.float32 or mid_lse.dtype != torch.float32:
-        raise ValueError("mid_o / mid_lse must be float32")
-    if mid_o.dim() != 3 or mid_lse.dim() != 2 or mid_lse.stride(1) != 1:
-        raise ValueError("mid_o must be [rows, heads, head_dim] and mid_lse [rows, heads]")
-    if mid_o.shape[1] < q.shape[1] or mid_o.shape[2] != q.shape[2] or mid_lse.shape[1] < q.shape[1]:
-        raise ValueError("mid_o / mid_lse are too small for the head count of q")
-    if k_buffer.shape != v_buffer.shape:
-        raise ValueError("k_buffer and v_buffer differ in shape")
-    tabs = [_table(n, t) for n, t in (
-        ("vnode_to_kv_entries", vnode_to_kv_entries), ("vnode_to_kv_offs", vnode_to_kv_offs),
-        ("vnode_to_kv_lens", vnode_to_kv_lens), ("vnode_to_q_entries", vnode_to_q_entries),
-        ("vnode_to_q_offs", vnode_to_q_offs), ("vnode_to_q_lens", vnode_to_q_lens),
-        ("req_to_vnode_entries", req_to_vnode_entries), ("req_to_vnode_offs", req_to_vnode_offs),
-        ("req_to_vnode_lens", req_to_vnode_lens))]
-    n0, n1 = _pair("phase_node_nums", phase_node_nums)
-    f0, f1 = _pair("phase_node_offsets", phase_node_offsets)
-    nv = vnode_to_kv_offs.numel()
-    if phase_info is not None:
-        _table("phase_info", phase_info)
-        if phase_info.numel() < 4:
-            raise ValueError("phase_info needs four entries: n0, n1, o0, o1")
-    if kv_entries_aux is not None:
-        _table("kv_entries_aux", kv_entries_aux)
-    for cnt, off in ((n0, f0), (n1, f1)):
-        if phase_info is None and (cnt < 0 or off < 0 or off + cnt > nv):
-            raise ValueError("phase_node_nums / phase_node_offsets do not fit the vnode tables")
-    if min(vnode_to_kv_lens.numel(), vnode_to_q_offs.numel(), vnode_to_q_lens.numel()) < nv:
-        raise ValueError("vnode tables differ in length")
-    batch = q.shape[0]
-    if req_to_vnode_offs.numel() < batch or req_to_vnode_lens.numel() < batch:
-        raise ValueError("request tables are shorter than the batch")
-    if o_lse is not None:
-        _require_cuda("o_lse", o_lse)
-        if o_lse.dtype != torch.float32 or not o_lse.is_contiguous() or o_lse.numel() < batch * q.shape[1]:
-            raise ValueError("o_lse must be a contiguous float32 [batch, heads] tensor")
-    if path not in _lib.PATHS:
-        raise ValueError(f"path must be one of {sorted(_lib.PATHS)}")
-
-    q_rows = vnode_to_q_entries.numel()
-    if isinstance(row_ranges, str):
-        if row_ranges != "detect":
-            raise ValueError("row_ranges must be 'detect', None or an int32 tensor")
-        q_rows, ranges = split_q_entries(vnode_to_q_entries)
-    else:
-        ranges = row_ranges
-    if ranges is not None:
-        _table("row ranges", ranges)
-        if ranges.numel() < 2 * q_rows:
-            raise ValueError("the row-range table needs two entries per partial row")
-
-    a = _lib.DecodeArgs()
-    a.vnode_q_kv_ranges = ranges.data_ptr() if ranges is not None else None
-    a.device_phase_info = phase_info.data_ptr() if phase_info is not None else None
-    a.vnode_to_kv_entries_aux = kv_entries_aux.data_ptr() if kv_entries_aux is not None else None
-    a.kv_entries_aux_len = kv_entries_aux.numel() if kv_entries_aux is not None else 0
-    a.q, a.k_buffer, a.v_buffer, a.o = q.data_ptr(), k_buffer.data_ptr(), v_buffer.data_ptr(), o.data_ptr()
-    a.o_lse = o_lse.data_ptr() if o_lse is not None else None
-    a.dtype = _DTYPES[q.dtype]
-    a.batch, a.num_qo_heads, a.head_dim = batch, q.shape[1], q.shape[2]
-    a.num_kv_heads = k_buffer.shape[1]
-    a.path = _lib.PATHS[path]
-    a.kv_rows = k_buffer.shape[0]
-    a.q_stride0, a.q_stride1 = q.stride(0), q.stride(1)
-    a.k_stride0, a.k_stride1 = k_buffer.stride(0), k_buffer.stride(1)
-    a.v_stride0, a.v_stride1 = v_buffer.stride(0), v_buffer.stride(1)
-    a.o_stride0, a.o_stride1 = o.stride(0), o.stride(1)
-    (a.vnode_to_kv_entries, a.vnode_to_kv_offs, a.vnode_to_kv_lens, a.vnode_to_q_entries,
-     a.vnode_to_q_offs, a.vnode_to_q_lens, a.req_to_vnode_entries, a.req_to_vnode_offs,
-     a.req_to_vnode_lens) = [t.data_ptr() for t in tabs]
-    a.kv_entries_len = vnode_to_kv_entries.numel()
-    a.num_partial_rows = min(mid_o.shape[0], mid_lse.shape[0], q_rows)
-    a.phase_node_nums[0], a.phase_node_nums[1] = n0, n1
-    a.phase_node_offsets[0], a.phase_node_offsets[1] = f0, f1
-    a.phase_q_tile_sizes[0], a.phase_q_tile_sizes[1] = _pair("phase_q_tile_sizes", phase_q_tile_sizes)
-    a.phase_kv_tile_sizes[0], a.phase_kv_tile_sizes[1] = _pair("phase_kv_tile_sizes", phase_kv_tile_sizes)
-    a.mid_o, a.mid_lse = mid_o.data_ptr(), mid_lse.data_ptr()
-    a.mid_o_stride0, a.mid_o_stride1 = mid_o.stride(0), mid_o.stride(1)
-    a.mid_lse_stride0 = mid_lse.stride(0)
-    a.sm_scale = float(sm_scale)
-    a.logit_cap = float(logit_cap)
-    a.stream = stream if stream is not None else torch.cuda.current_stream(q.device).cuda_stream
-    return a
+    if len(args) == 21:
+        args, logit_cap = args[:20], args[20]
+    code, ranges, rows = _resolve(args, path, row_ranges)
+    raw = _lib.call_module().args(args, logit_cap, code, o_lse, ranges, rows, phase_info, kv_entries_aux,
+                                  -1 if stream is None else stream)
+    return _lib.DecodeArgs.from_buffer_copy(raw)
 
 
-def _cached_args(tensors, rest, path, o_lse, row_ranges, phase_info=None, kv_entries_aux=None):
-    """Argument structs are memoised so that a steady-state decode loop pays for
-    one dict lookup and a few pointer stores instead of rebuilding ~45 fields.
-    The key names only what persists across calls - the K/V buffers, the plan
-    tables and the partial buffers (by tensor identity; the entry keeps them
-    alive, so an id cannot be recycled) - plus the scalar arguments and the
-    layout of ``q`` / ``o``.  ``q``, ``o`` and ``o_lse`` are new tensor objects
-    on every layer and step of a serving loop: their addresses are written into
-    the cached struct on each call and the cache holds no reference to them.  On
-    a hit the data pointers of the persistent tensors are compared with the
-    cached ones, which catches storage re-allocated behind the same object."""
-    q, k_buffer, v_buffer, o = tensors[:4]
-    persistent = tensors[1:3] + tensors[4:]
-    stream = torch.cuda.current_stream(q.device).cuda_stream
-    (pn, po, pq, pk, sm_scale, logit_cap) = rest
-    is_detect = isinstance(row_ranges, str)
-    ranges_key = row_ranges if is_detect or row_ranges is None else id(row_ranges)
-    key = (tuple(map(id, persistent)), pn[0], pn[1], po[0], po[1], pq[0], pq[1], pk[0], pk[1], sm_scale, logit_cap,
-           path, stream, ranges_key, q.shape, q.stride(), q.dtype, o.shape, o.stride(), o.dtype, o_lse is None,
-           id(phase_info) if phase_info is not None else None,
-           (id(kv_entries_aux), kv_entries_aux.data_ptr(), kv_entries_aux.numel()) if kv_entries_aux is not None else None)
-    ptrs = tuple([t.data_ptr() for t in persistent])
-    hit = _ARG_CACHE.get(key)
-    if hit is not None and hit[1] == ptrs and (not is_detect or hit[3] == _version_of(tensors[7])):
-        a = hit[0]
-        if not (q.is_cuda and o.is_cuda):
-            raise ValueError("q / o must live on a CUDA device; the engine has no CPU path")
-    else:
-        a = build_args(*tensors, pn, po, pq, pk, sm_scale, logit_cap, path=path, o_lse=o_lse, stream=stream,
-                       row_ranges=row_ranges, phase_info=phase_info, kv_entries_aux=kv_entries_aux)
-        if len(_ARG_CACHE) >= _ARG_CACHE_MAX:
-            _ARG_CACHE.clear()
-        keep = (row_ranges if isinstance(row_ranges, torch.Tensor) else None, phase_info, kv_entries_aux)
-        _ARG_CACHE[key] = (a, ptrs, persistent, _version_of(tensors[7]), keep)
-    a.q, a.o = q.data_ptr(), o.data_ptr()
-    if o_lse is not None:
-        if (not o_lse.is_cuda or o_lse.dtype != torch.float32 or not o_lse.is_contiguous()
-                or o_lse.numel() < q.shape[0] * q.shape[1]):
-            raise ValueError("o_lse must be a contiguous float32 [batch, heads] CUDA tensor")
-        a.o_lse = o_lse.data_ptr()
-    else:
-        a.o_lse = None
-    return a
+_ENTRIES = {"ft_decode": 0, "ft_stage1": 1, "ft_stage2": 2}
 
 
-def _call(fn_name, q, k_buffer, v_buffer, o, kv_entries, kv_offs, kv_lens, q_entries, q_offs, q_lens,
-          r2v_entries, r2v_offs, r2v_lens, mid_o, mid_lse, phase_node_nums, phase_node_offsets,
-          phase_q_tile_sizes, phase_kv_tile_sizes, sm_scale, logit_cap, path, o_lse, row_ranges="detect",
-          phase_info=None, kv_entries_aux=None):
-    tensors = (q, k_buffer, v_buffer, o, kv_entries, kv_offs, kv_lens, q_entries, q_offs, q_lens,
-               r2v_entries, r2v_offs, r2v_lens, mid_o, mid_lse)
-    rest = (phase_node_nums, phase_node_offsets, phase_q_tile_sizes, phase_kv_tile_sizes,
-            float(sm_scale), float(logit_cap))
-    a = _cached_args(tensors, rest, path, o_lse, row_ranges, phase_info, kv_entries_aux)
-    lib = _lib.load()
-    if q.device.index != torch.cuda.current_device():
-        with torch.cuda.device(q.device):
-            rc = getattr(lib, fn_name)(ctypes.byref(a))
-    else:
-        rc = getattr(lib, fn_name)(ctypes.byref(a))
-    _lib.check(rc)
+def _call(fn_name, args, logit_cap, path, o_lse, row_ranges, phase_info=None, kv_entries_aux=None):
+    code, ranges, rows = _resolve(args, path, row_ranges)
+    rc = _lib.call_module().call(_ENTRIES[fn_name], args, logit_cap, code, o_lse, ranges, rows, phase_info, kv_entries_aux, -1)
+    if rc != 0:
+        _lib.check(rc)
 
 
 def decode(*args, logit_cap=-1, path="auto", o_lse=None, row_ranges="detect", phase_info=None, kv_entries_aux=None):
     """Stage 1 + stage 2.  Positional arguments are those of the reference's
     ``fasttree_decode`` up to and including ``sm_scale``."""
-    _call("ft_decode", *args, logit_cap, path, o_lse, row_ranges, phase_info, kv_entries_aux)
+    _call("ft_decode", args, logit_cap, path, o_lse, row_ranges, phase_info, kv_entries_aux)
 
 
 def stage1(*args, logit_cap=-1, path="auto", row_ranges="detect", phase_info=None, kv_entries_aux=None):
-    _call("ft_stage1", *args, logit_cap, path, None, row_ranges, phase_info, kv_entries_aux)
+    _call("ft_stage1", args, logit_cap, path, None, row_ranges, phase_info, kv_entries_aux)
 
 
 def stage2(*args, logit_cap=-1, o_lse=None):
-    _call("ft_stage2", *args, logit_cap, "auto", o_lse, None)
+    _call("ft_stage2", args, logit_cap, "auto", o_lse, None)
 
 
 def decode_host_io(q_host, o_host, q_dev, k_buffer, v_buffer, o_dev, *rest, logit_cap=-1, path="auto",
@@ -313,7 +171,7 @@ def decode_host_io(q_host, o_host, q_dev, k_buffer, v_buffer, o_dev, *rest, logi
         raise ValueError("the device staging tensors must be packed")
     tensors = (q_dev, k_buffer, v_buffer, o_dev) + tuple(rest[:11])
     pn, po, pq, pk, sm_scale = rest[11:16]
-    a = _cached_args(tensors, (pn, po, pq, pk, float(sm_scale), float(logit_cap)), path, None, row_ranges)
+    a = build_args(*tensors, pn, po, pq, pk, sm_scale, logit_cap, path=path, row_ranges=row_ranges)
     lib = _lib.load()
     if q_dev.device.index != torch.cuda.current_device():
         with torch.cuda.device(q_dev.device):
@@ -332,7 +190,7 @@ def prepare_host_io(q_host, o_host, q_dev, k_buffer, v_buffer, o_dev, *rest, log
                    row_ranges=row_ranges, wait=True)          # validation, first-use costs, range look-up
     pn, po, pq, pk, sm_scale = rest[11:16]
     tensors = (q_dev, k_buffer, v_buffer, o_dev) + tuple(rest[:11])
-    a = build_args(*tensors, pn, po, pq, pk, float(sm_scale), logit_cap, path=path, row_ranges=row_ranges)
+    a = build_args(*tensors, pn, po, pq, pk, sm_scale, logit_cap, path=path, row_ranges=row_ranges)
     fn = _lib.load().ft_decode_host_io
     ref, qp, op, flag = ctypes.byref(a), q_host.data_ptr(), o_host.data_ptr(), 1 if wait else 0
     keep = (tensors, q_host, o_host, a)
@@ -348,8 +206,7 @@ def prepare_host_io(q_host, o_host, q_dev, k_buffer, v_buffer, o_dev, *rest, log
 
 
 def stage1_path_name(*args, logit_cap=-1, path="auto"):
-    tensors, rest = args[:15], args[15:]
-    a = build_args(*tensors, *rest, logit_cap, path=path)
+    a = build_args(*args, logit_cap, path=path)
     name = _lib.load().ft_stage1_path_name(ctypes.byref(a))
     if name is None:
         _lib.check(-1)

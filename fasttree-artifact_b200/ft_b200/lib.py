@@ -90,6 +90,7 @@ class DecodeArgs(ctypes.Structure):
 
 _lock = threading.Lock()
 _lib = None
+_call = None
 
 
 def library_path():
@@ -168,6 +169,32 @@ def load():
         lib.ft_plan_free.restype = None
         _lib = lib
     return _lib
+
+
+def call_module():
+    """The extension module that checks the tensors of a decode call, fills the argument block and calls the library
+    (csrc/ft_call.cpp), bound to the loaded library.  Built first when it is missing or stale, like the library."""
+    global _call
+    if _call is not None:
+        return _call
+    handle = load()
+    with _lock:
+        if _call is None:
+            if _build.call_module_stale():
+                try:
+                    _build.build_call_module(force=True)
+                except Exception as exc:
+                    raise FastTreeError(-3, f"ft_call.so is missing or older than its sources and could not be built: {exc}") from exc
+            import importlib.machinery
+            import importlib.util
+            import torch  # noqa: F401  its libraries must be loaded before the module that links to them
+            loader = importlib.machinery.ExtensionFileLoader("ft_call", _build.CALL_PATH)
+            mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("ft_call", loader))
+            loader.exec_module(mod)
+            mod.bind(*(ctypes.cast(getattr(handle, n), ctypes.c_void_p).value for n in ("ft_decode", "ft_stage1", "ft_stage2")),
+                     handle.ft_decode_args_size())
+            _call = mod
+    return _call
 
 
 def check(rc):
