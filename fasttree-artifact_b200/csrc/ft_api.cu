@@ -302,10 +302,11 @@ struct MapKey {
 };
 
 // Descriptor of a [rows, heads, head_dim] 16-bit tensor (element strides s0, s1), box 64 (head_dim) x box_heads x
-// box_rows, 128-byte swizzle.  Descriptors are cached by buffer identity (encoding one costs about a microsecond)
+// box_rows, 128-byte swizzle; with box_heads 0 the same tensor as [rows, all elements of a row] with a box of 64 x 1,
+// the form that gathers rows.  Descriptors are cached by buffer identity (encoding one costs about a microsecond)
 // in a hash table of 1024 slots, probed linearly over 8 slots; a full neighbourhood evicts its first slot.  A
-// serving process holds two descriptors per layer's K/V buffer plus two per query shape - a few hundred at most.
-bool tensor_map_3d(CUtensorMap* out, const void* base, int dtype, int head_dim, int64_t rows, int heads, int64_t s0,
+// serving process holds four descriptors per layer's K/V buffers plus two per query shape - a few hundred at most.
+bool tensor_map(CUtensorMap* out, const void* base, int dtype, int head_dim, int64_t rows, int heads, int64_t s0,
                    int64_t s1, int box_heads, int box_rows) {
   constexpr int SLOTS = 1024, PROBES = 8;
   static std::mutex mu;
@@ -332,12 +333,15 @@ bool tensor_map_3d(CUtensorMap* out, const void* base, int dtype, int head_dim, 
   if (slot < 0) slot = home;
   EncodeTiledFn enc = encode_tiled_fn();
   if (enc == nullptr || rows <= 0 || rows > 0x7fffffffLL || heads <= 0) return false;
-  const cuuint64_t dims[3] = {(cuuint64_t)head_dim, (cuuint64_t)heads, (cuuint64_t)rows};
-  const cuuint64_t strides[2] = {(cuuint64_t)s1 * 2, (cuuint64_t)s0 * 2};  // bytes, for dimensions 1 and 2
-  const cuuint32_t box[3] = {64, (cuuint32_t)box_heads, (cuuint32_t)box_rows};
+  const bool flat = box_heads == 0;
+  const int64_t row_elems = (int64_t)(heads - 1) * s1 + head_dim;
+  if (flat && (s1 < 0 || row_elems > s0 || row_elems > 0x7fffffffLL)) return false;  // rows that overlap: no 2-D tensor
+  const cuuint64_t dims[3] = {(cuuint64_t)(flat ? row_elems : head_dim), (cuuint64_t)(flat ? rows : heads), (cuuint64_t)rows};
+  const cuuint64_t strides[2] = {(cuuint64_t)(flat ? s0 : s1) * 2, (cuuint64_t)s0 * 2};  // bytes, for dimensions 1 and 2
+  const cuuint32_t box[3] = {64, (cuuint32_t)(flat ? 1 : box_heads), (cuuint32_t)box_rows};
   const cuuint32_t estr[3] = {1, 1, 1};
   CUtensorMap m;
-  const CUresult rc = enc(&m, dtype == FT_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3,
+  const CUresult rc = enc(&m, dtype == FT_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, flat ? 2 : 3,
                           const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -354,17 +358,22 @@ ft::TcParams tc_params(const ft::Stage1Params& p, const ft_decode_args* a) {
   memset(&tp, 0, sizeof(tp));
   tp.p = p;
   const int d = a->head_dim;
-  tp.has_tma = tensor_map_3d(&tp.k_map, a->k_buffer, a->dtype, d, a->kv_rows, a->num_kv_heads, a->k_stride0,
+  tp.has_tma = tensor_map(&tp.k_map, a->k_buffer, a->dtype, d, a->kv_rows, a->num_kv_heads, a->k_stride0,
                              a->k_stride1, 1, 64) &&
-               tensor_map_3d(&tp.v_map, a->v_buffer, a->dtype, d, a->kv_rows, a->num_kv_heads, a->v_stride0,
+               tensor_map(&tp.v_map, a->v_buffer, a->dtype, d, a->kv_rows, a->num_kv_heads, a->v_stride0,
                              a->v_stride1, 1, 64);
+  tp.has_gather4 = tp.has_tma &&
+                   tensor_map(&tp.k_rows_map, a->k_buffer, a->dtype, d, a->kv_rows, a->num_kv_heads, a->k_stride0,
+                                 a->k_stride1, 0, 1) &&
+                   tensor_map(&tp.v_rows_map, a->v_buffer, a->dtype, d, a->kv_rows, a->num_kv_heads, a->v_stride0,
+                                 a->v_stride1, 0, 1);
   // Q by TMA (tcgen05 kernel): one box per request covering its G heads (at most 8 per box), or one
   // box for a whole tile of consecutive requests, when G is a power of two up to 128
   const int g = p.group;
   if (tp.has_tma && g >= 1 && g <= 128 && (g & (g - 1)) == 0) {
     const int box_heads = g < 8 ? g : 8;
-    if (tensor_map_3d(&tp.q_map, a->q, a->dtype, d, a->batch, a->num_qo_heads, a->q_stride0, a->q_stride1, box_heads, 1) &&
-        tensor_map_3d(&tp.q_map_tile, a->q, a->dtype, d, a->batch, a->num_qo_heads, a->q_stride0, a->q_stride1, g, 128 / g))
+    if (tensor_map(&tp.q_map, a->q, a->dtype, d, a->batch, a->num_qo_heads, a->q_stride0, a->q_stride1, box_heads, 1) &&
+        tensor_map(&tp.q_map_tile, a->q, a->dtype, d, a->batch, a->num_qo_heads, a->q_stride0, a->q_stride1, g, 128 / g))
       tp.q_box_rows = box_heads;
   }
   return tp;

@@ -15,8 +15,11 @@ struct alignas(64) TcParams {
   CUtensorMap v_map;
   CUtensorMap q_map;       // [batch, heads, head_dim], box 64 x q_box_rows x 1: one request
   CUtensorMap q_map_tile;  // same tensor, box 64 x G x 128 / G: a whole Q tile of consecutive requests
+  CUtensorMap k_rows_map;  // K and V as [rows, all heads' elements], box 64 x 1: rows picked one by one (tile::gather4)
+  CUtensorMap v_rows_map;
   Stage1Params p;
   int has_tma;
+  int has_gather4;    // the two row maps are valid
   int q_box_rows;     // 0: gather Q with cp.async (group size not a power of two <= 128, or no descriptor)
   unsigned int* sched;  // persistent kernel: {tasks claimed beyond the first per CTA, CTAs finished}, zero between launches
 };
@@ -45,6 +48,15 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map
       "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];\n" ::
           "r"(dst),
       "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(bar)
+      : "memory");
+}
+
+// four rows r0..r3 of a 2-D map whose box is one row, 64 elements from column c0, to 4 x 128 bytes at dst (swizzled by address)
+__device__ __forceinline__ void tma_gather4(uint32_t dst, const CUtensorMap* map, int c0, int r0, int r1, int r2, int r3, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.tile::gather4.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, %6}], [%7];\n" ::
+          "r"(dst),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(r0), "r"(r1), "r"(r2), "r"(r3), "r"(bar)
       : "memory");
 }
 

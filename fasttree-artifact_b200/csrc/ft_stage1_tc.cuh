@@ -28,8 +28,9 @@
 //   warp 5     K loads.  A tile whose 64 row ids are consecutive is fetched
 //              with two tiled TMA copies (cp.async.bulk.tensor, 128-byte
 //              swizzle, no multicast) straight into the operand layout; any
-//              other tile (scattered pool slots, the ragged last tile) is
-//              gathered with 16-byte cp.async copies.  Row ids reach a small
+//              other tile (scattered pool slots) is gathered four rows at a time
+//              (tile::gather4), the odd rows and the padding of a ragged last
+//              tile with 16-byte cp.async copies.  Row ids reach a small
 //              shared ring with cp.async two tiles ahead.
 //   warps 6-7  Q gather (by request id), concurrent with the first K loads:
 //              when G is a power of two, two TMA boxes for the whole tile if the
@@ -232,42 +233,52 @@ __device__ __forceinline__ bool tc_wait(uint32_t bar, uint32_t parity, volatile 
   return false;
 }
 
-// Row-by-row gather of one 64-token operand tile (scattered pool slots, the ragged last tile): 16-byte copies that
-// zero-fill invalid rows themselves, so the loop has no branch.  Kept out of line: tiles of consecutive rows - every
-// tile of the benchmark shapes - never come here, and their loaders' code stays as small as it was.
-// ids in shared memory (K loader); returns true when a row id inside the chunk was out of range
+// Gather of one 64-token operand tile whose rows are not consecutive (scattered pool slots, the ragged last tile); the
+// row ids are in registers, row r in slot r >> 5 of lane r & 31.  Whole groups of four valid rows go through the TMA unit
+// (tile::gather4: one instruction per four rows and 64 elements, one per lane at head_dim 128); the up to three rows
+// left, the padding, and a tile with a bad row id anywhere use 16-byte cp.async copies, which zero-fill invalid rows.
+// Issuing the 1024 16-byte copies of a tile took a loader warp longer than the tile's share of the memory bandwidth:
+// 75 776 scattered tokens x 8 heads (303 MB), decode 113 -> 93 us (77 us when the rows are consecutive); either operand
+// alone through the TMA unit 105 us.
+// The buffer's full barrier counts an arrival of every lane, which the caller makes with mbar_arrive_on_cp_async.
+// Kept out of line: tiles of consecutive rows never come here, and their loaders' code stays as small as it was.
+// Returns true when a row id inside the chunk was out of range.
 template <typename T, int D>
-__device__ __noinline__ bool tc_gather_tile_smem(uint32_t buf, const T* base, int64_t stride, const int* ids, int t, int id_lim,
-                                                 uint32_t row_lim, int lane) {
+__device__ __noinline__ bool tc_gather_tile(uint32_t buf, const CUtensorMap* rows_map, int col0, const T* base, int64_t stride,
+                                            int id0, int id1, int t, int id_lim, uint32_t row_lim, int lane, uint32_t full) {
   using C = TcCfg<D>;
-  const int c = lane % C::CPR;
-  bool bad = false;
-#pragma unroll 4
-  for (int i = 0; i < C::TILE / C::RPI; ++i) {
-    const int r = lane / C::CPR + C::RPI * i, pos = t * C::TILE + r;
-    const uint32_t row = pos < id_lim ? (uint32_t)ids[r] : 0xffffffffu;
-    const bool ok = row < row_lim;  // padding (0xffffffff), negative and too-large ids all fail this test
-    bad |= !ok && pos < id_lim;
-    cp_async16_zfill(buf + tc_swz(r, c, 8192), base + (int64_t)(ok ? row : 0u) * stride + c * 8, ok);
+  const int n = max(min(id_lim - t * C::TILE, C::TILE), 0);  // row ids the chunk has for this tile
+  int done = 0;
+  if (rows_map != nullptr &&
+      __all_sync(0xffffffffu, (lane >= n || (uint32_t)id0 < row_lim) && (lane + 32 >= n || (uint32_t)id1 < row_lim))) {
+    done = n & ~3;
+    if (lane == 0 && done > 0) mbar_expect_tx(full, (uint32_t)done * (2u * D));
+    __syncwarp();
+#pragma unroll
+    for (int i0 = 0; i0 < C::TILE / 4 * C::NB; i0 += 32) {
+      const int i = i0 + lane, blk = i % C::NB, r = i / C::NB * 4;
+      int row[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int lo = __shfl_sync(0xffffffffu, id0, (r + k) & 31), hi = __shfl_sync(0xffffffffu, id1, (r + k) & 31);
+        row[k] = r < 32 ? lo : hi;
+      }
+      if (r < done) tma_gather4(buf + blk * 8192 + r * 128, rows_map, col0 + 64 * blk, row[0], row[1], row[2], row[3], full);
+    }
+    if (done == C::TILE) return false;
   }
-  return bad;
-}
-// ids in registers, two per lane: row r is slot r >> 5 of lane r & 31 (V loader)
-template <typename T, int D>
-__device__ __noinline__ bool tc_gather_tile_regs(uint32_t buf, const T* base, int64_t stride, int id0, int id1, int t, int id_lim,
-                                                 uint32_t row_lim, int lane) {
-  using C = TcCfg<D>;
   const int c = lane % C::CPR;
   bool bad = false;
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
 #pragma unroll 4
     for (int i = 0; i < 32 / C::RPI; ++i) {
-      const int r = lane / C::CPR + C::RPI * i + 32 * h, pos = t * C::TILE + r;
+      const int r = lane / C::CPR + C::RPI * i + 32 * h;
       const int id = __shfl_sync(0xffffffffu, h == 0 ? id0 : id1, r & 31);
-      const uint32_t row = pos < id_lim ? (uint32_t)id : 0xffffffffu;
-      const bool ok = row < row_lim;
-      bad |= !ok && pos < id_lim;
+      if (r < done) continue;
+      const uint32_t row = r < n ? (uint32_t)id : 0xffffffffu;
+      const bool ok = row < row_lim;  // padding (0xffffffff), negative and too-large ids all fail this test
+      bad |= !ok && r < n;
       cp_async16_zfill(buf + tc_swz(r, c, 8192), base + (int64_t)(ok ? row : 0u) * stride + c * 8, ok);
     }
   }
@@ -312,6 +323,10 @@ __device__ __forceinline__ void tc_body(const TcParams& tp, uint8_t* smem, const
   if (tid == 32 && tp.has_tma) {  // the first TMA copy would otherwise pay for fetching its descriptor
     asm volatile("prefetch.tensormap [%0];\n" ::"l"(reinterpret_cast<uint64_t>(&tp.k_map)) : "memory");
     asm volatile("prefetch.tensormap [%0];\n" ::"l"(reinterpret_cast<uint64_t>(&tp.v_map)) : "memory");
+    if (tp.has_gather4) {
+      asm volatile("prefetch.tensormap [%0];\n" ::"l"(reinterpret_cast<uint64_t>(&tp.k_rows_map)) : "memory");
+      asm volatile("prefetch.tensormap [%0];\n" ::"l"(reinterpret_cast<uint64_t>(&tp.v_rows_map)) : "memory");
+    }
     if (tp.q_box_rows > 0) {
       asm volatile("prefetch.tensormap [%0];\n" ::"l"(reinterpret_cast<uint64_t>(&tp.q_map_tile)) : "memory");
       asm volatile("prefetch.tensormap [%0];\n" ::"l"(reinterpret_cast<uint64_t>(&tp.q_map)) : "memory");
@@ -659,6 +674,7 @@ __device__ __forceinline__ void tc_body(const TcParams& tp, uint8_t* smem, const
           // Row ids live in registers, two per lane and one tile ahead, so this role shares nothing with the K
           // loader: same dense test (64 consecutive pool rows -> two TMA boxes), same gather otherwise.
           const T* vbase = reinterpret_cast<const T*>(p.v) + (int64_t)kvh * p.v_s1;
+          const CUtensorMap* v_rows = tp.has_gather4 ? &tp.v_rows_map : nullptr;
           auto fetch_ids = [&](int t, int (&dst)[2]) {
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
@@ -695,7 +711,8 @@ __device__ __forceinline__ void tc_body(const TcParams& tp, uint8_t* smem, const
                 mbar_arrive(full);
               }
             } else {
-              const bool bad = tc_gather_tile_regs<T, D>(buf, vbase, p.v_s0, cur[0], cur[1], t, id_lim, row_lim, lane);
+              const bool bad = tc_gather_tile<T, D>(buf, v_rows, kvh * (int)p.v_s1, vbase, p.v_s0, cur[0], cur[1], t, id_lim,
+                                                       row_lim, lane, full);
               if (bad) flag_error(FT_DEV_BAD_KV_INDEX);
               mbar_arrive_on_cp_async(full);
             }
@@ -717,25 +734,8 @@ __device__ __forceinline__ void tc_body(const TcParams& tp, uint8_t* smem, const
             if (pos < id_lim) cp_async4(idx_sm + ((t % C::IDX_SLOTS) * C::TILE + i) * 4, ids_of_chunk + pos);
           }
         };
-        // one operand tile (K or V of tile t) into `buf`, signalling `full`
-        auto load_tile = [&](int t, uint32_t buf, uint32_t full, const CUtensorMap* map, const T* base, int64_t stride,
-                             bool dense, int first_row) {
-          if (dense) {
-            if (lane == 0) {
-              mbar_arrive_expect_tx(full, C::TILE_BYTES);
-#pragma unroll
-              for (int h = 0; h < C::NB; ++h) tma_load_3d(buf + h * 8192, map, 64 * h, kvh, first_row, full);
-            } else {
-              mbar_arrive(full);
-            }
-            return;
-          }
-          const int* ids = ring + (t % C::IDX_SLOTS) * C::TILE;
-          const bool bad = tc_gather_tile_smem<T, D>(buf, base, stride, ids, t, id_lim, row_lim, lane);
-          if (bad) flag_error(FT_DEV_BAD_KV_INDEX);
-          mbar_arrive_on_cp_async(full);
-        };
         const T* kbase = reinterpret_cast<const T*>(p.k) + (int64_t)kvh * p.k_s1;
+        const CUtensorMap* k_rows = tp.has_gather4 ? &tp.k_rows_map : nullptr;
         if (ntiles > 0) issue_ids(0);
         cp_async_commit();
         if (ntiles > 1) issue_ids(1);
@@ -749,11 +749,12 @@ __device__ __forceinline__ void tc_body(const TcParams& tp, uint8_t* smem, const
           if (s == 0 && lane == 0) FT_TL_COARSE_MARK(5);
           // dense tile: 64 valid, consecutive row ids inside the buffer -> TMA
           const int* ids = ring + (s % C::IDX_SLOTS) * C::TILE;
+          const int id0 = ids[lane], id1 = ids[lane + 32];  // (stale past the end of the chunk: not used there)
           bool dense = false;
           int first_row = 0;
           if (tp.has_tma && (s + 1) * C::TILE <= id_lim) {
-            first_row = ids[0];
-            const bool mine = ids[lane] == first_row + lane && ids[lane + 32] == first_row + lane + 32;
+            first_row = __shfl_sync(0xffffffffu, id0, 0);
+            const bool mine = id0 == first_row + lane && id1 == first_row + lane + 32;
             dense = __all_sync(0xffffffffu, mine) && first_row >= 0 && (uint32_t)(first_row + C::TILE) <= row_lim;
           }
           if (!tc_wait(bar(C::K_EMPTY + b), ((uint32_t)(g / C::NSK) & 1u) ^ 1u, abort_flag)) {
@@ -763,7 +764,21 @@ __device__ __forceinline__ void tc_body(const TcParams& tp, uint8_t* smem, const
 #ifdef FT_TL_LOADERS
           if (s == FT_TL_TILE && lane == 0) FT_TL_MARK(5);
 #endif
-          load_tile(s, k_buf(g), bar(C::K_FULL + b), &tp.k_map, kbase, p.k_s0, dense, first_row);
+          const uint32_t buf = k_buf(g), full = bar(C::K_FULL + b);
+          if (dense) {
+            if (lane == 0) {
+              mbar_arrive_expect_tx(full, C::TILE_BYTES);
+#pragma unroll
+              for (int h = 0; h < C::NB; ++h) tma_load_3d(buf + h * 8192, &tp.k_map, 64 * h, kvh, first_row, full);
+            } else {
+              mbar_arrive(full);
+            }
+          } else {
+            const bool bad = tc_gather_tile<T, D>(buf, k_rows, kvh * (int)p.k_s1, kbase, p.k_s0, id0, id1, s, id_lim, row_lim,
+                                                  lane, full);
+            if (bad) flag_error(FT_DEV_BAD_KV_INDEX);
+            mbar_arrive_on_cp_async(full);
+          }
 #ifdef FT_TL_LOADERS
           if (s == FT_TL_TILE && lane == 0) FT_TL_MARK(6);
 #endif
