@@ -115,6 +115,7 @@ int build_plan(const int32_t* parent, const int32_t* seqlen, int32_t n_nodes, co
     m.rows_per_cta = 128;  // the tcgen05 stage-1 kernel holds 128 query rows per CTA
     m.ridge_flop_per_byte = (head_dim == 64 ? 2 : 4) * m.ridge_flop_per_byte;
     if (head_dim == 256) m.ctas_per_sm = 1;
+    if (head_dim != 128) m.group_member_tokens = 0;  // a caller that reads row ranges at these sizes asks with a model
   }
   ft_plan* plan = new (std::nothrow) ft_plan();
   if (plan == nullptr) return FT_ERR_TOO_LARGE;
@@ -266,15 +267,16 @@ int build_plan(const int32_t* parent, const int32_t* seqlen, int32_t n_nodes, co
       s.chunk = ceil_div(ceil_div(s.length, n_chunks), m.tile_tokens) * m.tile_tokens;
     }
 
-    // ---- groups of short nodes (table-building mode, head_dim 128, 16-bit elements: the shape whose kernels honour
-    // per-row token ranges).  Candidates - at most small_tile requests, at most group_member_tokens tokens - are
+    // ---- groups of short nodes (table-building mode, 16-bit elements, head_dim 64, 128 or 256: the shapes whose
+    // kernels honour per-row token ranges; serving path: head_dim 128).  Candidates - at most small_tile requests, at most group_member_tokens tokens - are
     // taken in order; a group is closed when the next candidate would exceed q_tile requests or 16 tiles of tokens,
     // would exceed the per-task token target (at least 4 tiles) once the group has more than small_tile requests,
     // or shares a request with it; groups with fewer than
     // group_min_members members, or not more requests than small_tile, are dissolved.  Result: the other virtual
     // nodes in their order, then groups and dissolved candidates in the order they were closed.
     bool any_groups = false;
-    if ((direct == nullptr || direct->tail_room >= 0) && head_dim == 128 && m.elem_bytes == 2 && m.group_member_tokens > 0) {
+    const bool tc_dim = head_dim == 128 || (direct == nullptr && (head_dim == 64 || head_dim == 256));
+    if ((direct == nullptr || direct->tail_room >= 0) && tc_dim && m.elem_bytes == 2 && m.group_member_tokens > 0) {
       const int64_t tile = m.tile_tokens;
       const int64_t target_tokens = (int64_t)std::floor(target / (double)row_bytes);
       int64_t hard_cap = 16 * tile;

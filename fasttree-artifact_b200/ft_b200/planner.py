@@ -421,7 +421,7 @@ def plan_b200(tree, kv_ptrs, batch_size, num_qo_heads, num_kv_heads, head_dim, p
     m = b200_model_for(params, head_dim, model)
     vnodes, assign, q_tile, small_tile, target = b200_virtual_nodes(
         tree, num_qo_heads, num_kv_heads, head_dim, m, lambda a, i: _chain_ranges(tree, kv_ptrs, a, i))
-    if head_dim == 128 and m.elem_bytes == 2:      # the kernels that honour row ranges exist for this shape
+    if head_dim in (64, 128, 256) and m.elem_bytes == 2:      # the kernels that honour row ranges exist for these shapes
         vnodes = b200_group_short_nodes(vnodes, q_tile, small_tile, m,
                                         int(math.floor(target / (2 * head_dim * m.elem_bytes))), num_kv_heads=num_kv_heads)
     vnodes = b200_split_tail(vnodes, q_tile, small_tile, m, num_kv_heads)
@@ -719,6 +719,13 @@ def b200_model_for(params, head_dim, model=None):
         # time, covers half the flops, and at 256 one CTA fills an SM
         m = replace(m, rows_per_cta=128, ridge_flop_per_byte=(2 if head_dim == 64 else 4) * m.ridge_flop_per_byte,
                     ctas_per_sm=1 if head_dim == 256 else m.ctas_per_sm)
+        # Short nodes are grouped at head_dim 64 and 256 when the storage type was stated.  Unstated, K/V may be fp32,
+        # whose kernels do the work of a group's masked rows on the CUDA cores (at 128 it is taken to be 16-bit).
+        # Measured per step, 32/8 heads, leaves of 16 / 32 / 100 tokens under 1,16 nodes, ungrouped -> grouped: 512 leaves
+        # of 64 60.3 -> 24.8 / 62.4 -> 31.9 / 82.3 -> 55.4 us, of 256 370 -> 61 / 376 -> 72 / 391 -> 139 us; 64 leaves of 64
+        # 14.0 -> 12.4 / 14.0 -> 13.3 / 14.9 -> 14.9 us.
+        if head_dim != 128 and not getattr(params, "kv_dtype_stated", False):
+            m = replace(m, group_member_tokens=0)
     if explicit is None and getattr(params, "kv_elem_bytes", 2) == 4:
         # fp32 storage runs on the CUDA-core kernel: 32-token tiles, one warp per scheduler, so a chunk costs
         # several microseconds per tile and a small problem is better cut down to single tiles

@@ -33,7 +33,8 @@ class FastTreeParams:
     overwrite ``TSQs``/``TSKs`` with the tile sizes it settled on.
     ``kv_elem_bytes`` (B200 splitter only, no counterpart in the reference, whose
     preparation never sees the dtype): 4 tells the splitter that K/V are fp32, which
-    run on the 32-token CUDA-core kernel and are cut as fine as 32 tokens."""
+    run on the 32-token CUDA-core kernel and are cut as fine as 32 tokens.  Stated with
+    ``set_kv_dtype`` it also lets short nodes be grouped at head_dim 64 and 256."""
     alpha = 0.66
     beta = 0.33
     gamma = 0.1
@@ -44,6 +45,7 @@ class FastTreeParams:
     native_planner = True
     verbose = False
     kv_elem_bytes = 2
+    kv_dtype_stated = False
 
     def set_values(self, alpha, beta, gamma):
         self.alpha = alpha
@@ -65,6 +67,7 @@ class FastTreeParams:
         if size not in (2, 4):
             raise ValueError("K/V are 16-bit or fp32")
         self.kv_elem_bytes = size
+        self.kv_dtype_stated = True
 
     def set_planner(self, name):
         if name not in ("b200", "reference"):

@@ -337,8 +337,8 @@ int ft_plan_copy_tables(const ft_plan* plan, int32_t* vnode_to_kv_entries, int32
                         int32_t* vnode_to_q_lens, int32_t* req_to_vnode_entries, int32_t* req_to_vnode_offs,
                         int32_t* req_to_vnode_lens, int32_t* node_assignments);
 /* The optional tenth table, vnode_q_kv_ranges of ft_decode_args ([partial_rows][2] int32): only when
- * ft_plan_info.has_row_ranges is 1 (ft_plan_b200_build at head_dim 128 with 16-bit elements, when short nodes were
- * packed into groups); FT_ERR_INVALID_ARGUMENT otherwise. */
+ * ft_plan_info.has_row_ranges is 1 (ft_plan_b200_build with 16-bit elements, at head_dim 128 or, given a model, 64 or 256,
+ * when short nodes were packed into groups); FT_ERR_INVALID_ARGUMENT otherwise. */
 int ft_plan_copy_row_ranges(const ft_plan* plan, int32_t* vnode_q_kv_ranges);
 void ft_plan_free(ft_plan* plan);
 

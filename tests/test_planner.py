@@ -484,3 +484,21 @@ def test_cascade_levels_describe_the_tree():
         assert sorted(x for lv in idx for x in lv) == list(range(ptrs[-1]))
         for q, k in zip(qo, kv):
             assert q[0] == 0 and q[-1] == batch and len(q) == len(k) and all(b > a for a, b in zip(q, q[1:]))
+
+
+@pytest.mark.parametrize("d", [64, 256])
+@pytest.mark.parametrize("sizes,lens", [([1, 16, 256], [64, 32, 16]), ([1, 3, 50], [100, 1, 127]), ([1, 5], [10, 128])])
+def test_groups_at_other_head_dims_once_the_storage_type_is_stated(d, sizes, lens):
+    """Stated 16-bit storage: groups, the same from both builders.  Stated fp32: none."""
+    tree, batch, ptrs = product_tree(ref_inputs.layered_tree(sizes, lens))
+    plans = []
+    for native in (False, True):
+        p = make_params(32, 8, [16, 4], planner_name="b200")
+        p.native_planner = native
+        p.set_kv_dtype(torch.float32)
+        assert fasttree.build_plan(tree, ptrs, batch, 32, 8, d, [1024, 128], [132, 528], [132, 132], p).vnode_q_kv_ranges is None
+        p.set_kv_dtype(torch.bfloat16)
+        plans.append(fasttree.build_plan(tree, ptrs, batch, 32, 8, d, [1024, 128], [132, 528], [132, 132], p))
+    check_plan_covers_every_path_once(tree, ptrs, batch, plans[0])
+    assert plans[0].vnode_q_kv_ranges is not None
+    _same_plan(*plans)
