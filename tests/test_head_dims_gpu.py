@@ -79,7 +79,7 @@ def test_head_dims_with_scattered_rows_and_row_ranges(d):
 
 @pytest.mark.parametrize("d", [64, 256])
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16], ids=["fp16", "bf16"])
-@pytest.mark.parametrize("spec", [([1, 16, 256], [64, 32, 16], 32, 8), ([1, 3, 50], [100, 1, 127], 16, 1),
+@pytest.mark.parametrize("spec", [([1, 16, 256], [64, 32, 16], 32, 8), ([1, 3, 50], [100, 1, 40], 16, 1),
                                   ([1, 40], [10, 33], 8, 8)], ids=["g4", "g16", "g1"])
 def test_groups_of_short_nodes(d, dtype, spec):
     """Leaves grouped into many-row tasks with token ranges, through every kernel family that takes the head size."""
