@@ -18,7 +18,6 @@
 #include "ft_stage1_narrow.cuh"
 #include "ft_stage1_stream.cuh"
 #include "ft_stage1_tc.cuh"
-#include "ft_stage1_persist.cuh"
 #include "ft_stage2.cuh"
 
 namespace {
@@ -398,11 +397,11 @@ static __device__ unsigned int g_sched_counters[64][2];
 
 template <typename T>
 int launch_persist(ft::TcParams p, int hkv, cudaStream_t st) {
-  using C = ft::PsCfg;
+  using C = ft::TcCfg<128>;
   if (dry_run("stage1_persist_kernel")) return FT_OK;
   static OncePerDevice once;
   int dev = 0;
-  FT_CUDA_OK(raise_smem_limit(once, ft::stage1_persist_kernel<T>, C::SMEM_BYTES, &dev));
+  FT_CUDA_OK(raise_smem_limit(once, ft::stage1_persist_kernel<T, 128>, C::SMEM_BYTES, &dev));
   if (dev < 0 || dev >= 64) return fail(FT_ERR_UNSUPPORTED, "device ordinal %d outside 0..63", dev);
   static std::atomic<unsigned int*> counters_of_device[64];
   unsigned int* base = counters_of_device[dev].load(std::memory_order_acquire);
@@ -418,7 +417,7 @@ int launch_persist(ft::TcParams p, int hkv, cudaStream_t st) {
   if (tasks <= 0) return FT_OK;
   if (tasks > 0x7fffffffLL) return fail(FT_ERR_TOO_LARGE, "vnodes x kv heads exceeds the task limit");
   const unsigned grid = (unsigned)(tasks < slots ? tasks : slots);
-  FT_CUDA_OK(launch_early(ft::stage1_persist_kernel<T>, grid, C::THREADS, C::SMEM_BYTES, st, p));
+  FT_CUDA_OK(launch_early(ft::stage1_persist_kernel<T, 128>, grid, C::THREADS, C::SMEM_BYTES, st, p));
   count_launch();
   return FT_OK;
 }
@@ -636,6 +635,7 @@ int ft_stage1(const ft_decode_args* a) {
       ft::Stage1Params p = stage1_params(a);
       p.node_offset = ph == 0 ? o0 : o1;
       p.node_count = joined ? n0 + n1 : (ph == 0 ? n0 : n1);
+      p.node_split = ph == 0 ? n0 : 0;
       if (p.node_count <= 0) continue;
       const ft::TcParams tp = tc_params(p, a);
       rc = a->dtype == FT_F16 ? launch_persist<__half>(tp, a->num_kv_heads, st)

@@ -47,6 +47,9 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
+// Barrier of the four warps that run a task (the CTA may hold other warps beside them)
+__device__ __forceinline__ void four_warps_sync() { asm volatile("bar.sync 3, 128;\n" ::: "memory"); }
+
 __device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], uint32_t addr) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
@@ -190,7 +193,7 @@ struct KvPipe {
   }
   __device__ __forceinline__ void wait_indices() {
     cp_async_wait<0>();
-    __syncthreads();
+    four_warps_sync();
   }
   __device__ __forceinline__ void prime_indices() {
     issue_first_indices();
@@ -229,7 +232,7 @@ struct KvPipe {
   // top of iteration j: tile j has landed; refill the stage freed by tile j-1
   __device__ __forceinline__ void advance(int j) {
     cp_async_wait<C::STAGES - 2>();
-    __syncthreads();
+    four_warps_sync();
     const int nt = j + C::STAGES - 1;
     if (nt < ntiles) {
       issue_tile(nt);
@@ -242,7 +245,7 @@ struct KvPipe {
   __device__ __forceinline__ uint32_t v_stage(int j) const { return k_stage(j) + C::STAGE_BYTES; }
   __device__ __forceinline__ void drain() {
     cp_async_wait<0>();
-    __syncthreads();
+    four_warps_sync();
   }
 };
 

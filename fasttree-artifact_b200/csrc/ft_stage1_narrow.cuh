@@ -46,7 +46,8 @@ struct NarrowCfg {
 };
 
 template <typename T, int D, int NQ>
-__device__ __forceinline__ void narrow_body(const Stage1Params& p, uint8_t* smem, const int vn, const int kvh) {
+__device__ __forceinline__ void narrow_body(const Stage1Params& p, uint8_t* smem, const int kvh, const int q_off, const int q_len,
+                                            const int kv_off, const int kv_len) {
   using C = MmaCfg<D>;
   using N = NarrowCfg<D, NQ>;
   const uint32_t q_sm = smem_u32(smem);
@@ -58,8 +59,6 @@ __device__ __forceinline__ void narrow_body(const Stage1Params& p, uint8_t* smem
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g8 = lane >> 2, t4 = lane & 3;
-  const int q_off = p.q_offs[vn], q_len = p.q_lens[vn];
-  const int kv_off = p.kv_offs[vn], kv_len = max(p.kv_lens[vn], 0);
   const int G = p.group;
   const int rows = q_len * G;
   if (rows <= 0) return;
@@ -229,7 +228,7 @@ __device__ __forceinline__ void narrow_body(const Stage1Params& p, uint8_t* smem
         epi_l[warp * N::ROWS + r + 1] = lb;
       }
     }
-    __syncthreads();
+    four_warps_sync();
 
     // ---- merge the four warps, normalise, write the partial rows
     {
@@ -272,7 +271,7 @@ __device__ __forceinline__ void narrow_body(const Stage1Params& p, uint8_t* smem
         }
       }
     }
-    __syncthreads();
+    four_warps_sync();
   }
 }
 
@@ -280,11 +279,11 @@ __device__ __forceinline__ void narrow_body(const Stage1Params& p, uint8_t* smem
 // two-block body (which also loops if a task has more than 16 rows).
 template <typename T, int D>
 __device__ __forceinline__ void narrow_dispatch(const Stage1Params& p, uint8_t* smem, const int vn, const int kvh) {
-  const int rows = p.q_lens[vn] * p.group;
-  if (rows <= 8)
-    narrow_body<T, D, 1>(p, smem, vn, kvh);
+  const int q_off = p.q_offs[vn], q_len = p.q_lens[vn], kv_off = p.kv_offs[vn], kv_len = max(p.kv_lens[vn], 0);
+  if (q_len * p.group <= 8)
+    narrow_body<T, D, 1>(p, smem, kvh, q_off, q_len, kv_off, kv_len);
   else
-    narrow_body<T, D, 2>(p, smem, vn, kvh);
+    narrow_body<T, D, 2>(p, smem, kvh, q_off, q_len, kv_off, kv_len);
 }
 
 template <typename T, int D>

@@ -97,7 +97,9 @@ struct TcCfg {
   static constexpr int NBARS = 18;
   static constexpr int ABORT_OFF = BAR_OFF + NBARS * 8;
   static constexpr int TMEM_SLOT_OFF = ABORT_OFF + 4;
-  static constexpr int SMEM_BYTES = TMEM_SLOT_OFF + 4;
+  static constexpr int NEXT_OFF = TMEM_SLOT_OFF + 4;  // looping kernel: {task, q_off, q_len, kv_off, kv_len, few rows} of the next task, twice
+  static constexpr int TOTALS_OFF = NEXT_OFF + 2 * 24;  // looping kernel: {tasks, many-row tasks, first vnode}
+  static constexpr int SMEM_BYTES = TOTALS_OFF + 12;
   static constexpr int TMEM_COLS = D == 256 ? 512 : 256;
   static constexpr int S_COL = 0, O_COL = 128;        // S is double-buffered: columns [0,64) and [64,128)
   static constexpr int WAIT_LIMIT = 1 << 16;          // probes of mbarrier.try_wait before a wait gives up
@@ -217,6 +219,20 @@ __device__ __forceinline__ float exp2_fma(float x) {
 #define FT_EXP2_FMA_EVERY 0  // n > 0: every n-th pair of a row's 32 score pairs takes exp2_fma instead of ex2.approx
 #endif
 
+// First wait of the looping kernel that gave up since the record was last read: {wait id (0 = none), block, warp, task
+// sequence number, tile counter, 0...}.  Wait ids: 2 S tile, 3 P.V before O is touched, 4 P.V before the epilogue, 5 Q
+// tile, 6 P or V tile, 8 K tile, 10 K/V stage free.
+__device__ int g_wait_diag[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+
+__device__ __forceinline__ void note_wait(int id, int seq, int counter) {
+  if (atomicCAS(&g_wait_diag[0], 0, id) == 0) {
+    g_wait_diag[1] = (int)blockIdx.x;
+    g_wait_diag[2] = (int)(threadIdx.x >> 5);
+    g_wait_diag[3] = seq;
+    g_wait_diag[4] = counter;
+  }
+}
+
 // Bounded wait for the phase of `bar` with the given parity.  Gives up after WAIT_LIMIT probes or as soon as
 // another role has raised the CTA's abort flag; the caller then raises the flag itself and unwinds.
 __device__ __forceinline__ bool tc_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
@@ -285,8 +301,9 @@ __device__ __noinline__ bool tc_gather_tile(uint32_t buf, const CUtensorMap* row
   return bad;
 }
 
-template <typename T, int D>
-__device__ __forceinline__ void tc_body(const TcParams& tp, uint8_t* smem, const int vn, const int kvh) {
+// LOOP false: one task (vn, kvh).  LOOP true: the CTA works through tasks of the whole launch, claimed from a counter.
+template <typename T, int D, bool LOOP>
+__device__ __forceinline__ void tc_body(const TcParams& tp, uint8_t* smem, int vn, int kvh) {
   using C = TcCfg<D>;
   const Stage1Params& p = tp.p;
   const uint32_t sm = smem_u32(smem);
@@ -308,7 +325,7 @@ __device__ __forceinline__ void tc_body(const TcParams& tp, uint8_t* smem, const
   // hides the reads' latency as well.
   uint32_t num_sms;
   asm("mov.u32 %0, %%nsmid;" : "=r"(num_sms));
-  const bool first_wave = blockIdx.x < 2u * num_sms;
+  const bool first_wave = LOOP || blockIdx.x < 2u * num_sms;
   int q_off = 0, q_len = 0, kv_off = 0, kv_len = 0;
   auto read_task = [&]() {
     wait_for_prior_grid();
@@ -360,16 +377,104 @@ __device__ __forceinline__ void tc_body(const TcParams& tp, uint8_t* smem, const
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  if (first_wave) read_task();
+  // Looping form: tasks [0, total) are (vnode, kv head) pairs, kv head fastest, the many-row ones first; a CTA starts
+  // with the task of its index and claims the others.  The K loader claims during the last tiles of a task, reads the
+  // new task's table entries and leaves them in shared memory (two slots: it can be one task ahead of a slow warp).
+  int task = (int)blockIdx.x, seq = 0;
+  volatile int* next = reinterpret_cast<volatile int*>(smem + C::NEXT_OFF);
+  volatile int* totals = reinterpret_cast<volatile int*>(smem + C::TOTALS_OFF);
+  // Few-row tasks (at most eight rows: the two-block body needs more registers than these warps have) run on the softmax
+  // warps with the memory-bound body, which knows no token ranges: a task with a row that does not attend to the whole
+  // chunk takes the tensor-core path like the many-row ones.  (All lanes of a warp.)
+  auto few_rows = [&](int t_q_off, int t_q_len, int t_kv_len) {
+    if (D == 256 || t_q_len * p.group > 8) return 0;
+    bool narrowed = false;
+    if (p.q_ranges != nullptr && lane < t_q_len) {
+      const int64_t part = (int64_t)t_q_off + lane;
+      if (part >= 0 && part < p.num_partial_rows) narrowed = p.q_ranges[2 * part] > 0 || p.q_ranges[2 * part + 1] < t_kv_len;
+    }
+    return __any_sync(0xffffffffu, narrowed) ? 0 : 1;
+  };
+  if constexpr (LOOP) {
+    wait_for_prior_grid();
+    int node_offset = p.node_offset;
+    int n0 = p.node_split, n1 = p.node_count - p.node_split;
+    if (p.dev_phase != nullptr) {
+      n0 = max(__ldg(p.dev_phase + 0), 0);
+      n1 = max(__ldg(p.dev_phase + 1), 0);
+      node_offset = max(__ldg(p.dev_phase + 2), 0);
+      const int o1 = __ldg(p.dev_phase + 3);
+      if (n0 > 0 && n1 > 0 && o1 != node_offset + n0) {  // the phases must be adjacent
+        if (tid == 0) flag_error(FT_DEV_BAD_ROW_INDEX);
+        n1 = 0;
+      }
+    }
+    const int total = (int)min((long long)(n0 + n1) * p.num_kv_heads, 0x7fffffffLL - (long long)gridDim.x);
+    vn = node_offset + task / p.num_kv_heads;
+    kvh = task - task / p.num_kv_heads * p.num_kv_heads;
+    if (task < total) {
+      q_off = p.q_offs[vn];
+      q_len = p.q_lens[vn];
+      kv_off = p.kv_offs[vn];
+      kv_len = max(p.kv_lens[vn], 0);
+    }
+    if (warp == 0) {
+      const int few = task < total && task >= n0 * p.num_kv_heads ? few_rows(q_off, q_len, kv_len) : 0;
+      if (lane == 0) next[5] = few;
+    }
+    if (tid == 0) {
+      totals[0] = total;
+      totals[1] = (int)min((long long)n0 * p.num_kv_heads, (long long)total);
+      totals[2] = node_offset;
+    }
+    __syncthreads();
+  } else {
+    if (first_wave) read_task();
+  }
   if (tid == 0) FT_TL_MARK(0);
   const int G = p.group;
-  const int rows = q_len * G;  // <= 0: nothing to do but to give the tensor memory back
   const float scale2 = p.sm_scale * 1.4426950408889634f;
-  const int ntiles = (kv_len + C::TILE - 1) / C::TILE;
-  // row ids past the end of the table are a plan error: flag once, treat those tokens as padding
-  const int id_lim = kv_ids_limit(p, kv_off, kv_len);
-  const int32_t* ids_of_chunk = kv_ids_base(p, kv_off);
-  if (rows > 0 && id_lim < kv_len && tid == 0) flag_error(FT_DEV_BAD_KV_INDEX);
+  int rows = 0, ntiles = 0, id_lim = 0;
+  const int32_t* ids_of_chunk = nullptr;
+  auto enter_task = [&]() {
+    rows = q_len * G;  // <= 0: nothing to do but to give the tensor memory back
+    ntiles = (kv_len + C::TILE - 1) / C::TILE;
+    // row ids past the end of the table are a plan error: flag once, treat those tokens as padding
+    id_lim = kv_ids_limit(p, kv_off, kv_len);
+    ids_of_chunk = kv_ids_base(p, kv_off);
+    if (rows > 0 && id_lim < kv_len && tid == 0) flag_error(FT_DEV_BAD_KV_INDEX);
+  };
+  if (!LOOP || task < totals[0]) enter_task();
+  // warp 5, all lanes: the task after this one
+  auto claim_next = [&]() {
+    int t = 0;
+    if (lane == 0) t = (int)gridDim.x + (int)atomicAdd(tp.sched, 1u);
+    t = __shfl_sync(0xffffffffu, t, 0);
+    volatile int* slot = next + 6 * ((seq + 1) & 1);
+    if (t < totals[0]) {
+      const int32_t* tab = (lane & 3) == 0 ? p.q_offs : (lane & 3) == 1 ? p.q_lens : (lane & 3) == 2 ? p.kv_offs : p.kv_lens;
+      const int v = __ldg(tab + totals[2] + t / p.num_kv_heads);
+      if (lane < 4) slot[1 + lane] = v;
+      int few = 0;
+      if (t >= totals[1])
+        few = few_rows(__shfl_sync(0xffffffffu, v, 0), __shfl_sync(0xffffffffu, v, 1), max(__shfl_sync(0xffffffffu, v, 3), 0));
+      if (lane == 0) slot[5] = few;
+    }
+    if (lane == 0) slot[0] = t;
+  };
+  auto next_task = [&]() {  // after the barrier that ends a task
+    ++seq;
+    const volatile int* slot = next + 6 * (seq & 1);
+    task = slot[0];
+    if (task >= totals[0]) return false;
+    kvh = task - task / p.num_kv_heads * p.num_kv_heads;
+    q_off = slot[1];
+    q_len = slot[2];
+    kv_off = slot[3];
+    kv_len = max(slot[4], 0);
+    enter_task();
+    return true;
+  };
   const uint32_t row_lim = (uint32_t)(p.kv_rows < 0x7fffffffLL ? p.kv_rows : 0x7fffffffLL);
   auto k_buf = [&](int t) { return sm + C::K_OFF + (t % C::NSK) * C::TILE_BYTES; };
   auto v_buf = [&](int t) { return sm + C::V_OFF + (t & 1) * C::TILE_BYTES; };
@@ -378,7 +483,8 @@ __device__ __forceinline__ void tc_body(const TcParams& tp, uint8_t* smem, const
   // buffer g % NSK for the (g / NSK)-th time, which gives every wait its barrier phase without per-barrier counters.
   int g0 = 0, pass = 0;
   bool dead = false;
-  auto give_up = [&]() {
+  auto give_up = [&](int wait_id) {
+    if (LOOP && *abort_flag == 0) note_wait(wait_id, seq, g0);  // only the wait that gave up first is of interest
     *abort_flag = 1;
     flag_error(FT_DEV_WAIT_TIMEOUT);
     dead = true;
@@ -395,10 +501,38 @@ __device__ __forceinline__ void tc_body(const TcParams& tp, uint8_t* smem, const
     return true;
   };
 
+  // end of a task without passes
+  auto task_end = [&]() {
+    __syncthreads();
+    return *abort_flag == 0;
+  };
+  // A role's code over the CTA's tasks: pass_of_role(row0) for each pass of 128 rows, few() for a few-row task.
+  auto run_tasks = [&](auto&& few, auto&& pass_of_role) {
+    bool more = !LOOP || task < totals[0];
+    while (more) {
+      if (LOOP && (rows <= 0 || next[6 * (seq & 1) + 5] != 0)) {
+        few();
+        more = task_end() && next_task();
+        continue;
+      }
+      for (int row0 = 0; row0 < rows && more; row0 += C::ROWS) {
+        pass_of_role(row0);
+        more = pass_end();
+      }
+      more = LOOP && more && next_task();
+    }
+  };
+
   // Each warpgroup sets its register budget on entry to its own code, so that the budget holds for all of it.
   if (warp < 4) {
     reg_grow<C::REGS_SOFTMAX>();
-    for (int row0 = 0; row0 < rows; row0 += C::ROWS) {
+    auto few_row_task = [&]() {
+      if constexpr (LOOP && D <= 128) {
+        if (rows > 0) narrow_body<T, D, 1>(p, smem, kvh, q_off, q_len, kv_off, kv_len);
+        proxy_fence();  // what these warps wrote to the operand buffers comes before the next task's TMA copies
+      }
+    };
+    run_tasks(few_row_task, [&](const int row0) {
       {
         // ================================================================ softmax (one query row per thread)
         const uint32_t t_lane = tmem + ((uint32_t)(warp * 32) << 16);  // this warp's 32-lane quadrant
@@ -417,7 +551,7 @@ __device__ __forceinline__ void tc_body(const TcParams& tp, uint8_t* smem, const
         for (int j = 0; j < ntiles && !dead; ++j) {
           const int g = g0 + j, b = g & 1;
           if (!tc_wait(bar(C::S_FULL + b), (uint32_t)(g >> 1) & 1u, abort_flag)) {
-            give_up();
+            give_up(2);
             break;
           }
           tc_fence_after();
@@ -499,7 +633,7 @@ __device__ __forceinline__ void tc_body(const TcParams& tp, uint8_t* smem, const
           if (j == FT_TL_TILE && tid == 0) FT_TL_SOFTMAX_MARK(11);
           if (j > 0 && __any_sync(0xffffffffu, grow)) {
             if (!tc_wait(bar(C::PV_DONE + ((g - 1) & 1)), (uint32_t)((g - 1) >> 1) & 1u, abort_flag)) {
-              give_up();
+              give_up(3);
               break;
             }
             tc_fence_after();
@@ -524,7 +658,7 @@ __device__ __forceinline__ void tc_body(const TcParams& tp, uint8_t* smem, const
         // ---- epilogue: wait for the last P.V, normalise, write this thread's partial row
         if (!dead && ntiles > 0 &&
             !tc_wait(bar(C::PV_DONE + ((g0 + ntiles - 1) & 1)), (uint32_t)((g0 + ntiles - 1) >> 1) & 1u, abort_flag))
-          give_up();
+          give_up(4);
         if (!dead) {
           tc_fence_after();
           if (tid == 0) FT_TL_MARK(3);
@@ -579,14 +713,15 @@ __device__ __forceinline__ void tc_body(const TcParams& tp, uint8_t* smem, const
             }
           }
           if (tid == 0) FT_TL_MARK(9);
+          if (LOOP) proxy_fence();  // the staged rows come before the next task's TMA copies
         }
       }
-      if (!pass_end()) break;
-    }
+    });
   } else {
     reg_shrink<C::REGS_OTHER>();
-    for (int row0 = 0; row0 < rows; row0 += C::ROWS) {
-      if (warp >= 6) {
+    auto no_role = [&]() {};
+    if (warp >= 6) {
+      run_tasks(no_role, [&](const int row0) {
         // ================================================================ Q gather (64 threads)
         // request ids of this pass's slots -> the (still unused) V buffers, then the rows themselves
         const int qt = tid - 192, ld_c = qt % C::CPR, ld_r = qt / C::CPR;
@@ -695,7 +830,7 @@ __device__ __forceinline__ void tc_body(const TcParams& tp, uint8_t* smem, const
               dense = __all_sync(0xffffffffu, mine) && first_row >= 0 && (uint32_t)(first_row + C::TILE) <= row_lim;
             }
             if (!tc_wait(bar(C::V_EMPTY + b), ((uint32_t)(g >> 1) & 1u) ^ 1u, abort_flag)) {
-              give_up();
+              give_up(10);
               break;
             }
             const uint32_t buf = v_buf(g), full = bar(C::V_FULL + b);
@@ -724,7 +859,9 @@ __device__ __forceinline__ void tc_body(const TcParams& tp, uint8_t* smem, const
           }
           cp_async_wait<0>();
         }
-      } else if (warp == 5) {
+      });
+    } else if (warp == 5) {
+      run_tasks(claim_next, [&](const int row0) {
         // ================================================================ loader
         const int* ring = reinterpret_cast<const int*>(smem + C::IDX_OFF);
         auto issue_ids = [&](int t) {  // 64 row ids of tile t -> slot t % 3, two per lane
@@ -758,7 +895,7 @@ __device__ __forceinline__ void tc_body(const TcParams& tp, uint8_t* smem, const
             dense = __all_sync(0xffffffffu, mine) && first_row >= 0 && (uint32_t)(first_row + C::TILE) <= row_lim;
           }
           if (!tc_wait(bar(C::K_EMPTY + b), ((uint32_t)(g / C::NSK) & 1u) ^ 1u, abort_flag)) {
-            give_up();
+            give_up(10);
             break;
           }
 #ifdef FT_TL_LOADERS
@@ -786,7 +923,10 @@ __device__ __forceinline__ void tc_body(const TcParams& tp, uint8_t* smem, const
           cp_async_commit();
         }
         cp_async_wait<0>();
-      } else {
+        if (LOOP && row0 + C::ROWS >= rows) claim_next();
+      });
+    } else {
+      run_tasks(no_role, [&](const int row0) {
         // ================================================================ MMA issue
         if (lane == 0) {
           const uint32_t idesc_s = tc_idesc<T>(128, C::TILE, false);
@@ -815,14 +955,14 @@ __device__ __forceinline__ void tc_body(const TcParams& tp, uint8_t* smem, const
             tc_commit(bar(C::PV_DONE + b));
             return true;
           };
-          if (ntiles > 0 && !tc_wait(bar(C::Q_FULL), (uint32_t)pass & 1u, abort_flag)) give_up();
+          if (ntiles > 0 && !tc_wait(bar(C::Q_FULL), (uint32_t)pass & 1u, abort_flag)) give_up(5);
           FT_TL_COARSE_MARK(7);
           for (int t = 0; t < ntiles && !dead; ++t) {
             const int g = g0 + t, b = g & 1, kb = g % C::NSK;
             // S_t = Q K_t^T into S buffer b.  The buffer's previous tenant, P of tile t-2, was consumed by a P.V issued
             // before this point, and same-shape MMAs execute in issue order.
             if (!tc_wait(bar(C::K_FULL + kb), (uint32_t)(g / C::NSK) & 1u, abort_flag)) {
-              give_up();
+              give_up(8);
               break;
             }
             if (t == 0) FT_TL_COARSE_MARK(6);
@@ -841,15 +981,14 @@ __device__ __forceinline__ void tc_body(const TcParams& tp, uint8_t* smem, const
             tc_commit(bar(C::K_EMPTY + kb));
             tc_commit(bar(C::S_FULL + b));
             if (t > 0 && !issue_pv(t - 1)) {
-              give_up();
+              give_up(6);
               break;
             }
           }
-          if (!dead && ntiles > 0 && !issue_pv(ntiles - 1)) give_up();
+          if (!dead && ntiles > 0 && !issue_pv(ntiles - 1)) give_up(6);
         }
         __syncwarp();
-      }
-      if (!pass_end()) break;
+      });
     }
   }
 
@@ -871,7 +1010,7 @@ __global__ void __launch_bounds__(TcCfg<D>::THREADS, 2) stage1_tc_kernel(const _
   int vn, kvh;
   task_of_block(tp.p, blockIdx.x, vn, kvh);
   FT_TL_BEGIN();
-  tc_body<T, D>(tp, smem, vn, kvh);
+  tc_body<T, D, false>(tp, smem, vn, kvh);
   FT_TL_END(1);
 }
 
@@ -895,7 +1034,7 @@ __global__ void __launch_bounds__(TcCfg<D>::THREADS, 2) stage1_fused_kernel(cons
   FT_TL_BEGIN();
   if (b < p.lead_wide || b >= p.lead_wide + few_ctas) {
     const int task = b < p.lead_wide ? b : b - few_ctas;
-    tc_body<T, D>(tp, smem, p.node_offset + task / H, task % H);
+    tc_body<T, D, false>(tp, smem, p.node_offset + task / H, task % H);
     FT_TL_END(1);
   } else {
     // This CTA will not allocate tensor memory.  Saying so at once matters: the SM admits no second CTA of a
@@ -915,6 +1054,23 @@ __global__ void __launch_bounds__(TcCfg<D>::THREADS, 2) stage1_fused_kernel(cons
       narrow_dispatch<T, D>(p, smem, p.node_offset + task / H, task % H);
     }
     FT_TL_END(2);
+  }
+}
+
+// Every task of a step from one grid whose size does not depend on the plan.
+template <typename T, int D>
+__global__ void __launch_bounds__(TcCfg<D>::THREADS, 2) stage1_persist_kernel(const __grid_constant__ TcParams tp) {
+  allow_dependent_launch();
+  extern __shared__ __align__(1024) uint8_t smem[];
+  tc_body<T, D, true>(tp, smem, 0, 0);
+  // the last CTA to get here re-arms the claim counter for the next launch
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(tp.sched + 1, 1u) == gridDim.x - 1) {
+      tp.sched[0] = 0u;
+      tp.sched[1] = 0u;
+      __threadfence();
+    }
   }
 }
 

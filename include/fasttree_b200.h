@@ -38,7 +38,7 @@ enum ft_path {
   FT_PATH_TCGEN05 = 3, /* tcgen05/TMEM kernel for 128-row tasks, 16-bit types, head_dim 64/128/256 */
   FT_PATH_MMA_WIDE = 4, /* the wide mma.sync kernel for every task (ablation / cross-check) */
   FT_PATH_STREAM = 5,   /* like AUTO, but few-row phases run the persistent kernel that pipelines across tasks */
-  FT_PATH_PERSIST = 6   /* one persistent tcgen05 kernel (a CTA per SM) for every task: 16-bit types, head_dim 128 */
+  FT_PATH_PERSIST = 6   /* one plan-independent grid (two CTAs per SM) that loops over all tasks: 16-bit types, head_dim 128 */
 };
 
 /* Status codes. */
@@ -249,7 +249,7 @@ int ft_selftest_bounded_wait(int limit, int* result_host, void* stream);
 
 /* Which bounded wait of the persistent stage-1 kernel gave up first since the last call (after
  * FT_DEV_WAIT_TIMEOUT): out8 = {wait id (0: none), block, warp, task sequence number, tile counter, 0, 0, 0};
- * the ids are listed next to the kernel (csrc/ft_stage1_persist.cuh).  Synchronises the device and clears the
+ * the ids are listed next to the kernel (csrc/ft_stage1_tc.cuh).  Synchronises the device and clears the
  * record.  A diagnostic aid; no counterpart in the reference. */
 int ft_read_wait_diagnostics(int32_t* out8);
 

@@ -1,0 +1,45 @@
+"""The plan-independent kernel: few-row tasks on its memory-bound body (at most eight rows), on the tensor cores (more
+rows, or token ranges that narrow a row), and plans with one phase empty, against the CPU oracle's partials."""
+import pytest
+import torch
+
+import gpu_utils
+from test_decode_gpu import ATOL16, adhoc
+from oracle import ref_attention
+
+from ft_b200 import engine, lib
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = [
+    ([1, 20], [300, 200], 8, 4),      # 40 rows on the root, leaves of 2 rows
+    ([1, 3], [700, 130], 8, 4),       # few-row tasks only, 6 and 2 rows
+    ([1, 6], [64, 129], 16, 1),       # leaves of 16 rows
+    ([1, 40], [200, 3], 8, 8),        # groups of short leaves: many-row tasks only
+    ([1, 700], [10, 150], 4, 4),      # thousands of one-row tasks: several per CTA
+]
+
+
+@pytest.mark.parametrize("narrow", [False, True], ids=["whole_chunks", "row_ranges"])
+@pytest.mark.parametrize("spec", SHAPES, ids=lambda s: "n%s_h%d-%d" % ("-".join(map(str, s[0])), s[2], s[3]))
+def test_persistent_kernel_partials(spec, narrow):
+    sizes, lens, hq, hkv = spec
+    c = adhoc(sizes, lens, hq, hkv, 128, torch.float16, seed=8, q_scale=0.5)
+    run = gpu_utils.EngineRun(c["nodes"], c["ptrs"], c["batch"], c["q"], c["k"], c["v"], hq, hkv, 128, c["tsq"])
+    args = (run.q, run.k, run.v, run.o, *run.aux, run.tiles[0], run.tiles[1], run.scale)
+    n = run.mid_o.shape[0]
+    tabs = [t.cpu().numpy() for t in run.aux[:6]]
+    tabs[3] = tabs[3][:n]
+    ranges = None
+    if narrow:     # every third row loses its first tokens, every third its last ones
+        begin = torch.where(torch.arange(n) % 3 == 1, 2, 0)
+        ranges = torch.stack([begin, torch.where(torch.arange(n) % 3 == 2, 60, 1 << 30)], dim=1).to(torch.int32).contiguous()
+    elif run.aux[3].numel() >= 3 * n:      # the plan's own ranges ride behind the request ids
+        ranges = run.aux[3][n:3 * n].reshape(n, 2).cpu().contiguous()
+    mid_o, mid_lse = ref_attention.stage1_partials(c["q"], c["k"], c["v"], *tabs, run.scale,
+                                                   q_ranges=None if ranges is None else ranges.numpy())
+    engine.stage1(*args, path="persist", row_ranges=None if ranges is None else ranges.cuda())
+    torch.cuda.synchronize()
+    assert lib.read_device_status() == 0
+    torch.testing.assert_close(run.mid_lse.cpu(), mid_lse, rtol=1e-4, atol=2e-5)
+    assert (run.mid_o.cpu() - mid_o).abs().max().item() <= ATOL16
