@@ -26,8 +26,9 @@ def test_persistent_kernel_partials(spec, narrow):
     sizes, lens, hq, hkv = spec
     c = adhoc(sizes, lens, hq, hkv, 128, torch.float16, seed=8, q_scale=0.5)
     run = gpu_utils.EngineRun(c["nodes"], c["ptrs"], c["batch"], c["q"], c["k"], c["v"], hq, hkv, 128, c["tsq"])
-    args = (run.q, run.k, run.v, run.o, *run.aux, run.tiles[0], run.tiles[1], run.scale)
     n = run.mid_o.shape[0]
+    args = (run.q, run.k, run.v, run.o, *run.aux[:3], run.aux[3][:n].contiguous(), *run.aux[4:], run.tiles[0], run.tiles[1],
+            run.scale)
     tabs = [t.cpu().numpy() for t in run.aux[:6]]
     tabs[3] = tabs[3][:n]
     ranges = None
