@@ -20,7 +20,7 @@ struct alignas(64) TcParams {
   Stage1Params p;
   int has_tma;
   int has_gather4;    // the two row maps are valid
-  int q_box_rows;     // 0: gather Q with cp.async (group size not a power of two <= 128, or no descriptor)
+  int q_box_rows;     // 0: gather Q with cp.async (group size above 128, or no descriptor)
   unsigned int* sched;  // persistent kernel: {tasks claimed beyond the first per CTA, CTAs finished}, zero between launches
 };
 

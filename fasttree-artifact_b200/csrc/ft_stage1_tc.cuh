@@ -33,9 +33,10 @@
 //              tile with 16-byte cp.async copies.  Row ids reach a small
 //              shared ring with cp.async two tiles ahead.
 //   warps 6-7  Q gather (by request id), concurrent with the first K loads:
-//              when G is a power of two, two TMA boxes for the whole tile if the
-//              request ids are consecutive, else one box per request (its G
-//              adjacent heads); 16-byte cp.async copies otherwise.
+//              two TMA boxes for the whole tile if the request ids are
+//              consecutive, else one box per request (its G adjacent heads);
+//              16-byte cp.async copies when G exceeds 128 or passes of a task
+//              do not start on a request.
 //   warp 6     then loads the V tiles the same way as warp 5 loads K, with the
 //              row ids in registers (two per lane, one tile ahead), so the two
 //              loaders share nothing and a gathered tile costs each of them
@@ -743,7 +744,9 @@ __device__ __forceinline__ void tc_body(const TcParams& tp, uint8_t* smem, int v
         // Requests with consecutive ids (the usual case: the leaves under a node are numbered in tree order) make
         // the whole Q tile one strided block of the Q tensor: two boxes of [128 / G requests][G heads][64].
         bool in_order = false;
-        if (tp.q_box_rows > 0) {
+        // (a box is a whole request: passes that do not start on one - G does not divide 128 - copy row by row)
+        const bool boxes = tp.q_box_rows > 0 && (C::ROWS % G == 0 || rows <= C::ROWS);
+        if (boxes) {
           const int req0 = req_of[0];
           bool mine = true;
           for (int i = lane; i < nslots; i += 32) mine &= req_of[i] == req0 + i;
@@ -751,16 +754,17 @@ __device__ __forceinline__ void tc_body(const TcParams& tp, uint8_t* smem, int v
         }
         if (in_order) {
           if (qt == 0) {
-            mbar_arrive_expect_tx(bar(C::Q_FULL), C::NB * 16384);  // full boxes: rows past the task's requests are dead rows
+            mbar_arrive_expect_tx(bar(C::Q_FULL), (uint32_t)(C::NB * 128 * (C::ROWS / G * G)));  // full boxes: rows past the task's requests are dead rows
 #pragma unroll
             for (int h = 0; h < C::NB; ++h)
               tma_load_3d(q_sm + h * 16384, &tp.q_map_tile, 64 * h, kvh * G, req_of[0], bar(C::Q_FULL));
           } else {
             mbar_arrive(bar(C::Q_FULL));
           }
-        } else if (tp.q_box_rows > 0) {
-          // The G rows of a request are adjacent heads of one Q row: one box of up to 8 rows x 64 elements per
-          // half.  G divides 128 here, so passes start on a request and a box never straddles an 8-row group.
+        } else if (boxes) {
+          // The G rows of a request are adjacent heads of one Q row: one box of q_box_rows rows x 64 elements per
+          // half, 128 bytes per row.  The swizzle goes by shared-memory address, so a box may start anywhere in an
+          // 8-row group and run on into the next.
           const int br = tp.q_box_rows;
           uint32_t bytes = 0;
           for (int i = qt; i < nslots; i += 64) {
@@ -776,7 +780,7 @@ __device__ __forceinline__ void tc_body(const TcParams& tp, uint8_t* smem, int v
             if (req >= 0 && req < p.batch) {
               for (int sub = 0; sub < G; sub += br) {
                 const int r = i * G + sub;
-                const uint32_t dst = q_sm + (uint32_t)((r >> 3) * 1024 + (r & 7) * 128);
+                const uint32_t dst = q_sm + (uint32_t)(r * 128);
 #pragma unroll
                 for (int h = 0; h < C::NB; ++h)
                   tma_load_3d(dst + h * 16384, &tp.q_map, 64 * h, kvh * G + sub, req, bar(C::Q_FULL));

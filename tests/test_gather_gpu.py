@@ -47,3 +47,43 @@ def test_scattered_rows_give_the_same_bits(d, layout, length):
     torch.cuda.synchronize()
     assert lib.read_device_status() == 0
     assert torch.equal(o.float().cpu(), want)
+
+
+@pytest.mark.parametrize("group", [3, 5, 6, 7, 8, 12, 24, 48, 100, 128])
+@pytest.mark.parametrize("d", [64, 128, 256])
+@pytest.mark.parametrize("rows_per_task", [128, 384])      # one pass; passes that start inside a request
+def test_query_tiles_of_any_group_size(group, d, rows_per_task):
+    """Q by whole-tile boxes (requests in order), by one box per request (ids shuffled) and row by row (a pass that
+    starts inside a request): the same partial rows."""
+    import fasttree
+    from ft_b200.planner import B200Model
+    from oracle import ref_attention
+    c = adhoc([1, max(2, 300 // group)], [130, 9], 2 * group, 2, d, torch.bfloat16, seed=2, q_scale=0.5)
+    params = gpu_utils.make_params(c["hq"], c["hkv"], c["tsq"], "b200")
+    params.b200_model = B200Model(rows_per_cta=rows_per_task)
+    tree = gpu_utils.product_tree(c["nodes"])
+    aux, _ = fasttree.fasttree_preparation(tree, c["ptrs"], c["batch"], c["hq"], c["hkv"], d, [1024, 128], [132, 528],
+                                           [132, 132], params, device="cuda")
+    n = aux[9].shape[0]
+    req = aux[3][:n].clone()
+    ranges = aux[3][n:3 * n].reshape(n, 2).contiguous() if aux[3].numel() > 2 * n else None
+    k, v = c["k"].cuda(), c["v"].cuda()
+    tabs = [t.cpu().numpy() for t in aux[:6]]
+    tabs[3] = tabs[3][:n]
+    want_o, want_lse = ref_attention.stage1_partials(c["q"], c["k"], c["v"], *tabs, d ** -0.5,
+                                                     q_ranges=None if ranges is None else ranges.cpu().numpy())
+    perm = torch.randperm(c["batch"], generator=torch.Generator().manual_seed(1))
+    shuffled = torch.empty_like(c["q"])
+    shuffled[perm] = c["q"]
+    got = []
+    for q, entries in ((c["q"], req), (shuffled, perm.cuda()[req.long()].to(torch.int32))):
+        q = q.cuda()
+        aux[9].fill_(float("nan"))
+        engine.stage1(q, k, v, torch.empty_like(q), *aux[:3], entries, *aux[4:], list(params.TSQs), list(params.TSKs),
+                      d ** -0.5, path="tcgen05", row_ranges=ranges)
+        torch.cuda.synchronize()
+        assert lib.read_device_status() == 0
+        got.append(aux[9].clone())
+        torch.testing.assert_close(aux[10].cpu(), want_lse, rtol=1e-4, atol=2e-5)
+        assert (aux[9].cpu() - want_o).abs().max().item() <= 2e-3 + 2 ** -8 * want_o.abs().max().item()
+    assert torch.equal(*got)
