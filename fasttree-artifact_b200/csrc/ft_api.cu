@@ -424,6 +424,17 @@ int launch_persist(ft::TcParams p, int hkv, cudaStream_t st) {
   return FT_OK;
 }
 
+// Few-row tasks: persistent workers with a task pipeline, or one CTA per task?  The workers hide a short task's start-up
+// but deal the tasks out statically; the hardware hands one-CTA tasks to whichever slot is free.  Workers are faster only
+// where very many tasks of about a tile each meet few slots (the plan's mean chunk, from the length of its row-id table,
+// tells the task length).  Measured per step, one CTA per task / workers, 296 slots, leaves under a 1000-token node, 32/8
+// heads of 128, ungrouped: 1024 leaves of 64 tokens 171 / 140 us, of 100 190 / 203, of 300 285 / 314; 512 leaves of 32
+// 84 / 98, of 64 89 / 89, of 130 125 / 155, of 900 324 / 374; a ragged tree of 117 tasks x 16 heads, 20 to 1948 tokens,
+// 140 / 247.
+bool few_rows_by_workers(const ft::Stage1Params& p, int64_t few, int64_t slots) {
+  return few >= 20 * slots && p.kv_entries_len <= 80LL * p.node_count;
+}
+
 template <typename T, int D>
 int launch_fused(ft::TcParams p, int hkv, cudaStream_t st) {
   constexpr int smem_a = ft::TcCfg<D>::SMEM_BYTES > ft::StreamCfg<D>::SMEM_BYTES ? ft::TcCfg<D>::SMEM_BYTES
@@ -434,17 +445,16 @@ int launch_fused(ft::TcParams p, int hkv, cudaStream_t st) {
   static OncePerDevice once;
   int dev = 0;
   FT_CUDA_OK(raise_smem_limit(once, ft::stage1_fused_kernel<T, D>, smem, &dev));
-  // Few-row tasks: a full set of persistent workers when each would get several tasks and the many-row CTAs
-  // do not fill the device more than once (the task pipeline then hides the per-task start-up; the workers
-  // take the slots the many-row CTAs leave and, as those finish, theirs too); one CTA per task otherwise (the
-  // hardware then slots the small CTAs in wherever a many-row CTA finishes).  Many-row CTAs go first.
+  // Few-row tasks by persistent workers only when the many-row CTAs do not fill the device more than once (the workers
+  // take the slots those leave and, as they finish, theirs too); one CTA per task otherwise (the hardware then slots
+  // the small CTAs in wherever a many-row CTA finishes).  Many-row CTAs go first.
   const int64_t wide = (int64_t)p.p.node_split * hkv;
   const int64_t few = (int64_t)(p.p.node_count - p.p.node_split) * hkv;
   const int64_t slots = 2LL * sm_count(dev);
 #ifdef FT_FORCE_WORKERS  // developer builds: persistent workers in every free slot, whatever the task count
   const int64_t workers = few < slots - wide ? few : (slots - wide > slots / 4 ? slots - wide : slots);
 #else
-  const int64_t workers = few >= 4 * slots && wide <= slots ? slots : 0;
+  const int64_t workers = few_rows_by_workers(p.p, few, slots) && wide <= slots ? slots : 0;
 #endif
   const int64_t few_ctas = workers > 0 ? workers : few;
   const int64_t lead = wide;
@@ -465,10 +475,9 @@ int launch_tensor(const ft::Stage1Params& p, const ft_decode_args* a, int hkv, c
     return launch_tc<T, D>(tc_params(p, a), hkv, st);
   if constexpr (D != 256) {
     if (max_rows <= 16) {
-      // few-row tasks only: persistent workers when there are several tasks per CTA slot, else one CTA per task
       int dev = 0;
       FT_CUDA_OK(cudaGetDevice(&dev));
-      const bool many = (int64_t)p.node_count * hkv >= 8LL * sm_count(dev);
+      const bool many = few_rows_by_workers(p, (int64_t)p.node_count * hkv, 2LL * sm_count(dev));
       if (path == FT_PATH_STREAM || (path == FT_PATH_AUTO && many)) return launch_stream<T, D>(tc_params(p, a), hkv, st);
     }
     if (path != FT_PATH_MMA_WIDE && max_rows <= 16) return launch_narrow<T, D>(p, hkv, st);
