@@ -134,12 +134,12 @@ __device__ __forceinline__ uint64_t tc_desc(uint32_t addr, uint32_t lbo_bytes, u
          (2ull << 61) /* SWIZZLE_128B */;
 }
 
-// kind::f16 instruction descriptor: fp32 accumulate, A K-major, dense
+// kind::f16 instruction descriptor: fp32 accumulate, A K-major, dense; negate_a: D = -A . B
 template <typename T>
-__device__ __forceinline__ uint32_t tc_idesc(int m, int n, bool b_mn_major) {
+__device__ __forceinline__ uint32_t tc_idesc(int m, int n, bool b_mn_major, bool negate_a = false) {
   const uint32_t fmt = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
-  return (1u << 4) | (fmt << 7) | (fmt << 10) | ((b_mn_major ? 1u : 0u) << 16) | ((uint32_t)(n >> 3) << 17) |
-         ((uint32_t)(m >> 4) << 24);
+  return (1u << 4) | (fmt << 7) | (fmt << 10) | ((negate_a ? 1u : 0u) << 13) | ((b_mn_major ? 1u : 0u) << 16) |
+         ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
 __device__ __forceinline__ void tc_mma(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t acc) {
@@ -434,7 +434,12 @@ __device__ __forceinline__ void tc_body(const TcParams& tp, uint8_t* smem, int v
   }
   if (tid == 0) FT_TL_MARK(0);
   const int G = p.group;
-  const float scale2 = p.sm_scale * 1.4426950408889634f;
+  // The scale is applied after the mask and the maximum (one packed FMA per pair of scores), which is only right for a
+  // positive one: a masked -inf would come out as +inf or NaN, and the largest product would not be the largest score.  A
+  // negative scale's sign therefore goes into the products (the MMA negates Q), and zero becomes the smallest normal
+  // number, under which every finite score is as good as 0.  A multiplication ahead of the mask for such scales, behind a
+  // branch in the tile loop, cost every other call: 512 leaves in four levels at head_dim 64 36.6 -> 37.1 us.
+  const float scale2 = p.sm_scale == 0.f ? 1.17549435e-38f : fabsf(p.sm_scale) * 1.4426950408889634f;
   int rows = 0, ntiles = 0, id_lim = 0;
   const int32_t* ids_of_chunk = nullptr;
   auto enter_task = [&]() {
@@ -925,7 +930,7 @@ __device__ __forceinline__ void tc_body(const TcParams& tp, uint8_t* smem, int v
   auto mma_pass = [&](const int row0) {
         // ================================================================ MMA issue
         if (lane == 0) {
-          const uint32_t idesc_s = tc_idesc<T>(128, C::TILE, false);
+          const uint32_t idesc_s = tc_idesc<T>(128, C::TILE, false, p.sm_scale < 0.f);
           const uint32_t idesc_o = tc_idesc<T>(128, 64, true);  // P.V in 64-column pieces: the shape of S
           const uint64_t q_desc = tc_desc(q_sm, 16, 1024);
           auto issue_pv = [&](int t) {  // O += P_t V_t : per 64 columns of O, 4 k-steps of 16 tokens, A = P_t in tensor memory
