@@ -18,6 +18,7 @@
 #pragma once
 
 #include "ft_common.cuh"
+#include "ft_stage1_row.cuh"
 
 namespace ft {
 
@@ -34,7 +35,7 @@ struct F32Cfg {
 };
 
 template <int D>
-__global__ void __launch_bounds__(256) stage1_f32_kernel(Stage1Params p) {
+__global__ void __launch_bounds__(256, D == 64 ? 4 : 3) stage1_f32_kernel(const __grid_constant__ Stage1Params p) {
   using C = F32Cfg<D>;
   allow_dependent_launch();
   wait_for_prior_grid();  // nothing of the preceding kernel's is read or overwritten before this
@@ -210,6 +211,12 @@ __global__ void __launch_bounds__(256) stage1_f32_kernel(Stage1Params p) {
 #pragma unroll
     for (int j = 0; j < D / 32; ++j) op[lane + 32 * j] = acc[i][j] * inv;
     if (lane == 0) p.mid_lse[part * p.ml_s0 + head] = l_run[i] > 0.f ? logf(l_run[i]) + m_run[i] : -INFINITY;
+    if (r_lo[i] > 0 || r_hi[i] < kv_len) {
+      float finite = 0.f;  // 0 x every element: 0, or NaN
+#pragma unroll
+      for (int j = 0; j < D / 32; ++j) finite = fmaf(acc[i][j], 0.f, finite);
+      if (__any_sync(0xffffffffu, !(finite == 0.f))) redo_narrowed_row<float>(p, kvh, q_off, kv_off, kv_len, prow);
+    }
   }
 }
 

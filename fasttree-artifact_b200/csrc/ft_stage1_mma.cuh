@@ -20,6 +20,7 @@
 #pragma once
 
 #include "ft_common.cuh"
+#include "ft_stage1_row.cuh"
 
 namespace ft {
 
@@ -340,7 +341,7 @@ __device__ __forceinline__ void mma_tile(const uint32_t k_sm, const uint32_t v_s
 }
 
 template <typename T, int D>
-__global__ void __launch_bounds__(128, 2) stage1_mma_kernel(Stage1Params p) {
+__global__ void __launch_bounds__(128, 2) stage1_mma_kernel(const __grid_constant__ Stage1Params p) {
   allow_dependent_launch();
   wait_for_prior_grid();  // nothing of the preceding kernel's is read or overwritten before this
   using C = MmaCfg<D>;
@@ -477,39 +478,51 @@ __global__ void __launch_bounds__(128, 2) stage1_mma_kernel(Stage1Params p) {
       const int r = tid >> 3, seg = tid & 7;
       for (int rb = 0; rb < n_rb; ++rb) {
         const int prow = row0 + rb * 16 + r;
-        if (prow >= rows) continue;
         const int slot = prow / G, gg = prow - slot * G;
         const int64_t part = (int64_t)q_off + slot;
-        if (part < 0 || part >= p.num_partial_rows) continue;  // flagged above
-        float M = -INFINITY;
-        for (int w = 0; w < ways; ++w) M = fmaxf(M, epi_m[(rb + (w << rb_log)) * 16 + r]);
-        float L = 0.f;
-        float4 out[D / 32];
+        bool spoiled = false;  // a row that attends to part of the chunk and is not finite (redo_narrowed_row)
+        if (prow < rows && part >= 0 && part < p.num_partial_rows) {  // bad rows were flagged above
+          float M = -INFINITY;
+          for (int w = 0; w < ways; ++w) M = fmaxf(M, epi_m[(rb + (w << rb_log)) * 16 + r]);
+          float L = 0.f;
+          float4 out[D / 32];
 #pragma unroll
-        for (int i = 0; i < D / 32; ++i) out[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (int w = 0; w < ways; ++w) {
-          const int ww = rb + (w << rb_log);
-          const float mw = epi_m[ww * 16 + r];
-          const float f = mw == -INFINITY ? 0.f : fast_exp2(mw - M);
-          L = fmaf(epi_l[ww * 16 + r], f, L);
-          const float4* src = reinterpret_cast<const float4*>(epi_o + (ww * 16 + r) * C::OSTRIDE);
+          for (int i = 0; i < D / 32; ++i) out[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+          for (int w = 0; w < ways; ++w) {
+            const int ww = rb + (w << rb_log);
+            const float mw = epi_m[ww * 16 + r];
+            const float f = mw == -INFINITY ? 0.f : fast_exp2(mw - M);
+            L = fmaf(epi_l[ww * 16 + r], f, L);
+            const float4* src = reinterpret_cast<const float4*>(epi_o + (ww * 16 + r) * C::OSTRIDE);
 #pragma unroll
-          for (int i = 0; i < D / 32; ++i) {
-            const float4 x = src[seg + 8 * i];
-            out[i].x = fmaf(f, x.x, out[i].x);
-            out[i].y = fmaf(f, x.y, out[i].y);
-            out[i].z = fmaf(f, x.z, out[i].z);
-            out[i].w = fmaf(f, x.w, out[i].w);
+            for (int i = 0; i < D / 32; ++i) {
+              const float4 x = src[seg + 8 * i];
+              out[i].x = fmaf(f, x.x, out[i].x);
+              out[i].y = fmaf(f, x.y, out[i].y);
+              out[i].z = fmaf(f, x.z, out[i].z);
+              out[i].w = fmaf(f, x.w, out[i].w);
+            }
+          }
+          const float inv = L > 0.f ? 1.f / L : 0.f;
+          const int head = kvh * G + gg;
+          float4* dst = reinterpret_cast<float4*>(p.mid_o + part * p.mo_s0 + (int64_t)head * p.mo_s1);
+#pragma unroll
+          for (int i = 0; i < D / 32; ++i)
+            dst[seg + 8 * i] = make_float4(out[i].x * inv, out[i].y * inv, out[i].z * inv, out[i].w * inv);
+          if (seg == 0)
+            p.mid_lse[part * p.ml_s0 + head] = L > 0.f ? (M + log2f(L)) * 0.6931471805599453f : -INFINITY;
+          if (p.q_ranges != nullptr && (p.q_ranges[2 * part] > 0 || p.q_ranges[2 * part + 1] < kv_len)) {
+            float finite = 0.f;
+#pragma unroll
+            for (int i = 0; i < D / 32; ++i) finite += (out[i].x * 0.f + out[i].y * 0.f) + (out[i].z * 0.f + out[i].w * 0.f);
+            spoiled = !(finite == 0.f);
           }
         }
-        const float inv = L > 0.f ? 1.f / L : 0.f;
-        const int head = kvh * G + gg;
-        float4* dst = reinterpret_cast<float4*>(p.mid_o + part * p.mo_s0 + (int64_t)head * p.mo_s1);
-#pragma unroll
-        for (int i = 0; i < D / 32; ++i)
-          dst[seg + 8 * i] = make_float4(out[i].x * inv, out[i].y * inv, out[i].z * inv, out[i].w * inv);
-        if (seg == 0)
-          p.mid_lse[part * p.ml_s0 + head] = L > 0.f ? (M + log2f(L)) * 0.6931471805599453f : -INFINITY;
+        if (p.q_ranges != nullptr) {
+          const uint32_t todo = __ballot_sync(0xffffffffu, spoiled);  // eight lanes per row
+          for (int i = 0; i < 4; ++i)
+            if ((todo >> (8 * i)) & 0xffu) redo_narrowed_row<T>(p, kvh, q_off, kv_off, kv_len, row0 + rb * 16 + warp * 4 + i);
+        }
       }
     }
     __syncthreads();  // staging area and Q tile are reused by the next 64-row block

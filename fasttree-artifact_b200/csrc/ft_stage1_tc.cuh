@@ -71,6 +71,7 @@
 #include "ft_common.cuh"
 #include "ft_stage1_mma.cuh"
 #include "ft_stage1_narrow.cuh"
+#include "ft_stage1_row.cuh"
 #include "ft_stage1_stream.cuh"
 
 namespace ft {
@@ -677,6 +678,7 @@ __device__ __forceinline__ void tc_body(const TcParams& tp, uint8_t* smem, int v
           const bool store = live && part >= 0 && part < p.num_partial_rows;
           const int head = kvh * G + gg;
           const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
+          float2 finite[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};  // 0 x every element: 0, or NaN
           // stage the normalised row in shared memory (every operand buffer is idle by now)
           const uint32_t out_row = sm + (uint32_t)tid * C::OUT_STRIDE;
 #pragma unroll
@@ -689,10 +691,15 @@ __device__ __forceinline__ void tc_body(const TcParams& tp, uint8_t* smem, int v
               for (int c = 0; c < 32; ++c) o[c] = 0.f;
             }
 #pragma unroll
-            for (int c = 0; c < 8; ++c)
-              asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};\n" ::"r"(out_row + (cb * 8 + c) * 16),
-                           "f"(o[4 * c] * inv), "f"(o[4 * c + 1] * inv), "f"(o[4 * c + 2] * inv), "f"(o[4 * c + 3] * inv)
+            for (int c = 0; c < 8; ++c) {
+              const float2 a = __fmul2_rn(make_float2(o[4 * c], o[4 * c + 1]), make_float2(inv, inv));
+              const float2 b = __fmul2_rn(make_float2(o[4 * c + 2], o[4 * c + 3]), make_float2(inv, inv));
+              finite[0] = __ffma2_rn(a, make_float2(0.f, 0.f), finite[0]);
+              finite[1] = __ffma2_rn(b, make_float2(0.f, 0.f), finite[1]);
+              asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};\n" ::"r"(out_row + (cb * 8 + c) * 16), "f"(a.x), "f"(a.y),
+                           "f"(b.x), "f"(b.y)
                            : "memory");
+            }
           }
           if (tid == 0) FT_TL_MARK(8);
           if (store)
@@ -716,6 +723,10 @@ __device__ __forceinline__ void tc_body(const TcParams& tp, uint8_t* smem, int v
               if (dst != nullptr) reinterpret_cast<float4*>(dst)[lane % LPR + 32 * h] = x;
             }
           }
+          const bool spoiled = !(finite[0].x + finite[0].y + finite[1].x + finite[1].y == 0.f) && p.q_ranges != nullptr && store &&
+                               (r_lo > 0 || r_hi < kv_len);  // a row that attends to part of its chunk and is not finite
+          for (uint32_t todo = __ballot_sync(0xffffffffu, spoiled); todo != 0; todo &= todo - 1)
+            redo_narrowed_row<T>(p, kvh, q_off, kv_off, kv_len, row0 + warp * 32 + __ffs(todo) - 1);
           if (tid == 0) FT_TL_MARK(9);
           if (LOOP) proxy_fence();  // the staged rows come before the next task's TMA copies
         }
