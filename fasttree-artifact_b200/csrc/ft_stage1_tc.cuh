@@ -734,6 +734,10 @@ __device__ __forceinline__ void tc_body(const TcParams& tp, uint8_t* smem, int v
   };
   auto q_v_pass = [&](const int row0) {
         // ================================================================ Q gather (64 threads)
+        if (ntiles == 0) {  // no product will wait for Q: loads issued here could land in the next pass's or task's buffers
+          mbar_arrive(bar(C::Q_FULL));  // (the barrier's phase is one per pass)
+          return;
+        }
         // request ids of this pass's slots -> the (still unused) V buffers, then the rows themselves
         const int qt = tid - 192, ld_c = qt % C::CPR, ld_r = qt / C::CPR;
         const int row_end = min(rows, row0 + C::ROWS);

@@ -44,3 +44,28 @@ def test_persistent_kernel_partials(spec, narrow):
     assert lib.read_device_status() == 0
     torch.testing.assert_close(run.mid_lse.cpu(), mid_lse, rtol=1e-4, atol=2e-5)
     assert (run.mid_o.cpu() - mid_o).abs().max().item() <= ATOL16
+
+
+@pytest.mark.parametrize("d,path", [(128, "persist"), (128, "tcgen05"), (64, "tcgen05"), (256, "tcgen05")])
+def test_empty_chunks_between_others(d, path):
+    """Every third task has query rows but no tokens: its partial rows are zero with an LSE of -inf, and the tasks that
+    the same CTA runs before and after it are untouched."""
+    c = adhoc([1, 150], [300, 130], 64, 4, d, torch.float16, seed=13, q_scale=0.5)      # 16 rows and more per task
+    run = gpu_utils.EngineRun(c["nodes"], c["ptrs"], c["batch"], c["q"], c["k"], c["v"], 64, 4, d, c["tsq"])
+    n = run.mid_o.shape[0]
+    lens = run.aux[2].clone()
+    lens[1::3] = 0
+    tabs = [t.cpu().numpy() for t in run.aux[:6]]
+    tabs[2], tabs[3] = lens.cpu().numpy(), tabs[3][:n]
+    mid_o, mid_lse = ref_attention.stage1_partials(c["q"], c["k"], c["v"], *tabs, run.scale)
+    mid_o, mid_lse = torch.nan_to_num(mid_o, nan=0.0), torch.nan_to_num(mid_lse, nan=float("-inf"), neginf=float("-inf"))
+    assert int((tabs[2] == 0).sum()) * 4 > 148 and bool(mid_lse.isinf().any())
+    for _ in range(3):
+        run.mid_o.fill_(float("nan"))
+        run.mid_lse.fill_(float("nan"))
+        engine.stage1(run.q, run.k, run.v, run.o, *run.aux[:2], lens, run.aux[3][:n].contiguous(), *run.aux[4:], run.tiles[0],
+                      run.tiles[1], run.scale, path=path, row_ranges=None)
+        torch.cuda.synchronize()
+        assert lib.read_device_status() == 0
+        torch.testing.assert_close(run.mid_lse.cpu(), mid_lse, rtol=1e-4, atol=2e-5)
+        assert (run.mid_o.cpu() - mid_o).abs().max().item() <= ATOL16
