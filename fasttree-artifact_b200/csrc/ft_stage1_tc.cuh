@@ -728,7 +728,7 @@ __device__ __forceinline__ void tc_body(const TcParams& tp, uint8_t* smem, int v
           for (uint32_t todo = __ballot_sync(0xffffffffu, spoiled); todo != 0; todo &= todo - 1)
             redo_narrowed_row<T>(p, kvh, q_off, kv_off, kv_len, row0 + warp * 32 + __ffs(todo) - 1);
           if (tid == 0) FT_TL_MARK(9);
-          if (LOOP) proxy_fence();  // the staged rows come before the next task's TMA copies
+          if (LOOP || row0 + C::ROWS < rows) proxy_fence();  // the staged rows come before the next pass's or task's TMA copies
         }
       }
   };
@@ -821,6 +821,7 @@ __device__ __forceinline__ void tc_body(const TcParams& tp, uint8_t* smem, int v
           mbar_arrive_on_cp_async(bar(C::Q_FULL));  // one arrival per thread once its copies have landed
           cp_async_wait<0>();
         }
+        proxy_fence();                                      // the request ids come before the TMA copies of V that replace them
         asm volatile("bar.sync 1, 64;\n" ::: "memory");  // both warps are done with the staged request ids: V may land there
         if (warp == 6) {
           // ============================================================== V loader (this warp, once Q is on its way)

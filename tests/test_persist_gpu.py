@@ -69,3 +69,28 @@ def test_empty_chunks_between_others(d, path):
         assert lib.read_device_status() == 0
         torch.testing.assert_close(run.mid_lse.cpu(), mid_lse, rtol=1e-4, atol=2e-5)
         assert (run.mid_o.cpu() - mid_o).abs().max().item() <= ATOL16
+
+
+@pytest.mark.parametrize("d,path", [(128, "persist"), (128, "tcgen05"), (64, "tcgen05"), (256, "tcgen05")])
+@pytest.mark.parametrize("rows", [132, 256, 260, 384])      # packed rows of the root's tasks: two and three passes
+def test_tasks_of_several_passes(rows, d, path):
+    """Tasks of more than 128 query rows: the passes of a task reuse the buffers their predecessor staged its output in,
+    and the looping kernel claims its next task on the last pass."""
+    import fasttree
+    from ft_b200.planner import B200Model
+    c = adhoc([1, rows // 4], [1500, 40], 32, 8, d, torch.float16, seed=14, q_scale=0.5)
+    params = gpu_utils.make_params(32, 8, c["tsq"], "b200")
+    params.b200_model = B200Model(rows_per_cta=384, min_chunk=64, group_member_tokens=0)
+    aux, _ = fasttree.fasttree_preparation(gpu_utils.product_tree(c["nodes"]), c["ptrs"], c["batch"], 32, 8, d, [1024, 128],
+                                           [132, 528], [132, 132], params, device="cuda")
+    tabs = [t.cpu().numpy() for t in aux[:6]]
+    assert int(tabs[5].max()) * 4 == rows
+    mid_o, mid_lse = ref_attention.stage1_partials(c["q"], c["k"], c["v"], *tabs, d ** -0.5)
+    q, k, v = c["q"].cuda(), c["k"].cuda(), c["v"].cuda()
+    for _ in range(3):
+        aux[9].fill_(float("nan"))
+        engine.stage1(q, k, v, torch.empty_like(q), *aux, list(params.TSQs), list(params.TSKs), d ** -0.5, path=path)
+        torch.cuda.synchronize()
+        assert lib.read_device_status() == 0
+        torch.testing.assert_close(aux[10].cpu(), mid_lse, rtol=1e-4, atol=2e-5)
+        assert (aux[9].cpu() - mid_o).abs().max().item() <= ATOL16
