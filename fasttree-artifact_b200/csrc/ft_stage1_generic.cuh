@@ -1,8 +1,10 @@
 // Stage 1, scalar fp32 kernel: any storage type, any head_dim <= 256.
 //
 // One CTA per (vnode, kv head), as in the reference launch grid
-// (kernel_bench/fasttree.py:448-451).  Each warp owns one packed query row
-// (request slot x group member) at a time (attend_row).  It is the correctness
+// (kernel_bench/fasttree.py:448-451), and block of four query rows, one per warp
+// (attend_row; packed row = request slot x group member): the rows of a task
+// share nothing here, so no step waits for the task that the plan gave the most
+// of them.  It is the correctness
 // path for unusual head sizes, types and layouts; the 16-bit cases of head_dim
 // 64, 128 and 256 go to the tensor-core kernels, fp32 at 64 and 128 to the tiled
 // fp32 kernel.
@@ -29,7 +31,7 @@ __global__ void __launch_bounds__(128) stage1_generic_kernel(Stage1Params p) {
   const T* __restrict__ kbase = reinterpret_cast<const T*>(p.k) + (int64_t)kvh * p.k_s1;
   const T* __restrict__ vbase = reinterpret_cast<const T*>(p.v) + (int64_t)kvh * p.v_s1;
 
-  for (int row = warp; row < rows; row += 4) {
+  for (int row = warp + 4 * (int)blockIdx.z; row < rows; row += 4 * (int)gridDim.z) {
     const int slot = row / G, g = row - slot * G;
     const int64_t prow = (int64_t)q_off + slot;
     if (prow < 0 || prow >= p.num_partial_rows) {

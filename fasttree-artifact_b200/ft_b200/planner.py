@@ -717,6 +717,8 @@ def b200_model_for(params, head_dim, model=None):
     if explicit is None and (head_dim == 128 or (head_dim in (64, 256) and getattr(params, "kv_elem_bytes", 2) == 2)):
         # the tcgen05 stage-1 kernel holds 128 query rows per CTA; at head_dim 64 its softmax, which sets the tile's
         # time, covers half the flops, and at 256 one CTA fills an SM
+        # (unstated K/V may be fp32: the fp32 and scalar kernels cut a task's rows into blocks of their own, so they do not
+        # follow this tile)
         m = replace(m, rows_per_cta=128, ridge_flop_per_byte=(2 if head_dim == 64 else 4) * m.ridge_flop_per_byte,
                     ctas_per_sm=1 if head_dim == 256 else m.ctas_per_sm)
         # Short nodes are grouped at head_dim 64 and 256 when the storage type was stated.  Unstated, K/V may be fp32,
