@@ -198,6 +198,7 @@ __global__ void __launch_bounds__(256, D == 64 ? 4 : 3) stage1_f32_kernel(const 
   }
 
   // ---- normalise and write the partial rows
+  uint32_t todo = 0;
 #pragma unroll
   for (int i = 0; i < RPW; ++i) {
     const int r = warp + NW * i;
@@ -215,9 +216,11 @@ __global__ void __launch_bounds__(256, D == 64 ? 4 : 3) stage1_f32_kernel(const 
       float finite = 0.f;  // 0 x every element: 0, or NaN
 #pragma unroll
       for (int j = 0; j < D / 32; ++j) finite = fmaf(acc[i][j], 0.f, finite);
-      if (__any_sync(0xffffffffu, !(finite == 0.f))) redo_narrowed_row<float>(p, kvh, q_off, kv_off, kv_len, prow);
+      if (__any_sync(0xffffffffu, !(finite == 0.f))) todo |= 1u << i;
     }
   }
+#pragma unroll 1
+  for (; todo != 0; todo &= todo - 1) redo_narrowed_row<float>(p, kvh, q_off, kv_off, kv_len, row0 + warp + NW * (__ffs(todo) - 1));
 }
 
 }  // namespace ft
