@@ -96,8 +96,16 @@ def row_ranges_of(vnode_to_q_entries):
     return split_q_entries(vnode_to_q_entries)[1]
 
 
+_ARG_NAMES = ("q", "k_buffer", "v_buffer", "o", "vnode_to_kv_entries", "vnode_to_kv_offs", "vnode_to_kv_lens",
+              "vnode_to_q_entries", "vnode_to_q_offs", "vnode_to_q_lens", "req_to_vnode_entries", "req_to_vnode_offs",
+              "req_to_vnode_lens", "mid_o", "mid_lse", "phase_node_nums", "phase_node_offsets", "phase_q_tile_sizes",
+              "phase_kv_tile_sizes", "sm_scale")
+
+
 def _resolve(args, path, row_ranges):
     """``(path code, row-range tensor or None, partial rows or -1)`` of a call's arguments."""
+    if len(args) != len(_ARG_NAMES):
+        raise TypeError(f"expected {len(_ARG_NAMES)} positional arguments, got {len(args)}")
     code = _lib.PATHS.get(path)
     if code is None:
         raise ValueError(f"path must be one of {sorted(_lib.PATHS)}")
@@ -111,9 +119,10 @@ def _resolve(args, path, row_ranges):
 
 
 def build_args(*args, path="auto", o_lse=None, stream=None, row_ranges="detect", phase_info=None, kv_entries_aux=None,
-               logit_cap=-1):
+               logit_cap=-1, **named):
     """A filled :class:`DecodeArgs` struct; raises ``ValueError`` where a tensor does not fit.  Positional arguments
-    are those of the reference's ``fasttree_decode`` up to and including ``sm_scale`` (and ``logit_cap``).
+    are those of the reference's ``fasttree_decode`` up to and including ``sm_scale`` (and ``logit_cap``); they may also
+    be given by name.
     ``kv_entries_aux``: an int32 CUDA tensor, the second row-id table that vnodes with bit 30 of their
     ``vnode_to_kv_offs`` value set read (grouped private tails of the serving path).  ``phase_info``: an
     int32 CUDA tensor ``[n0, n1, o0, o1]`` that stage 1 reads on the device in
@@ -122,8 +131,13 @@ def build_args(*args, path="auto", o_lse=None, stream=None, row_ranges="detect",
     ``"detect"`` looks for ranges packed into ``vnode_to_q_entries`` (see
     :func:`pack_row_ranges`), ``None`` says the plan has none (no look-up, no
     device read), a tensor gives the table explicitly."""
-    if len(args) == 21:
-        args, logit_cap = args[:20], args[20]
+    if len(args) == len(_ARG_NAMES) + 1:
+        args, logit_cap = args[:-1], args[-1]
+    if named:
+        missing = [n for n in _ARG_NAMES[len(args):] if n not in named]
+        if missing or len(named) != len(_ARG_NAMES) - len(args):
+            raise TypeError(f"build_args: missing {missing}, unknown or repeated {sorted(set(named) - set(_ARG_NAMES[len(args):]))}")
+        args = args + tuple(named[n] for n in _ARG_NAMES[len(args):])
     code, ranges, rows = _resolve(args, path, row_ranges)
     raw = _lib.call_module().args(args, logit_cap, code, o_lse, ranges, rows, phase_info, kv_entries_aux,
                                   -1 if stream is None else stream)

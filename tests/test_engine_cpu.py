@@ -1,5 +1,6 @@
 """Host-side pieces of the engine binding that need no GPU."""
 import numpy as np
+import pytest
 import torch
 
 from ft_b200 import engine
@@ -36,3 +37,20 @@ def test_range_lookup_works_on_inference_tensors():
         t = torch.arange(23, dtype=torch.int32)
         rows, got = engine.split_q_entries(t)
     assert rows == 23 and got is None
+
+
+def test_build_args_takes_its_tensors_by_position_and_by_name():
+    """Both forms reach the same check (tensors here live on the CPU, which it refuses); wrong counts and names do not."""
+    q = torch.zeros(2, 4, 64)
+    table = torch.zeros(4, dtype=torch.int32)
+    values = [q, q, q, q] + [table] * 9 + [q, q[..., 0], [1, 1], [0, 1], [2, 2], [32, 32], 0.1]
+    names = engine._ARG_NAMES
+    assert len(names) == len(values)
+    for split in (20, 15, 4, 0):
+        with pytest.raises(ValueError, match="q is on cpu"):
+            engine.build_args(*values[:split], **dict(zip(names[split:], values[split:])), row_ranges=None)
+    with pytest.raises(ValueError, match="q is on cpu"):
+        engine.build_args(*values, -1, row_ranges=None)
+    for args, named in ((values[:19], {}), (values[:19], {"scale": 0.1}), (values, {"q": q}), (values[:7], {}), (values * 2, {})):
+        with pytest.raises(TypeError):
+            engine.build_args(*args, **named)
