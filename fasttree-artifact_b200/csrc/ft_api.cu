@@ -426,13 +426,17 @@ int launch_persist(ft::TcParams p, int hkv, cudaStream_t st) {
 
 // Few-row tasks: persistent workers with a task pipeline, or one CTA per task?  The workers hide a short task's start-up
 // but deal the tasks out statically; the hardware hands one-CTA tasks to whichever slot is free.  Workers are faster only
-// where very many tasks of about a tile each meet few slots (the plan's mean chunk, from the length of its row-id table,
-// tells the task length).  Measured per step, one CTA per task / workers, 296 slots, leaves under a 1000-token node, 32/8
-// heads of 128, ungrouped: 1024 leaves of 64 tokens 171 / 140 us, of 100 190 / 203, of 300 285 / 314; 512 leaves of 32
-// 84 / 98, of 64 89 / 89, of 130 125 / 155, of 900 324 / 374; a ragged tree of 117 tasks x 16 heads, 20 to 1948 tokens,
-// 140 / 247.
-bool few_rows_by_workers(const ft::Stage1Params& p, int64_t few, int64_t slots) {
-  return few >= 20 * slots && p.kv_entries_len <= 80LL * p.node_count;
+// where very many tasks of about a tile each meet few slots.  The host does not see the tasks' lengths: the length of the
+// row-id table, of which every few-row chunk has a part of its own, bounds their sum from above, so workers are taken
+// where even that bound leaves a mean of at most 80 tokens per few-row node.  The table also holds the many-row phase's
+// row ids, and on the serving path it is the whole req_to_token pool: a plan with short few-row tasks beside a long prefix runs one CTA per task although workers would
+// be quicker (1024 leaves of 64 tokens under a 32 000-token node).  The splitter groups such leaves; what is left for
+// the workers are plans of its reference mode, ungrouped plans and hand-made ones.  Measured per step, one CTA per task /
+// workers, 296 slots, leaves under a 1000-token node, 32/8 heads of 128, ungrouped: 1024 leaves of 64 tokens 171 / 140 us,
+// of 100 190 / 203, of 300 285 / 314; 512 leaves of 32 84 / 98, of 64 89 / 89, of 130 125 / 155, of 900 324 / 374; a ragged
+// tree of 117 tasks x 16 heads, 20 to 1948 tokens, 140 / 247.
+bool few_rows_by_workers(int64_t few_nodes, int64_t kv_entries_len, int hkv, int64_t slots) {
+  return few_nodes * hkv >= 20 * slots && kv_entries_len <= 80 * few_nodes;
 }
 
 template <typename T, int D>
@@ -454,7 +458,7 @@ int launch_fused(ft::TcParams p, int hkv, cudaStream_t st) {
 #ifdef FT_FORCE_WORKERS  // developer builds: persistent workers in every free slot, whatever the task count
   const int64_t workers = few < slots - wide ? few : (slots - wide > slots / 4 ? slots - wide : slots);
 #else
-  const int64_t workers = few_rows_by_workers(p.p, few, slots) && wide <= slots ? slots : 0;
+  const int64_t workers = few_rows_by_workers(p.p.node_count - p.p.node_split, p.p.kv_entries_len, hkv, slots) && wide <= slots ? slots : 0;
 #endif
   const int64_t few_ctas = workers > 0 ? workers : few;
   const int64_t lead = wide;
@@ -477,7 +481,7 @@ int launch_tensor(const ft::Stage1Params& p, const ft_decode_args* a, int hkv, c
     if (max_rows <= 16) {
       int dev = 0;
       FT_CUDA_OK(cudaGetDevice(&dev));
-      const bool many = few_rows_by_workers(p, (int64_t)p.node_count * hkv, 2LL * sm_count(dev));
+      const bool many = few_rows_by_workers(p.node_count, p.kv_entries_len, hkv, 2LL * sm_count(dev));
       if (path == FT_PATH_STREAM || (path == FT_PATH_AUTO && many)) return launch_stream<T, D>(tc_params(p, a), hkv, st);
     }
     if (path != FT_PATH_MMA_WIDE && max_rows <= 16) return launch_narrow<T, D>(p, hkv, st);
