@@ -578,7 +578,7 @@ class Problem:
     def release(self):
         self.ks = self.vs = None
         self.aux = None
-        self.engine._ARG_CACHE.clear()
+        self.engine._RANGE_CACHE.clear()
         torch.cuda.empty_cache()
 
 

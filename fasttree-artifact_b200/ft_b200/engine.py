@@ -15,7 +15,7 @@ from . import lib as _lib
 
 # What is remembered about a plan: per vnode_to_q_entries table (by tensor object, weakly) whether it carries row ranges
 # (:func:`split_q_entries`).  id(tensor) -> (weak reference to it, (version, data_ptr, numel), rows or -1)
-_ARG_CACHE = {}
+_RANGE_CACHE = {}
 
 
 def _require_cuda(name, t):
@@ -75,18 +75,17 @@ def split_q_entries(vnode_to_q_entries):
     must not fall inside a CUDA graph capture."""
     t = vnode_to_q_entries
     n = t.numel()
+    if n < 5 or (n - 2) % 3 != 0:                 # too short for a trailer, or no multiple of three entries before it
+        return n, None
     state = (_version_of(t), t.data_ptr(), n)
     ident = id(t)
-    known = _ARG_CACHE.get(ident)
+    known = _RANGE_CACHE.get(ident)
     if known is not None and known[0]() is t and known[1] == state:
         hit = known[2]
     else:
-        hit = -1
-        if n >= 5 and (n - 2) % 3 == 0:
-            magic, rows = t.view(-1)[-2:].tolist()
-            if magic == ROW_RANGE_MAGIC and 3 * rows + 2 == n:
-                hit = rows
-        _ARG_CACHE[ident] = (weakref.ref(t, lambda _r, k=ident: _ARG_CACHE.pop(k, None)), state, hit)
+        magic, rows = t.view(-1)[-2:].tolist()
+        hit = rows if magic == ROW_RANGE_MAGIC and 3 * rows + 2 == n else -1
+        _RANGE_CACHE[ident] = (weakref.ref(t, lambda _r, k=ident: _RANGE_CACHE.pop(k, None)), state, hit)
     if hit < 0:
         return n, None
     return hit, t.view(-1)[hit:3 * hit].view(hit, 2)

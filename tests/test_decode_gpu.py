@@ -211,30 +211,42 @@ def test_short_nodes_run_as_groups_with_row_ranges(spec):
     assert torch.equal(o2.float().cpu(), grouped.decode(path="auto"))
 
 
-def test_argument_cache_keeps_no_query_tensors():
-    """A serving loop hands the engine new q / o tensor objects on every layer and step.  The memoised argument
-    structs are keyed on the persistent tensors only: 1000 calls with fresh q / o leave one entry and keep none
-    of the q storages alive."""
+def test_calls_keep_nothing_of_their_tensors():
+    """A serving loop hands the engine new q / o tensor objects on every layer and step, and new tables with every plan:
+    each call reads the tensors it is given, none outlives its caller's reference, and what is remembered about a
+    ``vnode_to_q_entries`` table (whether row ranges ride in it) goes with the table."""
     import gc
     import weakref
     c = cases.build_decode_case("mini3_fp16")
     run = gpu_utils.EngineRun(c["nodes"], c["ptrs"], c["batch"], c["q"], c["k"], c["v"], c["hq"], c["hkv"],
                               c["d"], c["tsq"], planner="b200")
     want = run.decode(path="auto")
-    engine._ARG_CACHE.clear()
+    side = torch.cuda.Stream()
+    engine._RANGE_CACHE.clear()
     refs = []
     for i in range(1000):
-        q = run.q.clone()
-        o = torch.empty_like(q)
-        engine.decode(q, run.k, run.v, o, *run.aux, run.tiles[0], run.tiles[1], run.scale)
-        if i % 100 == 0:
-            refs.append(weakref.ref(q))
+        fresh = i % 100 == 0        # a new plan: table objects of their own, K/V buffers at other addresses
+        k, v = (run.k.clone(), run.v.clone()) if fresh else (run.k, run.v)
+        aux = tuple(t.clone() if isinstance(t, torch.Tensor) else list(t) for t in run.aux) if fresh else run.aux
+        q = run.q.clone() * (2.0 if i % 2 else 1.0)
+        o = torch.full_like(q, float("nan"))
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side) if i % 200 == 100 else torch.cuda.stream(torch.cuda.current_stream()):
+            engine.decode(q, k, v, o, *aux, run.tiles[0], run.tiles[1], run.scale / (2.0 if i % 2 else 1.0))
+        if i % 50 == 0 or i % 100 == 51:
             torch.cuda.synchronize()
-            assert torch.equal(o.float().cpu(), want)
-    assert len(engine._ARG_CACHE) == 1
-    del q, o
+            assert torch.equal(o.float().cpu(), want)       # doubling q and halving the scale are exact
+            refs += [weakref.ref(t) for t in (q, o) + ((k, v, aux[3], aux[9]) if fresh else ())]
+    torch.cuda.synchronize()
+    del q, o, k, v, aux
     gc.collect()
     assert all(r() is None for r in refs)
+    assert run.aux[3].numel() > 2 * run.mid_o.shape[0] and len(engine._RANGE_CACHE) == 1    # the plan's own table, no clone
+    # a refused argument launches nothing
+    before = lib.load().ft_launch_count()
+    with pytest.raises(ValueError):
+        engine.decode(run.q, run.k, run.v, torch.empty_like(run.q[:1]), *run.aux, run.tiles[0], run.tiles[1], run.scale)
+    assert lib.load().ft_launch_count() == before
 
 
 @pytest.mark.parametrize("seed", range(10))
