@@ -251,6 +251,29 @@ __device__ __forceinline__ bool tc_wait(uint32_t bar, uint32_t parity, volatile 
   return false;
 }
 
+// Rows [done, 64) of a tile with 16-byte copies: row ids up to n, zeros behind them (copies that read nothing).  Returns
+// true when a row id was out of range; such a row becomes zeros too.
+template <typename T, int D>
+__device__ __noinline__ bool tc_copy_rows(uint32_t buf, const T* base, int64_t stride, int id0, int id1, int done, int n,
+                                          uint32_t row_lim, int lane) {
+  using C = TcCfg<D>;
+  const int c = lane % C::CPR, sub = lane / C::CPR;  // 16-byte chunk and row of an instruction's C::RPI rows
+  base += c * 8;
+  bool bad = false;
+#pragma unroll 4
+  for (int r0 = done; r0 < n; r0 += C::RPI) {
+    const int r = r0 + sub;
+    const int lo = __shfl_sync(0xffffffffu, id0, r & 31), hi = __shfl_sync(0xffffffffu, id1, r & 31);
+    const uint32_t row = (uint32_t)(r < 32 ? lo : hi);
+    const bool ok = row < row_lim;  // negative and too-large ids fail this test
+    bad |= !ok && r < n;
+    if (r < n) cp_async16_zfill(buf + tc_swz(r, c, 8192), base + (int64_t)(ok ? row : 0u) * stride, ok);
+  }
+#pragma unroll 4
+  for (int r = n + sub; r < C::TILE; r += C::RPI) cp_async16_zfill(buf + tc_swz(r, c, 8192), base, false);
+  return bad;
+}
+
 // Gather of one 64-token operand tile whose rows are not consecutive (scattered pool slots, the ragged last tile); the
 // row ids are in registers, row r in slot r >> 5 of lane r & 31.  Whole groups of four valid rows go through the TMA unit
 // (tile::gather4: one instruction per four rows and 64 elements, one per lane at head_dim 128); the up to three rows
@@ -258,10 +281,16 @@ __device__ __forceinline__ bool tc_wait(uint32_t bar, uint32_t parity, volatile 
 // Issuing the 1024 16-byte copies of a tile took a loader warp longer than the tile's share of the memory bandwidth:
 // 75 776 scattered tokens x 8 heads (303 MB), decode 113 -> 93 us (77 us when the rows are consecutive); either operand
 // alone through the TMA unit 105 us.
+// The copies are a function of their own (tc_copy_rows): one loop here that skipped the rows the TMA unit has taken was
+// slower than 64 plain copies, which showed wherever a one-tile task is on the critical path.  One such loop / apart, per
+// step: ten requests on 4000 tokens, 16/1 heads 14.2 / 13.0 us (12.8 when ragged tiles were copied whole), nine on 700,
+// 32/8 heads 12.7 / 12.2, search tree of 1024 requests 128.2 / 126.6; 16 documents of 1500 tokens, scattered, 33.0 / 32.0.
+// The looping kernel (LOOP) keeps the one loop: apart, its loaders' calls cost registers they do not have (scattered
+// 64 requests on 4096 tokens 37.3 -> 39.0 us, documents 37.7 -> 38.2; consecutive 33.2 -> 32.4).
 // The buffer's full barrier counts an arrival of every lane, which the caller makes with mbar_arrive_on_cp_async.
 // Kept out of line: tiles of consecutive rows never come here, and their loaders' code stays as small as it was.
 // Returns true when a row id inside the chunk was out of range.
-template <typename T, int D>
+template <typename T, int D, bool LOOP>
 __device__ __noinline__ bool tc_gather_tile(uint32_t buf, const CUtensorMap* rows_map, int col0, const T* base, int64_t stride,
                                             int id0, int id1, int t, int id_lim, uint32_t row_lim, int lane, uint32_t full) {
   using C = TcCfg<D>;
@@ -285,22 +314,26 @@ __device__ __noinline__ bool tc_gather_tile(uint32_t buf, const CUtensorMap* row
     }
     if (done == C::TILE) return false;
   }
-  const int c = lane % C::CPR;
-  bool bad = false;
+  if constexpr (!LOOP) {
+    return tc_copy_rows<T, D>(buf, base, stride, id0, id1, done, n, row_lim, lane);
+  } else {
+    const int c = lane % C::CPR;
+    bool bad = false;
 #pragma unroll
-  for (int h = 0; h < 2; ++h) {
+    for (int h = 0; h < 2; ++h) {
 #pragma unroll 4
-    for (int i = 0; i < 32 / C::RPI; ++i) {
-      const int r = lane / C::CPR + C::RPI * i + 32 * h;
-      const int id = __shfl_sync(0xffffffffu, h == 0 ? id0 : id1, r & 31);
-      if (r < done) continue;
-      const uint32_t row = r < n ? (uint32_t)id : 0xffffffffu;
-      const bool ok = row < row_lim;  // padding (0xffffffff), negative and too-large ids all fail this test
-      bad |= !ok && r < n;
-      cp_async16_zfill(buf + tc_swz(r, c, 8192), base + (int64_t)(ok ? row : 0u) * stride + c * 8, ok);
+      for (int i = 0; i < 32 / C::RPI; ++i) {
+        const int r = lane / C::CPR + C::RPI * i + 32 * h;
+        const int id = __shfl_sync(0xffffffffu, h == 0 ? id0 : id1, r & 31);
+        if (r < done) continue;
+        const uint32_t row = r < n ? (uint32_t)id : 0xffffffffu;
+        const bool ok = row < row_lim;  // padding (0xffffffff), negative and too-large ids all fail this test
+        bad |= !ok && r < n;
+        cp_async16_zfill(buf + tc_swz(r, c, 8192), base + (int64_t)(ok ? row : 0u) * stride + c * 8, ok);
+      }
     }
+    return bad;
   }
-  return bad;
 }
 
 // LOOP false: one task (vn, kvh).  LOOP true: the CTA works through tasks of the whole launch, claimed from a counter.
@@ -865,7 +898,7 @@ __device__ __forceinline__ void tc_body(const TcParams& tp, uint8_t* smem, int v
                 mbar_arrive(full);
               }
             } else {
-              const bool bad = tc_gather_tile<T, D>(buf, v_rows, kvh * (int)p.v_s1, vbase, p.v_s0, cur[0], cur[1], t, id_lim,
+              const bool bad = tc_gather_tile<T, D, LOOP>(buf, v_rows, kvh * (int)p.v_s1, vbase, p.v_s0, cur[0], cur[1], t, id_lim,
                                                        row_lim, lane, full);
               if (bad) flag_error(FT_DEV_BAD_KV_INDEX);
               mbar_arrive_on_cp_async(full);
@@ -929,7 +962,7 @@ __device__ __forceinline__ void tc_body(const TcParams& tp, uint8_t* smem, int v
               mbar_arrive(full);
             }
           } else {
-            const bool bad = tc_gather_tile<T, D>(buf, k_rows, kvh * (int)p.k_s1, kbase, p.k_s0, id0, id1, s, id_lim, row_lim,
+            const bool bad = tc_gather_tile<T, D, LOOP>(buf, k_rows, kvh * (int)p.k_s1, kbase, p.k_s0, id0, id1, s, id_lim, row_lim,
                                                   lane, full);
             if (bad) flag_error(FT_DEV_BAD_KV_INDEX);
             mbar_arrive_on_cp_async(full);
