@@ -6,8 +6,8 @@
 // rows (requests x GQA group) per pass against the vnode's KV chunk, 64 tokens
 // per tile:
 //
-//   S[128 x 64]   = Q[128 x 128] . K_tile^T        tcgen05.mma, A and B K-major
-//   O[128 x 128] += P[128 x 64]  . V_tile          tcgen05.mma, B MN-major
+//   S[128 x 64] = Q[128 x D] . K_tile^T        tcgen05.mma, A and B K-major     (D = head_dim: 64, 128 or 256)
+//   O[128 x D] += P[128 x 64] . V_tile         tcgen05.mma, B MN-major
 //
 // Roles
 //   warps 0-3  softmax: thread t owns query row t = TMEM lane t.  It reads its
@@ -20,8 +20,9 @@
 //              same offset, so the result is unchanged).  Only that rescale
 //              waits for the previous tile's P.V.
 //              At the end it stages its normalised row in shared memory and
-//              each warp writes its 32 rows to the partial buffer with full-row
-//              (512-byte) store instructions.
+//              each warp writes its 32 rows to the partial buffer with 512-byte
+//              store instructions.  Rows that attend to part of the chunk and did not
+//              come out finite are computed again (ft_stage1_row.cuh).
 //   warp 4     MMA issue (one elected lane): S_t is issued before the softmax of
 //              tile t-1 has finished (two S buffers in TMEM), P.V of tile t-1
 //              as soon as its P is written.
@@ -52,8 +53,9 @@
 //
 // Q, K and V use the canonical 128-byte-swizzled operand layout (64-element
 // blocks, 8-row groups of 1024 bytes).  TMEM: two 64-column S buffers (P of a
-// tile, 16-bit, takes the first 32 columns of its S buffer) and 128 columns of O
-// in a 256-column allocation, so two CTAs share an SM.
+// tile, 16-bit, takes the first 32 columns of its S buffer) and D columns of O
+// in a 256-column allocation, so two CTAs share an SM (512 columns and one CTA at
+// head_dim 256).
 // S buffer b is written again by S_{t+2} while it may still hold P_t.  Nothing
 // but issue order protects it: every MMA of this kernel has the same shape
 // (M 128, N 64, K 16 - P.V is issued as two 64-column halves of O for that
