@@ -3,6 +3,7 @@
 // Python entry points are in include/fasttree_b200.h.
 #include <cuda.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cstdarg>
 #include <mutex>
@@ -196,6 +197,7 @@ ft::Stage1Params stage1_params(const ft_decode_args* a) {
   p.node_split = 0;
   p.lead_wide = 0;
   p.workers = 0;
+  p.few_form = ft::FEW_ONE;
   p.num_kv_heads = a->num_kv_heads;
   p.sm_scale = a->sm_scale;
   return p;
@@ -229,18 +231,6 @@ int launch_mma(const ft::Stage1Params& p, int hkv, cudaStream_t st) {
   FT_CUDA_OK(raise_smem_limit(once, ft::stage1_mma_kernel<T, D>, C::SMEM_BYTES));
   const unsigned grid = (unsigned)p.node_count * (unsigned)hkv;
   FT_CUDA_OK(launch_early(ft::stage1_mma_kernel<T, D>, grid, C::THREADS, C::SMEM_BYTES, st, p));
-  count_launch();
-  return FT_OK;
-}
-
-template <typename T, int D>
-int launch_narrow(const ft::Stage1Params& p, int hkv, cudaStream_t st) {
-  using C = ft::NarrowCfg<D, 2>;
-  if (dry_run("stage1_narrow_kernel")) return FT_OK;
-  static OncePerDevice once;
-  FT_CUDA_OK(raise_smem_limit(once, ft::stage1_narrow_kernel<T, D>, C::SMEM_BYTES));
-  const unsigned grid = (unsigned)p.node_count * (unsigned)hkv;
-  FT_CUDA_OK(launch_early(ft::stage1_narrow_kernel<T, D>, grid, 128, C::SMEM_BYTES, st, p));
   count_launch();
   return FT_OK;
 }
@@ -360,7 +350,11 @@ ft::TcParams tc_params(const ft::Stage1Params& p, const ft_decode_args* a) {
   tp.has_tma = tensor_map(&tp.k_map, a->k_buffer, a->dtype, d, a->kv_rows, a->num_kv_heads, a->k_stride0,
                              a->k_stride1, 1, 64) &&
                tensor_map(&tp.v_map, a->v_buffer, a->dtype, d, a->kv_rows, a->num_kv_heads, a->v_stride0,
-                             a->v_stride1, 1, 64);
+                             a->v_stride1, 1, 64) &&
+               tensor_map(&tp.k_slab_map, a->k_buffer, a->dtype, d, a->kv_rows, a->num_kv_heads, a->k_stride0,
+                             a->k_stride1, 1, 16) &&
+               tensor_map(&tp.v_slab_map, a->v_buffer, a->dtype, d, a->kv_rows, a->num_kv_heads, a->v_stride0,
+                             a->v_stride1, 1, 16);
   tp.has_gather4 = tp.has_tma &&
                    tensor_map(&tp.k_rows_map, a->k_buffer, a->dtype, d, a->kv_rows, a->num_kv_heads, a->k_stride0,
                                  a->k_stride1, 0, 1) &&
@@ -378,6 +372,56 @@ ft::TcParams tc_params(const ft::Stage1Params& p, const ft_decode_args* a) {
       tp.q_box_rows = box_heads;
   }
   return tp;
+}
+
+// How the few-row tasks of a launch are run (ft::FEW_*; -1: by the tcgen05 kernel, head_dim 256 only); wide: its many-row CTAs.
+// Two tasks per CTA keep an SM streaming while a task starts up, but they share the SM's copy rate: below about 1.2 CTAs per
+// slot (1.6 at head_dim 64) some SMs hold four tasks and others two, and one task per CTA, dealt out as slots come free, is
+// the better balanced; tasks of about 130 tokens, mostly start-up, gain from one CTA per slot on.  One / two tasks per CTA, us
+// per step, leaves under a 1000-token node, 32/8 heads of 128: 60 of 130 tokens (1.03 CTAs per slot) 19.9 / 18.7, 60 of 400
+// (0.86) 28.2 / 31.9, 74 of 400 (1.16) 33.7 / 35.4, 90 of 400 (1.3) 39.0 / 37.3, 90 of 130 25.4 / 21.2; 64 requests of 256
+// tokens on 4096 (1.4) 27.7 / 25.6; the ragged tree of six levels (8.9) 595 / 546.  Heads of 64: 100 of 300 (1.45) 26.3 /
+// 32.5, 120 of 300 (1.7) 29.6 / 24.2.  More than eight heads per KV head: every task needs the two-block body, which does not
+// fit 128 registers (600 requests at 16/1 heads: nothing gained).
+// Head_dim 256, one CTA per SM: one round on the tcgen05 kernel, whose tile loads are the larger (16 leaves of 400 tokens 21.4
+// / 23.7 us with eight warps per task), up to two tasks per SM eight warps each (18 of 400 31.1 / 24.6), two at a time above
+// (60 of 130 47.5 / 30.0, 60 of 1500 144 / 125; 64 requests of 256 tokens on 4096 58 / 42).
+int few_rows_form(const ft::Stage1Params& p, int64_t few_nodes, int64_t wide, int hkv, int head_dim, int64_t slots) {
+  const int64_t few = few_nodes * hkv;
+  if (head_dim == 256) {
+    if (p.group > 8 || few + wide <= slots) return -1;
+    return few + wide > 2 * slots ? ft::FEW_PAIR : ft::FEW_EIGHT;
+  }
+  if (p.group > 8) return ft::FEW_ONE;
+  const int64_t ctas = (few + 1) / 2 + wide;
+  if (head_dim == 64) return 5 * ctas >= 8 * slots ? ft::FEW_PAIR : ft::FEW_ONE;
+  return 5 * ctas >= 6 * slots || (ctas >= slots && p.kv_entries_len <= 170 * few_nodes) ? ft::FEW_PAIR : ft::FEW_ONE;
+}
+
+template <typename T, int D>
+int launch_narrow(ft::TcParams p, int hkv, cudaStream_t st, int form) {
+  if (dry_run("stage1_narrow_kernel")) return FT_OK;
+  const int64_t tasks = (int64_t)p.p.node_count * hkv;
+  if constexpr (D <= 128) {
+    if (form == ft::FEW_ONE) {
+      using C = ft::NarrowCfg<D, 2>;
+      static OncePerDevice once;
+      void (*kernel)(ft::Stage1Params) = ft::stage1_narrow_kernel<T, D>;
+      FT_CUDA_OK(raise_smem_limit(once, kernel, C::SMEM_BYTES));
+      FT_CUDA_OK(launch_early(kernel, (unsigned)tasks, 128, C::SMEM_BYTES, st, p.p));
+      count_launch();
+      return FT_OK;
+    }
+  }
+  using C = ft::PairCfg<D>;
+  static OncePerDevice once;
+  void (*kernel)(ft::TcParams) = ft::stage1_narrow_kernel<T, D>;
+  FT_CUDA_OK(raise_smem_limit(once, kernel, C::SMEM_BYTES));
+  p.p.few_form = form;
+  const int per = ft::few_per_cta(form);
+  FT_CUDA_OK(launch_early(kernel, (unsigned)((tasks + per - 1) / per), C::THREADS, C::SMEM_BYTES, st, p));
+  count_launch();
+  return FT_OK;
 }
 
 template <typename T, int D>
@@ -439,52 +483,68 @@ bool few_rows_by_workers(int64_t few_nodes, int64_t kv_entries_len, int hkv, int
   return few_nodes * hkv >= 20 * slots && kv_entries_len <= 80 * few_nodes;
 }
 
-template <typename T, int D>
-int launch_fused(ft::TcParams p, int hkv, cudaStream_t st) {
-  constexpr int smem_a = ft::TcCfg<D>::SMEM_BYTES > ft::StreamCfg<D>::SMEM_BYTES ? ft::TcCfg<D>::SMEM_BYTES
-                                                                                    : ft::StreamCfg<D>::SMEM_BYTES;
-  constexpr int smem = smem_a > ft::NarrowCfg<D, 2>::SMEM_BYTES ? smem_a : ft::NarrowCfg<D, 2>::SMEM_BYTES;
-  static_assert(smem <= 115712, "two CTAs must fit in one SM's shared memory");
+template <typename T, int D, bool PAIR>
+int launch_fused_as(const ft::TcParams& p, int64_t ctas, cudaStream_t st) {
+  constexpr int few_smem = [] {
+    if constexpr (PAIR) return ft::PairCfg<D>::SMEM_BYTES;
+    else return std::max(ft::StreamCfg<D>::SMEM_BYTES, ft::NarrowCfg<D, 2>::SMEM_BYTES);
+  }();
+  constexpr int smem = std::max(ft::TcCfg<D>::SMEM_BYTES, few_smem);
+  static_assert(smem <= (D == 256 ? 232448 : 115712), "the resident CTAs must fit in one SM's shared memory");
   if (dry_run("stage1_fused_kernel")) return FT_OK;
+  if (ctas > 0x7fffffffLL) return fail(FT_ERR_TOO_LARGE, "vnodes x kv heads exceeds the grid limit");
   static OncePerDevice once;
-  int dev = 0;
-  FT_CUDA_OK(raise_smem_limit(once, ft::stage1_fused_kernel<T, D>, smem, &dev));
-  // Few-row tasks by persistent workers only when the many-row CTAs do not fill the device more than once (the workers
-  // take the slots those leave and, as they finish, theirs too); one CTA per task otherwise (the hardware then slots
-  // the small CTAs in wherever a many-row CTA finishes).  Many-row CTAs go first.
-  const int64_t wide = (int64_t)p.p.node_split * hkv;
-  const int64_t few = (int64_t)(p.p.node_count - p.p.node_split) * hkv;
-  const int64_t slots = 2LL * sm_count(dev);
-#ifdef FT_FORCE_WORKERS  // developer builds: persistent workers in every free slot, whatever the task count
-  const int64_t workers = few < slots - wide ? few : (slots - wide > slots / 4 ? slots - wide : slots);
-#else
-  const int64_t workers = few_rows_by_workers(p.p.node_count - p.p.node_split, p.p.kv_entries_len, hkv, slots) && wide <= slots ? slots : 0;
-#endif
-  const int64_t few_ctas = workers > 0 ? workers : few;
-  const int64_t lead = wide;
-  if (wide + few_ctas > 0x7fffffffLL) return fail(FT_ERR_TOO_LARGE, "vnodes x kv heads exceeds the grid limit");
-  p.p.workers = (int)workers;
-  p.p.lead_wide = (int)lead;
-  FT_CUDA_OK(launch_early(ft::stage1_fused_kernel<T, D>, (unsigned)(wide + few_ctas), ft::TcCfg<D>::THREADS, smem, st, p));
+  FT_CUDA_OK(raise_smem_limit(once, ft::stage1_fused_kernel<T, D, PAIR>, smem));
+  FT_CUDA_OK(launch_early(ft::stage1_fused_kernel<T, D, PAIR>, (unsigned)ctas, ft::TcCfg<D>::THREADS, smem, st, p));
   count_launch();
   return FT_OK;
 }
 
-// path: AUTO (<= 16 rows: persistent workers or narrow; above: tcgen05; head_dim 256 has the tcgen05 kernel only),
+template <typename T, int D>
+int launch_fused(ft::TcParams p, int hkv, cudaStream_t st) {
+  int dev = 0;
+  FT_CUDA_OK(cudaGetDevice(&dev));
+  const int64_t wide = (int64_t)p.p.node_split * hkv;
+  const int64_t few_nodes = p.p.node_count - p.p.node_split, few = few_nodes * hkv;
+  const int64_t slots = (int64_t)ft::TcCfg<D>::CTAS * sm_count(dev);
+  p.p.lead_wide = (int)wide;  // many-row CTAs go first
+  p.p.few_form = few_rows_form(p.p, few_nodes, wide, hkv, D, slots);
+  if constexpr (D <= 128) {
+    // Few-row tasks by persistent workers only when the many-row CTAs do not fill the device more than once (the workers
+    // take the slots those leave and, as they finish, theirs too).
+    if (few_rows_by_workers(few_nodes, p.p.kv_entries_len, hkv, slots) && wide <= slots) {
+      p.p.workers = (int)slots;
+      return launch_fused_as<T, D, false>(p, wide + slots, st);
+    }
+    if (p.p.few_form == ft::FEW_ONE) return launch_fused_as<T, D, false>(p, wide + few, st);
+  }
+  if (p.p.few_form < 0) return launch_tc<T, D>(p, hkv, st);  // the whole range on the tcgen05 kernel
+  const int per = ft::few_per_cta(p.p.few_form);
+  return launch_fused_as<T, D, true>(p, wide + (few + per - 1) / per, st);
+}
+
+// path: AUTO (<= 16 rows: persistent workers or narrow, in the form few_rows_form chooses; above: tcgen05),
 // STREAM (like AUTO, always the persistent workers), MMA (narrow / wide), MMA_WIDE (wide for everything),
 // TCGEN05 (tcgen05 for everything)
 template <typename T, int D>
 int launch_tensor(const ft::Stage1Params& p, const ft_decode_args* a, int hkv, cudaStream_t st, int max_rows, int path) {
-  if (D == 256 || path == FT_PATH_TCGEN05 || ((path == FT_PATH_AUTO || path == FT_PATH_STREAM) && max_rows > 16))
+  if (path == FT_PATH_TCGEN05 || ((path == FT_PATH_AUTO || path == FT_PATH_STREAM) && max_rows > 16))
     return launch_tc<T, D>(tc_params(p, a), hkv, st);
-  if constexpr (D != 256) {
+  int dev = 0;
+  FT_CUDA_OK(cudaGetDevice(&dev));
+  const int64_t slots = (int64_t)ft::TcCfg<D>::CTAS * sm_count(dev);
+  if constexpr (D == 256) {
+    const ft::TcParams tp = tc_params(p, a);
+    const int form = few_rows_form(p, p.node_count, 0, hkv, D, slots);
+    return form < 0 ? launch_tc<T, D>(tp, hkv, st) : launch_narrow<T, D>(tp, hkv, st, form);
+  } else {
     if (max_rows <= 16) {
-      int dev = 0;
-      FT_CUDA_OK(cudaGetDevice(&dev));
-      const bool many = few_rows_by_workers(p.node_count, p.kv_entries_len, hkv, 2LL * sm_count(dev));
+      const bool many = few_rows_by_workers(p.node_count, p.kv_entries_len, hkv, slots);
       if (path == FT_PATH_STREAM || (path == FT_PATH_AUTO && many)) return launch_stream<T, D>(tc_params(p, a), hkv, st);
     }
-    if (path != FT_PATH_MMA_WIDE && max_rows <= 16) return launch_narrow<T, D>(p, hkv, st);
+    if (path != FT_PATH_MMA_WIDE && max_rows <= 16)
+      return launch_narrow<T, D>(tc_params(p, a), hkv, st,
+                                 path == FT_PATH_AUTO ? few_rows_form(p, p.node_count, 0, hkv, D, slots) : ft::FEW_ONE);
     return launch_mma<T, D>(p, hkv, st);
   }
 }
@@ -639,7 +699,7 @@ int ft_stage1(const ft_decode_args* a) {
   const int64_t r1 = a->phase_q_tile_sizes[1] > 0 ? (int64_t)a->phase_q_tile_sizes[1] * group : 1 << 30;
   const int rows0 = (int)(r0 < (1 << 30) ? r0 : (1 << 30)), rows1 = (int)(r1 < (1 << 30) ? r1 : (1 << 30));
   const bool same_kernel = path == FT_PATH_GENERIC || path == FT_PATH_MMA_WIDE || path == FT_PATH_TCGEN05 ||
-                           a->head_dim == 256 || ((rows0 > 16) == (rows1 > 16));
+                           ((rows0 > 16) == (rows1 > 16));
   // the persistent kernel takes every task of the launch, whatever its row count
   if (path == FT_PATH_PERSIST && a->device_phase_info != nullptr) {
     ft::Stage1Params p = stage1_params(a);  // node_offset / node_count come from the device array
@@ -664,8 +724,8 @@ int ft_stage1(const ft_decode_args* a) {
     }
     return FT_OK;
   }
-  // head_dim 64 / 128, many-row phase followed directly by the few-row phase: one grid with both kernel bodies
-  if (path == FT_PATH_AUTO && a->head_dim <= 128 && n0 > 0 && n1 > 0 && o1 == o0 + n0 && rows0 > 16 && rows1 <= 16) {
+  // many-row phase followed directly by the few-row phase: one grid with both kernel bodies
+  if (path == FT_PATH_AUTO && (a->head_dim == 64 || a->head_dim == 128 || a->head_dim == 256) && n0 > 0 && n1 > 0 && o1 == o0 + n0 && rows0 > 16 && rows1 <= 16) {
     ft::Stage1Params p = stage1_params(a);
     p.node_offset = o0;
     p.node_count = n0 + n1;
@@ -675,6 +735,9 @@ int ft_stage1(const ft_decode_args* a) {
     if (a->head_dim == 64)
       return a->dtype == FT_F16 ? launch_fused<__half, 64>(tp, a->num_kv_heads, st)
                                 : launch_fused<__nv_bfloat16, 64>(tp, a->num_kv_heads, st);
+    if (a->head_dim == 256)
+      return a->dtype == FT_F16 ? launch_fused<__half, 256>(tp, a->num_kv_heads, st)
+                                : launch_fused<__nv_bfloat16, 256>(tp, a->num_kv_heads, st);
     return a->dtype == FT_F16 ? launch_fused<__half, 128>(tp, a->num_kv_heads, st)
                               : launch_fused<__nv_bfloat16, 128>(tp, a->num_kv_heads, st);
   }

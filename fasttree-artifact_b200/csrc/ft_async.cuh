@@ -17,6 +17,8 @@ struct alignas(64) TcParams {
   CUtensorMap q_map_tile;  // same tensor, box 64 x G x 128 / G: a whole Q tile of consecutive requests
   CUtensorMap k_rows_map;  // K and V as [rows, all heads' elements], box 64 x 1: rows picked one by one (tile::gather4)
   CUtensorMap v_rows_map;
+  CUtensorMap k_slab_map;  // K and V like k_map, box 64 x 1 x 16: the few-row kernel's slabs
+  CUtensorMap v_slab_map;
   Stage1Params p;
   int has_tma;
   int has_gather4;    // the two row maps are valid
@@ -42,6 +44,10 @@ __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
 // the barrier gets one arrival when all earlier cp.async copies of this thread have landed
 __device__ __forceinline__ void mbar_arrive_on_cp_async(uint32_t bar) {
   asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];\n" ::"r"(bar) : "memory");
+}
+// the same for a barrier that does not count on this thread: one more arrival is owed, and made by the copies
+__device__ __forceinline__ void mbar_arrive_after_cp_async(uint32_t bar) {
+  asm volatile("cp.async.mbarrier.arrive.shared::cta.b64 [%0];\n" ::"r"(bar) : "memory");
 }
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, uint32_t bar) {
   asm volatile(

@@ -97,7 +97,8 @@ struct Stage1Params {
   int32_t num_kv_heads;
   int32_t node_split;   // fused launch: vnodes [0, node_split) of the launch are many-row tasks
   int32_t lead_wide;    // fused launch: many-row CTAs placed before the few-row CTAs in block order
-  int32_t workers;      // fused launch: persistent few-row workers (0: one CTA per few-row task)
+  int32_t workers;      // fused launch: persistent few-row workers (0: one CTA per task or two)
+  int32_t few_form;     // how a CTA runs few-row tasks: FEW_ONE, FEW_PAIR or FEW_EIGHT
   float sm_scale;
 };
 
@@ -116,6 +117,10 @@ __device__ __forceinline__ int kv_ids_limit(const Stage1Params& p, int kv_off, i
   const int64_t readable = aux ? p.kv_entries_aux_len - (int64_t)(kv_off & (FT_AUX_BIT - 1)) : p.kv_entries_len - (int64_t)kv_off;
   return (int)(readable < (int64_t)kv_len ? (readable < 0 ? 0 : readable) : kv_len);
 }
+
+// Few-row tasks of a CTA: one by four warps, two by four warps each, or one by eight warps
+enum { FEW_ONE = 0, FEW_PAIR = 1, FEW_EIGHT = 2 };
+__host__ __device__ __forceinline__ int few_per_cta(int form) { return form == FEW_PAIR ? 2 : 1; }
 
 struct Stage2Params {
   const int32_t* r2v_entries;

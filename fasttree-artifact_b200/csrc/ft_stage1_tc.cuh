@@ -73,6 +73,7 @@
 #include "ft_common.cuh"
 #include "ft_stage1_mma.cuh"
 #include "ft_stage1_narrow.cuh"
+#include "ft_stage1_pair.cuh"
 #include "ft_stage1_row.cuh"
 #include "ft_stage1_stream.cuh"
 
@@ -111,6 +112,7 @@ struct TcCfg {
   static constexpr int K_FULL = 0, K_EMPTY = 3, V_FULL = 6, V_EMPTY = 8, S_FULL = 10, P_FULL = 12, PV_DONE = 14,
                        Q_FULL = 16;
   static constexpr int OUT_STRIDE = D * 4 + 16;       // bytes between staged output rows (+ 16: conflict-free 16-byte stores)
+  static constexpr int CTAS = D == 256 ? 1 : 2;       // resident CTAs per SM
   static constexpr int REGS_SOFTMAX = 184, REGS_OTHER = 72;
   static constexpr int REGS_WORKER = 232;             // few-row workers of the fused kernel: four warps, the other four leave
   static constexpr int CPR = D / 8, RPI = 32 / CPR;   // gathers: 16-byte chunks per row, rows per warp instruction
@@ -1099,22 +1101,24 @@ __global__ void __launch_bounds__(TcCfg<D>::THREADS, 2) stage1_tc_kernel(const _
   FT_TL_END(1);
 }
 
-// Both task families in one grid (head_dim 64 and 128): the tensor-bound many-row CTAs (tcgen05 body, one task each)
+// Both task families in one grid: the tensor-bound many-row CTAs (tcgen05 body, one task each)
 // and the memory-bound few-row CTAs (swapped-operand body) share the SMs instead of running back to back.
 // Block order, which is the order the hardware starts them in:
 //   [0, lead)                 many-row tasks 0 .. lead-1
 //   [lead, lead + few_ctas)   few-row CTAs: persistent workers that split the few-row tasks between them
-//                             (p.workers > 0), or one CTA per few-row task (p.workers == 0)
+//                             (p.workers > 0), or one CTA per one or two few-row tasks (p.workers == 0)
 //   the rest                  the remaining many-row tasks
 // `lead` leaves room for the few-row CTAs to start at once beside the first many-row CTAs.
-template <typename T, int D>
+// PAIR: few-row tasks by pair_cta (p.few_form), else by the workers or the one-task body; a kernel each, because in one
+// kernel they cost the one-task plans 2-3 % (45 leaves of 130 tokens under a 1000-token node 17.2 -> 17.6 us).
+template <typename T, int D, bool PAIR>
 __global__ void __launch_bounds__(TcCfg<D>::THREADS, 2) stage1_fused_kernel(const __grid_constant__ TcParams tp) {
   allow_dependent_launch();
   extern __shared__ __align__(1024) uint8_t smem[];
   const Stage1Params& p = tp.p;
   const int H = p.num_kv_heads;
   const int wide_tasks = p.node_split * H, few_tasks = (p.node_count - p.node_split) * H;
-  const int few_ctas = p.workers > 0 ? p.workers : few_tasks;
+  const int few_ctas = PAIR ? (few_tasks + few_per_cta(p.few_form) - 1) / few_per_cta(p.few_form) : p.workers > 0 ? p.workers : few_tasks;
   const int b = (int)blockIdx.x;
   FT_TL_BEGIN();
   if (b < p.lead_wide || b >= p.lead_wide + few_ctas) {
@@ -1125,19 +1129,26 @@ __global__ void __launch_bounds__(TcCfg<D>::THREADS, 2) stage1_fused_kernel(cons
     // This CTA will not allocate tensor memory.  Saying so at once matters: the SM admits no second CTA of a
     // kernel that uses tensor memory while a resident one still holds the right to allocate.
     if (threadIdx.x < 32) asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
-    if (threadIdx.x >= 128) {  // the few-row bodies are written for four warps: the others hand over their registers
-      reg_shrink<24>();
+    const int w = b - p.lead_wide;
+    if constexpr (!PAIR) {
+      if (threadIdx.x >= 128) {  // these bodies are written for four warps: the others hand over their registers
+        reg_shrink<24>();
+        return;
+      }
+      reg_grow<TcCfg<D>::REGS_WORKER>();
+      wait_for_prior_grid();  // nothing of the preceding kernel's is read or overwritten before this
+      if (p.workers > 0) {
+        stream_worker<T, D>(tp, smem, wide_tasks, few_tasks, w, p.workers);
+      } else {
+        const int task = wide_tasks + w;
+        narrow_dispatch<T, D>(p, smem, p.node_offset + task / H, task % H);
+      }
+      FT_TL_END(2);
       return;
     }
-    reg_grow<TcCfg<D>::REGS_WORKER>();
-    wait_for_prior_grid();  // nothing of the preceding kernel's is read or overwritten before this
-    const int w = b - p.lead_wide;
-    if (p.workers > 0) {
-      stream_worker<T, D>(tp, smem, wide_tasks, few_tasks, w, p.workers);
-    } else {
-      const int task = wide_tasks + w;
-      narrow_dispatch<T, D>(p, smem, p.node_offset + task / H, task % H);
-    }
+    if (D == 256) prefetch_slab_maps(tp);
+    wait_for_prior_grid();
+    if constexpr (PAIR) pair_cta<T, D>(tp, smem, p.few_form, wide_tasks + few_per_cta(p.few_form) * w, wide_tasks + few_tasks);
     FT_TL_END(2);
   }
 }
