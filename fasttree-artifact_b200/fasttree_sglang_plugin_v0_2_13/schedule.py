@@ -38,10 +38,12 @@ def _walk_requests(batch):
     node_to_reqs = defaultdict(list)
     covered = []
     for rid, req in enumerate(batch.reqs):
-        tokens = list(req.origin_input_ids) + list(req.output_ids)
+        prompt, output = req.origin_input_ids, req.output_ids
+        n_prompt = len(prompt)
+        n_tokens = n_prompt + len(output)
         node, pos = root, 0
-        while pos < len(tokens):
-            child = node.children.get(tokens[pos])
+        while pos < n_tokens:
+            child = node.children.get(prompt[pos] if pos < n_prompt else output[pos - n_prompt])
             if not child:
                 break
             node_to_reqs[child].append(rid)
@@ -52,8 +54,8 @@ def _walk_requests(batch):
 
 
 def _bfs(batch, node_to_reqs):
-    """Populated radix nodes in breadth-first order with their token offsets (schedule.py:74-85)."""
-    order, offsets, parents = [], [], []
+    """Populated radix nodes in breadth-first order with their token offsets, parents and lengths (schedule.py:74-85)."""
+    order, offsets, parents, lens = [], [], [], []
     todo = deque([(batch.tree_cache.root_node, 0, -1)])
     while todo:
         node, off, par = todo.popleft()
@@ -61,11 +63,12 @@ def _bfs(batch, node_to_reqs):
         order.append(node)
         offsets.append(off)
         parents.append(par)
-        nxt = off + len(node.value)
+        lens.append(len(node.value))
+        nxt = off + lens[me]
         for child in node.children.values():
             if child in node_to_reqs:
                 todo.append((child, nxt, me))
-    return order, offsets, parents
+    return order, offsets, parents, lens
 
 
 def _upload(md, tabs, last_vnodes, tail_state=None, src_table=None):
@@ -131,12 +134,11 @@ def _upload(md, tabs, last_vnodes, tail_state=None, src_table=None):
 
 
 # --------------------------------------------------------------- reference-compatible
-def _plan_reference(batch, md, node_to_reqs, order, offsets, req_idx, stride):
+def _plan_reference(batch, md, node_to_reqs, order, offsets, lens, req_idx, stride):
     tsq, tsk = list(md.TSQs), list(md.TSKs)
     split = [md.kv_split_sizes[0], md.kv_split_sizes[0]]
     heads = md.num_kv_heads
     counts = [len(node_to_reqs[n]) if n in node_to_reqs else 0 for n in order]
-    lens = [len(n.value) for n in order]
 
     def cta_counts():                                   # schedule.py:87-118 with the heuristic inert
         par = [0, 0]
@@ -170,7 +172,7 @@ def _plan_reference(batch, md, node_to_reqs, order, offsets, req_idx, stride):
         group = kids if kids else [node]
         reqs = [r for n in group for r in node_to_reqs[n]]
         first = node_to_reqs[group[0]][0]
-        start = stride * int(req_idx[first]) + off
+        start = stride * req_idx[first] + off
         ph = 0 if cnt > tsq[1] else 1
         # the reference sizes the request tiles from `cnt` but lists `reqs`; they agree whenever
         # every request of a node continues into one of its children (true for its workloads)
@@ -181,7 +183,7 @@ def _plan_reference(batch, md, node_to_reqs, order, offsets, req_idx, stride):
                                            q_tile=tsq[ph], kv_split=split[ph]))
     tails = []
     for rid, req in enumerate(batch.reqs):                                  # schedule.py:212-232
-        start = stride * int(req_idx[rid]) + len(req.origin_input_ids)
+        start = stride * req_idx[rid] + len(req.origin_input_ids)
         tails.append(_planner.VirtualNode([(start, start + len(req.output_ids) + 1)],
                                           np.asarray([rid], dtype=np.int32), q_tile=tsq[1], kv_split=split[1]))
     perm = []
@@ -206,13 +208,13 @@ class _RadixView:
         self.parent, self.id, self.seqlen, self.num_children, self.requests = parent, nid, seqlen, 0, requests
 
 
-def _plan_b200(batch, md, node_to_reqs, covered, order, offsets, parents, req_idx, stride):
+def _plan_b200(batch, md, node_to_reqs, covered, order, offsets, parents, lens, req_idx, stride):
     model = _planner.b200_model_for(md, md.head_dim)
     all_reqs = list(range(len(batch.reqs)))
     tree = []
     for i, (node, par) in enumerate(zip(order, parents)):
         reqs = all_reqs if i == 0 else sorted(node_to_reqs[node])
-        tree.append(_RadixView(par, i, len(node.value), reqs))
+        tree.append(_RadixView(par, i, lens[i], reqs))
         if par >= 0:
             tree[par].num_children += 1
 
@@ -223,7 +225,7 @@ def _plan_b200(batch, md, node_to_reqs, covered, order, offsets, parents, req_id
             up = tree[up].parent
             start = offsets[up]
         first = tree[i].requests[0]
-        base = stride * int(req_idx[first])
+        base = stride * req_idx[first]
         return [(base + start, base + offsets[i] + tree[i].seqlen)]
 
     # Radix nodes that only one request passes through (the unique end of its prompt) are contiguous with that
@@ -237,20 +239,25 @@ def _plan_b200(batch, md, node_to_reqs, covered, order, offsets, parents, req_id
                 tail_start[rid] = min(tail_start[rid], offsets[i])
                 tree[i].requests = []
                 tree[tree[i].parent].num_children -= 1
-    extra = []
-    for rid, req in enumerate(batch.reqs):
-        end = len(req.origin_input_ids) + len(req.output_ids) + 1
-        base = stride * int(req_idx[rid])
-        extra.append(([(base + tail_start[rid], base + end)], [rid]))
+    bsz = len(batch.reqs)
+    rids = np.arange(bsz, dtype=np.int64)
+    base = stride * np.asarray(req_idx, dtype=np.int64)
+    tail_end = base + np.fromiter((len(r.origin_input_ids) + len(r.output_ids) + 1 for r in batch.reqs), dtype=np.int64, count=bsz)
+    extra = np.stack([base + np.asarray(tail_start, dtype=np.int64), tail_end, rids], axis=1)
+    native = getattr(md, "native_planner", True)
+    if native:
+        arrays = _planner._tree_arrays(tree)
+        node_base = [stride * req_idx[nd.requests[0]] if nd.requests else 0 for nd in tree]
+
     def run(tail_room, model):
-        if getattr(md, "native_planner", True):
+        if native:
             # the native splitter of the shared library; the Python branch below is its specification
-            node_base = [stride * int(req_idx[nd.requests[0]]) if nd.requests else 0 for nd in tree]
             return _planner.b200_tables_native_direct(
-                tree, node_base, offsets, [(r[0][0], r[0][1], q[0]) for r, q in extra], len(batch.reqs),
-                md.num_qo_heads, md.num_kv_heads, md.head_dim, model, tail_room=tail_room)
+                tree, node_base, offsets, extra, bsz, md.num_qo_heads, md.num_kv_heads, md.head_dim, model,
+                tail_room=tail_room, arrays=arrays)
         vnodes, _assign, q_tile, small_tile, _target = _planner.b200_virtual_nodes(
-            tree, md.num_qo_heads, md.num_kv_heads, md.head_dim, model, ranges_of, extra=extra, tail_room=tail_room)
+            tree, md.num_qo_heads, md.num_kv_heads, md.head_dim, model, ranges_of,
+            extra=[([(b, e)], [r]) for b, e, r in extra.tolist()], tail_room=tail_room)
         tabs = _planner.emit_tables(vnodes, len(batch.reqs), small_tile=small_tile, direct_offsets=True,
                                     order_key=_planner.b200_task_order)
         return tabs, q_tile, small_tile, model.tile_tokens
@@ -269,39 +276,42 @@ def _plan_b200(batch, md, node_to_reqs, covered, order, offsets, parents, req_id
     md.phase_q_tile_sizes = [q_tile, small_tile]
     md.phase_kv_tile_sizes = [tile_tokens, tile_tokens]
     # the task holding the END of each request's tail (the one that grows during the burst)
-    ends = {}
-    for rid, req in enumerate(batch.reqs):
-        ends[stride * int(req_idx[rid]) + len(req.origin_input_ids) + len(req.output_ids) + 1] = rid
-    last = [-1] * len(batch.reqs)
+    last = np.full(bsz, -1, dtype=np.int64)
     kv_offs = tabs["vnode_to_kv_offs"].astype(np.int64)
-    kv_end = kv_offs + tabs["vnode_to_kv_lens"]
-    for task in np.flatnonzero((tabs["vnode_to_q_lens"] == 1) & (kv_offs < _planner.AUX_BIT)):
-        rid = ends.get(int(kv_end[task]))
-        if rid is not None and int(tabs["vnode_to_q_entries"][tabs["vnode_to_q_offs"][task]]) == rid:
-            last[rid] = int(task)
+    q_offs, q_lens, q_entries = tabs["vnode_to_q_offs"], tabs["vnode_to_q_lens"], tabs["vnode_to_q_entries"]
+    single = np.flatnonzero((q_lens == 1) & (kv_offs < _planner.AUX_BIT))
+    owner = q_entries[q_offs[single]]
+    ends_tail = kv_offs[single] + tabs["vnode_to_kv_lens"][single] == tail_end[owner]
+    last[owner[ends_tail]] = single[ends_tail]
     # tails that became members of a group: the run that ends where the request ends and has room behind it
-    state = np.full((len(batch.reqs), 4), -1, dtype=np.int32)
+    state = np.full((bsz, 4), -1, dtype=np.int32)
     segs = tabs.get("aux_segments")
     if segs is not None and len(segs):
+        segs = segs.astype(np.int64)
+        by_end = np.argsort(tail_end)
+        at = np.minimum(np.searchsorted(tail_end[by_end], segs[:, 0] + segs[:, 1]), bsz - 1)
+        rid = by_end[at]
+        tails = (tail_end[rid] == segs[:, 0] + segs[:, 1]) & (segs[:, 3] > 0)
+        rid, (src, length, dst, room) = rid[tails], segs[tails].T
         groups = np.flatnonzero(kv_offs >= _planner.AUX_BIT)
-        g_base = kv_offs[groups] - _planner.AUX_BIT
-        by_base = np.argsort(g_base)
-        for src, length, dst, room in segs.tolist():
-            rid = ends.get(src + length)
-            if rid is None or room <= 0:
-                continue
-            task = int(groups[by_base[np.searchsorted(g_base[by_base], dst, side="right") - 1]])
-            q0, qn = int(tabs["vnode_to_q_offs"][task]), int(tabs["vnode_to_q_lens"][task])
-            hit = np.flatnonzero(tabs["vnode_to_q_entries"][q0:q0 + qn] == rid)
-            if hit.size != 1:
-                raise RuntimeError("internal error: a grouped tail has no partial row of its own")
-            state[rid] = (dst + length, src + length, q0 + int(hit[0]), room)
-            last[rid] = task
-    if min(last, default=0) < 0:
+        groups = groups[np.argsort(kv_offs[groups], kind="stable")]
+        member_of = np.searchsorted(kv_offs[groups] - _planner.AUX_BIT, dst, side="right") - 1
+        # the groups' partial rows as (group, request) keys: a grouped tail has exactly one
+        g_len = q_lens[groups].astype(np.int64)
+        g_start = np.cumsum(g_len) - g_len
+        rows = np.arange(int(g_len.sum())) + np.repeat(q_offs[groups] - g_start, g_len)
+        keys = np.repeat(np.arange(groups.size), g_len) * bsz + q_entries[rows]
+        by_key = np.argsort(keys, kind="stable")
+        want = member_of * bsz + rid
+        lo, hi = (np.searchsorted(keys[by_key], want, side=side) for side in ("left", "right"))
+        if np.any(hi - lo != 1):
+            raise RuntimeError("internal error: a grouped tail has no partial row of its own")
+        state[rid] = np.stack([dst + length, src + length, rows[by_key[lo]], room], axis=1)
+        last[rid] = groups[member_of]
+    if bsz and last.min() < 0:
         raise RuntimeError("internal error: a request has no tail task")
-    for rid in range(len(batch.reqs)):
-        if state[rid, 0] < 0:
-            state[rid, 2] = last[rid]
+    own = state[:, 0] < 0
+    state[own, 2] = last[own]
     tabs["req_to_vnode_entries"] = tabs["req_to_vnode_entries"][:-_planner.PAD_ENTRIES]
     tabs["tail_state"] = state
     return tabs, last
@@ -312,13 +322,13 @@ def prepare_for_fasttree_meta(batch, fasttree_metadata):
     (reference: schedule.py:12-275).  Binds the metadata to the batch."""
     md = fasttree_metadata
     node_to_reqs, covered = _walk_requests(batch)
-    order, offsets, parents = _bfs(batch, node_to_reqs)
-    req_idx = batch.req_pool_indices.cpu()
+    order, offsets, parents, lens = _bfs(batch, node_to_reqs)
+    req_idx = batch.req_pool_indices.tolist()
     stride = batch.req_to_token_pool.req_to_token.stride(0)
     if md.planner == "reference":
-        tabs, last = _plan_reference(batch, md, node_to_reqs, order, offsets, req_idx, stride)
+        tabs, last = _plan_reference(batch, md, node_to_reqs, order, offsets, lens, req_idx, stride)
     else:
-        tabs, last = _plan_b200(batch, md, node_to_reqs, covered, order, offsets, parents, req_idx, stride)
+        tabs, last = _plan_b200(batch, md, node_to_reqs, covered, order, offsets, parents, lens, req_idx, stride)
     _upload(md, tabs, last, tail_state=tabs.get("tail_state"),
             src_table=batch.req_to_token_pool.req_to_token if getattr(md, "group_tails", False) else None)
     batch.fasttree_metadata = md

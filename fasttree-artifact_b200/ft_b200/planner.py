@@ -603,6 +603,7 @@ def b200_split_tail(vnodes, q_tile, small_tile, m, num_kv_heads):
 
 
 def _tree_arrays(tree):
+    """(parent, seqlen, request offsets, request ids) of a tree, as the native splitter takes them."""
     n = len(tree)
     parent = np.fromiter((nd.parent for nd in tree), dtype=np.int32, count=n)
     seqlen = np.fromiter((nd.seqlen for nd in tree), dtype=np.int32, count=n)
@@ -686,15 +687,16 @@ def plan_b200_native(tree, kv_ptrs, batch_size, num_qo_heads, num_kv_heads, head
 
 
 def b200_tables_native_direct(tree, node_base, node_offset, extra, batch_size, num_qo_heads, num_kv_heads, head_dim,
-                              model, tail_room=-1):
+                              model, tail_room=-1, arrays=None):
     """The serving path's tables from the native splitter (``ft_plan_b200_build_direct``): what
     :func:`b200_virtual_nodes` + :func:`emit_tables` (``direct_offsets=True``, ordered by
     :func:`b200_task_order`) produce for a tree whose node i covers positions
     ``[node_base[i] + node_offset[top carried ancestor], node_base[i] + node_offset[i] + seqlen_i)`` of an
     existing row-id table, plus the ``extra`` pairings ``(begin, end, request)``.
+    ``arrays``: :func:`_tree_arrays` of the tree, if at hand.
     Returns (tables dict, request tile, small request tile, tile tokens)."""
     import ctypes
-    parent, seqlen, req_offs, req_ids = _tree_arrays(tree)
+    parent, seqlen, req_offs, req_ids = arrays if arrays is not None else _tree_arrays(tree)
     base = np.ascontiguousarray(np.asarray(node_base, dtype=np.int64))
     offs = np.ascontiguousarray(np.asarray(node_offset, dtype=np.int64))
     ex = np.asarray(extra, dtype=np.int64).reshape(-1, 3)
