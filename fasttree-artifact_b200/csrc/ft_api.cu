@@ -385,17 +385,20 @@ ft::TcParams tc_params(const ft::Stage1Params& p, const ft_decode_args* a) {
 // fit 128 registers (600 requests at 16/1 heads: nothing gained).
 // Head_dim 256, one CTA per SM: one round on the tcgen05 kernel, whose tile loads are the larger (16 leaves of 400 tokens 21.4
 // / 23.7 us with eight warps per task), up to two tasks per SM eight warps each (18 of 400 31.1 / 24.6), two at a time above
-// (60 of 130 47.5 / 30.0, 60 of 1500 144 / 125; 64 requests of 256 tokens on 4096 58 / 42).
-int few_rows_form(const ft::Stage1Params& p, int64_t few_nodes, int64_t wide, int hkv, int head_dim, int64_t slots) {
+// (60 of 130 47.5 / 30.0, 60 of 1500 144 / 125; 64 requests of 256 tokens on 4096 58 / 45) unless many of them must have more
+// than eight rows: the partial rows that the many-row nodes (at most wide_rows) leave over say how many rows they share.
+int few_rows_form(const ft::Stage1Params& p, int64_t few_nodes, int64_t wide, int64_t wide_rows, int hkv, int head_dim, int64_t slots) {
   const int64_t few = few_nodes * hkv;
   if (head_dim == 256) {
     if (p.group > 8 || few + wide <= slots) return -1;
-    return few + wide > 2 * slots ? ft::FEW_PAIR : ft::FEW_EIGHT;
+    const bool small = (p.num_partial_rows - wide_rows) * p.group <= 8 * few_nodes;
+    return few + wide > 2 * slots && small ? ft::FEW_PAIR : ft::FEW_EIGHT;
   }
   if (p.group > 8) return ft::FEW_ONE;
   const int64_t ctas = (few + 1) / 2 + wide;
   if (head_dim == 64) return 5 * ctas >= 8 * slots ? ft::FEW_PAIR : ft::FEW_ONE;
-  return 5 * ctas >= 6 * slots || (ctas >= slots && p.kv_entries_len <= 170 * few_nodes) ? ft::FEW_PAIR : ft::FEW_ONE;
+  if (ctas >= 2 * slots || (5 * ctas >= 6 * slots && p.kv_entries_len <= 320 * few_nodes)) return ft::FEW_PAIR;
+  return ctas >= slots && p.kv_entries_len <= 170 * few_nodes ? ft::FEW_PAIR : ft::FEW_ONE;
 }
 
 template <typename T, int D>
@@ -501,14 +504,14 @@ int launch_fused_as(const ft::TcParams& p, int64_t ctas, cudaStream_t st) {
 }
 
 template <typename T, int D>
-int launch_fused(ft::TcParams p, int hkv, cudaStream_t st) {
+int launch_fused(ft::TcParams p, int hkv, cudaStream_t st, int64_t wide_rows) {
   int dev = 0;
   FT_CUDA_OK(cudaGetDevice(&dev));
   const int64_t wide = (int64_t)p.p.node_split * hkv;
   const int64_t few_nodes = p.p.node_count - p.p.node_split, few = few_nodes * hkv;
   const int64_t slots = (int64_t)ft::TcCfg<D>::CTAS * sm_count(dev);
   p.p.lead_wide = (int)wide;  // many-row CTAs go first
-  p.p.few_form = few_rows_form(p.p, few_nodes, wide, hkv, D, slots);
+  p.p.few_form = few_rows_form(p.p, few_nodes, wide, wide_rows, hkv, D, slots);
   if constexpr (D <= 128) {
     // Few-row tasks by persistent workers only when the many-row CTAs do not fill the device more than once (the workers
     // take the slots those leave and, as they finish, theirs too).
@@ -534,9 +537,7 @@ int launch_tensor(const ft::Stage1Params& p, const ft_decode_args* a, int hkv, c
   FT_CUDA_OK(cudaGetDevice(&dev));
   const int64_t slots = (int64_t)ft::TcCfg<D>::CTAS * sm_count(dev);
   if constexpr (D == 256) {
-    const ft::TcParams tp = tc_params(p, a);
-    const int form = few_rows_form(p, p.node_count, 0, hkv, D, slots);
-    return form < 0 ? launch_tc<T, D>(tp, hkv, st) : launch_narrow<T, D>(tp, hkv, st, form);
+    return launch_fused<T, D>(tc_params(p, a), hkv, st, 0);  // (no many-row phase)
   } else {
     if (max_rows <= 16) {
       const bool many = few_rows_by_workers(p.node_count, p.kv_entries_len, hkv, slots);
@@ -544,7 +545,7 @@ int launch_tensor(const ft::Stage1Params& p, const ft_decode_args* a, int hkv, c
     }
     if (path != FT_PATH_MMA_WIDE && max_rows <= 16)
       return launch_narrow<T, D>(tc_params(p, a), hkv, st,
-                                 path == FT_PATH_AUTO ? few_rows_form(p, p.node_count, 0, hkv, D, slots) : ft::FEW_ONE);
+                                 path == FT_PATH_AUTO ? few_rows_form(p, p.node_count, 0, 0, hkv, D, slots) : ft::FEW_ONE);
     return launch_mma<T, D>(p, hkv, st);
   }
 }
@@ -732,14 +733,15 @@ int ft_stage1(const ft_decode_args* a) {
     p.node_split = n0;
     cudaStream_t st = static_cast<cudaStream_t>(a->stream);
     const ft::TcParams tp = tc_params(p, a);
+    const int64_t wide_rows = (int64_t)n0 * a->phase_q_tile_sizes[0];
     if (a->head_dim == 64)
-      return a->dtype == FT_F16 ? launch_fused<__half, 64>(tp, a->num_kv_heads, st)
-                                : launch_fused<__nv_bfloat16, 64>(tp, a->num_kv_heads, st);
+      return a->dtype == FT_F16 ? launch_fused<__half, 64>(tp, a->num_kv_heads, st, wide_rows)
+                                : launch_fused<__nv_bfloat16, 64>(tp, a->num_kv_heads, st, wide_rows);
     if (a->head_dim == 256)
-      return a->dtype == FT_F16 ? launch_fused<__half, 256>(tp, a->num_kv_heads, st)
-                                : launch_fused<__nv_bfloat16, 256>(tp, a->num_kv_heads, st);
-    return a->dtype == FT_F16 ? launch_fused<__half, 128>(tp, a->num_kv_heads, st)
-                              : launch_fused<__nv_bfloat16, 128>(tp, a->num_kv_heads, st);
+      return a->dtype == FT_F16 ? launch_fused<__half, 256>(tp, a->num_kv_heads, st, wide_rows)
+                                : launch_fused<__nv_bfloat16, 256>(tp, a->num_kv_heads, st, wide_rows);
+    return a->dtype == FT_F16 ? launch_fused<__half, 128>(tp, a->num_kv_heads, st, wide_rows)
+                              : launch_fused<__nv_bfloat16, 128>(tp, a->num_kv_heads, st, wide_rows);
   }
   // Adjacent phases that want the same kernel go out as one grid.
   if (n0 > 0 && n1 > 0 && o1 == o0 + n0 && same_kernel)

@@ -58,7 +58,7 @@ struct SlabCfg {
 template <int D>
 struct PairCfg {
   static constexpr int NS = D == 64 ? 6 : 3;
-  static constexpr int MAX_NQ = D == 256 ? 1 : 2;     // 128 accumulators per thread do not fit: 9 to 16 rows in two passes
+  static constexpr int MAX_NQ = D == 256 ? 1 : 2;     // 128 accumulators per thread do not fit: 9 to 16 rows take two passes
   static constexpr int BODY_BYTES = (SlabCfg<D, MAX_NQ, NS>::bytes(4) + 1023) / 1024 * 1024;
   static constexpr int SMEM_BYTES = 2 * BODY_BYTES;
   static_assert(SlabCfg<D, MAX_NQ, NS>::bytes(8) <= SMEM_BYTES, "eight warps on one task");

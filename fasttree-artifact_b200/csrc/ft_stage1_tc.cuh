@@ -1121,8 +1121,18 @@ __global__ void __launch_bounds__(TcCfg<D>::THREADS, 2) stage1_fused_kernel(cons
   const int few_ctas = PAIR ? (few_tasks + few_per_cta(p.few_form) - 1) / few_per_cta(p.few_form) : p.workers > 0 ? p.workers : few_tasks;
   const int b = (int)blockIdx.x;
   FT_TL_BEGIN();
-  if (b < p.lead_wide || b >= p.lead_wide + few_ctas) {
-    const int task = b < p.lead_wide ? b : b - few_ctas;
+  bool many_rows = b < p.lead_wide || b >= p.lead_wide + few_ctas;
+  int task = b < p.lead_wide ? b : b - few_ctas;
+  if constexpr (D == 256) {
+    // Eight warps per task: a task of more than eight rows, which they would have to run in two passes over K and V, stays
+    // with the tcgen05 body (270 tasks of a five-level tree, 8/2 heads: two passes 61 us, this 44).
+    if (!many_rows && p.few_form == FEW_EIGHT) {
+      task = wide_tasks + b - p.lead_wide;
+      wait_for_prior_grid();
+      many_rows = p.q_lens[p.node_offset + task / H] * p.group > 8;
+    }
+  }
+  if (many_rows) {
     tc_body<T, D, false>(tp, smem, p.node_offset + task / H, task % H);
     FT_TL_END(1);
   } else {
@@ -1140,7 +1150,7 @@ __global__ void __launch_bounds__(TcCfg<D>::THREADS, 2) stage1_fused_kernel(cons
       if (p.workers > 0) {
         stream_worker<T, D>(tp, smem, wide_tasks, few_tasks, w, p.workers);
       } else {
-        const int task = wide_tasks + w;
+        task = wide_tasks + w;
         narrow_dispatch<T, D>(p, smem, p.node_offset + task / H, task % H);
       }
       FT_TL_END(2);
