@@ -323,7 +323,11 @@ def prepare_for_fasttree_meta(batch, fasttree_metadata):
     md = fasttree_metadata
     node_to_reqs, covered = _walk_requests(batch)
     order, offsets, parents, lens = _bfs(batch, node_to_reqs)
-    req_idx = batch.req_pool_indices.tolist()
+    # one row of the table per request; a tensor padded beyond the batch is fine, one that is too short is not
+    req_idx = batch.req_pool_indices[:len(batch.reqs)].cpu().reshape(-1).tolist()
+    if len(req_idx) != len(batch.reqs):
+        raise IndexError(f"req_pool_indices names {len(req_idx)} of {len(batch.reqs)} requests")
+    req_idx = [int(i) for i in req_idx]
     stride = batch.req_to_token_pool.req_to_token.stride(0)
     if md.planner == "reference":
         tabs, last = _plan_reference(batch, md, node_to_reqs, order, offsets, lens, req_idx, stride)

@@ -231,3 +231,23 @@ def test_monkey_patches_and_burst_loop(monkeypatch):
     server.running_batch = None
     server.forward_step()
     assert server.memory_checks == 1
+
+
+@pytest.mark.parametrize("planner", ["reference", "b200"])
+def test_request_indices_beyond_and_short_of_the_batch(planner):
+    """``req_pool_indices`` may be padded beyond the batch, hold one index per row or floats; one that is too short, even
+    by all but one entry, is refused."""
+    def tables(change):
+        batch, _rows, hq, hkv = plugin_cases.build("small_g4")
+        batch.req_pool_indices = change(batch.req_pool_indices)
+        md = make_md(hq, hkv, planner)
+        schedule.prepare_for_fasttree_meta(batch, md)
+        n = len(batch.reqs)
+        return [getattr(md, key)[:n].numpy() for key in KEYS] + [md.tail_state[:n].numpy(), md.req_last_vnodes]
+    want = tables(lambda idx: idx)
+    for change in (lambda idx: torch.cat([idx, idx.new_zeros(3)]), lambda idx: idx.view(-1, 1), lambda idx: idx.double()):
+        for got, exp in zip(tables(change), want):
+            np.testing.assert_array_equal(got, exp)
+    for n in (1, 3):
+        with pytest.raises(IndexError):
+            tables(lambda idx: idx[:n])
