@@ -1008,15 +1008,17 @@ int ft_refresh_tails(const int32_t* tail_state, int32_t n, const int32_t* src_ta
 
 namespace {
 // One warp waits on an mbarrier that nothing ever arrives at, through the same bounded waits the stage-1 kernels
-// use.  No copy, no MMA and no tensor memory is involved, so a wait that runs out leaves nothing in flight.
+// use, and on a completed one with too few probes in some lanes.  No copy, no MMA and no tensor memory is involved, so a wait that runs out leaves nothing in flight.
 __global__ void bounded_wait_selftest_kernel(int limit, int* result) {
-  __shared__ __align__(8) unsigned long long barrier_word;
+  __shared__ __align__(8) unsigned long long barrier_word[2];
   __shared__ int abort_word;
-  const uint32_t bar = ft::smem_u32(&barrier_word);
+  const uint32_t bar = ft::smem_u32(barrier_word), done = bar + 8;
   if (threadIdx.x == 0) {
     ft::mbar_init(bar, 1);
+    ft::mbar_init(done, 1);
     abort_word = 0;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    ft::mbar_arrive(done);
   }
   __syncthreads();
   // (1) the plain bounded wait of the persistent workers: gives up after `limit` probes
@@ -1026,9 +1028,12 @@ __global__ void bounded_wait_selftest_kernel(int limit, int* result) {
   if (threadIdx.x == 0) abort_word = 1;
   __syncthreads();
   const bool aborted = ft::tc_wait(bar, 0, &abort_word);
+  // (3) the few-row bodies' wait by whole warps, on a barrier that has completed: half of the lanes have no probe left,
+  // so all lanes must be told that the wait ran out
+  const bool split = __any_sync(0xffffffffu, ft::mbar_wait_warp(done, 0, threadIdx.x < 16 ? 0 : limit));
   if (threadIdx.x == 0) {
     if (!plain || !aborted) ft::flag_error(FT_DEV_WAIT_TIMEOUT);  // what the kernels do when a wait runs out
-    result[0] = plain ? 1 : 0;
+    result[0] = (plain ? 1 : 0) + (split ? 2 : 0);
     result[1] = aborted ? 1 : 0;
   }
 }

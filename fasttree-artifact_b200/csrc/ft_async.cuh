@@ -80,4 +80,10 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int lim
   return false;
 }
 
+// The same by a whole warp, with one answer for all lanes: "no" if any lane's probes have run out (a barrier that completes
+// at the limit would else split the warp, and its next shuffle would wait for lanes that have left).
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, int limit) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, limit));
+}
+
 }  // namespace ft

@@ -88,6 +88,14 @@ __device__ __forceinline__ void slab_body(const TcParams& tp, uint8_t* smem, con
   const uint32_t ring = q_sm + N::Q_BYTES + warp * N::RING_BYTES;
   auto body_sync = [&]() { asm volatile("bar.sync %0, %1;\n" ::"r"(barrier), "r"(32 * nw) : "memory"); };
 
+  // the same, and whether any thread of the body says yes
+  auto body_any = [&](bool mine) {
+    uint32_t any;
+    asm volatile("{\n\t.reg .pred a, b;\n\tsetp.ne.u32 a, %1, 0;\n\tbar.red.or.pred b, %2, %3, a;\n\tselp.u32 %0, 1, 0, b;\n\t}\n"
+                 : "=r"(any) : "r"((uint32_t)mine), "r"(barrier), "r"(32 * nw) : "memory");
+    return any != 0u;
+  };
+
   // row ids past the end of the table are a plan error: flagged once, those tokens become padding
   const int id_lim = kv_ids_limit(p, kv_off, kv_len);
   const int32_t* ids = kv_ids_base(p, kv_off);
@@ -99,7 +107,7 @@ __device__ __forceinline__ void slab_body(const TcParams& tp, uint8_t* smem, con
   // this warp's slabs: slab j holds tokens span * j + 16 warp ..
   const int span = 16 * nw;
   const int nslabs = kv_len > 16 * warp ? (kv_len - 16 * warp + span - 1) / span : 0;
-  bool bad = false, gathered = false, dead = false;
+  bool bad = false, gathered = false, dead = false;  // (dead: the same in all lanes)
   // one mbarrier per ring slot, one arrival each: lane 0's, with the bytes of a TMA copy or behind the lanes' cp.async copies
   const uint32_t bars = q_sm + N::Q_BYTES + nw * N::RING_BYTES + warp * NS * 8;
   if (N::TMA && lane == 0) {
@@ -123,9 +131,9 @@ __device__ __forceinline__ void slab_body(const TcParams& tp, uint8_t* smem, con
       __syncwarp();
     } else if (pending > 0) {  // (nothing pending: a wait has run out, nothing is issued any more)
       --pending;
-      if (!mbar_wait(bars + 8 * slot_use, phase_use, N::WAIT_LIMIT)) {
+      if (!mbar_wait_warp(bars + 8 * slot_use, phase_use, N::WAIT_LIMIT)) {
         dead = true;
-        flag_error(FT_DEV_WAIT_TIMEOUT);
+        if (lane == 0) flag_error(FT_DEV_WAIT_TIMEOUT);
       }
     }
     const uint32_t at = ring + slot_use * N::SLAB_BYTES;
@@ -348,8 +356,23 @@ __device__ __forceinline__ void slab_body(const TcParams& tp, uint8_t* smem, con
       }
       refill();
     }
-    if constexpr (!N::TMA) cp_async_wait<0>();
-    body_sync();  // rings idle: reuse them as the staging area
+    if constexpr (!N::TMA) {
+      cp_async_wait<0>();
+      body_sync();
+    } else if (body_any(dead)) {
+      // A wait ran out: that warp's copies may still arrive, so nothing is staged over the rings.  The rows left come out
+      // as if no token had been seen; the status word says why.
+      for (int r = row0 + (tid >> 3); r < rows; r += 4 * nw) {
+        const int slot = r / G, head = kvh * G + r - slot * G;
+        const int64_t part = (int64_t)q_off + slot;
+        if (part < 0 || part >= p.num_partial_rows) continue;
+        float4* dst = reinterpret_cast<float4*>(p.mid_o + part * p.mo_s0 + (int64_t)head * p.mo_s1);
+        for (int i = tid & 7; i < D / 4; i += 8) dst[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if ((tid & 7) == 0) p.mid_lse[part * p.ml_s0 + head] = -INFINITY;
+      }
+      return;
+    }
+    // rings idle: reuse them as the staging area
     if (tid == 0) FT_TL_MARK(6);
 
     // ---- stage this warp's (max, sum, O^T) partial

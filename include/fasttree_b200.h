@@ -242,7 +242,8 @@ int ft_read_device_status(void* stream, int32_t* flags);
 
 /* Runs one warp through the bounded mbarrier waits of the stage-1 kernels on a barrier nothing arrives at
  * (limit = probes before the plain wait gives up, 1 .. 2^20) and synchronises.  result_host[0] / [1] receive what
- * the plain wait and the abortable wait returned (0 = gave up, the expected answer); the kernel then raises
+ * the plain wait and the abortable wait returned (0 = gave up, the expected answer; [0] is 2 more if the wait of a whole
+ * warp, with too few probes in half of its lanes, gave them different answers); the kernel then raises
  * FT_DEV_WAIT_TIMEOUT in the device status word, as a stage-1 kernel whose wait ran out does.  No copy engine, tensor
  * core or tensor memory is used.  A health check for the failure-detection path; no counterpart in the reference. */
 int ft_selftest_bounded_wait(int limit, int* result_host, void* stream);
