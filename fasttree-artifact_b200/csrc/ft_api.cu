@@ -374,36 +374,68 @@ ft::TcParams tc_params(const ft::Stage1Params& p, const ft_decode_args* a) {
   return tp;
 }
 
+// What the plan says of its tasks' sizes; longest 0: nothing is known
+struct TaskSizes {
+  int64_t few_tokens = 0;
+  int64_t few_longest = 0, few_over_8_rows = 0, many_longest = 0;
+};
+
+// for a launch whose few-row tasks are phase 1's
+TaskSizes task_sizes(const ft_decode_args* a) {
+  TaskSizes z;
+  if (a->few_tokens > 0 && a->few_longest > 0)
+    z = {a->few_tokens, a->few_longest, a->few_over_8_rows, a->many_longest > 0 ? a->many_longest : 0};
+  return z;
+}
+
 // How the few-row tasks of a launch are run (ft::FEW_*; -1: by the tcgen05 kernel, head_dim 256 only); wide: its many-row CTAs.
-// Two tasks per CTA keep an SM streaming while a task starts up, but they share the SM's copy rate: below about 1.2 CTAs per
-// slot (1.6 at head_dim 64) some SMs hold four tasks and others two, and one task per CTA, dealt out as slots come free, is
-// the better balanced; tasks of about 130 tokens, mostly start-up, gain from one CTA per slot on.  One / two tasks per CTA, us
-// per step, leaves under a 1000-token node, 32/8 heads of 128: 60 of 130 tokens (1.03 CTAs per slot) 19.9 / 18.7, 60 of 400
-// (0.86) 28.2 / 31.9, 74 of 400 (1.16) 33.7 / 35.4, 90 of 400 (1.3) 39.0 / 37.3, 90 of 130 25.4 / 21.2; 64 requests of 256
-// tokens on 4096 (1.4) 27.7 / 25.6; the ragged tree of six levels (8.9) 595 / 546.  Heads of 64: 100 of 300 (1.45) 26.3 /
-// 32.5, 120 of 300 (1.7) 29.6 / 24.2.  More than eight heads per KV head: every task needs the two-block body, which does not
-// fit 128 registers (600 requests at 16/1 heads: nothing gained).
-// Head_dim 256, one CTA per SM: one round on the tcgen05 kernel, whose tile loads are the larger (16 leaves of 400 tokens 21.4
-// / 23.7 us with eight warps per task), up to two tasks per SM eight warps each (18 of 400 31.1 / 24.6), two at a time above
-// (60 of 130 47.5 / 30.0, 60 of 1500 144 / 125; 64 requests of 256 tokens on 4096 58 / 45) unless many of them must have more
-// than eight rows: the partial rows that the many-row nodes (at most wide_rows) leave over say how many rows they share.
-int few_rows_form(const ft::Stage1Params& p, int64_t few_nodes, int64_t wide, int64_t wide_rows, int hkv, int head_dim, int64_t slots) {
-  const int64_t few = few_nodes * hkv;
+// Two tasks per CTA keep an SM streaming while a task starts up, but four then share the SM's copy rate and they are dealt out
+// in pairs.  So they pay where the tasks are many for their longest one (their tokens fill 1.5 rounds of it at four tasks per
+// SM; 1.25 at head_dim 64), or about even, in enough rounds for their length; where few need the two-block body (more than
+// eight rows), which does not fit 128 registers; and where the step does not wait for a many-row chunk, which four neighbours
+// slow down (at head_dim 64 sooner: a token's rows are half as long, a many-row tile takes what it takes at 128).  us per step
+// with one / two tasks per CTA:
+//   head_dim 128  64 leaves of 256 tokens under 4096, 32/8 heads, 27.7 / 25.6, under 16000 40.2 / 37.2; 90 of 400 under 1000
+//                 39.1 / 36.7, 74 of 400 33.8 / 35.0; ragged trees: six levels (many for their longest) 577 / 566, four levels
+//                 58.6 / 81.2; 26 leaves of 275 under chunks of up to 1181, 32/32 heads, 54.5 / 68.4
+//   head_dim 64   448 leaves of 142 under 59, 16/16 heads, 142 / 89; ragged four levels 39.5 / 53.5; 322 leaves of 233 under
+//                 chunks of 7998, 64/8 heads, 139 / 188
+// Head_dim 256, one CTA per SM: one round on the tcgen05 kernel, whose tile loads are the larger.  Beyond it two at a time if
+// none has more than eight rows, which would be two passes over K and V, and they are many for their longest or short (beside
+// many-row CTAs, in whose rounds pairs fit worse, shorter); with eight warps each, and those of more than eight rows on the
+// tcgen05 body, if they are short or make more than two rounds.  us per step on the tcgen05 kernel / two at a time / eight warps each,
+// 16/8 heads: 64 of 256 under 4096 57.1 / 44.9 / 48.1; 60 of 130 under 1000 47.4 / 30.0 / 39.3, 60 of 1500 144 / 126 / 129,
+// 16 of 400 (one round) 21.5 / 23.1 / 24.1; 47 of 280 under 930, one task of 15 rows, 24/8 heads, 46.4 / 80.4 / 44.8; 29 of
+// 335 under 3 of 127 under 2013, 32/8 heads, 37.0 / 40.4 two at a time.
+// The bounds are where the ratio of both sides crosses one over 2700 trees drawn from the benchmark's ranges: the rule takes
+// two tasks (or eight warps) on 117 of 1030 at head_dim 128, 142 of 1085 at 64 and 134 of 628 at 256, which take 15, 21 and
+// 26 % less time for it, and at worst 3, 5 and 3 % more.
+int few_rows_form(const TaskSizes& z, int group, int64_t few_nodes, int64_t wide, int hkv, int head_dim, int64_t slots) {
+  const int64_t few = few_nodes * hkv, longest = z.few_longest, tokens = z.few_tokens * hkv;
+  const int without = head_dim == 256 ? -1 : ft::FEW_ONE;
+  if (longest == 0 || group > 8) return without;
   if (head_dim == 256) {
-    if (p.group > 8 || few + wide <= slots) return -1;
-    const bool small = (p.num_partial_rows - wide_rows) * p.group <= 8 * few_nodes;
-    return few + wide > 2 * slots && small ? ft::FEW_PAIR : ft::FEW_EIGHT;
+    if (few + wide <= slots) return without;
+    const int64_t short_of = 4 * wide <= slots ? 400 : 256;
+    if (z.few_over_8_rows == 0 && z.many_longest * slots <= 4 * tokens && (longest <= short_of || tokens >= 2 * slots * longest))
+      return ft::FEW_PAIR;
+    const bool brief = longest <= 320 && 8 * z.few_over_8_rows <= few_nodes && 5 * wide <= 3 * slots;
+    return 5 * few > 12 * slots || brief ? ft::FEW_EIGHT : without;
   }
-  if (p.group > 8) return ft::FEW_ONE;
-  const int64_t ctas = (few + 1) / 2 + wide;
-  if (head_dim == 64) return 5 * ctas >= 8 * slots ? ft::FEW_PAIR : ft::FEW_ONE;
-  if (ctas >= 2 * slots || (5 * ctas >= 6 * slots && p.kv_entries_len <= 320 * few_nodes)) return ft::FEW_PAIR;
-  return ctas >= slots && p.kv_entries_len <= 170 * few_nodes ? ft::FEW_PAIR : ft::FEW_ONE;
+  if (4 * z.few_over_8_rows > few_nodes) return without;
+  const bool even = 4 * longest * few_nodes <= 5 * z.few_tokens;
+  bool two;
+  if (head_dim == 64)
+    two = z.many_longest * slots <= tokens && (2 * tokens >= 5 * slots * longest || (even && few >= 2 * slots && longest <= 512));
+  else
+    two = z.many_longest * slots <= 4 * tokens &&
+          (tokens >= 3 * slots * longest || (even && (5 * few >= 12 * slots ? longest <= 640 : 5 * few >= 8 * slots && longest <= 320)));
+  return two ? ft::FEW_PAIR : without;
 }
 
 template <typename T, int D>
 int launch_narrow(ft::TcParams p, int hkv, cudaStream_t st, int form) {
-  if (dry_run("stage1_narrow_kernel")) return FT_OK;
+  if (dry_run(form == ft::FEW_ONE ? "stage1_narrow_kernel" : "stage1_narrow_kernel/pair")) return FT_OK;
   const int64_t tasks = (int64_t)p.p.node_count * hkv;
   if constexpr (D <= 128) {
     if (form == ft::FEW_ONE) {
@@ -494,7 +526,8 @@ int launch_fused_as(const ft::TcParams& p, int64_t ctas, cudaStream_t st) {
   }();
   constexpr int smem = std::max(ft::TcCfg<D>::SMEM_BYTES, few_smem);
   static_assert(smem <= (D == 256 ? 232448 : 115712), "the resident CTAs must fit in one SM's shared memory");
-  if (dry_run("stage1_fused_kernel")) return FT_OK;
+  if (dry_run(!PAIR ? "stage1_fused_kernel" : p.p.few_form == ft::FEW_PAIR ? "stage1_fused_kernel/pair" : "stage1_fused_kernel/eight"))
+    return FT_OK;
   if (ctas > 0x7fffffffLL) return fail(FT_ERR_TOO_LARGE, "vnodes x kv heads exceeds the grid limit");
   static OncePerDevice once;
   FT_CUDA_OK(raise_smem_limit(once, ft::stage1_fused_kernel<T, D, PAIR>, smem));
@@ -504,14 +537,14 @@ int launch_fused_as(const ft::TcParams& p, int64_t ctas, cudaStream_t st) {
 }
 
 template <typename T, int D>
-int launch_fused(ft::TcParams p, int hkv, cudaStream_t st, int64_t wide_rows) {
+int launch_fused(ft::TcParams p, const TaskSizes& sizes, int hkv, cudaStream_t st) {
   int dev = 0;
   FT_CUDA_OK(cudaGetDevice(&dev));
   const int64_t wide = (int64_t)p.p.node_split * hkv;
   const int64_t few_nodes = p.p.node_count - p.p.node_split, few = few_nodes * hkv;
   const int64_t slots = (int64_t)ft::TcCfg<D>::CTAS * sm_count(dev);
   p.p.lead_wide = (int)wide;  // many-row CTAs go first
-  p.p.few_form = few_rows_form(p.p, few_nodes, wide, wide_rows, hkv, D, slots);
+  p.p.few_form = few_rows_form(sizes, p.p.group, few_nodes, wide, hkv, D, slots);
   if constexpr (D <= 128) {
     // Few-row tasks by persistent workers only when the many-row CTAs do not fill the device more than once (the workers
     // take the slots those leave and, as they finish, theirs too).
@@ -531,13 +564,14 @@ int launch_fused(ft::TcParams p, int hkv, cudaStream_t st, int64_t wide_rows) {
 // TCGEN05 (tcgen05 for everything)
 template <typename T, int D>
 int launch_tensor(const ft::Stage1Params& p, const ft_decode_args* a, int hkv, cudaStream_t st, int max_rows, int path) {
+  const TaskSizes sizes = p.node_offset == a->phase_node_offsets[1] && p.node_count == a->phase_node_nums[1] ? task_sizes(a) : TaskSizes();
   if (path == FT_PATH_TCGEN05 || ((path == FT_PATH_AUTO || path == FT_PATH_STREAM) && max_rows > 16))
     return launch_tc<T, D>(tc_params(p, a), hkv, st);
   int dev = 0;
   FT_CUDA_OK(cudaGetDevice(&dev));
   const int64_t slots = (int64_t)ft::TcCfg<D>::CTAS * sm_count(dev);
   if constexpr (D == 256) {
-    return launch_fused<T, D>(tc_params(p, a), hkv, st, 0);  // (no many-row phase)
+    return launch_fused<T, D>(tc_params(p, a), sizes, hkv, st);  // (no many-row phase)
   } else {
     if (max_rows <= 16) {
       const bool many = few_rows_by_workers(p.node_count, p.kv_entries_len, hkv, slots);
@@ -545,7 +579,7 @@ int launch_tensor(const ft::Stage1Params& p, const ft_decode_args* a, int hkv, c
     }
     if (path != FT_PATH_MMA_WIDE && max_rows <= 16)
       return launch_narrow<T, D>(tc_params(p, a), hkv, st,
-                                 path == FT_PATH_AUTO ? few_rows_form(p, p.node_count, 0, 0, hkv, D, slots) : ft::FEW_ONE);
+                                 path == FT_PATH_AUTO ? few_rows_form(sizes, p.group, p.node_count, 0, hkv, D, slots) : ft::FEW_ONE);
     return launch_mma<T, D>(p, hkv, st);
   }
 }
@@ -733,15 +767,15 @@ int ft_stage1(const ft_decode_args* a) {
     p.node_split = n0;
     cudaStream_t st = static_cast<cudaStream_t>(a->stream);
     const ft::TcParams tp = tc_params(p, a);
-    const int64_t wide_rows = (int64_t)n0 * a->phase_q_tile_sizes[0];
+    const TaskSizes sizes = task_sizes(a);
     if (a->head_dim == 64)
-      return a->dtype == FT_F16 ? launch_fused<__half, 64>(tp, a->num_kv_heads, st, wide_rows)
-                                : launch_fused<__nv_bfloat16, 64>(tp, a->num_kv_heads, st, wide_rows);
+      return a->dtype == FT_F16 ? launch_fused<__half, 64>(tp, sizes, a->num_kv_heads, st)
+                                : launch_fused<__nv_bfloat16, 64>(tp, sizes, a->num_kv_heads, st);
     if (a->head_dim == 256)
-      return a->dtype == FT_F16 ? launch_fused<__half, 256>(tp, a->num_kv_heads, st, wide_rows)
-                                : launch_fused<__nv_bfloat16, 256>(tp, a->num_kv_heads, st, wide_rows);
-    return a->dtype == FT_F16 ? launch_fused<__half, 128>(tp, a->num_kv_heads, st, wide_rows)
-                              : launch_fused<__nv_bfloat16, 128>(tp, a->num_kv_heads, st, wide_rows);
+      return a->dtype == FT_F16 ? launch_fused<__half, 256>(tp, sizes, a->num_kv_heads, st)
+                                : launch_fused<__nv_bfloat16, 256>(tp, sizes, a->num_kv_heads, st);
+    return a->dtype == FT_F16 ? launch_fused<__half, 128>(tp, sizes, a->num_kv_heads, st)
+                              : launch_fused<__nv_bfloat16, 128>(tp, sizes, a->num_kv_heads, st);
   }
   // Adjacent phases that want the same kernel go out as one grid.
   if (n0 > 0 && n1 > 0 && o1 == o0 + n0 && same_kernel)

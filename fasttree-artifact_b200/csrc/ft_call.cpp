@@ -66,6 +66,25 @@ void pair(const char* name, PyObject* o, int64_t (&out)[2]) {
   Py_DECREF(seq);
 }
 
+// The task sizes that a plan's phase_node_nums carries (ft_b200.planner.PhaseNodeNums); a plain list or tuple has none.
+void task_sizes(PyObject* o, ft_decode_args& a) {
+  if (PyList_CheckExact(o) || PyTuple_CheckExact(o)) return;
+  PyObject* sizes = PyObject_GetAttrString(o, "task_sizes");
+  if (sizes == nullptr) {
+    PyErr_Clear();
+    return;
+  }
+  long long n[4] = {0, 0, 0, 0};
+  const bool ok = PyTuple_Check(sizes) && PyTuple_GET_SIZE(sizes) == 4;
+  for (int i = 0; ok && i < 4; ++i) n[i] = PyLong_AsLongLong(PyTuple_GET_ITEM(sizes, i));
+  Py_DECREF(sizes);
+  if (PyErr_Occurred()) throw Refused();
+  a.few_tokens = n[0];
+  a.few_longest = (int32_t)n[1];
+  a.few_over_8_rows = (int32_t)n[2];
+  a.many_longest = (int32_t)n[3];
+}
+
 // Positional arguments of the reference's fasttree_decode (kernel_bench/fasttree.py:582-601), in order.
 enum { Q, K, V, O, KV_ENTRIES, KV_OFFS, KV_LENS, Q_ENTRIES, Q_OFFS, Q_LENS, R2V_ENTRIES, R2V_OFFS, R2V_LENS, MID_O, MID_LSE,
        NODE_NUMS, NODE_OFFSETS, Q_TILES, KV_TILES, SM_SCALE, N_ARGS };
@@ -113,6 +132,7 @@ void fill(PyObject* const* x, ft_decode_args& a, c10::DeviceIndex& device) {
   }
   int64_t nums[2], offs[2], q_tiles[2], kv_tiles[2];
   pair("phase_node_nums", arg(NODE_NUMS), nums);
+  task_sizes(arg(NODE_NUMS), a);
   pair("phase_node_offsets", arg(NODE_OFFSETS), offs);
   pair("phase_q_tile_sizes", arg(Q_TILES), q_tiles);
   pair("phase_kv_tile_sizes", arg(KV_TILES), kv_tiles);

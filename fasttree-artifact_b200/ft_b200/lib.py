@@ -85,6 +85,8 @@ class DecodeArgs(ctypes.Structure):
         ("device_phase_info", ctypes.c_void_p),
         ("vnode_to_kv_entries_aux", ctypes.c_void_p),
         ("kv_entries_aux_len", ctypes.c_int64),
+        ("few_tokens", ctypes.c_int64), ("few_longest", ctypes.c_int32), ("few_over_8_rows", ctypes.c_int32),
+        ("many_longest", ctypes.c_int32),
     ]
 
 

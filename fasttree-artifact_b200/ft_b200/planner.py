@@ -81,6 +81,22 @@ class Plan:
                 self.req_to_vnode_entries, self.req_to_vnode_offs, self.req_to_vnode_lens)
 
 
+class PhaseNodeNums(list):
+    """``phase_node_nums`` of a plan, with the task sizes that the launch chooses between its kernels by and cannot read from
+    the device tables: ``task_sizes = (tokens of phase 1's chunks together, the longest of them, vnodes of phase 1 with more
+    than 8 query rows, longest chunk of phase 0)``.  A plain list in its place works too; the launch then assumes nothing."""
+
+    def __init__(self, nums, kv_lens=None, q_lens=None, group=1):
+        """``kv_lens`` / ``q_lens``: the plan's ``vnode_to_kv_lens`` / ``vnode_to_q_lens`` (phase 0 first, as emitted)."""
+        super().__init__(nums)
+        self.task_sizes = (0, 0, 0, 0)
+        if kv_lens is not None:
+            n0, n1 = nums
+            many, few = kv_lens[:n0], kv_lens[n0:n0 + n1]
+            self.task_sizes = (int(few.sum(dtype=np.int64)), int(few.max(initial=0)),
+                               int(np.count_nonzero(q_lens[n0:n0 + n1].astype(np.int64) * group > 8)), int(many.max(initial=0)))
+
+
 # --------------------------------------------------------------------- emitter
 def emit_tables(vnodes, batch_size, small_tile, order_key=None, order_out=None, direct_offsets=False):
     """Cut every virtual node into (KV chunk x request tile) tasks and build the

@@ -144,6 +144,11 @@ typedef struct ft_decode_args {
                                          serving plan has one few-row task per request tail
                                          (fasttree_sglang_plugin_v0_2_13/schedule.py:212-232). */
   int64_t kv_entries_aux_len;         /* readable entries of vnode_to_kv_entries_aux */
+  int64_t few_tokens;                 /* sizes of the plan's tasks, which the host cannot read from the device tables: */
+  int32_t few_longest;                /* tokens of phase 1's chunks together, the longest of them, how many of its vnodes */
+  int32_t few_over_8_rows;            /* have more than 8 query rows, the longest chunk of phase 0.  They choose between */
+  int32_t many_longest;               /* ways to run phase 1 with the same results; few_longest 0 = unknown: one task per
+                                         CTA (head_dim 256: the tcgen05 kernel for both phases) */
 } ft_decode_args;
 
 /* Library version (major*10000 + minor*100 + patch). */

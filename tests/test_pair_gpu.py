@@ -1,19 +1,27 @@
 """Few-row tasks two to a CTA (and, at head_dim 256, one by eight warps), on their own and beside many-row tasks in one grid,
-against the CPU oracle's partials.  Chunk lengths around the slabs of 16 tokens and the 64 or 128 tokens that a body's warps
-take per turn; consecutive rows, scattered rows and both in one chunk; 1 to 16 query rows.  Tolerances as in
-test_decode_gpu.py."""
+against the CPU oracle's partials; and which plans take them.  Chunk lengths around the slabs of 16 tokens and the 64 or 128
+tokens that a body's warps take per turn; consecutive rows, scattered rows and both in one chunk; 1 to 16 query rows, so
+that at head_dim 256 a body runs one pass and two.  The task sizes a plan states choose the form and nothing else: each case
+states what brings its form about and asserts it.  Tolerances as in test_decode_gpu.py."""
 import numpy as np
 import pytest
 import torch
 
+import fasttree
+import gpu_utils
+import kv_tree_simple
+import tree_generation
 from oracle import ref_attention
 from test_decode_gpu import ATOL16
 
 from ft_b200 import engine, lib
+from ft_b200.planner import PhaseNodeNums
 
 pytestmark = pytest.mark.gpu
 
 LENS = [1, 2, 15, 16, 17, 31, 33, 47, 48, 49, 63, 64, 65, 112, 113, 127, 128, 129, 191, 193, 255, 256, 257, 320, 400]
+FEW = 31
+SIZES = {"one": (0, 0, 0, 0), "pair": (10 ** 9, 1, 0, 0), "eight": (1, 1, 1, 1)}
 
 
 def _plan(few, many, group, seed):
@@ -36,14 +44,12 @@ def _plan(few, many, group, seed):
     return rows, [np.concatenate(entries), off(lens), np.array(lens), q_entries, off(qs), np.array(qs)]
 
 
-@pytest.mark.parametrize("d,few", [(64, 130), (128, 130), (256, 130), (256, 31)], ids=["64", "128", "256", "256-eight"])
+@pytest.mark.parametrize("d,form", [(64, "pair"), (128, "pair"), (256, "pair"), (256, "eight")])
 @pytest.mark.parametrize("many", [0, 2])
 @pytest.mark.parametrize("group,hkv,dtype", [(1, 8, torch.bfloat16), (4, 8, torch.float16), (7, 8, torch.float16)])
 @pytest.mark.parametrize("extra", ["", "ranges", "bad_id"])
-def test_few_row_tasks(d, few, many, group, hkv, dtype, extra):
-    if few == 130 and (few * hkv // 2) * 5 < 8 * 296:
-        hkv = 8 * -(-8 * 296 // (5 * few * 4))
-    rows, tabs = _plan(few, many, group, seed=d + group)
+def test_few_row_tasks(d, form, many, group, hkv, dtype, extra):
+    rows, tabs = _plan(FEW, many, group, seed=d + group)
     gen = torch.Generator().manual_seed(group)
     k, v = (torch.randn(rows, hkv, d, generator=gen).to(dtype) for _ in range(2))
     q = (torch.randn(64, hkv * group, d, generator=gen) * 0.5).to(dtype)
@@ -58,9 +64,13 @@ def test_few_row_tasks(d, few, many, group, hkv, dtype, extra):
     mid_o, mid_lse = torch.full((parts, hkv * group, d), float("nan"), device="cuda"), torch.empty(parts, hkv * group, device="cuda")
     none = torch.zeros(64, dtype=torch.int32, device="cuda")
     qd = q.cuda()
-    engine.stage1(qd, k.cuda(), v.cuda(), torch.empty_like(qd), *dev, none, none, none, mid_o, mid_lse, [many, few], [0, many],
-                  [40, max(1, 16 // group)], [64, 64], d ** -0.5,
-                  row_ranges=None if ranges is None else torch.from_numpy(ranges.astype(np.int32)).cuda())
+    nums = PhaseNodeNums([many, FEW])
+    nums.task_sizes = SIZES[form]
+    args = (qd, k.cuda(), v.cuda(), torch.empty_like(qd), *dev, none, none, none, mid_o, mid_lse, nums, [0, many],
+            [40, max(1, 16 // group)], [64, 64], d ** -0.5)
+    kernel = "stage1_fused_kernel" if many or d == 256 else "stage1_narrow_kernel"
+    assert engine.stage1_path_name(*args) == f"{kernel}/{form}"
+    engine.stage1(*args, row_ranges=None if ranges is None else torch.from_numpy(ranges.astype(np.int32)).cuda())
     torch.cuda.synchronize()
     assert lib.read_device_status() == (lib.FT_DEV_BAD_KV_INDEX if extra == "bad_id" else 0)
     want_o, want_lse = ref_attention.stage1_partials(q, k, v, *tabs, d ** -0.5, q_ranges=ranges)
@@ -70,3 +80,43 @@ def test_few_row_tasks(d, few, many, group, hkv, dtype, extra):
     tol = ATOL16 + (float(want_o.abs().max()) * 2 ** -8 if dtype == torch.bfloat16 else 0.0)
     torch.testing.assert_close(mid_lse.cpu(), want_lse, rtol=1e-4, atol=2e-5)
     assert (mid_o.cpu() - want_o).abs().max().item() <= tol
+
+
+ONE, PAIR, EIGHT, TC = "stage1_fused_kernel", "stage1_fused_kernel/pair", "stage1_fused_kernel/eight", "stage1_tc_kernel"
+
+
+@pytest.mark.parametrize("tree,hq,hkv,d,want", [
+    (("1,64", "4096,256"), 32, 8, 128, PAIR),            # even leaves in two rounds, whatever the prefix's length
+    (("1,64", "8192,256"), 32, 8, 128, PAIR),
+    (("1,8", "4096,256"), 32, 8, 128, ONE),              # too few
+    (("1,74", "1000,400"), 32, 8, 128, ONE),             # too few for their length
+    (("1,90", "1000,400"), 32, 8, 128, PAIR),
+    ((5, 51848), 64, 8, 128, ONE),                       # ragged and long, 2.7 rounds
+    ((4, 28143), 32, 8, 64, ONE),
+    (("1,10,322", "7998,1052,233"), 64, 8, 64, ONE),     # the step waits for many-row chunks of 7998 tokens
+    (("1,59,448", "16,59,142"), 16, 16, 64, PAIR),
+    (("1,64", "4096,256"), 16, 8, 256, PAIR),
+    (("1,47", "930,280"), 24, 8, 256, EIGHT),            # one of the tasks has 15 rows: two passes for eight, one on tcgen05
+    (("1,12,24,48", "2000,400,300,200"), 64, 8, 256, EIGHT),
+    (("1,18", "1000,400"), 16, 8, 256, PAIR),
+    (("1,16", "1000,400"), 16, 8, 256, TC),              # one round
+    (("1,9", "11165,203"), 32, 8, 256, TC),              # a round and a quarter, most of it many-row
+    (("1,2,4", "16011,518,10"), 32, 8, 256, TC),         # long tasks
+], ids=lambda x: "-".join(map(str, x)).replace(",", ".") if isinstance(x, tuple) else str(x).replace("stage1_", ""))
+def test_which_plans_take_two_tasks_per_cta(tree, hq, hkv, d, want):
+    assert torch.cuda.get_device_properties(0).multi_processor_count == 148
+    if isinstance(tree[0], int):
+        rows = tree_generation.generate_random_tree(*tree)
+    else:
+        rows = tree_generation.generate_tree(*([int(x) for x in t.split(",")] for t in tree))
+    nodes = kv_tree_simple.tree_from_rows(rows)
+    batch, ptrs = kv_tree_simple.assign_requests(nodes)
+    params = gpu_utils.make_params(hq, hkv, [max(1, 64 * hkv // hq), max(1, 16 * hkv // hq)], "b200")
+    params.set_kv_dtype(torch.float16)
+    aux, _ = fasttree.fasttree_preparation(nodes, ptrs, batch, hq, hkv, d, [1024, 128], [132, 528], [132, 132], params)
+    q = torch.zeros(batch, hq, d, dtype=torch.float16, device="cuda")
+    kv = torch.zeros(ptrs[-1], hkv, d, dtype=torch.float16, device="cuda")
+    name = lambda aux: engine.stage1_path_name(q, kv, kv, torch.empty_like(q), *aux, params.TSQs, params.TSKs, d ** -0.5)
+    assert name(aux) == want
+    # a plan that does not state its sizes, as one made by hand: nothing is assumed
+    assert name(aux[:11] + (list(aux[11]),) + aux[12:]) == (TC if d == 256 else ONE)
