@@ -294,7 +294,8 @@ struct MapKey {
 // box_rows, 128-byte swizzle; with box_heads 0 the same tensor as [rows, all elements of a row] with a box of 64 x 1,
 // the form that gathers rows.  Descriptors are cached by buffer identity (encoding one costs about a microsecond)
 // in a hash table of 1024 slots, probed linearly over 8 slots; a full neighbourhood evicts its first slot.  A
-// serving process holds four descriptors per layer's K/V buffers plus two per query shape - a few hundred at most.
+// serving process holds four descriptors per layer's K/V buffers (six at head_dim 256) plus two per query shape - a few
+// hundred at most.
 bool tensor_map(CUtensorMap* out, const void* base, int dtype, int head_dim, int64_t rows, int heads, int64_t s0,
                    int64_t s1, int box_heads, int box_rows) {
   constexpr int SLOTS = 1024, PROBES = 8;
@@ -350,11 +351,7 @@ ft::TcParams tc_params(const ft::Stage1Params& p, const ft_decode_args* a) {
   tp.has_tma = tensor_map(&tp.k_map, a->k_buffer, a->dtype, d, a->kv_rows, a->num_kv_heads, a->k_stride0,
                              a->k_stride1, 1, 64) &&
                tensor_map(&tp.v_map, a->v_buffer, a->dtype, d, a->kv_rows, a->num_kv_heads, a->v_stride0,
-                             a->v_stride1, 1, 64) &&
-               tensor_map(&tp.k_slab_map, a->k_buffer, a->dtype, d, a->kv_rows, a->num_kv_heads, a->k_stride0,
-                             a->k_stride1, 1, 16) &&
-               tensor_map(&tp.v_slab_map, a->v_buffer, a->dtype, d, a->kv_rows, a->num_kv_heads, a->v_stride0,
-                             a->v_stride1, 1, 16);
+                             a->v_stride1, 1, 64);
   tp.has_gather4 = tp.has_tma &&
                    tensor_map(&tp.k_rows_map, a->k_buffer, a->dtype, d, a->kv_rows, a->num_kv_heads, a->k_stride0,
                                  a->k_stride1, 0, 1) &&
@@ -433,28 +430,23 @@ int few_rows_form(const TaskSizes& z, int group, int64_t few_nodes, int64_t wide
   return two ? ft::FEW_PAIR : without;
 }
 
+// few-row tasks alone, at head_dim 64 or 128
 template <typename T, int D>
-int launch_narrow(ft::TcParams p, int hkv, cudaStream_t st, int form) {
-  if (dry_run(form == ft::FEW_ONE ? "stage1_narrow_kernel" : "stage1_narrow_kernel/pair")) return FT_OK;
-  const int64_t tasks = (int64_t)p.p.node_count * hkv;
-  if constexpr (D <= 128) {
-    if (form == ft::FEW_ONE) {
-      using C = ft::NarrowCfg<D, 2>;
-      static OncePerDevice once;
-      void (*kernel)(ft::Stage1Params) = ft::stage1_narrow_kernel<T, D>;
-      FT_CUDA_OK(raise_smem_limit(once, kernel, C::SMEM_BYTES));
-      FT_CUDA_OK(launch_early(kernel, (unsigned)tasks, 128, C::SMEM_BYTES, st, p.p));
-      count_launch();
-      return FT_OK;
-    }
+int launch_narrow(const ft::Stage1Params& p, int hkv, cudaStream_t st, int form) {
+  const bool pair = form == ft::FEW_PAIR;
+  if (dry_run(pair ? "stage1_pair_kernel" : "stage1_narrow_kernel")) return FT_OK;
+  const int64_t tasks = (int64_t)p.node_count * hkv;
+  if (pair) {
+    using C = ft::PairCfg<D>;
+    static OncePerDevice once;
+    FT_CUDA_OK(raise_smem_limit(once, ft::stage1_pair_kernel<T, D>, C::SMEM_BYTES));
+    FT_CUDA_OK(launch_early(ft::stage1_pair_kernel<T, D>, (unsigned)((tasks + 1) / 2), C::THREADS, C::SMEM_BYTES, st, p));
+  } else {
+    using C = ft::NarrowCfg<D, 2>;
+    static OncePerDevice once;
+    FT_CUDA_OK(raise_smem_limit(once, ft::stage1_narrow_kernel<T, D>, C::SMEM_BYTES));
+    FT_CUDA_OK(launch_early(ft::stage1_narrow_kernel<T, D>, (unsigned)tasks, 128, C::SMEM_BYTES, st, p));
   }
-  using C = ft::PairCfg<D>;
-  static OncePerDevice once;
-  void (*kernel)(ft::TcParams) = ft::stage1_narrow_kernel<T, D>;
-  FT_CUDA_OK(raise_smem_limit(once, kernel, C::SMEM_BYTES));
-  p.p.few_form = form;
-  const int per = ft::few_per_cta(form);
-  FT_CUDA_OK(launch_early(kernel, (unsigned)((tasks + per - 1) / per), C::THREADS, C::SMEM_BYTES, st, p));
   count_launch();
   return FT_OK;
 }
@@ -519,7 +511,7 @@ bool few_rows_by_workers(int64_t few_nodes, int64_t kv_entries_len, int hkv, int
 }
 
 template <typename T, int D, bool PAIR>
-int launch_fused_as(const ft::TcParams& p, int64_t ctas, cudaStream_t st) {
+int launch_fused_as(const ft::FusedParams<D, PAIR>& p, int64_t ctas, cudaStream_t st) {
   constexpr int few_smem = [] {
     if constexpr (PAIR) return ft::PairCfg<D>::SMEM_BYTES;
     else return std::max(ft::StreamCfg<D>::SMEM_BYTES, ft::NarrowCfg<D, 2>::SMEM_BYTES);
@@ -537,7 +529,7 @@ int launch_fused_as(const ft::TcParams& p, int64_t ctas, cudaStream_t st) {
 }
 
 template <typename T, int D>
-int launch_fused(ft::TcParams p, const TaskSizes& sizes, int hkv, cudaStream_t st) {
+int launch_fused(ft::TcParams p, const ft_decode_args* a, const TaskSizes& sizes, int hkv, cudaStream_t st) {
   int dev = 0;
   FT_CUDA_OK(cudaGetDevice(&dev));
   const int64_t wide = (int64_t)p.p.node_split * hkv;
@@ -556,7 +548,17 @@ int launch_fused(ft::TcParams p, const TaskSizes& sizes, int hkv, cudaStream_t s
   }
   if (p.p.few_form < 0) return launch_tc<T, D>(p, hkv, st);  // the whole range on the tcgen05 kernel
   const int per = ft::few_per_cta(p.p.few_form);
-  return launch_fused_as<T, D, true>(p, wide + (few + per - 1) / per, st);
+  const int64_t ctas = wide + (few + per - 1) / per;
+  if constexpr (D == 256) {
+    ft::SlabParams sp;
+    memset(&sp, 0, sizeof(sp));
+    static_cast<ft::TcParams&>(sp) = p;
+    sp.has_slabs = tensor_map(&sp.k_slab_map, a->k_buffer, a->dtype, D, a->kv_rows, hkv, a->k_stride0, a->k_stride1, 1, 16) &&
+                   tensor_map(&sp.v_slab_map, a->v_buffer, a->dtype, D, a->kv_rows, hkv, a->v_stride0, a->v_stride1, 1, 16);
+    return launch_fused_as<T, D, true>(sp, ctas, st);
+  } else {
+    return launch_fused_as<T, D, true>(p, ctas, st);
+  }
 }
 
 // path: AUTO (<= 16 rows: persistent workers or narrow, in the form few_rows_form chooses; above: tcgen05),
@@ -571,14 +573,14 @@ int launch_tensor(const ft::Stage1Params& p, const ft_decode_args* a, int hkv, c
   FT_CUDA_OK(cudaGetDevice(&dev));
   const int64_t slots = (int64_t)ft::TcCfg<D>::CTAS * sm_count(dev);
   if constexpr (D == 256) {
-    return launch_fused<T, D>(tc_params(p, a), sizes, hkv, st);  // (no many-row phase)
+    return launch_fused<T, D>(tc_params(p, a), a, sizes, hkv, st);  // (no many-row phase)
   } else {
     if (max_rows <= 16) {
       const bool many = few_rows_by_workers(p.node_count, p.kv_entries_len, hkv, slots);
       if (path == FT_PATH_STREAM || (path == FT_PATH_AUTO && many)) return launch_stream<T, D>(tc_params(p, a), hkv, st);
     }
     if (path != FT_PATH_MMA_WIDE && max_rows <= 16)
-      return launch_narrow<T, D>(tc_params(p, a), hkv, st,
+      return launch_narrow<T, D>(p, hkv, st,
                                  path == FT_PATH_AUTO ? few_rows_form(sizes, p.group, p.node_count, 0, hkv, D, slots) : ft::FEW_ONE);
     return launch_mma<T, D>(p, hkv, st);
   }
@@ -769,13 +771,13 @@ int ft_stage1(const ft_decode_args* a) {
     const ft::TcParams tp = tc_params(p, a);
     const TaskSizes sizes = task_sizes(a);
     if (a->head_dim == 64)
-      return a->dtype == FT_F16 ? launch_fused<__half, 64>(tp, sizes, a->num_kv_heads, st)
-                                : launch_fused<__nv_bfloat16, 64>(tp, sizes, a->num_kv_heads, st);
+      return a->dtype == FT_F16 ? launch_fused<__half, 64>(tp, a, sizes, a->num_kv_heads, st)
+                                : launch_fused<__nv_bfloat16, 64>(tp, a, sizes, a->num_kv_heads, st);
     if (a->head_dim == 256)
-      return a->dtype == FT_F16 ? launch_fused<__half, 256>(tp, sizes, a->num_kv_heads, st)
-                                : launch_fused<__nv_bfloat16, 256>(tp, sizes, a->num_kv_heads, st);
-    return a->dtype == FT_F16 ? launch_fused<__half, 128>(tp, sizes, a->num_kv_heads, st)
-                              : launch_fused<__nv_bfloat16, 128>(tp, sizes, a->num_kv_heads, st);
+      return a->dtype == FT_F16 ? launch_fused<__half, 256>(tp, a, sizes, a->num_kv_heads, st)
+                                : launch_fused<__nv_bfloat16, 256>(tp, a, sizes, a->num_kv_heads, st);
+    return a->dtype == FT_F16 ? launch_fused<__half, 128>(tp, a, sizes, a->num_kv_heads, st)
+                              : launch_fused<__nv_bfloat16, 128>(tp, a, sizes, a->num_kv_heads, st);
   }
   // Adjacent phases that want the same kernel go out as one grid.
   if (n0 > 0 && n1 > 0 && o1 == o0 + n0 && same_kernel)

@@ -17,14 +17,23 @@ struct alignas(64) TcParams {
   CUtensorMap q_map_tile;  // same tensor, box 64 x G x 128 / G: a whole Q tile of consecutive requests
   CUtensorMap k_rows_map;  // K and V as [rows, all heads' elements], box 64 x 1: rows picked one by one (tile::gather4)
   CUtensorMap v_rows_map;
-  CUtensorMap k_slab_map;  // K and V like k_map, box 64 x 1 x 16: the few-row kernel's slabs
-  CUtensorMap v_slab_map;
   Stage1Params p;
   int has_tma;
   int has_gather4;    // the two row maps are valid
   int q_box_rows;     // 0: gather Q with cp.async (group size above 128, or no descriptor)
   unsigned int* sched;  // persistent kernel: {tasks claimed beyond the first per CTA, CTAs finished}, zero between launches
 };
+
+// the same for a launch whose few-row tasks read slabs by TMA (head_dim 256)
+struct SlabParams : TcParams {
+  CUtensorMap k_slab_map;  // K and V like k_map, box 64 x 1 x 16
+  CUtensorMap v_slab_map;
+  int has_slabs;
+};
+
+// the common parameters of any parameter block
+__device__ __forceinline__ const Stage1Params& stage1_of(const Stage1Params& p) { return p; }
+__device__ __forceinline__ const Stage1Params& stage1_of(const TcParams& tp) { return tp.p; }
 
 __device__ __forceinline__ void proxy_fence() { asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory"); }
 

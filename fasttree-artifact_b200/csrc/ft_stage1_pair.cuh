@@ -21,12 +21,17 @@
 // during which its slot of the SM streams nothing.  Two bodies per CTA put four
 // tasks on an SM instead of two, each with half of the shared memory, so that one
 // task's start-up runs under the others' streaming.
+//
+// The price is 128 registers per thread: the two-block body (9 to 16 rows) spills
+// at head_dim 128 (72 bytes stored / 172 loaded per thread, 100 / 212 in the fused
+// kernel), which is why a plan with many such tasks keeps one per CTA.
 #pragma once
 
 #include "ft_async.cuh"
 #include "ft_common.cuh"
 #include "ft_stage1_mma.cuh"
 #include "ft_stage1_narrow.cuh"
+#include "ft_stage1_row.cuh"
 
 namespace ft {
 
@@ -66,12 +71,13 @@ struct PairCfg {
   static_assert(SMEM_BYTES <= (D == 256 ? 232448 : 115712), "two CTAs per SM, one at head_dim 256");
 };
 
-// nw: warps of the body, 4 or 8 (threads tid of 32 nw); barrier: a hardware barrier of its own
-template <typename T, int D, int NQ, int NS>
-__device__ __forceinline__ void slab_body(const TcParams& tp, uint8_t* smem, const int tid, const int nw, const int barrier,
+// Params: SlabParams at head_dim 256, any parameter block below; nw: warps of the body, 4 or 8 (threads tid of 32 nw);
+// barrier: a hardware barrier of its own
+template <typename T, int D, int NQ, int NS, typename Params>
+__device__ __forceinline__ void slab_body(const Params& tp, uint8_t* smem, const int tid, const int nw, const int barrier,
                                             const int kvh, const int q_off, const int q_len, const int kv_off, const int kv_len) {
   using N = SlabCfg<D, NQ, NS>;
-  const Stage1Params& p = tp.p;
+  const Stage1Params& p = stage1_of(tp);
   constexpr bool Q_IN_REGS = NQ == 1 && D <= 128;
   const uint32_t q_sm = smem_u32(smem);
   float* epi_o = reinterpret_cast<float*>(smem + N::Q_BYTES);
@@ -196,10 +202,11 @@ __device__ __forceinline__ void slab_body(const TcParams& tp, uint8_t* smem, con
     auto look_at_ids = [&](int b) {  // the pair of slabs in id_cur
       const int pos = span * (2 * b + (lane >> 4)) + 16 * warp + (lane & 15);
       bad |= pos < id_lim && (uint32_t)id_cur >= row_lim;
-      if constexpr (!N::TMA) return;
-      first = __shfl_sync(0xffffffffu, id_cur, lane & 16);
-      const uint32_t run = __ballot_sync(0xffffffffu, id_cur == first + (lane & 15) && first >= 0 && (uint32_t)first + 16 <= row_lim);
-      if (!tp.has_tma || ((run >> (lane & 16)) & 0xffffu) != 0xffffu) first = -1;
+      if constexpr (N::TMA) {
+        first = __shfl_sync(0xffffffffu, id_cur, lane & 16);
+        const uint32_t run = __ballot_sync(0xffffffffu, id_cur == first + (lane & 15) && first >= 0 && (uint32_t)first + 16 <= row_lim);
+        if (!tp.has_slabs || ((run >> (lane & 16)) & 0xffffu) != 0xffffu) first = -1;
+      }
     };
     auto issue = [&]() {
       const int j = u_issue >> 1;
@@ -211,11 +218,13 @@ __device__ __forceinline__ void slab_body(const TcParams& tp, uint8_t* smem, con
       const uint32_t dst = ring + slot_issue * N::SLAB_BYTES, full = bars + 8 * slot_issue;
       const int row0_of = N::TMA ? __shfl_sync(0xffffffffu, first, (j & 1) * 16) : -1;
       if (row0_of >= 0) {
-        if (lane == 0) {
-          mbar_arrive_expect_tx(full, N::SLAB_BYTES);
+        if constexpr (N::TMA) {
+          if (lane == 0) {
+            mbar_arrive_expect_tx(full, N::SLAB_BYTES);
 #pragma unroll
-          for (int h = 0; h < D / 64; ++h)
-            tma_load_3d(dst + h * (N::SLAB * 128), is_v ? &tp.v_slab_map : &tp.k_slab_map, 64 * h, kvh, row0_of, full);
+            for (int h = 0; h < D / 64; ++h)
+              tma_load_3d(dst + h * (N::SLAB * 128), is_v ? &tp.v_slab_map : &tp.k_slab_map, 64 * h, kvh, row0_of, full);
+          }
         }
       } else {
         const T* base = is_v ? vbase : kbase;
@@ -448,24 +457,25 @@ __device__ __forceinline__ void slab_body(const TcParams& tp, uint8_t* smem, con
   if (bad) flag_error(FT_DEV_BAD_KV_INDEX);
 }
 
-__device__ __forceinline__ void prefetch_slab_maps(const TcParams& tp) {
-  if (threadIdx.x == 0 && tp.has_tma) {
+__device__ __forceinline__ void prefetch_slab_maps(const SlabParams& tp) {
+  if (threadIdx.x == 0 && tp.has_slabs) {
     asm volatile("prefetch.tensormap [%0];\n" ::"l"(reinterpret_cast<uint64_t>(&tp.k_slab_map)) : "memory");
     asm volatile("prefetch.tensormap [%0];\n" ::"l"(reinterpret_cast<uint64_t>(&tp.v_slab_map)) : "memory");
   }
 }
 
 // One few-row CTA.  FEW_PAIR: its two bodies of four warps take tasks `first` and `first` + 1 (of `tasks`, kv head fastest);
-// FEW_EIGHT: all eight warps take task `first`.  Tasks with at most 8 query rows run the one-block body, the others the
-// two-block body (which also loops if a task has more than 16 rows).
-template <typename T, int D>
-__device__ __forceinline__ void pair_cta(const TcParams& tp, uint8_t* smem, const int form, const int first, const int tasks) {
+// FEW_EIGHT (head_dim 256): all eight warps take task `first`.  Tasks with at most 8 query rows run the one-block body, the
+// others the two-block body (which also loops if a task has more than 16 rows).
+template <typename T, int D, typename Params>
+__device__ __forceinline__ void pair_cta(const Params& tp, uint8_t* smem, const int form, const int first, const int tasks) {
   using P = PairCfg<D>;
-  const int body = form == FEW_PAIR ? threadIdx.x >> 7 : 0, task = first + body;
+  const Stage1Params& p = stage1_of(tp);
+  const bool pair = D != 256 || form == FEW_PAIR;
+  const int body = pair ? threadIdx.x >> 7 : 0, task = first + body;
   if (task >= tasks) return;
-  const int nw = form == FEW_PAIR ? 4 : 8, tid = threadIdx.x & (32 * nw - 1);
+  const int nw = pair ? 4 : 8, tid = threadIdx.x & (32 * nw - 1);
   int vn, kvh;
-  const Stage1Params& p = tp.p;
   task_of_block(p, task, vn, kvh);
   const int q_off = p.q_offs[vn], q_len = p.q_lens[vn], kv_off = p.kv_offs[vn], kv_len = max(p.kv_lens[vn], 0);
   smem += body * P::BODY_BYTES;
@@ -475,15 +485,15 @@ __device__ __forceinline__ void pair_cta(const TcParams& tp, uint8_t* smem, cons
     slab_body<T, D, P::MAX_NQ, P::NS>(tp, smem, tid, nw, 3 + body, kvh, q_off, q_len, kv_off, kv_len);
 }
 
+// Few-row tasks alone, two to a CTA (head_dim 256 runs them in the fused kernel: its CTAs of both kinds fill an SM each)
 template <typename T, int D>
-__global__ void __launch_bounds__(PairCfg<D>::THREADS, 2) stage1_narrow_kernel(const __grid_constant__ TcParams tp) {
+__global__ void __launch_bounds__(PairCfg<D>::THREADS, 2) stage1_pair_kernel(const __grid_constant__ Stage1Params p) {
+  static_assert(D <= 128, "at 256 the fused kernel runs them");
   allow_dependent_launch();
-  if (D == 256) prefetch_slab_maps(tp);
   wait_for_prior_grid();  // nothing of the preceding kernel's is read or overwritten before this
   extern __shared__ __align__(1024) uint8_t smem[];
-  const Stage1Params& p = tp.p;
   FT_TL_BEGIN();
-  pair_cta<T, D>(tp, smem, p.few_form, few_per_cta(p.few_form) * (int)blockIdx.x, p.node_count * p.num_kv_heads);
+  pair_cta<T, D>(p, smem, FEW_PAIR, 2 * (int)blockIdx.x, p.node_count * p.num_kv_heads);
   FT_TL_END(2);
 }
 

@@ -1101,6 +1101,9 @@ __global__ void __launch_bounds__(TcCfg<D>::THREADS, 2) stage1_tc_kernel(const _
   FT_TL_END(1);
 }
 
+template <int D, bool PAIR>
+using FusedParams = std::conditional_t<PAIR && D == 256, SlabParams, TcParams>;
+
 // Both task families in one grid: the tensor-bound many-row CTAs (tcgen05 body, one task each)
 // and the memory-bound few-row CTAs (swapped-operand body) share the SMs instead of running back to back.
 // Block order, which is the order the hardware starts them in:
@@ -1112,7 +1115,7 @@ __global__ void __launch_bounds__(TcCfg<D>::THREADS, 2) stage1_tc_kernel(const _
 // PAIR: few-row tasks by pair_cta (p.few_form), else by the workers or the one-task body; a kernel each, because in one
 // kernel they cost the one-task plans 2-3 % (45 leaves of 130 tokens under a 1000-token node 17.2 -> 17.6 us).
 template <typename T, int D, bool PAIR>
-__global__ void __launch_bounds__(TcCfg<D>::THREADS, 2) stage1_fused_kernel(const __grid_constant__ TcParams tp) {
+__global__ void __launch_bounds__(TcCfg<D>::THREADS, 2) stage1_fused_kernel(const __grid_constant__ FusedParams<D, PAIR> tp) {
   allow_dependent_launch();
   extern __shared__ __align__(1024) uint8_t smem[];
   const Stage1Params& p = tp.p;
@@ -1123,11 +1126,12 @@ __global__ void __launch_bounds__(TcCfg<D>::THREADS, 2) stage1_fused_kernel(cons
   FT_TL_BEGIN();
   bool many_rows = b < p.lead_wide || b >= p.lead_wide + few_ctas;
   int task = b < p.lead_wide ? b : b - few_ctas;
+  const int w = b - p.lead_wide;
   if constexpr (D == 256) {
     // Eight warps per task: a task of more than eight rows, which they would have to run in two passes over K and V, stays
     // with the tcgen05 body (270 tasks of a five-level tree, 8/2 heads: two passes 61 us, this 44).
     if (!many_rows && p.few_form == FEW_EIGHT) {
-      task = wide_tasks + b - p.lead_wide;
+      task = wide_tasks + w;
       wait_for_prior_grid();
       many_rows = p.q_lens[p.node_offset + task / H] * p.group > 8;
     }
@@ -1135,32 +1139,30 @@ __global__ void __launch_bounds__(TcCfg<D>::THREADS, 2) stage1_fused_kernel(cons
   if (many_rows) {
     tc_body<T, D, false>(tp, smem, p.node_offset + task / H, task % H);
     FT_TL_END(1);
-  } else {
-    // This CTA will not allocate tensor memory.  Saying so at once matters: the SM admits no second CTA of a
-    // kernel that uses tensor memory while a resident one still holds the right to allocate.
-    if (threadIdx.x < 32) asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
-    const int w = b - p.lead_wide;
-    if constexpr (!PAIR) {
-      if (threadIdx.x >= 128) {  // these bodies are written for four warps: the others hand over their registers
-        reg_shrink<24>();
-        return;
-      }
-      reg_grow<TcCfg<D>::REGS_WORKER>();
-      wait_for_prior_grid();  // nothing of the preceding kernel's is read or overwritten before this
-      if (p.workers > 0) {
-        stream_worker<T, D>(tp, smem, wide_tasks, few_tasks, w, p.workers);
-      } else {
-        task = wide_tasks + w;
-        narrow_dispatch<T, D>(p, smem, p.node_offset + task / H, task % H);
-      }
-      FT_TL_END(2);
+    return;
+  }
+  // This CTA will not allocate tensor memory.  Saying so at once matters: the SM admits no second CTA of a
+  // kernel that uses tensor memory while a resident one still holds the right to allocate.
+  if (threadIdx.x < 32) asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+  if constexpr (!PAIR) {
+    if (threadIdx.x >= 128) {  // these bodies are written for four warps: the others hand over their registers
+      reg_shrink<24>();
       return;
     }
-    if (D == 256) prefetch_slab_maps(tp);
+    reg_grow<TcCfg<D>::REGS_WORKER>();
+    wait_for_prior_grid();  // nothing of the preceding kernel's is read or overwritten before this
+    if (p.workers > 0) {
+      stream_worker<T, D>(tp, smem, wide_tasks, few_tasks, w, p.workers);
+    } else {
+      task = wide_tasks + w;
+      narrow_dispatch<T, D>(p, smem, p.node_offset + task / H, task % H);
+    }
+  } else {
+    if constexpr (D == 256) prefetch_slab_maps(tp);
     wait_for_prior_grid();
-    if constexpr (PAIR) pair_cta<T, D>(tp, smem, p.few_form, wide_tasks + few_per_cta(p.few_form) * w, wide_tasks + few_tasks);
-    FT_TL_END(2);
+    pair_cta<T, D>(tp, smem, p.few_form, wide_tasks + few_per_cta(p.few_form) * w, wide_tasks + few_tasks);
   }
+  FT_TL_END(2);
 }
 
 // Every task of a step from one grid whose size does not depend on the plan.

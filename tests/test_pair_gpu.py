@@ -68,8 +68,7 @@ def test_few_row_tasks(d, form, many, group, hkv, dtype, extra):
     nums.task_sizes = SIZES[form]
     args = (qd, k.cuda(), v.cuda(), torch.empty_like(qd), *dev, none, none, none, mid_o, mid_lse, nums, [0, many],
             [40, max(1, 16 // group)], [64, 64], d ** -0.5)
-    kernel = "stage1_fused_kernel" if many or d == 256 else "stage1_narrow_kernel"
-    assert engine.stage1_path_name(*args) == f"{kernel}/{form}"
+    assert engine.stage1_path_name(*args) == (f"stage1_fused_kernel/{form}" if many or d == 256 else "stage1_pair_kernel")
     engine.stage1(*args, row_ranges=None if ranges is None else torch.from_numpy(ranges.astype(np.int32)).cuda())
     torch.cuda.synchronize()
     assert lib.read_device_status() == (lib.FT_DEV_BAD_KV_INDEX if extra == "bad_id" else 0)
