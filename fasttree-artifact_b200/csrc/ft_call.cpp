@@ -48,7 +48,9 @@ const at::Tensor& table(const char* name, PyObject* o) {
 }
 
 void pair(const char* name, PyObject* o, int64_t (&out)[2]) {
-  PyObject* seq = PySequence_Fast(o, "expected a pair of integers");
+  // (a list subclass without an iterator of its own, such as a plan's counts, is read in place like a list)
+  const bool listed = PyList_Check(o) && Py_TYPE(o)->tp_iter == PyList_Type.tp_iter;
+  PyObject* seq = listed ? Py_NewRef(o) : PySequence_Fast(o, "expected a pair of integers");
   if (seq == nullptr) throw Refused();
   if (PySequence_Fast_GET_SIZE(seq) != 2) {
     Py_DECREF(seq);
@@ -69,7 +71,8 @@ void pair(const char* name, PyObject* o, int64_t (&out)[2]) {
 // The task sizes that a plan's phase_node_nums carries (ft_b200.planner.PhaseNodeNums); a plain list or tuple has none.
 void task_sizes(PyObject* o, ft_decode_args& a) {
   if (PyList_CheckExact(o) || PyTuple_CheckExact(o)) return;
-  PyObject* sizes = PyObject_GetAttrString(o, "task_sizes");
+  static PyObject* const name = PyUnicode_InternFromString("task_sizes");
+  PyObject* sizes = PyObject_GetAttr(o, name);
   if (sizes == nullptr) {
     PyErr_Clear();
     return;
@@ -132,7 +135,7 @@ void fill(PyObject* const* x, ft_decode_args& a, c10::DeviceIndex& device) {
   }
   int64_t nums[2], offs[2], q_tiles[2], kv_tiles[2];
   pair("phase_node_nums", arg(NODE_NUMS), nums);
-  task_sizes(arg(NODE_NUMS), a);
+  if (dtype != at::kFloat) task_sizes(arg(NODE_NUMS), a);  // (fp32 kernels have one form)
   pair("phase_node_offsets", arg(NODE_OFFSETS), offs);
   pair("phase_q_tile_sizes", arg(Q_TILES), q_tiles);
   pair("phase_kv_tile_sizes", arg(KV_TILES), kv_tiles);

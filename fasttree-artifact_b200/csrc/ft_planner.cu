@@ -556,6 +556,15 @@ int build_plan(const int32_t* parent, const int32_t* seqlen, int32_t n_nodes, co
     info.aux_segments = (int64_t)(plan->aux_segments.size() / 4);
     info.target_bytes = target;
     info.virtual_nodes = (int64_t)specs.size();
+    for (size_t i = 0; i < nv; ++i) {
+      if (i < big.size()) {
+        info.many_longest = std::max(info.many_longest, plan->kv_lens[i]);
+      } else {
+        info.few_tokens += plan->kv_lens[i];
+        info.few_longest = std::max(info.few_longest, plan->kv_lens[i]);
+        info.few_over_8_rows += (int64_t)plan->q_lens[i] * group > 8 ? 1 : 0;
+      }
+    }
   } catch (const std::bad_alloc&) {
     delete plan;
     return FT_ERR_TOO_LARGE;

@@ -127,8 +127,8 @@ def _upload(md, tabs, last_vnodes, tail_state=None, src_table=None):
                     md.kv_entries_aux[dst:dst + length] = flat[src:src + length]
                     md.kv_entries_aux[dst + length:dst + length + room] = flat[src]
         md.refresh_pending = md.num_grouped_tails > 0 or (md.graph_safe and md.refresh_layer is None)
-    md.phase_node_nums = _planner.PhaseNodeNums(tabs["phase_node_nums"], tabs["vnode_to_kv_lens"], tabs["vnode_to_q_lens"],
-                                                md.kv_group_num)
+    md.phase_node_nums = _planner.PhaseNodeNums.of_tables(tabs["phase_node_nums"], tabs["vnode_to_kv_lens"],
+                                                          tabs["vnode_to_q_lens"], md.kv_group_num)
     md.phase_node_offsets = list(tabs["phase_node_offsets"])
     md.req_last_vnodes = [int(v) for v in last_vnodes]
     md.num_vnodes, md.num_partial_rows = int(nv), int(rows)
@@ -325,10 +325,12 @@ def prepare_for_fasttree_meta(batch, fasttree_metadata):
     node_to_reqs, covered = _walk_requests(batch)
     order, offsets, parents, lens = _bfs(batch, node_to_reqs)
     # one row of the table per request; a tensor padded beyond the batch is fine, one that is too short is not
-    req_idx = batch.req_pool_indices[:len(batch.reqs)].cpu().reshape(-1).tolist()
-    if len(req_idx) != len(batch.reqs):
-        raise IndexError(f"req_pool_indices names {len(req_idx)} of {len(batch.reqs)} requests")
-    req_idx = [int(i) for i in req_idx]
+    bsz = len(batch.reqs)
+    req_idx = batch.req_pool_indices.tolist()[:bsz]
+    if bsz and not isinstance(req_idx[0], int):         # one index per row, or floats
+        req_idx = [int(i) for i in batch.req_pool_indices[:bsz].reshape(-1).tolist()]
+    if len(req_idx) != bsz:
+        raise IndexError(f"req_pool_indices names {len(req_idx)} of {bsz} requests")
     stride = batch.req_to_token_pool.req_to_token.stride(0)
     if md.planner == "reference":
         tabs, last = _plan_reference(batch, md, node_to_reqs, order, offsets, lens, req_idx, stride)

@@ -52,7 +52,9 @@ class PlanInfo(ctypes.Structure):
                 ("phase_node_nums", ctypes.c_int32 * 2), ("phase_node_offsets", ctypes.c_int32 * 2),
                 ("q_tile", ctypes.c_int32), ("small_tile", ctypes.c_int32), ("tile_tokens", ctypes.c_int32),
                 ("has_row_ranges", ctypes.c_int32), ("target_bytes", ctypes.c_double),
-                ("aux_entries", ctypes.c_int64), ("aux_segments", ctypes.c_int64)]
+                ("aux_entries", ctypes.c_int64), ("aux_segments", ctypes.c_int64),
+                ("few_tokens", ctypes.c_int64), ("few_longest", ctypes.c_int32), ("few_over_8_rows", ctypes.c_int32),
+                ("many_longest", ctypes.c_int32)]
 
 
 class DecodeArgs(ctypes.Structure):

@@ -86,15 +86,20 @@ class PhaseNodeNums(list):
     the device tables: ``task_sizes = (tokens of phase 1's chunks together, the longest of them, vnodes of phase 1 with more
     than 8 query rows, longest chunk of phase 0)``.  A plain list in its place works too; the launch then assumes nothing."""
 
-    def __init__(self, nums, kv_lens=None, q_lens=None, group=1):
-        """``kv_lens`` / ``q_lens``: the plan's ``vnode_to_kv_lens`` / ``vnode_to_q_lens`` (phase 0 first, as emitted)."""
+    def __init__(self, nums, task_sizes=(0, 0, 0, 0)):
         super().__init__(nums)
-        self.task_sizes = (0, 0, 0, 0)
-        if kv_lens is not None:
-            n0, n1 = nums
-            many, few = kv_lens[:n0], kv_lens[n0:n0 + n1]
-            self.task_sizes = (int(few.sum(dtype=np.int64)), int(few.max(initial=0)),
-                               int(np.count_nonzero(q_lens[n0:n0 + n1].astype(np.int64) * group > 8)), int(many.max(initial=0)))
+        self.task_sizes = task_sizes
+
+    @classmethod
+    def of_tables(cls, nums, kv_lens, q_lens, group):
+        """``kv_lens`` / ``q_lens``: the plan's ``vnode_to_kv_lens`` / ``vnode_to_q_lens`` (phase 0 first, as emitted).
+        Counts that state their sizes already, as the native splitter's do, are returned as they are."""
+        if isinstance(nums, cls):
+            return nums
+        n0, n1 = nums
+        few = kv_lens[n0:n0 + n1]
+        return cls(nums, (int(few.sum(dtype=np.int64)), int(few.max(initial=0)),
+                          int(np.count_nonzero(q_lens[n0:n0 + n1] > 8 // group)), int(kv_lens[:n0].max(initial=0))))
 
 
 # --------------------------------------------------------------------- emitter
@@ -664,7 +669,8 @@ def _native_tables(build, direct):
         L.ft_plan_free(handle)
     if direct:
         tabs["vnode_to_kv_entries"] = None
-    tabs["phase_node_nums"] = [int(x) for x in info.phase_node_nums]
+    tabs["phase_node_nums"] = PhaseNodeNums([int(x) for x in info.phase_node_nums],
+                                            (info.few_tokens, info.few_longest, info.few_over_8_rows, info.many_longest))
     tabs["phase_node_offsets"] = [int(x) for x in info.phase_node_offsets]
     return tabs, [int(a) for a in assign], info
 

@@ -308,6 +308,8 @@ typedef struct ft_plan_info {
   double target_bytes;  /* streamed bytes one task was sized for */
   int64_t aux_entries;  /* serving plans with groups: entries of the auxiliary row-id table the vnode offsets assume */
   int64_t aux_segments; /* ... and the number of segments ft_plan_copy_aux_segments reports */
+  int64_t few_tokens;   /* the task sizes to pass in the fields of these names of ft_decode_args */
+  int32_t few_longest, few_over_8_rows, many_longest;
 } ft_plan_info;
 
 /* Tree: n_nodes records in id order, node 0 the root, parents before children (parent[0] = -1); seqlen tokens per

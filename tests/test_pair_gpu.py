@@ -64,8 +64,7 @@ def test_few_row_tasks(d, form, many, group, hkv, dtype, extra):
     mid_o, mid_lse = torch.full((parts, hkv * group, d), float("nan"), device="cuda"), torch.empty(parts, hkv * group, device="cuda")
     none = torch.zeros(64, dtype=torch.int32, device="cuda")
     qd = q.cuda()
-    nums = PhaseNodeNums([many, FEW])
-    nums.task_sizes = SIZES[form]
+    nums = PhaseNodeNums([many, FEW], SIZES[form])
     args = (qd, k.cuda(), v.cuda(), torch.empty_like(qd), *dev, none, none, none, mid_o, mid_lse, nums, [0, many],
             [40, max(1, 16 // group)], [64, 64], d ** -0.5)
     assert engine.stage1_path_name(*args) == (f"stage1_fused_kernel/{form}" if many or d == 256 else "stage1_pair_kernel")
@@ -99,6 +98,7 @@ ONE, PAIR, EIGHT, TC = "stage1_fused_kernel", "stage1_fused_kernel/pair", "stage
     (("1,12,24,48", "2000,400,300,200"), 64, 8, 256, EIGHT),
     (("1,18", "1000,400"), 16, 8, 256, PAIR),
     (("1,16", "1000,400"), 16, 8, 256, TC),              # one round
+    (("1,26", "3441,314"), 32, 8, 256, TC),              # beside many-row tasks, and not short
     (("1,9", "11165,203"), 32, 8, 256, TC),              # a round and a quarter, most of it many-row
     (("1,2,4", "16011,518,10"), 32, 8, 256, TC),         # long tasks
 ], ids=lambda x: "-".join(map(str, x)).replace(",", ".") if isinstance(x, tuple) else str(x).replace("stage1_", ""))
