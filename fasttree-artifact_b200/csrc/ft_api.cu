@@ -736,8 +736,9 @@ int ft_stage1(const ft_decode_args* a) {
   const int64_t r0 = a->phase_q_tile_sizes[0] > 0 ? (int64_t)a->phase_q_tile_sizes[0] * group : 1 << 30;
   const int64_t r1 = a->phase_q_tile_sizes[1] > 0 ? (int64_t)a->phase_q_tile_sizes[1] * group : 1 << 30;
   const int rows0 = (int)(r0 < (1 << 30) ? r0 : (1 << 30)), rows1 = (int)(r1 < (1 << 30) ? r1 : (1 << 30));
+  // (head_dim 256: a few-row phase in front of a many-row one runs on the tcgen05 kernel with it)
   const bool same_kernel = path == FT_PATH_GENERIC || path == FT_PATH_MMA_WIDE || path == FT_PATH_TCGEN05 ||
-                           ((rows0 > 16) == (rows1 > 16));
+                           a->head_dim == 256 || ((rows0 > 16) == (rows1 > 16));
   // the persistent kernel takes every task of the launch, whatever its row count
   if (path == FT_PATH_PERSIST && a->device_phase_info != nullptr) {
     ft::Stage1Params p = stage1_params(a);  // node_offset / node_count come from the device array

@@ -119,3 +119,15 @@ def test_which_plans_take_two_tasks_per_cta(tree, hq, hkv, d, want):
     assert name(aux) == want
     # a plan that does not state its sizes, as one made by hand: nothing is assumed
     assert name(aux[:11] + (list(aux[11]),) + aux[12:]) == (TC if d == 256 else ONE)
+
+
+@pytest.mark.parametrize("d,want", [(256, TC), (128, "stage1_narrow_kernel+stage1_tc_kernel")])
+def test_a_few_row_phase_in_front_of_a_many_row_one(d, want):
+    """At head_dim 256 both go to the tcgen05 kernel in one launch."""
+    q = torch.zeros(64, 32, d, dtype=torch.float16, device="cuda")
+    kv = torch.zeros(64, 8, d, dtype=torch.float16, device="cuda")
+    ints = lambda n: torch.zeros(n, dtype=torch.int32, device="cuda")
+    name = engine.stage1_path_name(q, kv, kv, torch.empty_like(q), ints(900), *[ints(50)] * 2, ints(64), *[ints(50)] * 2,
+                                   ints(64), ints(64), ints(64), torch.zeros(64, 32, d, device="cuda"),
+                                   torch.zeros(64, 32, device="cuda"), [40, 10], [0, 40], [4, 32], [64, 64], 0.1)
+    assert name == want
