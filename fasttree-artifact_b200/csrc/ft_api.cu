@@ -153,7 +153,7 @@ int pick_path(const ft_decode_args* a) {
     if (a->path == FT_PATH_PERSIST && a->head_dim != 128)
       return fail(FT_ERR_UNSUPPORTED, "the persistent kernel needs head_dim 128, got %d", a->head_dim);
     if (a->path != FT_PATH_TCGEN05 && a->head_dim == 256)
-      return fail(FT_ERR_UNSUPPORTED, "head_dim 256 has the tcgen05 kernel only");
+      return fail(FT_ERR_UNSUPPORTED, "head_dim 256 runs on paths AUTO, TCGEN05 and GENERIC only");
     return a->path;
   }
   if (a->path != FT_PATH_AUTO) return fail(FT_ERR_INVALID_ARGUMENT, "unknown path %d", a->path);
@@ -404,20 +404,21 @@ TaskSizes task_sizes(const ft_decode_args* a) {
 // warps each, 16/8 heads: 64 of 256 under 4096 57.1 / 44.9 / 48.1; 60 of 130 under 1000 47.4 / 30.0 / 39.3, 60 of 1500
 // 144 / 126 / 129, 16 of 400 (one round) 21.5 / 23.1 / 24.1; 47 of 280 under 930, one task of 15 rows, 24/8 heads, 46.4 /
 // 80.4 / 44.8; 29 of 335 under 3 of 127 under 2013, 32/8 heads, 37.0 / 40.4 two at a time; 26 of 314 under 3441 35.2 / 37.1
-// with eight warps each.
+// with eight warps each; 4 of 60 beside groups of 17 x 60, which the step waits for, 32/32 heads, 33.4 / 35.3 so.
 // The bounds are where the ratio of both sides crosses one over 2700 trees drawn from the benchmark's ranges: the rule takes
-// two tasks (or eight warps) on 117 of 1030 at head_dim 128, 142 of 1085 at 64 and 125 of 628 at 256, which take 15, 21 and
-// 27 % less time for it, and at worst 3, 5 and 3 % more.
+// two tasks (or eight warps) on 117 of 1030 at head_dim 128, 142 of 1085 at 64 and 124 of 628 at 256, which take 15, 21 and
+// 27 % less time for it, and at worst 3, 5 and 0 % more.  Of 1700 trees drawn after
+// that it was more than 3 % behind one task per CTA (or the tcgen05 kernel) on one.
 int few_rows_form(const TaskSizes& z, int group, int64_t few_nodes, int64_t wide, int hkv, int head_dim, int64_t slots) {
   const int64_t few = few_nodes * hkv, longest = z.few_longest, tokens = z.few_tokens * hkv;
   const int without = head_dim == 256 ? -1 : ft::FEW_ONE;
   if (longest == 0 || group > 8) return without;
   if (head_dim == 256) {
     if (few + wide <= slots) return without;
-    const bool alone = 8 * wide <= slots;
-    if (z.few_over_8_rows == 0 && z.many_longest * slots <= 4 * tokens && (longest <= (alone ? 400 : 256) || tokens >= 2 * slots * longest))
+    const bool alone = 8 * wide <= slots, waits = z.many_longest * slots > 4 * tokens;
+    if (z.few_over_8_rows == 0 && !waits && (longest <= (alone ? 400 : 256) || tokens >= 2 * slots * longest))
       return ft::FEW_PAIR;
-    const bool brief = longest <= (alone ? 320 : 256) && 8 * z.few_over_8_rows <= few_nodes && 5 * wide <= 3 * slots;
+    const bool brief = longest <= (alone ? 320 : 256) && !waits && 8 * z.few_over_8_rows <= few_nodes && 5 * wide <= 3 * slots;
     return 5 * few > 12 * slots || brief ? ft::FEW_EIGHT : without;
   }
   if (4 * z.few_over_8_rows > few_nodes) return without;

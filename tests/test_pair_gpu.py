@@ -21,7 +21,7 @@ pytestmark = pytest.mark.gpu
 
 LENS = [1, 2, 15, 16, 17, 31, 33, 47, 48, 49, 63, 64, 65, 112, 113, 127, 128, 129, 191, 193, 255, 256, 257, 320, 400]
 FEW = 31
-SIZES = {"one": (0, 0, 0, 0), "pair": (10 ** 9, 1, 0, 0), "eight": (1, 1, 1, 1)}
+SIZES = {"one": (0, 0, 0, 0), "pair": (10 ** 9, 1, 0, 0), "eight": (1, 1, 1, 0)}
 
 
 def _plan(few, many, group, seed):
@@ -98,6 +98,7 @@ ONE, PAIR, EIGHT, TC = "stage1_fused_kernel", "stage1_fused_kernel/pair", "stage
     (("1,12,24,48", "2000,400,300,200"), 64, 8, 256, EIGHT),
     (("1,18", "1000,400"), 16, 8, 256, PAIR),
     (("1,16", "1000,400"), 16, 8, 256, TC),              # one round
+    (("1,21", "123,60"), 32, 32, 256, TC),               # the step waits for groups of 17 leaves
     (("1,26", "3441,314"), 32, 8, 256, TC),              # beside many-row tasks, and not short
     (("1,9", "11165,203"), 32, 8, 256, TC),              # a round and a quarter, most of it many-row
     (("1,2,4", "16011,518,10"), 32, 8, 256, TC),         # long tasks
