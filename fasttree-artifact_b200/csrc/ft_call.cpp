@@ -48,9 +48,7 @@ const at::Tensor& table(const char* name, PyObject* o) {
 }
 
 void pair(const char* name, PyObject* o, int64_t (&out)[2]) {
-  // (a list subclass without an iterator of its own, such as a plan's counts, is read in place like a list)
-  const bool listed = PyList_Check(o) && Py_TYPE(o)->tp_iter == PyList_Type.tp_iter;
-  PyObject* seq = listed ? Py_NewRef(o) : PySequence_Fast(o, "expected a pair of integers");
+  PyObject* seq = PySequence_Fast(o, "expected a pair of integers");
   if (seq == nullptr) throw Refused();
   if (PySequence_Fast_GET_SIZE(seq) != 2) {
     Py_DECREF(seq);
@@ -68,15 +66,13 @@ void pair(const char* name, PyObject* o, int64_t (&out)[2]) {
   Py_DECREF(seq);
 }
 
-// The task sizes that a plan's phase_node_nums carries (ft_b200.planner.PhaseNodeNums); a plain list or tuple has none.
-void task_sizes(PyObject* o, ft_decode_args& a) {
-  if (PyList_CheckExact(o) || PyTuple_CheckExact(o)) return;
+// The task sizes that a plan's vnode_to_kv_lens tensor carries as an attribute (ft_b200.planner.task_sizes); without it none
+// are known.
+void task_sizes(PyObject* table, ft_decode_args& a) {
   static PyObject* const name = PyUnicode_InternFromString("task_sizes");
-  PyObject* sizes = PyObject_GetAttr(o, name);
-  if (sizes == nullptr) {
-    PyErr_Clear();
-    return;
-  }
+  PyObject* sizes = nullptr;
+  if (_PyObject_LookupAttr(table, name, &sizes) < 0) throw Refused();
+  if (sizes == nullptr) return;
   long long n[4] = {0, 0, 0, 0};
   const bool ok = PyTuple_Check(sizes) && PyTuple_GET_SIZE(sizes) == 4;
   for (int i = 0; ok && i < 4; ++i) n[i] = PyLong_AsLongLong(PyTuple_GET_ITEM(sizes, i));
@@ -135,7 +131,7 @@ void fill(PyObject* const* x, ft_decode_args& a, c10::DeviceIndex& device) {
   }
   int64_t nums[2], offs[2], q_tiles[2], kv_tiles[2];
   pair("phase_node_nums", arg(NODE_NUMS), nums);
-  if (dtype != at::kFloat) task_sizes(arg(NODE_NUMS), a);  // (fp32 kernels have one form)
+  if (dtype != at::kFloat) task_sizes(arg(KV_LENS), a);  // (fp32 kernels have one form)
   pair("phase_node_offsets", arg(NODE_OFFSETS), offs);
   pair("phase_q_tile_sizes", arg(Q_TILES), q_tiles);
   pair("phase_kv_tile_sizes", arg(KV_TILES), kv_tiles);

@@ -127,8 +127,9 @@ def _upload(md, tabs, last_vnodes, tail_state=None, src_table=None):
                     md.kv_entries_aux[dst:dst + length] = flat[src:src + length]
                     md.kv_entries_aux[dst + length:dst + length + room] = flat[src]
         md.refresh_pending = md.num_grouped_tails > 0 or (md.graph_safe and md.refresh_layer is None)
-    md.phase_node_nums = _planner.PhaseNodeNums.of_tables(tabs["phase_node_nums"], tabs["vnode_to_kv_lens"],
-                                                          tabs["vnode_to_q_lens"], md.kv_group_num)
+    md.phase_node_nums = list(tabs["phase_node_nums"])
+    md.vnode_to_kv_lens.task_sizes = tabs.get("task_sizes") or _planner.task_sizes(
+        tabs["phase_node_nums"], tabs["vnode_to_kv_lens"], tabs["vnode_to_q_lens"], md.kv_group_num)
     md.phase_node_offsets = list(tabs["phase_node_offsets"])
     md.req_last_vnodes = [int(v) for v in last_vnodes]
     md.num_vnodes, md.num_partial_rows = int(nv), int(rows)

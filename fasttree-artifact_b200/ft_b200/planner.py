@@ -66,6 +66,7 @@ class Plan:
     phase_kv_tile_sizes: list = field(default_factory=list)
     kv_split_sizes: list = field(default_factory=list)
     info: dict = field(default_factory=dict)
+    task_sizes: tuple = None               # see :func:`task_sizes`; the native splitter counts them, for others the caller does
 
     @property
     def num_partial_rows(self):
@@ -81,25 +82,18 @@ class Plan:
                 self.req_to_vnode_entries, self.req_to_vnode_offs, self.req_to_vnode_lens)
 
 
-class PhaseNodeNums(list):
-    """``phase_node_nums`` of a plan, with the task sizes that the launch chooses between its kernels by and cannot read from
-    the device tables: ``task_sizes = (tokens of phase 1's chunks together, the longest of them, vnodes of phase 1 with more
-    than 8 query rows, longest chunk of phase 0)``.  A plain list in its place works too; the launch then assumes nothing."""
+def task_sizes(phase_node_nums, kv_lens, q_lens, group):
+    """What the launch chooses between its kernels by and cannot read from the device tables: ``(tokens of phase 1's chunks
+    together, the longest of them, vnodes of phase 1 with more than 8 query rows, longest chunk of phase 0)``, of the plan's
+    ``vnode_to_kv_lens`` / ``vnode_to_q_lens`` (phase 0 first, as emitted).
 
-    def __init__(self, nums, task_sizes=(0, 0, 0, 0)):
-        super().__init__(nums)
-        self.task_sizes = task_sizes
-
-    @classmethod
-    def of_tables(cls, nums, kv_lens, q_lens, group):
-        """``kv_lens`` / ``q_lens``: the plan's ``vnode_to_kv_lens`` / ``vnode_to_q_lens`` (phase 0 first, as emitted).
-        Counts that state their sizes already, as the native splitter's do, are returned as they are."""
-        if isinstance(nums, cls):
-            return nums
-        n0, n1 = nums
-        few = kv_lens[n0:n0 + n1]
-        return cls(nums, (int(few.sum(dtype=np.int64)), int(few.max(initial=0)),
-                          int(np.count_nonzero(q_lens[n0:n0 + n1] > 8 // group)), int(kv_lens[:n0].max(initial=0))))
+    They have no slot in the reference's 13-entry tuple and travel as the attribute ``task_sizes`` of the
+    ``vnode_to_kv_lens`` tensor, which saving, pickling and deepcopy keep; a table without it works too, the launch then
+    assumes nothing."""
+    n0, n1 = phase_node_nums
+    few = kv_lens[n0:n0 + n1]
+    return (int(few.sum(dtype=np.int64)), int(few.max(initial=0)), int(np.count_nonzero(q_lens[n0:n0 + n1] > 8 // group)),
+            int(kv_lens[:n0].max(initial=0)))
 
 
 # --------------------------------------------------------------------- emitter
@@ -669,8 +663,8 @@ def _native_tables(build, direct):
         L.ft_plan_free(handle)
     if direct:
         tabs["vnode_to_kv_entries"] = None
-    tabs["phase_node_nums"] = PhaseNodeNums([int(x) for x in info.phase_node_nums],
-                                            (info.few_tokens, info.few_longest, info.few_over_8_rows, info.many_longest))
+    tabs["phase_node_nums"] = [int(x) for x in info.phase_node_nums]
+    tabs["task_sizes"] = (info.few_tokens, info.few_longest, info.few_over_8_rows, info.many_longest)
     tabs["phase_node_offsets"] = [int(x) for x in info.phase_node_offsets]
     return tabs, [int(a) for a in assign], info
 

@@ -116,9 +116,9 @@ def fasttree_preparation(tree_info, KV_ptrs, batch_size, num_qo_heads, num_kv_he
     rows = plan.num_partial_rows
     mid_o = torch.empty((rows, num_qo_heads, head_dim), dtype=torch.float32, device=dev)
     mid_lse = torch.empty((rows, num_qo_heads), dtype=torch.float32, device=dev)
-    nums = _planner.PhaseNodeNums.of_tables(plan.phase_node_nums, plan.vnode_to_kv_lens, plan.vnode_to_q_lens,
-                                            max(1, num_qo_heads // num_kv_heads))
-    aux = tabs + (mid_o, mid_lse, nums, list(plan.phase_node_offsets))
+    tabs[2].task_sizes = plan.task_sizes or _planner.task_sizes(plan.phase_node_nums, plan.vnode_to_kv_lens, plan.vnode_to_q_lens,
+                                                                max(1, num_qo_heads // num_kv_heads))
+    aux = tabs + (mid_o, mid_lse, list(plan.phase_node_nums), list(plan.phase_node_offsets))
     return aux, plan.node_assignments
 
 

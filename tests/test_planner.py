@@ -507,23 +507,27 @@ def test_groups_at_other_head_dims_once_the_storage_type_is_stated(d, sizes, len
 
 @pytest.mark.parametrize("planner_name,native", [("reference", False), ("b200", False), ("b200", True)])
 def test_plans_state_their_task_sizes(planner_name, native):
-    """The sizes beside the phase counts are the emitted tables', they survive what a tuple of tables goes through, and the
-    counts stay an ordinary pair."""
+    """The sizes are the emitted tables'; as a tensor's attribute they survive what a tuple of tables goes through, and a
+    saved tuple still loads with torch's default of weights only."""
     import copy
-    import pickle
-    from ft_b200.planner import PhaseNodeNums
+    import io
+    import torch
     for sizes, lens, hq in (([1, 3, 12, 36], [300, 170, 900, 200], 32), ([1, 40], [2000, 130], 8), ([1], [77], 64)):
         tree, batch, ptrs = product_tree(ref_inputs.layered_tree(sizes, lens))
         p = make_params(hq, 8, [max(1, 512 // hq), max(1, 128 // hq)], planner_name=planner_name)
         p.native_planner = native
         plan = fasttree.build_plan(tree, ptrs, batch, hq, 8, 128, [1024, 128], [132, 528], [132, 132], p)
         n0, n1 = plan.phase_node_nums
-        nums = PhaseNodeNums.of_tables(plan.phase_node_nums, plan.vnode_to_kv_lens, plan.vnode_to_q_lens, hq // 8)
+        got = planner.task_sizes(plan.phase_node_nums, plan.vnode_to_kv_lens, plan.vnode_to_q_lens, hq // 8)
         few = plan.vnode_to_kv_lens[n0:n0 + n1].tolist()
         over = sum(hq // 8 * int(x) > 8 for x in plan.vnode_to_q_lens[n0:n0 + n1])
-        want = (sum(few), max(few, default=0), over, max(plan.vnode_to_kv_lens[:n0].tolist(), default=0))
-        for got in (nums, copy.deepcopy(nums), pickle.loads(pickle.dumps(nums))):
-            assert got == [n0, n1] and got.task_sizes == want
+        assert got == (sum(few), max(few, default=0), over, max(plan.vnode_to_kv_lens[:n0].tolist(), default=0))
+        assert plan.task_sizes == (got if native else None)
         if len(sizes) == 4:
             assert n1 > 0 and over > 0
-    assert PhaseNodeNums([3, 4]).task_sizes == (0, 0, 0, 0)
+        table = torch.from_numpy(plan.vnode_to_kv_lens)
+        table.task_sizes = got
+        saved = io.BytesIO()
+        torch.save((table, list(plan.phase_node_nums)), saved)
+        saved.seek(0)
+        assert torch.load(saved)[0].task_sizes == got and copy.deepcopy(table).task_sizes == got
