@@ -432,8 +432,9 @@ class Problem:
         self.engine.stage1(self.q, self.ks[c], self.vs[c], self.o, *self.aux, self.tsq, self.tsk, self.scale, path=self.path)
 
     def stage1_name(self):
-        return self.engine.stage1_path_name(self.q, self.ks[0], self.vs[0], self.o, *self.aux, self.tsq, self.tsk,
+        name = self.engine.stage1_path_name(self.q, self.ks[0], self.vs[0], self.o, *self.aux, self.tsq, self.tsk,
                                             self.scale, path=self.path)
+        return name.replace("/pair", "").replace("/eight", "")     # the forms of one kernel, by its own name
 
     def label(self):
         return workload_label(self.workload, self.desc, self.hq, self.hkv, self.dt)

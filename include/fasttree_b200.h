@@ -119,9 +119,10 @@ typedef struct ft_decode_args {
                                          nodes with disjoint request sets (their KV concatenated, each request
                                          seeing only its own node's tokens).  NULL = every row sees the whole
                                          chunk, as in the reference.  Honoured by the many-row kernels (tcgen05,
-                                         wide mma.sync) and by the generic kernel; the few-row kernels do not
-                                         read it, so rows of vnodes with <= 16 query rows must cover their whole
-                                         chunk (the planner of this library only narrows rows of many-row vnodes). */
+                                         wide mma.sync) and by the generic kernel; of the few-row kernels only the
+                                         one that runs two tasks per CTA reads it, so rows of vnodes with <= 16
+                                         query rows must cover their whole chunk (the planner of this library only
+                                         narrows rows of many-row vnodes). */
   const int32_t* device_phase_info;   /* NULL, or a DEVICE array {phase_node_nums[0], phase_node_nums[1],
                                          phase_node_offsets[0], phase_node_offsets[1]} that stage 1 reads at run
                                          time instead of the host values above (the two phases must be adjacent:
@@ -263,7 +264,8 @@ int ft_read_wait_diagnostics(int32_t* out8);
 int64_t ft_launch_count(void);
 
 /* Names of the kernels ft_stage1 would launch for these arguments, joined by '+' when there are two launches
- * (e.g. "stage1_fused_kernel", "stage1_tc_kernel+stage1_narrow_kernel"): the names a profiler shows.  Nothing is
+ * (e.g. "stage1_fused_kernel", "stage1_tc_kernel+stage1_narrow_kernel"): the names a profiler shows, the fused
+ * kernel's with "/pair" or "/eight" behind it where its few-row CTAs run two tasks, or one by eight warps.  Nothing is
  * launched.  NULL with ft_last_error() set when the arguments are rejected.  The text belongs to the calling
  * thread and is valid until its next call. */
 const char* ft_stage1_path_name(const ft_decode_args* args);
