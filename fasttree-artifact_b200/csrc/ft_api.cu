@@ -661,11 +661,7 @@ int launch_stage1_range(const ft_decode_args* a, int path, int offset, int count
 // the kernel be scheduled early (programmatic dependent launch): it reads the request tables before it waits for
 // the preceding kernel, which is safe after stage 1 (that kernel never writes them) but not after an arbitrary
 // kernel of the caller's that may still be building those tables.
-template <typename T>
-int launch_stage2(const ft::Stage2Params& p, cudaStream_t st, bool after_stage1) {
-  const int64_t pairs = (int64_t)p.batch * p.heads;
-  if (pairs == 0) return FT_OK;
-  const int64_t blocks = (pairs + 3) / 4;
+int launch_merge(void (*kernel)(ft::Stage2Params), const ft::Stage2Params& p, int64_t blocks, cudaStream_t st, bool after_stage1) {
   if (blocks > 0x7fffffffLL) return fail(FT_ERR_TOO_LARGE, "batch x heads too large for one launch");
   // launched with permission to be scheduled before the preceding kernel (stage 1) has drained; the kernel itself
   // waits for that kernel's completion before it touches the partial buffers
@@ -679,19 +675,44 @@ int launch_stage2(const ft::Stage2Params& p, cudaStream_t st, bool after_stage1)
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = after_stage1 ? 1 : 0;
-  int dev = 0;
-  FT_CUDA_OK(cudaGetDevice(&dev));
-  const bool one_round = blocks <= 6LL * sm_count(dev);  // latency-bound: more rows in flight per lane
-  if (p.head_dim > 128)
-    FT_CUDA_OK(cudaLaunchKernelEx(&cfg, ft::stage2_merge_kernel<T, 2, 4>, p));
-  else if (blocks <= 2LL * sm_count(dev))
-    FT_CUDA_OK(cudaLaunchKernelEx(&cfg, ft::stage2_merge_kernel<T, 1, 16>, p));
-  else if (one_round)
-    FT_CUDA_OK(cudaLaunchKernelEx(&cfg, ft::stage2_merge_kernel<T, 1, 8>, p));
-  else
-    FT_CUDA_OK(cudaLaunchKernelEx(&cfg, ft::stage2_merge_kernel<T, 1, 4>, p));
+  FT_CUDA_OK(cudaLaunchKernelEx(&cfg, kernel, p));
   count_launch();
   return FT_OK;
+}
+
+template <typename T, int C, int RB, int SPLIT>
+int launch_pieces(ft::Stage2Params p, cudaStream_t st, bool after_stage1) {
+  p.pieces = (uint32_t)((((int64_t)p.heads << p.dim_shift) + 128 * C - 1) / (128 * C));
+  const int64_t items = (int64_t)p.batch * p.pieces;
+  if (items > 0x7fffffffLL) return fail(FT_ERR_TOO_LARGE, "batch x heads too large for one launch");
+  p.items = (uint32_t)items;
+  return launch_merge(ft::stage2_piece_kernel<T, C, RB, SPLIT>, p, SPLIT == 1 ? (items + 3) / 4 : items, st, after_stage1);
+}
+
+// Which merge, by the 128-float pieces of the output and the mean number of partial rows per request (an upper bound where
+// the scratch buffers hold more rows than the plan).  us for the merge alone, replayed from a graph, and per decode step:
+//   few pieces, many rows: four warps per piece    160 pieces x 36 rows, one warp per head 5.9 / four 3.9 (step 13.8 / 11.8),
+//                                                  32 x 18 4.2 / 2.9 (12.2 / 9.9); 1024 x 9 3.7 / 3.4, 2048 x 9 4.1 / 5.2
+//   one round of CTAs with more than four rows, or six rows and more: weights by one lane per row
+//                                                  2048 x 7, step, 25.7 (by every lane 26.7); 8192 x 18 11.3 (14.1)
+//   fewer rows: weights by every lane              16384 heads of 64 x 3.4 9.0 -> 4.9 (step 37.0 -> 33.1), 8192 x 4 6.1 -> 5.6
+//   very many pieces: two of them per warp         65536 x 2 33.8 -> 21.2, 32768 x 3 20.9 -> 17.0 (one piece 18.7)
+// At head_dim 64 and below one lane per row would leave half of the lanes and more idle: 8192 pieces x 18 rows 19.3 / 13.8.
+template <typename T>
+int launch_stage2(const ft::Stage2Params& p, cudaStream_t st, bool after_stage1) {
+  const int64_t pieces = (((int64_t)p.batch * p.heads << p.dim_shift) + 127) / 128, heads = (int64_t)p.batch * p.heads;
+  if (pieces == 0) return FT_OK;
+  const int64_t rows = p.num_partial_rows, batch = p.batch;
+  if (pieces <= 1024 && rows >= 6 * batch)
+    return rows >= 12 * batch ? launch_pieces<T, 1, 8, 4>(p, st, after_stage1) : launch_pieces<T, 1, 4, 4>(p, st, after_stage1);
+  int dev = 0;
+  FT_CUDA_OK(cudaGetDevice(&dev));
+  const bool one_round = heads <= 24LL * sm_count(dev);
+  if (p.head_dim >= 128 && ((one_round && rows > 4 * batch) || rows >= 6 * batch)) {
+    auto* kernel = p.head_dim > 128 ? ft::stage2_merge_kernel<T, 2, 4> : one_round ? ft::stage2_merge_kernel<T, 1, 8> : ft::stage2_merge_kernel<T, 1, 4>;
+    return launch_merge(kernel, p, (heads + 3) / 4, st, after_stage1);
+  }
+  return pieces <= 16384 ? launch_pieces<T, 1, 4, 1>(p, st, after_stage1) : launch_pieces<T, 2, 2, 1>(p, st, after_stage1);
 }
 
 __global__ void bump_kv_lens_kernel(int32_t* kv_lens, const int32_t* last, int n) {
@@ -814,6 +835,7 @@ int stage2_impl(const ft_decode_args* a, bool after_stage1) {
   p.batch = a->batch;
   p.heads = a->num_qo_heads;
   p.head_dim = a->head_dim;
+  for (p.dim_shift = 0; (1 << p.dim_shift) < a->head_dim;) ++p.dim_shift;
   {
     const int64_t esz = a->dtype == FT_F32 ? 4 : 2, vec = 4 * esz;  // bytes of one 4-element store
     p.o_vec = (reinterpret_cast<uintptr_t>(a->o) % vec == 0 && (a->o_stride0 * esz) % vec == 0 &&

@@ -134,7 +134,10 @@ struct Stage2Params {
   int64_t num_partial_rows;
   int32_t batch;
   int32_t heads;
-  int32_t head_dim;
+  int32_t head_dim;   // a power of two, 1 << dim_shift
+  int32_t dim_shift;
+  uint32_t pieces;    // warps' worth of floats in a partial row
+  uint32_t items;      // requests x pieces
   int32_t o_vec;  // 1: o rows are aligned for 4-element vector stores
 };
 
