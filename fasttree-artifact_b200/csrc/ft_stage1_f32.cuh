@@ -10,8 +10,14 @@
 //                scheduler: the arithmetic of a tile is one dependent chain per warp,
 //                and with four warps of four rows a tile took twice as long)
 //   softmax      a row's 32 scores sit in the 32 lanes of one warp: shuffles
-//   O[16 x D]    thread owns columns lane, lane+32, ... of its warp's 2 rows; the
-//                probabilities are broadcast by shuffle, V read conflict-free
+//   O[16 x D]    thread owns D / 32 adjacent columns of its warp's 2 rows; the
+//                probabilities go through shared memory
+// Everything in shared memory is read 16 bytes at a time (8 of V at head_dim 64): the K
+// tile passes through shared memory once per warp, which bounds a tile's arithmetic, and
+// a word at a time the reads' issue did.  With that and the first reads sent off together
+// (before: the Q rows, then the row ids, then the K and V rows) stage 1 of 4 requests on
+// 512 tokens, 8/2 heads of 128, takes 7.0 us (7.6), of 40 requests of 300 tokens on 500,
+// 16/16 heads, 173 (196), of 64 requests of 100 on 1000, 32/8 heads of 64, 66 (78).
 // Same conventions as the other stage-1 kernels (kernel_bench/fasttree.py:360-413):
 // scores scaled after the dot product, normalised partial output, lse = log(sum) + max;
 // optional per-row token ranges; bad indices are skipped and flagged.
@@ -26,10 +32,11 @@ template <int D>
 struct F32Cfg {
   static constexpr int ROWS = 16, TILE = 32, THREADS = 256;
   static constexpr int WARPS = THREADS / 32, RPW = ROWS / WARPS;  // rows per warp
-  static constexpr int KSTRIDE = D + 1;              // floats between K rows: lane = token reads are conflict-free
+  static constexpr int KSTRIDE = D + 4;              // floats between K rows: lane = token 16-byte reads are conflict-free
   static constexpr int Q_FLOATS = ROWS * D, K_FLOATS = TILE * KSTRIDE, V_FLOATS = TILE * D;
   static constexpr int K_OFF = ((Q_FLOATS + 3) / 4) * 4, V_OFF = ((K_OFF + K_FLOATS + 3) / 4) * 4;
-  static constexpr int SMEM_BYTES = (V_OFF + V_FLOATS) * 4;
+  static constexpr int P_OFF = V_OFF + V_FLOATS;     // ROWS x TILE probabilities
+  static constexpr int SMEM_BYTES = (P_OFF + ROWS * TILE) * 4;
   static constexpr int C4 = D / 4;                   // float4 chunks per row
   static constexpr int LOADS = TILE * C4 / THREADS;  // float4 loads per thread per operand per tile
 };
@@ -43,6 +50,7 @@ __global__ void __launch_bounds__(256, D == 64 ? 4 : 3) stage1_f32_kernel(const 
   float* q_s = smem_f32;
   float* k_s = smem_f32 + C::K_OFF;
   float* v_s = smem_f32 + C::V_OFF;
+  float* p_s = smem_f32 + C::P_OFF;
   const int vn = blockIdx.x + p.node_offset, kvh = blockIdx.y, row0 = blockIdx.z * C::ROWS;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int q_off = p.q_offs[vn], q_len = p.q_lens[vn];
@@ -57,37 +65,42 @@ __global__ void __launch_bounds__(256, D == 64 ? 4 : 3) stage1_f32_kernel(const 
   const float* kbase = reinterpret_cast<const float*>(p.k) + (int64_t)kvh * p.k_s1;
   const float* vbase = reinterpret_cast<const float*>(p.v) + (int64_t)kvh * p.v_s1;
 
-  // ---- Q rows of this block -> shared memory (zeros for rows past the end or with a bad index)
-  for (int i = tid; i < C::ROWS * C::C4; i += C::THREADS) {
-    const int r = i / C::C4, c4 = i - r * C::C4;
-    float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+  // The reads that everything waits for go out together: a thread's row ids of tile 0 and the request ids of its Q rows,
+  // then the K, V and Q rows themselves.  (A row's Q float4s: thread tid has number tid % C4 of rows tid / C4 + RPQ u.)
+  constexpr int RPQ = C::THREADS / C::C4, QLOADS = C::ROWS / RPQ;
+  const int q_c4 = tid % C::C4;
+  int q_req[QLOADS];
+#pragma unroll
+  for (int u = 0; u < QLOADS; ++u) {
+    const int r = tid / C::C4 + RPQ * u;
+    q_req[u] = -1;
     if (r < rows) {
-      const int prow = row0 + r, slot = prow / G, gg = prow - slot * G;
-      const int64_t part = (int64_t)q_off + slot;
-      if (part >= 0 && part < p.num_partial_rows) {
-        const int req = p.q_entries[part];
-        if (req >= 0 && req < p.batch)
-          x = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p.q) + (int64_t)req * p.q_s0 +
-                                               (int64_t)(kvh * G + gg) * p.q_s1 + 4 * c4);
-        else if (c4 == 0)
-          flag_error(FT_DEV_BAD_Q_INDEX);
-      } else if (c4 == 0) {
+      const int64_t part = (int64_t)q_off + (row0 + r) / G;
+      if (part >= 0 && part < p.num_partial_rows)
+        q_req[u] = p.q_entries[part];
+      else if (q_c4 == 0)
         flag_error(FT_DEV_BAD_ROW_INDEX);
-      }
     }
-    *reinterpret_cast<float4*>(q_s + r * D + 4 * c4) = x;
   }
-
   // per-thread state: rows warp + WARPS * i
-  constexpr int RPW = C::RPW, NW = C::WARPS;
-  float m_run[RPW], l_run[RPW], acc[RPW][D / 32];
+  constexpr int RPW = C::RPW, NW = C::WARPS, CPL = D / 32;  // CPL: columns per lane
+  auto load_cols = [](float (&x)[CPL], const float* src) {
+    if constexpr (CPL == 4) {
+      const float4 y = *reinterpret_cast<const float4*>(src);
+      x[0] = y.x, x[1] = y.y, x[2] = y.z, x[3] = y.w;
+    } else {
+      const float2 y = *reinterpret_cast<const float2*>(src);
+      x[0] = y.x, x[1] = y.y;
+    }
+  };
+  float m_run[RPW], l_run[RPW], acc[RPW][CPL];
   int r_lo[RPW], r_hi[RPW];
 #pragma unroll
   for (int i = 0; i < RPW; ++i) {
     m_run[i] = -INFINITY;
     l_run[i] = 0.f;
 #pragma unroll
-    for (int j = 0; j < D / 32; ++j) acc[i][j] = 0.f;
+    for (int j = 0; j < CPL; ++j) acc[i][j] = 0.f;
     r_lo[i] = 0;
     r_hi[i] = kv_len;
     const int r = warp + NW * i;
@@ -102,25 +115,26 @@ __global__ void __launch_bounds__(256, D == 64 ? 4 : 3) stage1_f32_kernel(const 
 
   const int ntiles = (kv_len + C::TILE - 1) / C::TILE;
   float4 kreg[C::LOADS], vreg[C::LOADS];
-  // the tile's rows -> registers (zeros for padding and bad row ids)
+  // row ids of tile t (-1: padding), then its rows -> registers (zeros for padding and bad row ids)
+  int idreg[C::LOADS];
+  auto fetch_ids = [&](int t) {
+#pragma unroll
+    for (int u = 0; u < C::LOADS; ++u) {
+      const int pos = t * C::TILE + (u * C::THREADS + tid) / C::C4;
+      idreg[u] = pos < id_lim ? ids[pos] : -1;
+    }
+  };
   auto fetch = [&](int t) {
     bool bad = false;
 #pragma unroll
     for (int u = 0; u < C::LOADS; ++u) {
-      const int i = u * C::THREADS + tid, tok = i / C::C4, c4 = i - tok * C::C4;
-      const int pos = t * C::TILE + tok;
-      int64_t row = -1;
-      if (pos < kv_len) {
-        if (pos < id_lim) row = ids[pos];
-        if (row < 0 || row >= p.kv_rows) {
-          bad = true;
-          row = -1;
-        }
-      }
-      if (row >= 0) {
+      const int i = u * C::THREADS + tid, c4 = i % C::C4;
+      const int64_t row = idreg[u];
+      if (row >= 0 && row < p.kv_rows) {
         kreg[u] = __ldg(reinterpret_cast<const float4*>(kbase + row * p.k_s0) + c4);
         vreg[u] = __ldg(reinterpret_cast<const float4*>(vbase + row * p.v_s0) + c4);
       } else {
+        bad |= t * C::TILE + i / C::C4 < kv_len;
         kreg[u] = vreg[u] = make_float4(0.f, 0.f, 0.f, 0.f);
       }
     }
@@ -130,37 +144,50 @@ __global__ void __launch_bounds__(256, D == 64 ? 4 : 3) stage1_f32_kernel(const 
 #pragma unroll
     for (int u = 0; u < C::LOADS; ++u) {
       const int i = u * C::THREADS + tid, tok = i / C::C4, c4 = i - tok * C::C4;
-      float* kd = k_s + tok * C::KSTRIDE + 4 * c4;
-      kd[0] = kreg[u].x;
-      kd[1] = kreg[u].y;
-      kd[2] = kreg[u].z;
-      kd[3] = kreg[u].w;
+      *reinterpret_cast<float4*>(k_s + tok * C::KSTRIDE + 4 * c4) = kreg[u];
       *reinterpret_cast<float4*>(v_s + tok * D + 4 * c4) = vreg[u];
     }
   };
 
-  if (ntiles > 0) fetch(0);
+  fetch_ids(0);
+  fetch(0);
+  if (ntiles > 1) fetch_ids(1);
+  // ---- Q rows of this block -> shared memory (zeros for rows past the end or with a bad index)
+#pragma unroll
+  for (int u = 0; u < QLOADS; ++u) {
+    const int r = tid / C::C4 + RPQ * u;
+    float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (q_req[u] >= 0 && q_req[u] < p.batch)
+      x = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p.q) + (int64_t)q_req[u] * p.q_s0 +
+                                           (int64_t)(kvh * G + (row0 + r) % G) * p.q_s1 + 4 * q_c4);
+    else if (r < rows && q_c4 == 0)
+      flag_error(FT_DEV_BAD_Q_INDEX);
+    *reinterpret_cast<float4*>(q_s + r * D + 4 * q_c4) = x;
+  }
   for (int t = 0; t < ntiles; ++t) {
-    __syncthreads();  // the previous tile has been consumed (and, at t = 0, Q is in place)
+    if (t > 0) __syncthreads();  // the previous tile has been consumed
     stash();
-    __syncthreads();
-    if (t + 1 < ntiles) fetch(t + 1);  // in flight during the arithmetic below
+    __syncthreads();  // (at t = 0, Q is in place too)
+    if (t + 1 < ntiles) {  // in flight during the arithmetic below
+      fetch(t + 1);
+      if (t + 2 < ntiles) fetch_ids(t + 2);
+    }
 
     // ---- S = Q K^T for this thread's rows and its token
     float s[RPW];
 #pragma unroll
     for (int i = 0; i < RPW; ++i) s[i] = 0.f;
-    const float* kr = k_s + lane * C::KSTRIDE;
-#pragma unroll 4
+    const float4* kr = reinterpret_cast<const float4*>(k_s + lane * C::KSTRIDE);
+#pragma unroll 8
     for (int d4 = 0; d4 < C::C4; ++d4) {
-      const float k0 = kr[4 * d4], k1 = kr[4 * d4 + 1], k2 = kr[4 * d4 + 2], k3 = kr[4 * d4 + 3];
+      const float4 kv = kr[d4];
 #pragma unroll
       for (int i = 0; i < RPW; ++i) {
         const float4 qv = *reinterpret_cast<const float4*>(q_s + (warp + NW * i) * D + 4 * d4);
-        s[i] = fmaf(qv.x, k0, s[i]);
-        s[i] = fmaf(qv.y, k1, s[i]);
-        s[i] = fmaf(qv.z, k2, s[i]);
-        s[i] = fmaf(qv.w, k3, s[i]);
+        s[i] = fmaf(qv.x, kv.x, s[i]);
+        s[i] = fmaf(qv.y, kv.y, s[i]);
+        s[i] = fmaf(qv.z, kv.z, s[i]);
+        s[i] = fmaf(qv.w, kv.w, s[i]);
       }
     }
     // ---- online softmax per row (32 tokens = 32 lanes)
@@ -179,22 +206,31 @@ __global__ void __launch_bounds__(256, D == 64 ? 4 : 3) stage1_f32_kernel(const 
       pr[i] = seen ? expf(x - m_new) : 0.f;
       l_run[i] = l_run[i] * corr + warp_sum(pr[i]);
 #pragma unroll
-      for (int j = 0; j < D / 32; ++j) acc[i][j] *= corr;
+      for (int j = 0; j < CPL; ++j) acc[i][j] *= corr;
       m_run[i] = m_new;
     }
     // ---- O += P V
-#pragma unroll 4
-    for (int tok = 0; tok < C::TILE; ++tok) {
-      float vv[D / 32];
 #pragma unroll
-      for (int j = 0; j < D / 32; ++j) vv[j] = v_s[tok * D + lane + 32 * j];
+    for (int i = 0; i < RPW; ++i) p_s[(warp + NW * i) * C::TILE + lane] = pr[i];
+    __syncwarp();
+#pragma unroll 2
+    for (int t4 = 0; t4 < C::TILE; t4 += 4) {
+      float4 w[RPW];
 #pragma unroll
-      for (int i = 0; i < RPW; ++i) {
-        const float w = __shfl_sync(0xffffffffu, pr[i], tok);
+      for (int i = 0; i < RPW; ++i) w[i] = *reinterpret_cast<const float4*>(p_s + (warp + NW * i) * C::TILE + t4);
 #pragma unroll
-        for (int j = 0; j < D / 32; ++j) acc[i][j] = fmaf(w, vv[j], acc[i][j]);
+      for (int k = 0; k < 4; ++k) {
+        float vv[CPL];
+        load_cols(vv, v_s + (t4 + k) * D + CPL * lane);
+#pragma unroll
+        for (int i = 0; i < RPW; ++i) {
+          const float wk = k == 0 ? w[i].x : k == 1 ? w[i].y : k == 2 ? w[i].z : w[i].w;
+#pragma unroll
+          for (int j = 0; j < CPL; ++j) acc[i][j] = fmaf(wk, vv[j], acc[i][j]);
+        }
       }
     }
+    __syncwarp();  // before the next tile's probabilities
   }
 
   // ---- normalise and write the partial rows
@@ -208,14 +244,16 @@ __global__ void __launch_bounds__(256, D == 64 ? 4 : 3) stage1_f32_kernel(const 
     if (part < 0 || part >= p.num_partial_rows) continue;
     const int head = kvh * G + gg;
     const float inv = l_run[i] > 0.f ? 1.f / l_run[i] : 0.f;
-    float* op = p.mid_o + part * p.mo_s0 + (int64_t)head * p.mo_s1;
-#pragma unroll
-    for (int j = 0; j < D / 32; ++j) op[lane + 32 * j] = acc[i][j] * inv;
+    float* op = p.mid_o + part * p.mo_s0 + (int64_t)head * p.mo_s1 + CPL * lane;
+    if constexpr (CPL == 4)
+      *reinterpret_cast<float4*>(op) = make_float4(acc[i][0] * inv, acc[i][1] * inv, acc[i][2] * inv, acc[i][3] * inv);
+    else
+      *reinterpret_cast<float2*>(op) = make_float2(acc[i][0] * inv, acc[i][1] * inv);
     if (lane == 0) p.mid_lse[part * p.ml_s0 + head] = l_run[i] > 0.f ? logf(l_run[i]) + m_run[i] : -INFINITY;
     if (r_lo[i] > 0 || r_hi[i] < kv_len) {
       float finite = 0.f;  // 0 x every element: 0, or NaN
 #pragma unroll
-      for (int j = 0; j < D / 32; ++j) finite = fmaf(acc[i][j], 0.f, finite);
+      for (int j = 0; j < CPL; ++j) finite = fmaf(acc[i][j], 0.f, finite);
       if (__any_sync(0xffffffffu, !(finite == 0.f))) todo |= 1u << i;
     }
   }
