@@ -22,7 +22,7 @@ Two planners, selected by ``FastTreeMetadata.planner``:
   kernel) and starts each tail where the radix walk actually stopped, so prompt
   tokens that are not in the cache are still attended to.
 """
-from collections import defaultdict, deque
+from collections import deque
 
 import numpy as np
 import torch
@@ -35,7 +35,7 @@ def _walk_requests(batch):
     """Per request, follow the radix tree along prompt + generated tokens
     (schedule.py:18-35).  Returns (node -> request ids, tokens covered per request)."""
     root = batch.tree_cache.root_node
-    node_to_reqs = defaultdict(list)
+    seen = {}           # node -> (request ids, tokens)
     covered = []
     for rid, req in enumerate(batch.reqs):
         prompt, output = req.origin_input_ids, req.output_ids
@@ -46,11 +46,19 @@ def _walk_requests(batch):
             child = node.children.get(prompt[pos] if pos < n_prompt else output[pos - n_prompt])
             if not child:
                 break
-            node_to_reqs[child].append(rid)
+            entry = seen.get(child)
+            if entry is None:
+                entry = seen[child] = ([], len(child.key))
+            entry[0].append(rid)
             node = child
-            pos += len(child.key)
+            pos += entry[1]
         covered.append(pos)
-    return node_to_reqs, covered
+    return {node: reqs for node, (reqs, _) in seen.items()}, covered
+
+
+def _length(value):
+    """Entries of a radix node's value: a 1-D tensor, or a list (a tensor's ``len`` costs a microsecond per node)."""
+    return value.numel() if isinstance(value, torch.Tensor) else len(value)
 
 
 def _bfs(batch, node_to_reqs):
@@ -63,7 +71,7 @@ def _bfs(batch, node_to_reqs):
         order.append(node)
         offsets.append(off)
         parents.append(par)
-        lens.append(len(node.value))
+        lens.append(_length(node.value))
         nxt = off + lens[me]
         for child in node.children.values():
             if child in node_to_reqs:
@@ -264,14 +272,19 @@ def _plan_b200(batch, md, node_to_reqs, covered, order, offsets, parents, lens, 
                                     order_key=_planner.b200_task_order)
         return tabs, q_tile, small_tile, model.tile_tokens
 
-    tabs, q_tile, small_tile, tile_tokens = run(-1, model)
-    if getattr(md, "group_tails", False):
+    # Every request has a few-row tail task of its own in a plan without groups: where those alone pass the bound below,
+    # that plan would only be made to be replaced.
+    bound = md.group_tails_min_load * model.num_sms * model.ctas_per_sm if getattr(md, "group_tails", False) else None
+    tabs = None
+    if bound is None or bsz * md.num_kv_heads < bound:
+        tabs, q_tile, small_tile, tile_tokens = run(-1, model)
+    if bound is not None:
         # Groups pay when the few-row tasks alone would queue up several deep behind the resident CTAs; then the
         # burst is planned again with short runs packed into many-row vnodes.  A group needs more than 16 query
         # rows anyway (only the many-row kernels honour row ranges); past that, a handful of one-tile tails
         # already costs less as one task than as one task each.
-        few_row_ctas = tabs["phase_node_nums"][1] * md.num_kv_heads
-        if few_row_ctas >= md.group_tails_min_load * model.num_sms * model.ctas_per_sm:
+        few_row_ctas = (bsz if tabs is None else tabs["phase_node_nums"][1]) * md.num_kv_heads
+        if few_row_ctas >= bound:
             from dataclasses import replace
             tabs, q_tile, small_tile, tile_tokens = run(
                 md.tail_room, replace(model, group_min_members=min(model.group_min_members, 4)))
