@@ -267,6 +267,53 @@ int build_plan(const int32_t* parent, const int32_t* seqlen, int32_t n_nodes, co
       s.chunk = ceil_div(ceil_div(s.length, n_chunks), m.tile_tokens) * m.tile_tokens;
     }
 
+    // List schedule, in emission order, of the tasks that virtual nodes of these sizes are cut into (integer time: a fixed
+    // cost per task plus one unit per KV tile; a task = the CTAs of all KV heads of one chunk x request tile, which start
+    // side by side): its length, the time of all tasks together, and the end of every node's last task.
+    struct Piece {
+      int64_t length, chunk, nreq;
+    };
+    const int64_t sched_slots = std::max<int64_t>((int64_t)(m.num_sms * m.ctas_per_sm) / std::max(num_kv_heads, 1), 1);
+    auto simulate = [&](const std::vector<Piece>& pieces, std::vector<int64_t>& last_end, int64_t& total) {
+      const int64_t start_cost[2] = {5, 4};  // many-row / few-row task, in tile times
+      struct SimTask {
+        int phase;
+        int64_t key, dur;
+        size_t piece;
+      };
+      std::vector<SimTask> tasks;
+      for (size_t i = 0; i < pieces.size(); ++i) {
+        const Piece& s = pieces[i];
+        if (s.nreq == 0 || s.length <= 0) continue;
+        const int64_t n_kv = ceil_div(s.length, s.chunk), n_q = ceil_div(s.nreq, q_tile);
+        for (int64_t c = 0; c < n_kv; ++c) {
+          const int64_t c_len = std::min((c + 1) * s.chunk, s.length) - c * s.chunk;
+          for (int64_t t = 0; t < n_q; ++t) {
+            const int64_t q_len = std::min((t + 1) * (int64_t)q_tile, s.nreq) - t * q_tile;
+            const int phase = q_len > small_tile ? 0 : 1;
+            tasks.push_back({phase, c_len * 64 + std::min<int64_t>(q_len, 63), start_cost[phase] + ceil_div(c_len, m.tile_tokens), i});
+          }
+        }
+      }
+      std::stable_sort(tasks.begin(), tasks.end(), [](const SimTask& a, const SimTask& b) {
+        return a.phase != b.phase ? a.phase < b.phase : a.key > b.key;
+      });
+      std::priority_queue<int64_t, std::vector<int64_t>, std::greater<int64_t>> free_at;
+      for (int64_t k = 0; k < sched_slots; ++k) free_at.push(0);
+      last_end.assign(pieces.size(), 0);
+      int64_t makespan = 0;
+      total = 0;
+      for (const SimTask& t : tasks) {
+        const int64_t start = free_at.top();
+        free_at.pop();
+        free_at.push(start + t.dur);
+        last_end[t.piece] = std::max(last_end[t.piece], start + t.dur);
+        makespan = std::max(makespan, start + t.dur);
+        total += t.dur;
+      }
+      return makespan;
+    };
+
     // ---- groups of short nodes (table-building mode, 16-bit elements, head_dim 64, 128 or 256: the shapes whose
     // kernels honour per-row token ranges; serving path: head_dim 128).  Candidates - at most small_tile requests, at most group_member_tokens tokens - are
     // taken in order; a group is closed when the next candidate would exceed q_tile requests or 16 tiles of tokens,
@@ -282,9 +329,11 @@ int build_plan(const int32_t* parent, const int32_t* seqlen, int32_t n_nodes, co
       int64_t hard_cap = 16 * tile;
       int64_t cap = std::min(std::max(target_tokens / tile * tile, 4 * tile), hard_cap);
       if (direct != nullptr) {
-        // Serving path: the groups are sized so that the step fills two rounds of resident CTAs, the other tasks
-        // included (measured: their tiles are gathered row by row, and two shorter groups per slot hide that latency
-        // better than one long one, while a third round costs more than it hides), up to 24 tiles.
+        // Serving path: groups of up to 24 tiles, sized so that the step, the other tasks included, fills a number of rounds of
+        // resident CTAs: two, unless the simulated schedule of another of these numbers (in quarters) ends sooner.  How the
+        // longest tasks fall on the slots matters more than their mean (512 requests under 4 prompts, 16 other tasks on 37
+        // slots, us of stage 1 and the schedule's time units at 1 / 1.25 / 1.5 / 2 / 2.25 / 2.5 / 3 rounds:
+        // 48.3 / 40.7 / 48.2 / 43.8 / 42.1 / 55.9 / 52.9 and 26 / 24 / 29 / 27 / 26 / 36 / 33).
         int64_t cand_tokens = 0, other = 0;
         for (const Spec& s : specs) {
           const int64_t nreq = (int64_t)s.reqs.size();
@@ -292,9 +341,52 @@ int build_plan(const int32_t* parent, const int32_t* seqlen, int32_t n_nodes, co
           else other += ceil_div(s.length, s.chunk) * ceil_div(nreq, q_tile);
         }
         const int64_t round = std::max<int64_t>((int64_t)slots / std::max(num_kv_heads, 1), 1);
-        const int64_t free_tasks = std::max<int64_t>(std::max(2 * round - other, round / 2), 2);
         hard_cap = 24 * tile;
-        cap = std::min(std::max(ceil_div(ceil_div(cand_tokens, free_tasks), tile) * tile, 4 * tile), hard_cap);
+        std::vector<int64_t> tried, last_end;
+        std::vector<uint8_t> taken((size_t)std::max(batch, 1), 0);
+        int64_t best_end = -1;
+        for (const int64_t quarters : {8, 5, 9, 6, 7, 4}) {
+          const int64_t free_tasks = std::max<int64_t>(std::max(quarters * round / 4 - other, round / 2), 2);
+          const int64_t c = std::min(std::max(ceil_div(ceil_div(cand_tokens, free_tasks), tile) * tile, 4 * tile), hard_cap);
+          if (std::find(tried.begin(), tried.end(), c) != tried.end()) continue;
+          tried.push_back(c);
+          // the sizes that the grouping below would come out with
+          std::vector<Piece> kept, tail;
+          std::vector<const Spec*> cur;
+          int64_t cur_tokens = 0, cur_n = 0, total = 0;
+          auto close = [&]() {
+            for (const Spec* s : cur)
+              for (int32_t r : s->reqs) taken[r] = 0;
+            if ((int64_t)cur.size() >= m.group_min_members && cur_n > small_tile)
+              tail.push_back({cur_tokens, ceil_div(cur_tokens, tile) * tile, cur_n});
+            else
+              for (const Spec* s : cur) tail.push_back({s->length, s->chunk, (int64_t)s->reqs.size()});
+            cur.clear();
+            cur_tokens = cur_n = 0;
+          };
+          for (const Spec& s : specs) {
+            const int64_t nreq = (int64_t)s.reqs.size(), span = s.length + s.room;
+            if (nreq > small_tile || span > m.group_member_tokens) {
+              kept.push_back({s.length, s.chunk, nreq});
+              continue;
+            }
+            bool shared = false;
+            for (int32_t r : s.reqs) shared = shared || taken[r] != 0;
+            if (!cur.empty() && (cur_n + nreq > q_tile || cur_tokens + span > hard_cap || (cur_tokens >= c && cur_n > small_tile) || shared))
+              close();
+            for (int32_t r : s.reqs) taken[r] = 1;
+            cur_tokens += span;
+            cur_n += nreq;
+            cur.push_back(&s);
+          }
+          close();
+          kept.insert(kept.end(), tail.begin(), tail.end());
+          const int64_t end = simulate(kept, last_end, total);
+          if (best_end < 0 || end < best_end) {
+            best_end = end;
+            cap = c;
+          }
+        }
       }
       else {
         // One round: when the tasks at the default cap would spill a little past one round of resident CTAs while
@@ -370,64 +462,23 @@ int build_plan(const int32_t* parent, const int32_t* seqlen, int32_t n_nodes, co
     // task that ends in the later half of that excess is cut to half its chunk length (never below min_chunk); the
     // cut is kept if the simulated makespan drops.  (A step of one round lasts as long as its longest task: same cut.)
     if (direct == nullptr) {
-      const int64_t start_cost[2] = {5, 4};  // many-row / few-row task, in tile times
-      const int64_t sched_slots = std::max<int64_t>((int64_t)(m.num_sms * m.ctas_per_sm) / std::max(num_kv_heads, 1), 1);
-      struct SimTask {
-        int phase;
-        int64_t key, seq, dur;
-        size_t spec;
-      };
-      auto simulate = [&](const std::vector<int64_t>& chunk_of, std::vector<int64_t>& last_end, int64_t& total) {
-        std::vector<SimTask> tasks;
-        for (size_t si = 0; si < specs.size(); ++si) {
-          const Spec& s = specs[si];
-          const int64_t nreq = (int64_t)s.reqs.size();
-          if (nreq == 0 || s.length <= 0) continue;
-          const int64_t n_kv = ceil_div(s.length, chunk_of[si]), n_q = ceil_div(nreq, q_tile);
-          for (int64_t c = 0; c < n_kv; ++c) {
-            const int64_t c_len = std::min((c + 1) * chunk_of[si], s.length) - c * chunk_of[si];
-            for (int64_t t = 0; t < n_q; ++t) {
-              const int64_t q_len = std::min((t + 1) * (int64_t)q_tile, nreq) - t * q_tile;
-              const int phase = q_len > small_tile ? 0 : 1;
-              tasks.push_back({phase, c_len * 64 + std::min<int64_t>(q_len, 63), (int64_t)tasks.size(),
-                               start_cost[phase] + ceil_div(c_len, m.tile_tokens), si});
-            }
-          }
-        }
-        std::stable_sort(tasks.begin(), tasks.end(), [](const SimTask& a, const SimTask& b) {
-          return a.phase != b.phase ? a.phase < b.phase : a.key > b.key;
-        });
-        std::priority_queue<int64_t, std::vector<int64_t>, std::greater<int64_t>> free_at;
-        for (int64_t k = 0; k < sched_slots; ++k) free_at.push(0);
-        last_end.assign(specs.size(), 0);
-        int64_t makespan = 0;
-        total = 0;
-        for (const SimTask& t : tasks) {
-          const int64_t start = free_at.top();
-          free_at.pop();
-          free_at.push(start + t.dur);
-          last_end[t.spec] = std::max(last_end[t.spec], start + t.dur);
-          makespan = std::max(makespan, start + t.dur);
-          total += t.dur;
-        }
-        return makespan;
-      };
-      std::vector<int64_t> chunk_of(specs.size()), last_end;
-      for (size_t si = 0; si < specs.size(); ++si) chunk_of[si] = specs[si].chunk;
+      std::vector<Piece> pieces;
+      std::vector<int64_t> last_end;
+      for (const Spec& s : specs) pieces.push_back({s.length, s.chunk, (int64_t)s.reqs.size()});
       int64_t total = 0;
-      const int64_t makespan = simulate(chunk_of, last_end, total);
+      const int64_t makespan = simulate(pieces, last_end, total);
       const int64_t bound = ceil_div(total, sched_slots);
       if ((makespan - bound) * 8 > makespan) {
         const int64_t late_from = makespan - (makespan - bound + 1) / 2;
-        std::vector<int64_t> trial(chunk_of);
+        std::vector<Piece> trial(pieces);
         bool any = false;
         for (size_t si = 0; si < specs.size(); ++si) {
           const Spec& s = specs[si];
           if (!s.row_ranges.empty() || last_end[si] <= late_from) continue;
-          const int64_t cur = std::min(chunk_of[si], s.length);
+          const int64_t cur = std::min(s.chunk, s.length);
           const int64_t half = ceil_div(ceil_div(cur, 2), m.tile_tokens) * m.tile_tokens;
           if (half >= m.min_chunk && half < cur) {
-            trial[si] = half;
+            trial[si].chunk = half;
             any = true;
           }
         }
@@ -435,7 +486,7 @@ int build_plan(const int32_t* parent, const int32_t* seqlen, int32_t n_nodes, co
           std::vector<int64_t> fs2;
           int64_t total2 = 0;
           if (simulate(trial, fs2, total2) < makespan)
-            for (size_t si = 0; si < specs.size(); ++si) specs[si].chunk = trial[si];
+            for (size_t si = 0; si < specs.size(); ++si) specs[si].chunk = trial[si].chunk;
         }
       }
     }

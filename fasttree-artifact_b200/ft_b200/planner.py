@@ -30,6 +30,7 @@ import numpy as np
 PAD_ENTRIES = 32  # the reference appends 32 x -1 to both index lists (fasttree.py:261-262)
 AUX_BIT = 1 << 30     # FT_KV_OFFSET_AUX: a vnode_to_kv_offs value with this bit indexes the auxiliary row-id table
 GROUP_MAX_TILES_DIRECT = 24  # ... and a group of the serving path never more than this
+GROUP_ROUNDS = (8, 5, 9, 6, 7, 4)  # ... which aims at this many quarters of a round, the first unless another's schedule ends sooner
 GROUP_MAX_TILES = 16  # a group of short nodes never spans more KV tiles than this (same constant in csrc/ft_planner.cu)
 
 
@@ -472,10 +473,11 @@ def b200_group_short_nodes(vnodes, q_tile, small_tile, m, target_tokens, direct=
     hard_cap = GROUP_MAX_TILES * tile
     cap = min(max(target_tokens // tile * tile, 4 * tile), hard_cap)
     if direct:
-        # serving path: the groups are sized so that the step fills two rounds of resident CTAs, the other tasks
-        # included (measured on the 512-request burst, 16 other tasks on 37 slots: 36 / 53 / 73 / 80 / 120 tasks run
-        # 69.7 / 61.9 / 55.7 / 68.5 / 76.1 us - their tiles are gathered row by row, and two shorter groups per slot
-        # hide that latency better than one long one, while a third round costs more than it hides), up to 24 tiles
+        # Serving path: groups of up to 24 tiles, sized so that the step, the other tasks included, fills a number of
+        # rounds of resident CTAs.  Which number is decided on simulated schedules: two rounds unless another of
+        # GROUP_ROUNDS ends sooner - how the longest tasks fall on the slots matters more than the mean (512 requests
+        # under 4 prompts, 16 other tasks on 37 slots, us of stage 1 and the schedule's time units at 1 / 1.25 / 1.5 / 2 /
+        # 2.25 / 2.5 / 3 rounds: 48.3 / 40.7 / 48.2 / 43.8 / 42.1 / 55.9 / 52.9 and 26 / 24 / 29 / 27 / 26 / 36 / 33).
         cand_tokens = other = 0
         for vn in vnodes:
             length = sum(e - b for b, e in vn.kv_ranges)
@@ -484,9 +486,21 @@ def b200_group_short_nodes(vnodes, q_tile, small_tile, m, target_tokens, direct=
             else:
                 other += -(-length // vn.kv_split) * -(-len(vn.requests) // vn.q_tile)
         round_ = max(int(m.num_sms * m.ctas_per_sm * m.waves) // max(num_kv_heads, 1), 1)
-        free_tasks = max(2 * round_ - other, round_ // 2, 2)
         hard_cap = GROUP_MAX_TILES_DIRECT * tile
-        cap = min(max(-(-(-(-cand_tokens // free_tasks)) // tile) * tile, 4 * tile), hard_cap)
+        slots = max((m.num_sms * m.ctas_per_sm) // max(num_kv_heads, 1), 1)
+        best = best_end = None
+        tried = set()
+        for quarters in GROUP_ROUNDS:
+            free_tasks = max(quarters * round_ // 4 - other, round_ // 2, 2)
+            cap = min(max(-(-(-(-cand_tokens // free_tasks)) // tile) * tile, 4 * tile), hard_cap)
+            if cap in tried:
+                continue
+            tried.add(cap)
+            packed = _pack_short_nodes(vnodes, q_tile, small_tile, m, cap, hard_cap, direct)
+            end = b200_simulated_schedule(packed, q_tile, small_tile, m, slots)[0]
+            if best is None or end < best_end:
+                best, best_end = packed, end
+        return best
     else:
         # One round: when the tasks at the default cap would spill a little past one round of resident CTAs while
         # longer groups keep everything inside it, the cap grows to what fills the round exactly (cfg3 on a 4-head
@@ -503,6 +517,12 @@ def b200_group_short_nodes(vnodes, q_tile, small_tile, m, target_tokens, direct=
             fill = -(-(-(-cand_tokens // (round_ - other))) // tile) * tile
             if fill <= hard_cap:
                 cap = max(cap, fill)
+    return _pack_short_nodes(vnodes, q_tile, small_tile, m, cap, hard_cap, direct)
+
+
+def _pack_short_nodes(vnodes, q_tile, small_tile, m, cap, hard_cap, direct):
+    """:func:`b200_group_short_nodes` at a given size of the groups, in tokens."""
+    tile = m.tile_tokens
     kept, tail = [], []
     cur, cur_reqs, cur_tokens, cur_n = [], set(), 0, 0
 
@@ -556,7 +576,7 @@ def b200_simulated_schedule(vnodes, q_tile, small_tile, m, slots):
     task ends)."""
     tasks = []
     for vi, vn in enumerate(vnodes):
-        length = sum(e - b for b, e in vn.kv_ranges)
+        length = sum(e - b for b, e in vn.kv_ranges) + sum(vn.member_room or ())
         nreq = len(vn.requests)
         if nreq == 0 or length <= 0:
             continue

@@ -1,0 +1,43 @@
+"""Serving plans: the number of rounds that the groups of short nodes are sized for."""
+import numpy as np
+import pytest
+
+from ft_b200 import planner
+
+
+def _burst(requests, prompts, prompt_tokens, tail_tokens, spread):
+    """Shared prompts, then one private tail per request with room to grow, as the serving path hands them over."""
+    per = -(-requests // prompts)
+    nodes = []
+    for p in range(prompts):
+        ids = np.arange(p * per, min((p + 1) * per, requests), dtype=np.int32)
+        nodes.append(planner.VirtualNode([(1000 * p, 1000 * p + prompt_tokens)], ids, q_tile=32, kv_split=512))
+    for r in range(requests):
+        n = tail_tokens + r % (spread + 1)
+        nodes.append(planner.VirtualNode([(10 ** 6 + 300 * r, 10 ** 6 + 300 * r + n)], np.array([r], dtype=np.int32), q_tile=32,
+                                         kv_split=128, room=12))
+    return nodes
+
+
+@pytest.mark.parametrize("requests,prompts,prompt_tokens,tail_tokens,spread", [
+    (512, 4, 420, 36, 7), (300, 8, 300, 90, 9), (192, 4, 39, 65, 3), (209, 11, 262, 27, 5), (400, 2, 800, 12, 5), (150, 1, 64, 100, 0),
+])
+def test_another_number_of_rounds_only_where_its_schedule_ends_sooner(monkeypatch, requests, prompts, prompt_tokens, tail_tokens, spread):
+    m = planner.B200Model(rows_per_cta=128, group_min_members=4)
+    nodes = _burst(requests, prompts, prompt_tokens, tail_tokens, spread)
+    slots = m.num_sms * m.ctas_per_sm // 8
+
+    def grouped(rounds):
+        monkeypatch.setattr(planner, "GROUP_ROUNDS", rounds)
+        out = planner.b200_group_short_nodes(nodes, 32, 4, m, 0, direct=True, num_kv_heads=8)
+        # every request's tokens are still met exactly once, whatever the grouping
+        tails = sorted((r, e - b) for v in out for r, (b, e) in
+                       (zip(v.requests.tolist(), v.row_ranges) if v.row_ranges is not None else
+                        ((r, (0, sum(y - x for x, y in v.kv_ranges))) for r in v.requests.tolist() if len(v.requests) == 1)))
+        assert tails == sorted((int(v.requests[0]), v.kv_ranges[0][1] - v.kv_ranges[0][0]) for v in nodes if len(v.requests) == 1)
+        return planner.b200_simulated_schedule(out, 32, 4, m, slots)[0]
+
+    every = planner.GROUP_ROUNDS
+    ends = [grouped((q,)) for q in every]
+    chosen = grouped(every)
+    assert every[0] == 8 and chosen == min(ends) <= ends[0]
