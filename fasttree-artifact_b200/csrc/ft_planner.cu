@@ -272,6 +272,7 @@ int build_plan(const int32_t* parent, const int32_t* seqlen, int32_t n_nodes, co
     // side by side): its length, the time of all tasks together, and the end of every node's last task.
     struct Piece {
       int64_t length, chunk, nreq;
+      bool group;
     };
     const int64_t sched_slots = std::max<int64_t>((int64_t)(m.num_sms * m.ctas_per_sm) / std::max(num_kv_heads, 1), 1);
     auto simulate = [&](const std::vector<Piece>& pieces, std::vector<int64_t>& last_end, int64_t& total) {
@@ -314,6 +315,35 @@ int build_plan(const int32_t* parent, const int32_t* seqlen, int32_t n_nodes, co
       return makespan;
     };
 
+    // Tail split (table-building mode).  The hardware hands CTAs to slots in grid order, so a step of 2.05 or 2.6 rounds ends
+    // with a round in which a fraction of the slots run whole tasks while the rest of the GPU idles.  When the makespan
+    // exceeds the perfectly packed time by more than an eighth, every plain (ungrouped) virtual node with a task that ends in
+    // the later half of that excess is cut to half its chunk length (never below min_chunk); the cut is kept if the
+    // simulated makespan drops.  (A step of one round lasts as long as its longest task: same cut.)  Returns the makespan.
+    auto split_tail = [&](std::vector<Piece>& pieces) {
+      std::vector<int64_t> last_end, trial_end;
+      int64_t total = 0, total2 = 0;
+      const int64_t makespan = simulate(pieces, last_end, total);
+      const int64_t bound = ceil_div(total, sched_slots);
+      if ((makespan - bound) * 8 <= makespan) return makespan;
+      const int64_t late_from = makespan - (makespan - bound + 1) / 2;
+      std::vector<Piece> trial(pieces);
+      bool any = false;
+      for (size_t i = 0; i < pieces.size(); ++i) {
+        if (pieces[i].group || last_end[i] <= late_from) continue;
+        const int64_t cur = std::min(pieces[i].chunk, pieces[i].length);
+        const int64_t half = ceil_div(ceil_div(cur, 2), m.tile_tokens) * m.tile_tokens;
+        if (half >= m.min_chunk && half < cur) {
+          trial[i].chunk = half;
+          any = true;
+        }
+      }
+      const int64_t end = any ? simulate(trial, trial_end, total2) : makespan;
+      if (end >= makespan) return makespan;
+      pieces.swap(trial);
+      return end;
+    };
+
     // ---- groups of short nodes (table-building mode, 16-bit elements, head_dim 64, 128 or 256: the shapes whose
     // kernels honour per-row token ranges; serving path: head_dim 128).  Candidates - at most small_tile requests, at most group_member_tokens tokens - are
     // taken in order; a group is closed when the next candidate would exceed q_tile requests or 16 tiles of tokens,
@@ -328,6 +358,41 @@ int build_plan(const int32_t* parent, const int32_t* seqlen, int32_t n_nodes, co
       const int64_t target_tokens = (int64_t)std::floor(target / (double)row_bytes);
       int64_t hard_cap = 16 * tile;
       int64_t cap = std::min(std::max(target_tokens / tile * tile, 4 * tile), hard_cap);
+      // the sizes that the grouping below comes out with at groups of `cap` tokens
+      std::vector<uint8_t> taken((size_t)std::max(batch, 1), 0);
+      auto packed = [&](int64_t cap, int64_t hard_cap) {
+        std::vector<Piece> kept, tail;
+        std::vector<const Spec*> cur;
+        int64_t cur_tokens = 0, cur_n = 0;
+        auto close = [&]() {
+          for (const Spec* s : cur)
+            for (int32_t r : s->reqs) taken[r] = 0;
+          if ((int64_t)cur.size() >= m.group_min_members && cur_n > small_tile)
+            tail.push_back({cur_tokens, ceil_div(cur_tokens, tile) * tile, cur_n, true});
+          else
+            for (const Spec* s : cur) tail.push_back({s->length, s->chunk, (int64_t)s->reqs.size(), false});
+          cur.clear();
+          cur_tokens = cur_n = 0;
+        };
+        for (const Spec& s : specs) {
+          const int64_t nreq = (int64_t)s.reqs.size(), span = s.length + s.room;
+          if (nreq > small_tile || span > m.group_member_tokens) {
+            kept.push_back({s.length, s.chunk, nreq, false});
+            continue;
+          }
+          bool shared = false;
+          for (int32_t r : s.reqs) shared = shared || taken[r] != 0;
+          const bool full = direct != nullptr ? cur_tokens >= cap : cur_tokens + span > cap;
+          if (!cur.empty() && (cur_n + nreq > q_tile || cur_tokens + span > hard_cap || (full && cur_n > small_tile) || shared)) close();
+          for (int32_t r : s.reqs) taken[r] = 1;
+          cur_tokens += span;
+          cur_n += nreq;
+          cur.push_back(&s);
+        }
+        close();
+        kept.insert(kept.end(), tail.begin(), tail.end());
+        return kept;
+      };
       if (direct != nullptr) {
         // Serving path: groups of up to 24 tiles, sized so that the step, the other tasks included, fills a number of rounds of
         // resident CTAs: two, unless the simulated schedule of another of these numbers (in quarters) ends sooner.  How the
@@ -343,45 +408,14 @@ int build_plan(const int32_t* parent, const int32_t* seqlen, int32_t n_nodes, co
         const int64_t round = std::max<int64_t>((int64_t)slots / std::max(num_kv_heads, 1), 1);
         hard_cap = 24 * tile;
         std::vector<int64_t> tried, last_end;
-        std::vector<uint8_t> taken((size_t)std::max(batch, 1), 0);
         int64_t best_end = -1;
         for (const int64_t quarters : {8, 5, 9, 6, 7, 4}) {
           const int64_t free_tasks = std::max<int64_t>(std::max(quarters * round / 4 - other, round / 2), 2);
           const int64_t c = std::min(std::max(ceil_div(ceil_div(cand_tokens, free_tasks), tile) * tile, 4 * tile), hard_cap);
           if (std::find(tried.begin(), tried.end(), c) != tried.end()) continue;
           tried.push_back(c);
-          // the sizes that the grouping below would come out with
-          std::vector<Piece> kept, tail;
-          std::vector<const Spec*> cur;
-          int64_t cur_tokens = 0, cur_n = 0, total = 0;
-          auto close = [&]() {
-            for (const Spec* s : cur)
-              for (int32_t r : s->reqs) taken[r] = 0;
-            if ((int64_t)cur.size() >= m.group_min_members && cur_n > small_tile)
-              tail.push_back({cur_tokens, ceil_div(cur_tokens, tile) * tile, cur_n});
-            else
-              for (const Spec* s : cur) tail.push_back({s->length, s->chunk, (int64_t)s->reqs.size()});
-            cur.clear();
-            cur_tokens = cur_n = 0;
-          };
-          for (const Spec& s : specs) {
-            const int64_t nreq = (int64_t)s.reqs.size(), span = s.length + s.room;
-            if (nreq > small_tile || span > m.group_member_tokens) {
-              kept.push_back({s.length, s.chunk, nreq});
-              continue;
-            }
-            bool shared = false;
-            for (int32_t r : s.reqs) shared = shared || taken[r] != 0;
-            if (!cur.empty() && (cur_n + nreq > q_tile || cur_tokens + span > hard_cap || (cur_tokens >= c && cur_n > small_tile) || shared))
-              close();
-            for (int32_t r : s.reqs) taken[r] = 1;
-            cur_tokens += span;
-            cur_n += nreq;
-            cur.push_back(&s);
-          }
-          close();
-          kept.insert(kept.end(), tail.begin(), tail.end());
-          const int64_t end = simulate(kept, last_end, total);
+          int64_t total = 0;
+          const int64_t end = simulate(packed(c, hard_cap), last_end, total);
           if (best_end < 0 || end < best_end) {
             best_end = end;
             cap = c;
@@ -401,6 +435,27 @@ int build_plan(const int32_t* parent, const int32_t* seqlen, int32_t n_nodes, co
         if (other < round && other + ceil_div(cand_tokens, cap) > round) {
           const int64_t fill = ceil_div(ceil_div(cand_tokens, round - other), tile) * tile;
           if (fill <= hard_cap) cap = std::max(cap, fill);
+        }
+        // That size, or a half, three quarters or one and a half times as much where there are groups then too and the
+        // schedule of the step, its tail split included, ends a twentieth sooner.  Plans for one or two KV heads, where a
+        // long group outlasts the other tasks, want shorter ones (218 requests in three levels at 8/2 heads, us per step and
+        // time units at 1 / 0.5 / 0.75 / 1.5: 12.8 / 11.3 / 12.0 / 14.5 and 9 / 7 / 8 / 11), a search tree of 1024 requests
+        // longer ones (117.2 / 130.0 / 122.0 / 116.3, 76 / 91 / 77 / 71).  A smaller difference the model does not resolve
+        // (512 leaves at head_dim 64 31.6 / 33.6 at 29 / 28).
+        const int64_t base = cap, base_hard = hard_cap;
+        int64_t first_end = 0, best_end = 0;
+        for (const int64_t quarters : {4, 2, 3, 6}) {
+          const int64_t size = std::max(base * quarters / 4 / tile * tile, 2 * tile), hard = std::max(base_hard, size);
+          std::vector<Piece> pieces = packed(size, hard);
+          const bool any = std::any_of(pieces.begin(), pieces.end(), [](const Piece& p) { return p.group; });
+          if (quarters == 4 && !any) break;
+          const int64_t end = split_tail(pieces);
+          if (quarters == 4 || (any && end * 20 <= first_end * 19 && end < best_end)) {
+            best_end = end;
+            cap = size;
+            hard_cap = hard;
+          }
+          if (quarters == 4) first_end = end;
         }
       }
       std::vector<Spec> kept, tail;
@@ -454,41 +509,11 @@ int build_plan(const int32_t* parent, const int32_t* seqlen, int32_t n_nodes, co
       for (Spec& t : tail) specs.push_back(std::move(t));
     }
 
-    // ---- tail split (table-building mode).  The hardware hands CTAs to slots in grid order, so a step of 2.05 or 2.6
-    // rounds ends with a round in which a fraction of the slots run whole tasks while the rest of the GPU idles.  On a
-    // simulated list schedule of the tasks in emission order (integer time: a fixed cost per task plus one unit per
-    // KV tile; a task = the CTAs of all KV heads of one chunk x request tile, which start side by side), when the
-    // makespan exceeds the perfectly packed time by more than an eighth, every plain (ungrouped) virtual node with a
-    // task that ends in the later half of that excess is cut to half its chunk length (never below min_chunk); the
-    // cut is kept if the simulated makespan drops.  (A step of one round lasts as long as its longest task: same cut.)
-    if (direct == nullptr) {
+    if (direct == nullptr) {  // tail split
       std::vector<Piece> pieces;
-      std::vector<int64_t> last_end;
-      for (const Spec& s : specs) pieces.push_back({s.length, s.chunk, (int64_t)s.reqs.size()});
-      int64_t total = 0;
-      const int64_t makespan = simulate(pieces, last_end, total);
-      const int64_t bound = ceil_div(total, sched_slots);
-      if ((makespan - bound) * 8 > makespan) {
-        const int64_t late_from = makespan - (makespan - bound + 1) / 2;
-        std::vector<Piece> trial(pieces);
-        bool any = false;
-        for (size_t si = 0; si < specs.size(); ++si) {
-          const Spec& s = specs[si];
-          if (!s.row_ranges.empty() || last_end[si] <= late_from) continue;
-          const int64_t cur = std::min(s.chunk, s.length);
-          const int64_t half = ceil_div(ceil_div(cur, 2), m.tile_tokens) * m.tile_tokens;
-          if (half >= m.min_chunk && half < cur) {
-            trial[si].chunk = half;
-            any = true;
-          }
-        }
-        if (any) {
-          std::vector<int64_t> fs2;
-          int64_t total2 = 0;
-          if (simulate(trial, fs2, total2) < makespan)
-            for (size_t si = 0; si < specs.size(); ++si) specs[si].chunk = trial[si].chunk;
-        }
-      }
+      for (const Spec& s : specs) pieces.push_back({s.length, s.chunk, (int64_t)s.reqs.size(), !s.row_ranges.empty()});
+      split_tail(pieces);
+      for (size_t i = 0; i < specs.size(); ++i) specs[i].chunk = pieces[i].chunk;
     }
 
     // ---- emission: chunk-major, request-tile-minor; every chunk repeats the node's request list

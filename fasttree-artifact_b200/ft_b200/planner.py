@@ -31,7 +31,8 @@ PAD_ENTRIES = 32  # the reference appends 32 x -1 to both index lists (fasttree.
 AUX_BIT = 1 << 30     # FT_KV_OFFSET_AUX: a vnode_to_kv_offs value with this bit indexes the auxiliary row-id table
 GROUP_MAX_TILES_DIRECT = 24  # ... and a group of the serving path never more than this
 GROUP_ROUNDS = (8, 5, 9, 6, 7, 4)  # ... which aims at this many quarters of a round, the first unless another's schedule ends sooner
-GROUP_MAX_TILES = 16  # a group of short nodes never spans more KV tiles than this (same constant in csrc/ft_planner.cu)
+GROUP_CAPS = (4, 2, 3, 6)  # a group's size in quarters of what fills a task: the first unless another's schedule ends sooner
+GROUP_MAX_TILES = 16  # a group of short nodes never spans more KV tiles than this, or what another size asks for (same constants in csrc/ft_planner.cu)
 
 
 @dataclass
@@ -438,8 +439,7 @@ def plan_b200(tree, kv_ptrs, batch_size, num_qo_heads, num_kv_heads, head_dim, p
     vnodes, assign, q_tile, small_tile, target = b200_virtual_nodes(
         tree, num_qo_heads, num_kv_heads, head_dim, m, lambda a, i: _chain_ranges(tree, kv_ptrs, a, i))
     if head_dim in (64, 128, 256) and m.elem_bytes == 2:      # the kernels that honour row ranges exist for these shapes
-        vnodes = b200_group_short_nodes(vnodes, q_tile, small_tile, m,
-                                        int(math.floor(target / (2 * head_dim * m.elem_bytes))), num_kv_heads=num_kv_heads)
+        vnodes = b200_sized_groups(vnodes, q_tile, small_tile, m, int(math.floor(target / (2 * head_dim * m.elem_bytes))), num_kv_heads)
     vnodes = b200_split_tail(vnodes, q_tile, small_tile, m, num_kv_heads)
     tabs = emit_tables(vnodes, batch_size, small_tile=small_tile, order_key=b200_task_order)
     params.set_q_tile_sizes([q_tile, small_tile])
@@ -449,7 +449,7 @@ def plan_b200(tree, kv_ptrs, batch_size, num_qo_heads, num_kv_heads, head_dim, p
                 info={"planner": "b200", "target_bytes": float(target), "vnodes": len(vnodes)}, **tabs)
 
 
-def b200_group_short_nodes(vnodes, q_tile, small_tile, m, target_tokens, direct=False, num_kv_heads=1):
+def b200_group_short_nodes(vnodes, q_tile, small_tile, m, target_tokens, direct=False, num_kv_heads=1, quarters=4):
     """Packs short virtual nodes with pairwise disjoint request sets into groups
     that run as ONE many-row task: the members' KV is concatenated, their requests
     are concatenated, and each request attends only to its own member's tokens
@@ -469,7 +469,7 @@ def b200_group_short_nodes(vnodes, q_tile, small_tile, m, target_tokens, direct=
     the burst - counts as part of its length."""
     if m.group_member_tokens <= 0:
         return vnodes
-    tile = m.tile_tokens
+    tile = m.tile_tokens   # (quarters, for other groups: their size in quarters of the computed one)
     hard_cap = GROUP_MAX_TILES * tile
     cap = min(max(target_tokens // tile * tile, 4 * tile), hard_cap)
     if direct:
@@ -517,7 +517,33 @@ def b200_group_short_nodes(vnodes, q_tile, small_tile, m, target_tokens, direct=
             fill = -(-(-(-cand_tokens // (round_ - other))) // tile) * tile
             if fill <= hard_cap:
                 cap = max(cap, fill)
-    return _pack_short_nodes(vnodes, q_tile, small_tile, m, cap, hard_cap, direct)
+    size = max(cap * quarters // 4 // tile * tile, 2 * tile)
+    return _pack_short_nodes(vnodes, q_tile, small_tile, m, size, max(hard_cap, size), direct)
+
+
+def b200_sized_groups(vnodes, q_tile, small_tile, m, target_tokens, num_kv_heads):
+    """:func:`b200_group_short_nodes` at the size it computes, or at a half, three
+    quarters or one and a half times as much where there are groups then too and the
+    schedule of the step, its tail split included, ends a twentieth sooner.  Plans
+    for one or two KV heads, where a long group outlasts the other tasks, want
+    shorter ones (218 requests in three levels at 8/2 heads, us per step and time
+    units at 1 / 0.5 / 0.75 / 1.5: 12.8 / 11.3 / 12.0 / 14.5 and 9 / 7 / 8 / 11), a
+    search tree of 1024 requests longer ones (117.2 / 130.0 / 122.0 / 116.3, 76 / 91 /
+    77 / 71).  A smaller difference the model does not resolve (512 leaves at head_dim
+    64 31.6 / 33.6 at 29 / 28)."""
+    slots = max((m.num_sms * m.ctas_per_sm) // max(num_kv_heads, 1), 1)
+    best = best_end = first_end = None
+    for quarters in GROUP_CAPS:
+        packed = b200_group_short_nodes(vnodes, q_tile, small_tile, m, target_tokens, num_kv_heads=num_kv_heads, quarters=quarters)
+        any_group = any(vn.row_ranges is not None for vn in packed)
+        if best is None and not any_group:
+            return packed
+        end = b200_simulated_schedule(b200_split_tail(packed, q_tile, small_tile, m, num_kv_heads), q_tile, small_tile, m, slots)[0]
+        if best is None:
+            best, best_end, first_end = packed, end, end
+        elif any_group and end * 20 <= first_end * 19 and end < best_end:
+            best, best_end = packed, end
+    return best
 
 
 def _pack_short_nodes(vnodes, q_tile, small_tile, m, cap, hard_cap, direct):
