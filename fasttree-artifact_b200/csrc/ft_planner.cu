@@ -346,10 +346,10 @@ int build_plan(const int32_t* parent, const int32_t* seqlen, int32_t n_nodes, co
 
     // ---- groups of short nodes (table-building mode, 16-bit elements, head_dim 64, 128 or 256: the shapes whose
     // kernels honour per-row token ranges; serving path: head_dim 128).  Candidates - at most small_tile requests, at most group_member_tokens tokens - are
-    // taken in order; a group is closed when the next candidate would exceed q_tile requests or 16 tiles of tokens,
-    // would exceed the per-task token target (at least 4 tiles) once the group has more than small_tile requests,
-    // or shares a request with it; groups with fewer than
-    // group_min_members members, or not more requests than small_tile, are dissolved.  Result: the other virtual
+    // taken in order; a group is closed when the next candidate would exceed q_tile requests or 16 tiles of tokens
+    // (24 on the serving path and at one and a half times that), would exceed the group's token target (at least
+    // 4 tiles, or that share of them) once the group has more than small_tile requests, or shares a request with it;
+    // groups with fewer than group_min_members members, or not more requests than small_tile, are dissolved.  Result: the other virtual
     // nodes in their order, then groups and dissolved candidates in the order they were closed.
     bool any_groups = false;
     const bool tc_dim = head_dim == 128 || (direct == nullptr && (head_dim == 64 || head_dim == 256));
@@ -441,16 +441,21 @@ int build_plan(const int32_t* parent, const int32_t* seqlen, int32_t n_nodes, co
         // long group outlasts the other tasks, want shorter ones (218 requests in three levels at 8/2 heads, us per step and
         // time units at 1 / 0.5 / 0.75 / 1.5: 12.8 / 11.3 / 12.0 / 14.5 and 9 / 7 / 8 / 11), a search tree of 1024 requests
         // longer ones (117.2 / 130.0 / 122.0 / 116.3, 76 / 91 / 77 / 71).  A smaller difference the model does not resolve
-        // (512 leaves at head_dim 64 31.6 / 33.6 at 29 / 28).
+        // (512 leaves at head_dim 64 31.6 / 33.6 at 29 / 28).  The tail split that goes with another size may make more
+        // partial rows: never more than fit the library's own scratch where those of the first size do.
         const int64_t base = cap, base_hard = hard_cap;
-        int64_t first_end = 0, best_end = 0;
+        const int64_t scratch_rows = (int64_t)FT_STATIC_SCRATCH_BYTES / 4 / ((int64_t)num_qo_heads * (head_dim + 1));
+        int64_t first_end = 0, best_end = 0, rows_limit = 0;
         for (const int64_t quarters : {4, 2, 3, 6}) {
           const int64_t size = std::max(base * quarters / 4 / tile * tile, 2 * tile), hard = std::max(base_hard, size);
           std::vector<Piece> pieces = packed(size, hard);
           const bool any = std::any_of(pieces.begin(), pieces.end(), [](const Piece& p) { return p.group; });
           if (quarters == 4 && !any) break;
           const int64_t end = split_tail(pieces);
-          if (quarters == 4 || (any && end * 20 <= first_end * 19 && end < best_end)) {
+          int64_t rows = 0;
+          for (const Piece& p : pieces) rows += p.nreq * ceil_div(p.length, p.chunk);
+          if (quarters == 4) rows_limit = std::max(rows, scratch_rows);
+          if (quarters == 4 || (any && rows <= rows_limit && end * 20 <= first_end * 19 && end < best_end)) {
             best_end = end;
             cap = size;
             hard_cap = hard;

@@ -284,7 +284,7 @@ def _plan_b200(batch, md, node_to_reqs, covered, order, offsets, parents, lens, 
         tabs, q_tile, small_tile, tile_tokens = run(-1, model)
     if bound is not None:
         # Groups pay when the few-row tasks alone would queue up several deep behind the resident CTAs; then the
-        # burst is planned again with short runs packed into many-row vnodes.  A group needs more than 16 query
+        # burst is planned with short runs packed into many-row vnodes.  A group needs more than 16 query
         # rows anyway (only the many-row kernels honour row ranges); past that, a handful of one-tile tails
         # already costs less as one task than as one task each.
         few_row_ctas = (bsz if tabs is None else tabs["phase_node_nums"][1]) * md.num_kv_heads

@@ -435,11 +435,13 @@ def plan_b200(tree, kv_ptrs, batch_size, num_qo_heads, num_kv_heads, head_dim, p
     ``num_kv_heads`` is the LOCAL head count of this GPU (the grid is tasks x
     local KV heads), so a head-sharded rank plans finer chunks.  Writes the
     request/KV tile sizes it used back into ``params`` like the reference does."""
+    from . import lib as _lib
     m = b200_model_for(params, head_dim, model)
     vnodes, assign, q_tile, small_tile, target = b200_virtual_nodes(
         tree, num_qo_heads, num_kv_heads, head_dim, m, lambda a, i: _chain_ranges(tree, kv_ptrs, a, i))
     if head_dim in (64, 128, 256) and m.elem_bytes == 2:      # the kernels that honour row ranges exist for these shapes
-        vnodes = b200_sized_groups(vnodes, q_tile, small_tile, m, int(math.floor(target / (2 * head_dim * m.elem_bytes))), num_kv_heads)
+        vnodes = b200_sized_groups(vnodes, q_tile, small_tile, m, int(math.floor(target / (2 * head_dim * m.elem_bytes))), num_kv_heads,
+                                   _lib.FT_STATIC_SCRATCH_BYTES // 4 // (num_qo_heads * (head_dim + 1)))
     vnodes = b200_split_tail(vnodes, q_tile, small_tile, m, num_kv_heads)
     tabs = emit_tables(vnodes, batch_size, small_tile=small_tile, order_key=b200_task_order)
     params.set_q_tile_sizes([q_tile, small_tile])
@@ -458,9 +460,10 @@ def b200_group_short_nodes(vnodes, q_tile, small_tile, m, target_tokens, direct=
 
     Candidates are the virtual nodes with at most ``small_tile`` requests and at
     most ``group_member_tokens`` tokens, taken in order; a group is closed when
-    the next candidate would exceed ``q_tile`` requests or 16 tiles of tokens,
-    would exceed the per-task token target (at least 4 tiles) once the group has
-    more than ``small_tile`` requests, or shares a request with it.  Groups
+    the next candidate would exceed ``q_tile`` requests or 16 tiles of tokens (24
+    for ``direct``), would exceed the per-task token target (at least 4 tiles) once
+    the group has more than ``small_tile`` requests, or shares a request with it.
+    ``quarters``: the size in quarters of the target (the bound gives way to it).  Groups
     with fewer than ``group_min_members`` members, or not more requests than
     ``small_tile``, are dissolved.  Result: the other virtual nodes in their
     order, then groups and dissolved candidates in the order they were closed.
@@ -521,7 +524,7 @@ def b200_group_short_nodes(vnodes, q_tile, small_tile, m, target_tokens, direct=
     return _pack_short_nodes(vnodes, q_tile, small_tile, m, size, max(hard_cap, size), direct)
 
 
-def b200_sized_groups(vnodes, q_tile, small_tile, m, target_tokens, num_kv_heads):
+def b200_sized_groups(vnodes, q_tile, small_tile, m, target_tokens, num_kv_heads, scratch_rows):
     """:func:`b200_group_short_nodes` at the size it computes, or at a half, three
     quarters or one and a half times as much where there are groups then too and the
     schedule of the step, its tail split included, ends a twentieth sooner.  Plans
@@ -530,18 +533,22 @@ def b200_sized_groups(vnodes, q_tile, small_tile, m, target_tokens, num_kv_heads
     units at 1 / 0.5 / 0.75 / 1.5: 12.8 / 11.3 / 12.0 / 14.5 and 9 / 7 / 8 / 11), a
     search tree of 1024 requests longer ones (117.2 / 130.0 / 122.0 / 116.3, 76 / 91 /
     77 / 71).  A smaller difference the model does not resolve (512 leaves at head_dim
-    64 31.6 / 33.6 at 29 / 28)."""
+    64 31.6 / 33.6 at 29 / 28).  The tail split that goes with another size may make
+    more partial rows: never more than the ``scratch_rows`` of the library's own
+    scratch where those of the first size fit."""
     slots = max((m.num_sms * m.ctas_per_sm) // max(num_kv_heads, 1), 1)
-    best = best_end = first_end = None
+    best = best_end = first_end = rows_limit = None
     for quarters in GROUP_CAPS:
         packed = b200_group_short_nodes(vnodes, q_tile, small_tile, m, target_tokens, num_kv_heads=num_kv_heads, quarters=quarters)
         any_group = any(vn.row_ranges is not None for vn in packed)
         if best is None and not any_group:
             return packed
-        end = b200_simulated_schedule(b200_split_tail(packed, q_tile, small_tile, m, num_kv_heads), q_tile, small_tile, m, slots)[0]
+        split = b200_split_tail(packed, q_tile, small_tile, m, num_kv_heads)
+        end = b200_simulated_schedule(split, q_tile, small_tile, m, slots)[0]
+        rows = sum(len(vn.requests) * -(-sum(e - b for b, e in vn.kv_ranges) // vn.kv_split) for vn in split)
         if best is None:
-            best, best_end, first_end = packed, end, end
-        elif any_group and end * 20 <= first_end * 19 and end < best_end:
+            best, best_end, first_end, rows_limit = packed, end, end, max(rows, scratch_rows)
+        elif any_group and rows <= rows_limit and end * 20 <= first_end * 19 and end < best_end:
             best, best_end = packed, end
     return best
 

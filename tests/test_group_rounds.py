@@ -1,8 +1,12 @@
-"""Serving plans: the number of rounds that the groups of short nodes are sized for."""
+"""The size of the groups of short nodes: the number of rounds in serving plans, the share of a task in the others."""
 import numpy as np
 import pytest
+import torch
 
-from ft_b200 import planner
+import fasttree
+import kv_tree_simple
+import tree_generation
+from ft_b200 import lib, planner
 
 
 def _burst(requests, prompts, prompt_tokens, tail_tokens, spread):
@@ -41,3 +45,26 @@ def test_another_number_of_rounds_only_where_its_schedule_ends_sooner(monkeypatc
     ends = [grouped((q,)) for q in every]
     chosen = grouped(every)
     assert every[0] == 8 and chosen == min(ends) <= ends[0]
+
+
+@pytest.mark.parametrize("sizes,lens,hq,hkv", [
+    ([1, 9, 162], [1274, 157, 33], 64, 8), ([1, 14, 168], [500, 134, 14], 64, 8), ([1, 18, 216], [1990, 191, 43], 32, 4),
+    ([1, 65], [150, 9], 8, 2),
+])
+def test_another_group_size_needs_no_more_scratch_than_there_is(monkeypatch, sizes, lens, hq, hkv):
+    nodes = kv_tree_simple.tree_from_rows(tree_generation.generate_tree(sizes, lens))
+    batch, ptrs = kv_tree_simple.assign_requests(nodes)
+
+    def plan(make):
+        params = fasttree.FastTreeParams()
+        params.set_kv_group_num(hq // hkv)
+        params.set_kv_dtype(torch.bfloat16)
+        return make(nodes, ptrs, batch, hq, hkv, 128, params)
+
+    spec, native = plan(planner.plan_b200), plan(planner.plan_b200_native)
+    for name in ("vnode_to_q_entries", "vnode_to_q_offs", "vnode_to_kv_offs", "vnode_to_kv_lens", "req_to_vnode_entries"):
+        np.testing.assert_array_equal(getattr(spec, name), getattr(native, name))
+    monkeypatch.setattr(planner, "GROUP_CAPS", (4,))
+    first = plan(planner.plan_b200)
+    scratch_rows = lib.FT_STATIC_SCRATCH_BYTES // (4 * hq * 129)
+    assert len(spec.vnode_to_q_entries) <= max(len(first.vnode_to_q_entries), scratch_rows)
