@@ -160,8 +160,10 @@ __global__ void __launch_bounds__(256, D == 64 ? 4 : 3) stage1_f32_kernel(const 
     if (q_req[u] >= 0 && q_req[u] < p.batch)
       x = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p.q) + (int64_t)q_req[u] * p.q_s0 +
                                            (int64_t)(kvh * G + (row0 + r) % G) * p.q_s1 + 4 * q_c4);
-    else if (r < rows && q_c4 == 0)
-      flag_error(FT_DEV_BAD_Q_INDEX);
+    else if (r < rows && q_c4 == 0) {  // a bad row id has been flagged above: no request was read there
+      const int64_t part = (int64_t)q_off + (row0 + r) / G;
+      if (part >= 0 && part < p.num_partial_rows) flag_error(FT_DEV_BAD_Q_INDEX);
+    }
     *reinterpret_cast<float4*>(q_s + r * D + 4 * q_c4) = x;
   }
   for (int t = 0; t < ntiles; ++t) {
