@@ -16,8 +16,8 @@
 // tile passes through shared memory once per warp, which bounds a tile's arithmetic, and
 // a word at a time the reads' issue did.  With that and the first reads sent off together
 // (before: the Q rows, then the row ids, then the K and V rows) stage 1 of 4 requests on
-// 512 tokens, 8/2 heads of 128, takes 7.0 us (7.6), of 40 requests of 300 tokens on 500,
-// 16/16 heads, 173 (196), of 64 requests of 100 on 1000, 32/8 heads of 64, 66 (78).
+// 512 tokens, 8/2 heads of 128, takes 6.8 us (7.7), of 40 requests of 300 tokens on 500,
+// 16/16 heads, 171 (196), of 64 requests of 100 on 1000, 32/8 heads of 64, 66 (79).
 // Same conventions as the other stage-1 kernels (kernel_bench/fasttree.py:360-413):
 // scores scaled after the dot product, normalised partial output, lse = log(sum) + max;
 // optional per-row token ranges; bad indices are skipped and flagged.
@@ -115,21 +115,21 @@ __global__ void __launch_bounds__(256, D == 64 ? 4 : 3) stage1_f32_kernel(const 
 
   const int ntiles = (kv_len + C::TILE - 1) / C::TILE;
   float4 kreg[C::LOADS], vreg[C::LOADS];
-  // row ids of tile t (-1: padding), then its rows -> registers (zeros for padding and bad row ids)
-  int idreg[C::LOADS];
+  // Row ids of tile t (-1: padding), then its rows -> registers (zeros for padding and bad row ids).  A load fetches WPR
+  // rows per warp: lane l holds the id of row l % WPR of load l / WPR.  (A register per load, the same in every lane of the
+  // row, made the kernel of head_dim 128 spill 28 bytes: 7.2 and 173 us for the first two shapes above.)
+  constexpr int WPR = 32 / C::C4;
+  int idreg = -1;
   auto fetch_ids = [&](int t) {
-#pragma unroll
-    for (int u = 0; u < C::LOADS; ++u) {
-      const int pos = t * C::TILE + (u * C::THREADS + tid) / C::C4;
-      idreg[u] = pos < id_lim ? ids[pos] : -1;
-    }
+    const int pos = t * C::TILE + (lane / WPR) * (C::THREADS / C::C4) + warp * WPR + lane % WPR;
+    idreg = lane < WPR * C::LOADS && pos < id_lim ? ids[pos] : -1;
   };
   auto fetch = [&](int t) {
     bool bad = false;
 #pragma unroll
     for (int u = 0; u < C::LOADS; ++u) {
       const int i = u * C::THREADS + tid, c4 = i % C::C4;
-      const int64_t row = idreg[u];
+      const int64_t row = __shfl_sync(0xffffffffu, idreg, u * WPR + lane / C::C4);
       if (row >= 0 && row < p.kv_rows) {
         kreg[u] = __ldg(reinterpret_cast<const float4*>(kbase + row * p.k_s0) + c4);
         vreg[u] = __ldg(reinterpret_cast<const float4*>(vbase + row * p.v_s0) + c4);
