@@ -270,19 +270,28 @@ int build_plan(const int32_t* parent, const int32_t* seqlen, int32_t n_nodes, co
     // List schedule, in emission order, of the tasks that virtual nodes of these sizes are cut into (integer time: a fixed
     // cost per task plus one unit per KV tile; a task = the CTAs of all KV heads of one chunk x request tile, which start
     // side by side): its length, the time of all tasks together, and the end of every node's last task.
+    // Sizes of groups are compared at finer costs: each row of a group is masked in some tile, which makes its tiles longer
+    // (three levels of 256 requests: 1.8 us beside 0.95), and few-row tasks run two to a CTA when they fill more than two
+    // rounds.  Fitted to 680 drawn trees of 2 to 4 sizes each, the schedules then tell the ratio of two sizes' times to 6 %
+    // (mean square; 11 % without).
     struct Piece {
       int64_t length, chunk, nreq;
       bool group;
     };
+    struct Cost {
+      int64_t start[2], tile, group_tile;  // many-row / few-row task; a tile, a tile of a group
+      bool pairs;
+    };
+    const Cost cut_cost = {{5, 4}, 1, 1, false};
     const int64_t sched_slots = std::max<int64_t>((int64_t)(m.num_sms * m.ctas_per_sm) / std::max(num_kv_heads, 1), 1);
-    auto simulate = [&](const std::vector<Piece>& pieces, std::vector<int64_t>& last_end, int64_t& total) {
-      const int64_t start_cost[2] = {5, 4};  // many-row / few-row task, in tile times
+    auto simulate = [&](const std::vector<Piece>& pieces, const Cost& cost, std::vector<int64_t>& last_end, int64_t& total) {
       struct SimTask {
         int phase;
         int64_t key, dur;
         size_t piece;
       };
       std::vector<SimTask> tasks;
+      int64_t few = 0;
       for (size_t i = 0; i < pieces.size(); ++i) {
         const Piece& s = pieces[i];
         if (s.nreq == 0 || s.length <= 0) continue;
@@ -292,7 +301,9 @@ int build_plan(const int32_t* parent, const int32_t* seqlen, int32_t n_nodes, co
           for (int64_t t = 0; t < n_q; ++t) {
             const int64_t q_len = std::min((t + 1) * (int64_t)q_tile, s.nreq) - t * q_tile;
             const int phase = q_len > small_tile ? 0 : 1;
-            tasks.push_back({phase, c_len * 64 + std::min<int64_t>(q_len, 63), start_cost[phase] + ceil_div(c_len, m.tile_tokens), i});
+            few += phase;
+            tasks.push_back({phase, c_len * 64 + std::min<int64_t>(q_len, 63),
+                             cost.start[phase] + (s.group ? cost.group_tile : cost.tile) * ceil_div(c_len, m.tile_tokens), i});
           }
         }
       }
@@ -302,15 +313,20 @@ int build_plan(const int32_t* parent, const int32_t* seqlen, int32_t n_nodes, co
       std::priority_queue<int64_t, std::vector<int64_t>, std::greater<int64_t>> free_at;
       for (int64_t k = 0; k < sched_slots; ++k) free_at.push(0);
       last_end.assign(pieces.size(), 0);
-      int64_t makespan = 0;
+      const size_t many = tasks.size() - (size_t)few;
+      const bool pairs = cost.pairs && few > 2 * sched_slots;
+      int64_t makespan = 0, end = 0;
       total = 0;
-      for (const SimTask& t : tasks) {
-        const int64_t start = free_at.top();
-        free_at.pop();
-        free_at.push(start + t.dur);
-        last_end[t.piece] = std::max(last_end[t.piece], start + t.dur);
-        makespan = std::max(makespan, start + t.dur);
-        total += t.dur;
+      for (size_t k = 0; k < tasks.size(); ++k) {
+        const SimTask& t = tasks[k];
+        if (!pairs || k < many || (k - many) % 2 == 0) {  // (the second of a pair ends with the first, which is no shorter)
+          end = free_at.top() + t.dur;
+          free_at.pop();
+          free_at.push(end);
+          total += t.dur;
+        }
+        last_end[t.piece] = std::max(last_end[t.piece], end);
+        makespan = std::max(makespan, end);
       }
       return makespan;
     };
@@ -323,7 +339,7 @@ int build_plan(const int32_t* parent, const int32_t* seqlen, int32_t n_nodes, co
     auto split_tail = [&](std::vector<Piece>& pieces) {
       std::vector<int64_t> last_end, trial_end;
       int64_t total = 0, total2 = 0;
-      const int64_t makespan = simulate(pieces, last_end, total);
+      const int64_t makespan = simulate(pieces, cut_cost, last_end, total);
       const int64_t bound = ceil_div(total, sched_slots);
       if ((makespan - bound) * 8 <= makespan) return makespan;
       const int64_t late_from = makespan - (makespan - bound + 1) / 2;
@@ -338,7 +354,7 @@ int build_plan(const int32_t* parent, const int32_t* seqlen, int32_t n_nodes, co
           any = true;
         }
       }
-      const int64_t end = any ? simulate(trial, trial_end, total2) : makespan;
+      const int64_t end = any ? simulate(trial, cut_cost, trial_end, total2) : makespan;
       if (end >= makespan) return makespan;
       pieces.swap(trial);
       return end;
@@ -395,10 +411,12 @@ int build_plan(const int32_t* parent, const int32_t* seqlen, int32_t n_nodes, co
       };
       if (direct != nullptr) {
         // Serving path: groups of up to 24 tiles, sized so that the step, the other tasks included, fills a number of rounds of
-        // resident CTAs: two, unless the simulated schedule of another of these numbers (in quarters) ends sooner.  How the
-        // longest tasks fall on the slots matters more than their mean (512 requests under 4 prompts, 16 other tasks on 37
-        // slots, us of stage 1 and the schedule's time units at 1 / 1.25 / 1.5 / 2 / 2.25 / 2.5 / 3 rounds:
-        // 48.3 / 40.7 / 48.2 / 43.8 / 42.1 / 55.9 / 52.9 and 26 / 24 / 29 / 27 / 26 / 36 / 33).
+        // resident CTAs: two, unless there are groups then and the simulated schedule of another of these numbers (in quarters)
+        // ends a tenth sooner.  How the longest tasks fall on the slots matters more than their mean (512 requests under 4
+        // prompts, 16 other tasks on 37 slots, us per decode call and the schedule's units at 1 / 1.25 / 1.5 / 1.75 / 2 / 2.25
+        // rounds: 55.5 / 48.6 / 55.9 / 56.7 / 51.9 / 50.0 and 31.3 / 25.8 / 33.8 / 35.0 / 31.3 / 30.0).  Over 200 drawn bursts 96 take
+        // another number, 1.19 times as fast together, none slower; without the tenth, all tiles alike and from plans without
+        // groups as well, seven took one that was 4 to 18 % slower.
         int64_t cand_tokens = 0, other = 0;
         for (const Spec& s : specs) {
           const int64_t nreq = (int64_t)s.reqs.size();
@@ -408,15 +426,21 @@ int build_plan(const int32_t* parent, const int32_t* seqlen, int32_t n_nodes, co
         const int64_t round = std::max<int64_t>((int64_t)slots / std::max(num_kv_heads, 1), 1);
         hard_cap = 24 * tile;
         std::vector<int64_t> tried, last_end;
-        int64_t best_end = -1;
+        int64_t first_end = 0, best_end = -1;
         for (const int64_t quarters : {8, 5, 9, 6, 7, 4}) {
           const int64_t free_tasks = std::max<int64_t>(std::max(quarters * round / 4 - other, round / 2), 2);
           const int64_t c = std::min(std::max(ceil_div(ceil_div(cand_tokens, free_tasks), tile) * tile, 4 * tile), hard_cap);
           if (std::find(tried.begin(), tried.end(), c) != tried.end()) continue;
           tried.push_back(c);
+          const std::vector<Piece> pieces = packed(c, hard_cap);
+          if (best_end < 0 && std::none_of(pieces.begin(), pieces.end(), [](const Piece& p) { return p.group; })) {
+            cap = c;
+            break;
+          }
           int64_t total = 0;
-          const int64_t end = simulate(packed(c, hard_cap), last_end, total);
-          if (best_end < 0 || end < best_end) {
+          const int64_t end = simulate(pieces, {{20, 16}, 4, 5, false}, last_end, total);
+          if (best_end < 0) first_end = end;
+          if (best_end < 0 || (end * 11 <= first_end * 10 && end < best_end)) {
             best_end = end;
             cap = c;
           }
@@ -436,31 +460,32 @@ int build_plan(const int32_t* parent, const int32_t* seqlen, int32_t n_nodes, co
           const int64_t fill = ceil_div(ceil_div(cand_tokens, round - other), tile) * tile;
           if (fill <= hard_cap) cap = std::max(cap, fill);
         }
-        // That size, or a half, three quarters or one and a half times as much where there are groups then too and the
-        // schedule of the step, its tail split included, ends a twentieth sooner.  Plans for one or two KV heads, where a
-        // long group outlasts the other tasks, want shorter ones (218 requests in three levels at 8/2 heads, us per step and
-        // time units at 1 / 0.5 / 0.75 / 1.5: 12.8 / 11.3 / 12.0 / 14.5 and 9 / 7 / 8 / 11), a search tree of 1024 requests
-        // longer ones (117.2 / 130.0 / 122.0 / 116.3, 76 / 91 / 77 / 71).  A smaller difference the model does not resolve
-        // (512 leaves at head_dim 64 31.6 / 33.6 at 29 / 28).  The tail split that goes with another size may make more
-        // partial rows: never more than fit the library's own scratch where those of the first size do.
+        // That size, or a half, three quarters or one and a half times as much where there are groups then too, no more
+        // partial rows for the merge, and a schedule of the step, its tail split included, that ends a twentieth and two and a
+        // half units sooner.  Of 680 drawn trees with groups 122 take another size, 1.12 times as fast together; two steps
+        // of 11.4 us are 4 and 5 % slower though their stage 1 alone is quicker, one of 56 is 3 % slower; of 250 others 38, 1.12
+        // times as fast, none slower.  At the tail split's costs, rows allowed to grow, 264 of the 680 took another size, eighteen
+        // of which were 3 to 24 % slower.
         const int64_t base = cap, base_hard = hard_cap;
-        const int64_t scratch_rows = (int64_t)FT_STATIC_SCRATCH_BYTES / 4 / ((int64_t)num_qo_heads * (head_dim + 1));
-        int64_t first_end = 0, best_end = 0, rows_limit = 0;
+        int64_t first_end = 0, best_end = 0, first_rows = 0;
         for (const int64_t quarters : {4, 2, 3, 6}) {
           const int64_t size = std::max(base * quarters / 4 / tile * tile, 2 * tile), hard = std::max(base_hard, size);
           std::vector<Piece> pieces = packed(size, hard);
           const bool any = std::any_of(pieces.begin(), pieces.end(), [](const Piece& p) { return p.group; });
           if (quarters == 4 && !any) break;
-          const int64_t end = split_tail(pieces);
-          int64_t rows = 0;
+          split_tail(pieces);
+          std::vector<int64_t> last_end;
+          int64_t rows = 0, total = 0;
           for (const Piece& p : pieces) rows += p.nreq * ceil_div(p.length, p.chunk);
-          if (quarters == 4) rows_limit = std::max(rows, scratch_rows);
-          if (quarters == 4 || (any && rows <= rows_limit && end * 20 <= first_end * 19 && end < best_end)) {
+          const int64_t end = simulate(pieces, {{28, 16}, 4, 5, true}, last_end, total);
+          if (quarters == 4) {
+            first_end = best_end = end;
+            first_rows = rows;
+          } else if (any && rows <= first_rows && end * 21 <= first_end * 20 && end + 10 <= first_end && end < best_end) {
             best_end = end;
             cap = size;
             hard_cap = hard;
           }
-          if (quarters == 4) first_end = end;
         }
       }
       std::vector<Spec> kept, tail;

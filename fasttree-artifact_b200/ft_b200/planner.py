@@ -435,13 +435,11 @@ def plan_b200(tree, kv_ptrs, batch_size, num_qo_heads, num_kv_heads, head_dim, p
     ``num_kv_heads`` is the LOCAL head count of this GPU (the grid is tasks x
     local KV heads), so a head-sharded rank plans finer chunks.  Writes the
     request/KV tile sizes it used back into ``params`` like the reference does."""
-    from . import lib as _lib
     m = b200_model_for(params, head_dim, model)
     vnodes, assign, q_tile, small_tile, target = b200_virtual_nodes(
         tree, num_qo_heads, num_kv_heads, head_dim, m, lambda a, i: _chain_ranges(tree, kv_ptrs, a, i))
     if head_dim in (64, 128, 256) and m.elem_bytes == 2:      # the kernels that honour row ranges exist for these shapes
-        vnodes = b200_sized_groups(vnodes, q_tile, small_tile, m, int(math.floor(target / (2 * head_dim * m.elem_bytes))), num_kv_heads,
-                                   _lib.FT_STATIC_SCRATCH_BYTES // 4 // (num_qo_heads * (head_dim + 1)))
+        vnodes = b200_sized_groups(vnodes, q_tile, small_tile, m, int(math.floor(target / (2 * head_dim * m.elem_bytes))), num_kv_heads)
     vnodes = b200_split_tail(vnodes, q_tile, small_tile, m, num_kv_heads)
     tabs = emit_tables(vnodes, batch_size, small_tile=small_tile, order_key=b200_task_order)
     params.set_q_tile_sizes([q_tile, small_tile])
@@ -472,15 +470,15 @@ def b200_group_short_nodes(vnodes, q_tile, small_tile, m, target_tokens, direct=
     the burst - counts as part of its length."""
     if m.group_member_tokens <= 0:
         return vnodes
-    tile = m.tile_tokens   # (quarters, for other groups: their size in quarters of the computed one)
+    tile = m.tile_tokens
     hard_cap = GROUP_MAX_TILES * tile
     cap = min(max(target_tokens // tile * tile, 4 * tile), hard_cap)
     if direct:
         # Serving path: groups of up to 24 tiles, sized so that the step, the other tasks included, fills a number of
-        # rounds of resident CTAs.  Which number is decided on simulated schedules: two rounds unless another of
-        # GROUP_ROUNDS ends sooner - how the longest tasks fall on the slots matters more than the mean (512 requests
-        # under 4 prompts, 16 other tasks on 37 slots, us of stage 1 and the schedule's time units at 1 / 1.25 / 1.5 / 2 /
-        # 2.25 / 2.5 / 3 rounds: 48.3 / 40.7 / 48.2 / 43.8 / 42.1 / 55.9 / 52.9 and 26 / 24 / 29 / 27 / 26 / 36 / 33).
+        # rounds of resident CTAs: two, unless there are groups then and the simulated schedule of another of GROUP_ROUNDS
+        # ends a tenth sooner - how the longest tasks fall on the slots matters more than the mean (512 requests under 4 prompts, 16 other tasks on
+        # 37 slots, us per decode call and the schedule's units at 1 / 1.25 / 1.5 / 1.75 / 2 / 2.25 rounds:
+        # 55.5 / 48.6 / 55.9 / 56.7 / 51.9 / 50.0 and 31.3 / 25.8 / 33.8 / 35.0 / 31.3 / 30.0).
         cand_tokens = other = 0
         for vn in vnodes:
             length = sum(e - b for b, e in vn.kv_ranges)
@@ -491,7 +489,7 @@ def b200_group_short_nodes(vnodes, q_tile, small_tile, m, target_tokens, direct=
         round_ = max(int(m.num_sms * m.ctas_per_sm * m.waves) // max(num_kv_heads, 1), 1)
         hard_cap = GROUP_MAX_TILES_DIRECT * tile
         slots = max((m.num_sms * m.ctas_per_sm) // max(num_kv_heads, 1), 1)
-        best = best_end = None
+        best = best_end = first_end = None
         tried = set()
         for quarters in GROUP_ROUNDS:
             free_tasks = max(quarters * round_ // 4 - other, round_ // 2, 2)
@@ -500,8 +498,12 @@ def b200_group_short_nodes(vnodes, q_tile, small_tile, m, target_tokens, direct=
                 continue
             tried.add(cap)
             packed = _pack_short_nodes(vnodes, q_tile, small_tile, m, cap, hard_cap, direct)
-            end = b200_simulated_schedule(packed, q_tile, small_tile, m, slots)[0]
-            if best is None or end < best_end:
+            if best is None and all(vn.row_ranges is None for vn in packed):
+                return packed
+            end = b200_simulated_schedule(packed, q_tile, small_tile, m, slots, SERVING_GROUP_COST)[0]
+            if best is None:
+                first_end = end
+            if best is None or (end * 11 <= first_end * 10 and end < best_end):
                 best, best_end = packed, end
         return best
     else:
@@ -524,31 +526,24 @@ def b200_group_short_nodes(vnodes, q_tile, small_tile, m, target_tokens, direct=
     return _pack_short_nodes(vnodes, q_tile, small_tile, m, size, max(hard_cap, size), direct)
 
 
-def b200_sized_groups(vnodes, q_tile, small_tile, m, target_tokens, num_kv_heads, scratch_rows):
+def b200_sized_groups(vnodes, q_tile, small_tile, m, target_tokens, num_kv_heads):
     """:func:`b200_group_short_nodes` at the size it computes, or at a half, three
-    quarters or one and a half times as much where there are groups then too and the
-    schedule of the step, its tail split included, ends a twentieth sooner.  Plans
-    for one or two KV heads, where a long group outlasts the other tasks, want
-    shorter ones (218 requests in three levels at 8/2 heads, us per step and time
-    units at 1 / 0.5 / 0.75 / 1.5: 12.8 / 11.3 / 12.0 / 14.5 and 9 / 7 / 8 / 11), a
-    search tree of 1024 requests longer ones (117.2 / 130.0 / 122.0 / 116.3, 76 / 91 /
-    77 / 71).  A smaller difference the model does not resolve (512 leaves at head_dim
-    64 31.6 / 33.6 at 29 / 28).  The tail split that goes with another size may make
-    more partial rows: never more than the ``scratch_rows`` of the library's own
-    scratch where those of the first size fit."""
+    quarters or one and a half times as much where there are groups then too, no more
+    partial rows for the merge, and a schedule of the step, its tail split included,
+    that ends a twentieth and ten of its units sooner."""
     slots = max((m.num_sms * m.ctas_per_sm) // max(num_kv_heads, 1), 1)
-    best = best_end = first_end = rows_limit = None
+    best = best_end = first_end = first_rows = None
     for quarters in GROUP_CAPS:
         packed = b200_group_short_nodes(vnodes, q_tile, small_tile, m, target_tokens, num_kv_heads=num_kv_heads, quarters=quarters)
         any_group = any(vn.row_ranges is not None for vn in packed)
         if best is None and not any_group:
             return packed
         split = b200_split_tail(packed, q_tile, small_tile, m, num_kv_heads)
-        end = b200_simulated_schedule(split, q_tile, small_tile, m, slots)[0]
+        end = b200_simulated_schedule(split, q_tile, small_tile, m, slots, GROUP_COST)[0]
         rows = sum(len(vn.requests) * -(-sum(e - b for b, e in vn.kv_ranges) // vn.kv_split) for vn in split)
         if best is None:
-            best, best_end, first_end, rows_limit = packed, end, end, max(rows, scratch_rows)
-        elif any_group and rows <= rows_limit and end * 20 <= first_end * 19 and end < best_end:
+            best, best_end, first_end, first_rows = packed, end, end, rows
+        elif any_group and rows <= first_rows and end * 21 <= first_end * 20 and end + 10 <= first_end and end < best_end:
             best, best_end = packed, end
     return best
 
@@ -596,17 +591,20 @@ def _pack_short_nodes(vnodes, q_tile, small_tile, m, cap, hard_cap, direct):
     return kept + tail
 
 
-TAIL_START_COST = (5, 4)   # fixed cost of a many-row / few-row task, in units of one 64-token tile's time
+# Costs of a simulated schedule: fixed part of a many-row / few-row task, a KV tile, a KV tile of a group, whether few-row
+# tasks that fill more than two rounds run two to a CTA
+CUT_COST = (5, 4, 1, 1, False)
+SERVING_GROUP_COST = (20, 16, 4, 5, False)   # ... where sizes of groups are compared (each of their rows is masked in some tile)
+GROUP_COST = (28, 16, 4, 5, True)
 TAIL_ROUNDS = 1            # a late task is halved this many times at most (measured: quarters cost more in partial rows than they gain)
 
 
-def b200_simulated_schedule(vnodes, q_tile, small_tile, m, slots):
+def b200_simulated_schedule(vnodes, q_tile, small_tile, m, slots, cost=CUT_COST):
     """List schedule of the tasks the virtual nodes will be cut into, in emission
     order (phase, then longest chunk first), on ``slots`` task slots - a task being
     the CTAs of all KV heads of one (chunk, request tile), which start side by side.
-    Integer time: :data:`TAIL_START_COST` per task plus one unit per KV tile.
-    Returns (makespan, total time of all tasks, per virtual node the time its last
-    task ends)."""
+    Integer time, in the units of ``cost``.  Returns (makespan, total time of all
+    tasks, per virtual node the time its last task ends)."""
     tasks = []
     for vi, vn in enumerate(vnodes):
         length = sum(e - b for b, e in vn.kv_ranges) + sum(vn.member_room or ())
@@ -621,18 +619,22 @@ def b200_simulated_schedule(vnodes, q_tile, small_tile, m, slots):
                 q_len = min((t + 1) * vn.q_tile, nreq) - t * vn.q_tile
                 phase = 0 if q_len > small_tile else 1
                 tasks.append((phase, -(c_len * 64 + min(q_len, 63)), len(tasks), vi,
-                              TAIL_START_COST[phase] + -(-c_len // m.tile_tokens)))
+                              cost[phase] + cost[2 if vn.row_ranges is None else 3] * -(-c_len // m.tile_tokens)))
     tasks.sort(key=lambda t: t[:3])
-    free = [0] * max(slots, 1)
+    many = sum(t[0] == 0 for t in tasks)
+    slots = max(slots, 1)
+    pairs = cost[4] and len(tasks) - many > 2 * slots
+    free = [0] * slots
     heapq.heapify(free)
     last_end = [0] * len(vnodes)
-    makespan = total = 0
-    for _, _, _, vi, dur in tasks:
-        start = heapq.heappop(free)
-        heapq.heappush(free, start + dur)
-        last_end[vi] = max(last_end[vi], start + dur)
-        makespan = max(makespan, start + dur)
-        total += dur
+    makespan = total = end = 0
+    for k, (_, _, _, vi, dur) in enumerate(tasks):
+        if not pairs or k < many or (k - many) % 2 == 0:      # (the second of a pair ends with the first, which is no shorter)
+            end = heapq.heappop(free) + dur
+            heapq.heappush(free, end)
+            total += dur
+        last_end[vi] = max(last_end[vi], end)
+        makespan = max(makespan, end)
     return makespan, total, last_end
 
 

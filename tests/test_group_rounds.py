@@ -68,3 +68,41 @@ def test_another_group_size_needs_no_more_scratch_than_there_is(monkeypatch, siz
     first = plan(planner.plan_b200)
     scratch_rows = lib.FT_STATIC_SCRATCH_BYTES // (4 * hq * 129)
     assert len(spec.vnode_to_q_entries) <= max(len(first.vnode_to_q_entries), scratch_rows)
+
+
+@pytest.mark.parametrize("sizes,lens,hq,hkv,d,quarters", [
+    # sizes that a schedule of equal tiles called quicker, and what they took of the first size's time
+    ([1, 1, 50, 75, 301], [1993, 46, 10, 10, 32], 4, 1, 128, 4),      # 1.33: longer groups
+    ([1, 2, 5, 24, 29], [300, 1178, 253, 16, 23], 32, 8, 256, 4),     # 1.22
+    ([1, 343, 408], [9116, 40, 12], 24, 8, 128, 2),                   # 1.14 (the half as long ones 0.93)
+    ([1, 4, 199], [590, 144, 54], 24, 8, 64, 4),                      # 1.13
+    ([1, 2, 4, 8, 26], [61, 244, 25, 8, 59], 32, 8, 256, 4),          # 1.11
+    ([1, 179], [740, 9], 16, 16, 128, 4),                             # 1.11
+    ([1, 2, 25], [1218, 63, 9], 64, 8, 128, 4),                       # 1.07: half as many rows again for the merge
+    ([1, 3, 99], [109, 30, 29], 64, 8, 128, 4),                       # 1.05
+])
+def test_a_group_size_that_runs_slower_is_not_taken(monkeypatch, sizes, lens, hq, hkv, d, quarters):
+    nodes = kv_tree_simple.tree_from_rows(tree_generation.generate_tree(sizes, lens))
+    batch, ptrs = kv_tree_simple.assign_requests(nodes)
+
+    def tables(make):
+        params = fasttree.FastTreeParams()
+        params.set_kv_group_num(hq // hkv)
+        params.set_kv_dtype(torch.bfloat16)
+        plan = make(nodes, ptrs, batch, hq, hkv, d, params)
+        return [plan.vnode_to_kv_lens, plan.vnode_to_q_lens, plan.vnode_to_q_entries]
+
+    chosen, native = tables(planner.plan_b200), tables(planner.plan_b200_native)
+    monkeypatch.setattr(planner, "GROUP_CAPS", (quarters,))
+    for a, b, c in zip(chosen, native, tables(planner.plan_b200)):
+        np.testing.assert_array_equal(a, c)
+        np.testing.assert_array_equal(b, c)
+
+
+def test_a_burst_without_groups_at_two_rounds_keeps_its_tails_apart():
+    """168 tails of one or two tiles under 7 prompts at 64/8 heads: two rounds leave them alone, and so they run quickest
+    (30.5 us per decode call; grouped 33.0 to 41.0)."""
+    m = planner.B200Model(rows_per_cta=128, group_min_members=4)
+    nodes = _burst(168, 7, 213, 82, 1)
+    out = planner.b200_group_short_nodes(nodes, 16, 2, m, 0, direct=True, num_kv_heads=8)
+    assert len(out) == len(nodes) and all(v.row_ranges is None for v in out)
