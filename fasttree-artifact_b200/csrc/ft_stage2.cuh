@@ -2,8 +2,8 @@
 // rows (kernel_bench/fasttree.py:482-546).  Memory-bound on the partial buffers;
 // those are written by stage 1 just before and are normally still in L2.
 //
-// stage2_merge_kernel: one warp per (request, head); lanes span head_dim in float4
-// chunks, so a partial row of head_dim 128 is one 512-byte coalesced warp load.
+// stage2_merge_kernel: one warp per (request, head) of head_dim 128 or 256; lanes span
+// it in float4 chunks, so a partial row of 128 is one 512-byte coalesced warp load.
 // The weights exp(lse_i - max) are computed lane-parallel (32 partial rows at a
 // time, running maximum across batches) and broadcast by shuffle, which keeps the
 // dependent chain per partial to one FMA.
@@ -22,12 +22,63 @@
 
 namespace ft {
 
-// MAXC: float4 chunks per lane (1: head_dim <= 128, 2: head_dim <= 256).  RB: partial rows in flight per lane.  A
-// request's merge is a chain of L2 round trips, one per batch of RB rows.  A launch that fits one round of CTAs is
-// bound by that chain and runs with RB = 8 at six CTAs per SM; a launch of several rounds is bound by how many warps
-// the SM holds and runs with RB = 4 at nine (head_dim <= 128).
+// Four columns of an output row.
+template <typename T>
+__device__ __forceinline__ void store_columns(const Stage2Params& p, int req, int head, int at, const float4& acc, float inv) {
+  T* __restrict__ dst = reinterpret_cast<T*>(p.o) + (int64_t)req * p.o_s0 + (int64_t)head * p.o_s1 + at;
+  alignas(16) T out[4] = {from_float<T>(acc.x * inv), from_float<T>(acc.y * inv), from_float<T>(acc.z * inv), from_float<T>(acc.w * inv)};
+  if (p.o_vec) {  // in one store when the output rows allow it
+    if constexpr (sizeof(T) == 2)
+      *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(out);
+    else
+      *reinterpret_cast<float4*>(dst) = *reinterpret_cast<const float4*>(out);
+  } else {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) dst[e] = out[e];
+  }
+}
+
+// A partial row counts only if its weight, relative to the request's largest LSE, is not zero - else infinities and NaN in
+// rows that do not count would come into the sum as 0 x Inf.  While rows are still being met the largest LSE is not known,
+// and one that is added may turn out not to count.  A sum that came out finite met none of that; any other is formed once
+// more here, row by row with the largest LSE known, and so depends neither on the order of the rows nor on the kernel.
+// That the kernels hold this code costs them 0.02 to 0.05 us (1024 pieces x 2 rows 2.31 -> 2.36, 2048 x 7 no change), the
+// form of two float4s per lane 3 to 5 % (65536 x 2 17.8 -> 18.4).
+// Called by each lane for the four columns from `column` on of its request's row, which it has stored already.
+template <typename T>
+__device__ __noinline__ void merge_again(const Stage2Params& p, int req, int column) {
+  const int head = column >> p.dim_shift, at = column & (p.head_dim - 1), off = p.r2v_offs[req], n = p.r2v_lens[req];
+  auto lse_of = [&](int i, int& row) {  // -inf: an empty partial, or a bad row id (flagged where it was met first)
+    row = p.r2v_entries[off + i];
+    return row >= 0 && row < p.num_partial_rows ? __ldcg(p.mid_lse + (int64_t)row * p.ml_s0 + head) : -INFINITY;
+  };
+  float mx = -INFINITY, sum = 0.f;
+  int row;
+  for (int i = 0; i < n; ++i) mx = fmaxf(mx, lse_of(i, row));
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int i = 0; i < n; ++i) {
+    const float lse = lse_of(i, row), w = lse > -INFINITY ? expf(lse - mx) : 0.f;
+    if (w == 0.f) continue;
+    const float4 x = __ldcg(reinterpret_cast<const float4*>(p.mid_o + (int64_t)row * p.mo_s0 + (int64_t)head * p.mo_s1 + at));
+    sum += w;
+    acc.x = fmaf(w, x.x, acc.x);
+    acc.y = fmaf(w, x.y, acc.y);
+    acc.z = fmaf(w, x.z, acc.z);
+    acc.w = fmaf(w, x.w, acc.w);
+  }
+  store_columns<T>(p, req, head, at, acc, sum > 0.f ? 1.f / sum : 0.f);
+}
+
+__device__ __forceinline__ bool all_finite(const float4& x) {  // 0 x every element: 0, or NaN
+  return fmaf(x.x, 0.f, fmaf(x.y, 0.f, fmaf(x.z, 0.f, x.w * 0.f))) == 0.f;
+}
+
+// MAXC: float4 chunks per lane (1: head_dim 128, 2: head_dim 256; smaller heads go to the other kernel).  RB: partial rows
+// in flight per lane.  A request's merge is a chain of L2 round trips, one per batch of RB rows.  A launch that fits one
+// round of CTAs is bound by that chain and runs with RB = 8 at six CTAs per SM; a launch of several rounds is bound by how
+// many warps the SM holds and runs with RB = 4 at nine (head_dim 128).
 template <typename T, int MAXC, int RB>
-__global__ void __launch_bounds__(128, MAXC == 1 && RB == 4 ? 9 : 6) stage2_merge_kernel(Stage2Params p) {
+__global__ void __launch_bounds__(128, MAXC == 1 && RB == 4 ? 9 : 6) stage2_merge_kernel(const __grid_constant__ Stage2Params p) {
   allow_dependent_launch();  // a following stage-1 launch may set itself up under this kernel's tail
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t pair = (int64_t)blockIdx.x * 4 + warp;
@@ -107,30 +158,22 @@ __global__ void __launch_bounds__(128, MAXC == 1 && RB == 4 ? 9 : 6) stage2_merg
   }
   wsum = warp_sum(wsum);
   const float inv = wsum > 0.f ? 1.f / wsum : 0.f;
-  T* __restrict__ dst = reinterpret_cast<T*>(p.o) + (int64_t)req * p.o_s0 + (int64_t)head * p.o_s1;
 #pragma unroll
-  for (int c = 0; c < MAXC; ++c) {
-    const int ch = lane + 32 * c;
-    if (ch < chunks) {
-      alignas(16) T out[4] = {from_float<T>(acc[c].x * inv), from_float<T>(acc[c].y * inv), from_float<T>(acc[c].z * inv),
-                  from_float<T>(acc[c].w * inv)};
-      if (p.o_vec) {  // four elements in one store when the output rows allow it
-        if constexpr (sizeof(T) == 2)
-          *reinterpret_cast<uint2*>(dst + 4 * ch) = *reinterpret_cast<const uint2*>(out);
-        else
-          *reinterpret_cast<float4*>(dst + 4 * ch) = *reinterpret_cast<const float4*>(out);
-      } else {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) dst[4 * ch + e] = out[e];
-      }
-    }
-  }
+  for (int c = 0; c < MAXC; ++c)
+    if (lane + 32 * c < chunks) store_columns<T>(p, req, head, 4 * (lane + 32 * c), acc[c], inv);
   if (p.o_lse != nullptr && lane == 0)
     p.o_lse[(int64_t)req * p.heads + head] = wsum > 0.f ? mx + logf(wsum) : -INFINITY;
+  if (n <= 32) return;  // all rows were met with their largest LSE known
+  unsigned again = 0;
+#pragma unroll
+  for (int c = 0; c < MAXC; ++c)
+    if (lane + 32 * c < chunks && !all_finite(acc[c])) again |= 1u << c;
+#pragma unroll 1
+  for (; again != 0; again &= again - 1) merge_again<T>(p, req, (head << p.dim_shift) + 4 * (lane + 32 * (__ffs(again) - 1)));
 }
 
 template <typename T, int C, int RB, int SPLIT>
-__global__ void __launch_bounds__(128, RB * C == 4 ? (C == 1 ? 10 : 9) : 1) stage2_piece_kernel(Stage2Params p) {
+__global__ void __launch_bounds__(128, RB * C == 4 ? (C == 1 ? 10 : 9) : 1) stage2_piece_kernel(const __grid_constant__ Stage2Params p) {
   static_assert(SPLIT == 1 || SPLIT == 4, "a warp or the whole block per item");
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const unsigned item = SPLIT == 1 ? blockIdx.x * 4 + warp : blockIdx.x;
@@ -255,6 +298,7 @@ __global__ void __launch_bounds__(128, RB * C == 4 ? (C == 1 ? 10 : 9) : 1) stag
   for (int c = 0; c < C; ++c) {
     if (head[c] < 0) continue;
     const float inv = sum[c] > 0.f ? 1.f / sum[c] : 0.f;
+    // (through store_columns the two-float4 form spills 36 bytes)
     T* __restrict__ dst = reinterpret_cast<T*>(p.o) + (int64_t)req * p.o_s0 + (int64_t)head[c] * p.o_s1 + at[c];
     alignas(16) T out[4] = {from_float<T>(acc[c].x * inv), from_float<T>(acc[c].y * inv), from_float<T>(acc[c].z * inv),
                             from_float<T>(acc[c].w * inv)};
@@ -270,6 +314,13 @@ __global__ void __launch_bounds__(128, RB * C == 4 ? (C == 1 ? 10 : 9) : 1) stag
     if (p.o_lse != nullptr && at[c] == 0)
       p.o_lse[(int64_t)req * p.heads + head[c]] = sum[c] > 0.f ? mx[c] + logf(sum[c]) : -INFINITY;
   }
+  if (SPLIT == 1 && n_all <= RB) return;  // all rows were met with their largest LSE known
+  unsigned again = 0;
+#pragma unroll
+  for (int c = 0; c < C; ++c)
+    if (head[c] >= 0 && !all_finite(acc[c])) again |= 1u << c;
+#pragma unroll 1
+  for (; again != 0; again &= again - 1) merge_again<T>(p, req, 4 * (lane + 32 * (__ffs(again) - 1 + C * piece)));
 }
 
 }  // namespace ft
