@@ -689,8 +689,8 @@ int launch_pieces(ft::Stage2Params p, cudaStream_t st, bool after_stage1) {
   return launch_merge(ft::stage2_piece_kernel<T, C, RB, SPLIT>, p, SPLIT == 1 ? (items + 3) / 4 : items, st, after_stage1);
 }
 
-// Which merge, by the 128-float pieces of the output and the mean number of partial rows per request (an upper bound where
-// the scratch buffers hold more rows than the plan).  us for the merge alone, replayed from a graph, and per decode step:
+// Which merge, by the 128-float pieces of the output and the mean number of partial rows per request (of the plan, where
+// the caller states it: its scratch buffers may hold more).  us for the merge alone, replayed from a graph, and per decode step:
 //   few pieces, many rows: four warps per piece    160 pieces x 36 rows, one warp per head 5.9 / four 3.9 (step 13.8 / 11.8),
 //                                                  32 x 18 4.2 / 2.9 (12.2 / 9.9); 1024 x 9 3.7 / 3.4, 2048 x 9 4.1 / 5.2
 //   one round of CTAs with more than four rows, or six rows and more: weights by one lane per row
@@ -699,10 +699,10 @@ int launch_pieces(ft::Stage2Params p, cudaStream_t st, bool after_stage1) {
 //   very many pieces: two of them per warp         65536 x 2 33.8 -> 21.2, 32768 x 3 20.9 -> 17.0 (one piece 18.7)
 // At head_dim 64 and below one lane per row would leave half of the lanes and more idle: 8192 pieces x 18 rows 19.3 / 13.8.
 template <typename T>
-int launch_stage2(const ft::Stage2Params& p, cudaStream_t st, bool after_stage1) {
+int launch_stage2(const ft::Stage2Params& p, int64_t rows, cudaStream_t st, bool after_stage1) {
   const int64_t pieces = (((int64_t)p.batch * p.heads << p.dim_shift) + 127) / 128, heads = (int64_t)p.batch * p.heads;
   if (pieces == 0) return FT_OK;
-  const int64_t rows = p.num_partial_rows, batch = p.batch;
+  const int64_t batch = p.batch;
   if (pieces <= 1024 && rows >= 6 * batch)
     return rows >= 12 * batch ? launch_pieces<T, 1, 8, 4>(p, st, after_stage1) : launch_pieces<T, 1, 4, 4>(p, st, after_stage1);
   int dev = 0;
@@ -844,10 +844,11 @@ int stage2_impl(const ft_decode_args* a, bool after_stage1) {
                   : 0;
   }
   cudaStream_t st = static_cast<cudaStream_t>(a->stream);
+  const int64_t rows = a->plan_rows > 0 && a->plan_rows < a->num_partial_rows ? a->plan_rows : a->num_partial_rows;
   switch (a->dtype) {
-    case FT_F16: return launch_stage2<__half>(p, st, after_stage1);
-    case FT_BF16: return launch_stage2<__nv_bfloat16>(p, st, after_stage1);
-    default: return launch_stage2<float>(p, st, after_stage1);
+    case FT_F16: return launch_stage2<__half>(p, rows, st, after_stage1);
+    case FT_BF16: return launch_stage2<__nv_bfloat16>(p, rows, st, after_stage1);
+    default: return launch_stage2<float>(p, rows, st, after_stage1);
   }
 }
 }  // namespace

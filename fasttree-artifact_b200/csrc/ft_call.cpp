@@ -66,22 +66,23 @@ void pair(const char* name, PyObject* o, int64_t (&out)[2]) {
   Py_DECREF(seq);
 }
 
-// The task sizes that a plan's vnode_to_kv_lens tensor carries as an attribute (ft_b200.planner.task_sizes); without it none
-// are known.
+// The task sizes that a plan's vnode_to_kv_lens tensor carries as an attribute (ft_b200.planner.task_sizes), with the plan's
+// partial rows behind them where the scratch buffers hold more; without it none are known.
 void task_sizes(PyObject* table, ft_decode_args& a) {
   static PyObject* const name = PyUnicode_InternFromString("task_sizes");
   PyObject* sizes = nullptr;
   if (_PyObject_LookupAttr(table, name, &sizes) < 0) throw Refused();
   if (sizes == nullptr) return;
-  long long n[4] = {0, 0, 0, 0};
-  const bool ok = PyTuple_Check(sizes) && PyTuple_GET_SIZE(sizes) == 4;
-  for (int i = 0; ok && i < 4; ++i) n[i] = PyLong_AsLongLong(PyTuple_GET_ITEM(sizes, i));
+  long long n[5] = {0, 0, 0, 0, 0};
+  const int count = PyTuple_Check(sizes) ? (int)PyTuple_GET_SIZE(sizes) : 0;
+  for (int i = 0; (count == 4 || count == 5) && i < count; ++i) n[i] = PyLong_AsLongLong(PyTuple_GET_ITEM(sizes, i));
   Py_DECREF(sizes);
   if (PyErr_Occurred()) throw Refused();
   a.few_tokens = n[0];
   a.few_longest = (int32_t)n[1];
   a.few_over_8_rows = (int32_t)n[2];
   a.many_longest = (int32_t)n[3];
+  a.plan_rows = (int32_t)n[4];
 }
 
 // Positional arguments of the reference's fasttree_decode (kernel_bench/fasttree.py:582-601), in order.
@@ -131,7 +132,7 @@ void fill(PyObject* const* x, ft_decode_args& a, c10::DeviceIndex& device) {
   }
   int64_t nums[2], offs[2], q_tiles[2], kv_tiles[2];
   pair("phase_node_nums", arg(NODE_NUMS), nums);
-  if (dtype != at::kFloat) task_sizes(arg(KV_LENS), a);  // (fp32 kernels have one form)
+  task_sizes(arg(KV_LENS), a);
   pair("phase_node_offsets", arg(NODE_OFFSETS), offs);
   pair("phase_q_tile_sizes", arg(Q_TILES), q_tiles);
   pair("phase_kv_tile_sizes", arg(KV_TILES), kv_tiles);

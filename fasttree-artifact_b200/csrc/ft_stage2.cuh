@@ -87,7 +87,6 @@ __global__ void __launch_bounds__(128, MAXC == 1 && RB == 4 ? 9 : 6) stage2_merg
   const int head = (int)(pair - (int64_t)req * p.heads);
   const int off = p.r2v_offs[req];
   const int n = p.r2v_lens[req];
-  const int chunks = p.head_dim >> 2;
   int batch_rows = lane < n ? p.r2v_entries[off + lane] : -1;  // plan data: readable before stage 1 is done
   wait_for_prior_grid();                                       // the partial buffers are complete from here on
 
@@ -122,8 +121,7 @@ __global__ void __launch_bounds__(128, MAXC == 1 && RB == 4 ? 9 : 6) stage2_merg
             reinterpret_cast<const float4*>(p.mid_o + (int64_t)(rows[r] >= 0 ? rows[r] : 0) * p.mo_s0 + (int64_t)head * p.mo_s1);
 #pragma unroll
         for (int c = 0; c < MAXC; ++c) {
-          const int ch = lane + 32 * c;
-          x[r][c] = rows[r] >= 0 && ch < chunks ? __ldcg(src + ch) : make_float4(0.f, 0.f, 0.f, 0.f);
+          x[r][c] = rows[r] >= 0 ? __ldcg(src + lane + 32 * c) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
       }
       if (i0 == 0) {  // the batch's LSEs are needed only now: rescale what has been summed so far to the new maximum
@@ -159,15 +157,14 @@ __global__ void __launch_bounds__(128, MAXC == 1 && RB == 4 ? 9 : 6) stage2_merg
   wsum = warp_sum(wsum);
   const float inv = wsum > 0.f ? 1.f / wsum : 0.f;
 #pragma unroll
-  for (int c = 0; c < MAXC; ++c)
-    if (lane + 32 * c < chunks) store_columns<T>(p, req, head, 4 * (lane + 32 * c), acc[c], inv);
+  for (int c = 0; c < MAXC; ++c) store_columns<T>(p, req, head, 4 * (lane + 32 * c), acc[c], inv);
   if (p.o_lse != nullptr && lane == 0)
     p.o_lse[(int64_t)req * p.heads + head] = wsum > 0.f ? mx + logf(wsum) : -INFINITY;
   if (n <= 32) return;  // all rows were met with their largest LSE known
   unsigned again = 0;
 #pragma unroll
   for (int c = 0; c < MAXC; ++c)
-    if (lane + 32 * c < chunks && !all_finite(acc[c])) again |= 1u << c;
+    if (!all_finite(acc[c])) again |= 1u << c;
 #pragma unroll 1
   for (; again != 0; again &= again - 1) merge_again<T>(p, req, (head << p.dim_shift) + 4 * (lane + 32 * (__ffs(again) - 1)));
 }

@@ -92,7 +92,6 @@ class FastTreeMetadata:
             self.kv_entries_aux = self.vnode_q_kv_ranges = self.aux_segments = None
         self.mid_o = torch.empty((max_vnode_to_q_entries, num_qo_heads, head_dim), dtype=torch.float32, device=device)
         self.mid_lse = torch.empty((max_vnode_to_q_entries, num_qo_heads), dtype=torch.float32, device=device)
-        self.plan_mid_o, self.plan_mid_lse = self.mid_o, self.mid_lse    # the rows a decode call is given
 
         self.phase_node_nums: Tuple[int, int] = None
         self.phase_node_offsets: Tuple[int, int] = None

@@ -58,7 +58,7 @@ def _replace_radix_attn():
             md.vnode_to_kv_offs, md.vnode_to_kv_lens,
             md.vnode_to_q_entries, md.vnode_to_q_offs, md.vnode_to_q_lens,
             md.req_to_vnode_entries, md.req_to_vnode_offs, md.req_to_vnode_lens,
-            md.plan_mid_o, md.plan_mid_lse,
+            md.mid_o, md.mid_lse,
             md.phase_node_nums, md.phase_node_offsets, md.phase_q_tile_sizes, md.phase_kv_tile_sizes,
             sm_scale=self.scaling, logit_cap=self.logit_cap,
             phase_info=md.phase_info_dev if md.graph_safe else None,

@@ -136,15 +136,16 @@ def _upload(md, tabs, last_vnodes, tail_state=None, src_table=None):
                     md.kv_entries_aux[dst + length:dst + length + room] = flat[src]
         md.refresh_pending = md.num_grouped_tails > 0 or (md.graph_safe and md.refresh_layer is None)
     md.phase_node_nums = list(tabs["phase_node_nums"])
-    md.vnode_to_kv_lens.task_sizes = tabs.get("task_sizes") or _planner.task_sizes(
-        tabs["phase_node_nums"], tabs["vnode_to_kv_lens"], tabs["vnode_to_q_lens"], md.kv_group_num)
+    sizes = tabs.get("task_sizes") or _planner.task_sizes(tabs["phase_node_nums"], tabs["vnode_to_kv_lens"],
+                                                          tabs["vnode_to_q_lens"], md.kv_group_num)
+    if not md.graph_safe:
+        # The plan's rows, far fewer than the buffers': the merge kernel is chosen by their number (512 requests 13 270 ->
+        # 13 150 us per burst).  A captured step has to fit every later plan and to give what an eager call gives.
+        sizes = (*sizes, int(rows))
+    md.vnode_to_kv_lens.task_sizes = sizes
     md.phase_node_offsets = list(tabs["phase_node_offsets"])
     md.req_last_vnodes = [int(v) for v in last_vnodes]
     md.num_vnodes, md.num_partial_rows = int(nv), int(rows)
-    # The plan's own rows: the merge kernel is chosen by their number (512 requests 13 270 -> 13 150 us per burst).  A captured
-    # step has to fit every later plan.
-    n = md.mid_o.shape[0] if md.graph_safe else max(int(rows), 1)
-    md.plan_mid_o, md.plan_mid_lse = md.mid_o[:n], md.mid_lse[:n]
 
 
 # --------------------------------------------------------------- reference-compatible

@@ -88,7 +88,7 @@ class DecodeArgs(ctypes.Structure):
         ("vnode_to_kv_entries_aux", ctypes.c_void_p),
         ("kv_entries_aux_len", ctypes.c_int64),
         ("few_tokens", ctypes.c_int64), ("few_longest", ctypes.c_int32), ("few_over_8_rows", ctypes.c_int32),
-        ("many_longest", ctypes.c_int32),
+        ("many_longest", ctypes.c_int32), ("plan_rows", ctypes.c_int32),
     ]
 
 

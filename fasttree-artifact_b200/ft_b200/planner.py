@@ -91,7 +91,8 @@ def task_sizes(phase_node_nums, kv_lens, q_lens, group):
 
     They have no slot in the reference's 13-entry tuple and travel as the attribute ``task_sizes`` of the
     ``vnode_to_kv_lens`` tensor, which saving, pickling and deepcopy keep; a table without it works too, the launch then
-    assumes nothing."""
+    assumes nothing.  A fifth entry, the plan's partial rows, goes with scratch buffers that hold more of them: the merge
+    kernel is chosen by their number."""
     n0, n1 = phase_node_nums
     few = kv_lens[n0:n0 + n1]
     return (int(few.sum(dtype=np.int64)), int(few.max(initial=0)), int(np.count_nonzero(q_lens[n0:n0 + n1] > 8 // group)),

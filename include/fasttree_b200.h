@@ -150,6 +150,9 @@ typedef struct ft_decode_args {
   int32_t few_over_8_rows;            /* have more than 8 query rows, the longest chunk of phase 0.  They choose between */
   int32_t many_longest;               /* ways to run phase 1 with the same results; few_longest 0 = unknown: one task per
                                          CTA (head_dim 256: the tcgen05 kernel for both phases) */
+  int32_t plan_rows;                  /* partial rows of the plan (ft_plan_info.partial_rows), by whose number per request
+                                         the merge kernel is chosen; 0 = num_partial_rows, which buffers sized for more than
+                                         one plan overstate.  Stays below 2^31; bounds nothing. */
 } ft_decode_args;
 
 /* Library version (major*10000 + minor*100 + patch). */
