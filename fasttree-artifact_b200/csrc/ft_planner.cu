@@ -374,40 +374,71 @@ int build_plan(const int32_t* parent, const int32_t* seqlen, int32_t n_nodes, co
       const int64_t target_tokens = (int64_t)std::floor(target / (double)row_bytes);
       int64_t hard_cap = 16 * tile;
       int64_t cap = std::min(std::max(target_tokens / tile * tile, 4 * tile), hard_cap);
-      // the sizes that the grouping below comes out with at groups of `cap` tokens
+      // The grouping at groups of `cap` tokens: virtual nodes order[begin, end), in the order of the result.
+      struct Bundle {
+        size_t begin, end;
+        int64_t tokens, nreq;
+        bool group;
+      };
+      struct Packing {
+        std::vector<size_t> order;
+        std::vector<Bundle> bundles;
+      };
       std::vector<uint8_t> taken((size_t)std::max(batch, 1), 0);
-      auto packed = [&](int64_t cap, int64_t hard_cap) {
-        std::vector<Piece> kept, tail;
-        std::vector<const Spec*> cur;
+      auto pack = [&](int64_t cap, int64_t hard_cap) {
+        Packing kept, tail;
+        auto single = [&](Packing& to, size_t i) {
+          to.bundles.push_back({to.order.size(), to.order.size() + 1, specs[i].length, (int64_t)specs[i].reqs.size(), false});
+          to.order.push_back(i);
+        };
+        std::vector<size_t> cur;
         int64_t cur_tokens = 0, cur_n = 0;
         auto close = [&]() {
-          for (const Spec* s : cur)
-            for (int32_t r : s->reqs) taken[r] = 0;
-          if ((int64_t)cur.size() >= m.group_min_members && cur_n > small_tile)
-            tail.push_back({cur_tokens, ceil_div(cur_tokens, tile) * tile, cur_n, true});
-          else
-            for (const Spec* s : cur) tail.push_back({s->length, s->chunk, (int64_t)s->reqs.size(), false});
+          for (size_t i : cur)
+            for (int32_t r : specs[i].reqs) taken[r] = 0;
+          if ((int64_t)cur.size() >= m.group_min_members && cur_n > small_tile) {
+            tail.bundles.push_back({tail.order.size(), tail.order.size() + cur.size(), cur_tokens, cur_n, true});
+            tail.order.insert(tail.order.end(), cur.begin(), cur.end());
+          } else {
+            for (size_t i : cur) single(tail, i);
+          }
           cur.clear();
           cur_tokens = cur_n = 0;
         };
-        for (const Spec& s : specs) {
+        for (size_t i = 0; i < specs.size(); ++i) {
+          const Spec& s = specs[i];
           const int64_t nreq = (int64_t)s.reqs.size(), span = s.length + s.room;
           if (nreq > small_tile || span > m.group_member_tokens) {
-            kept.push_back({s.length, s.chunk, nreq, false});
+            single(kept, i);
             continue;
           }
           bool shared = false;
           for (int32_t r : s.reqs) shared = shared || taken[r] != 0;
+          // (serving path: a group is closed once it has reached the cap, not before it would pass it, so that
+          // the groups number no more than the tasks they were sized for)
           const bool full = direct != nullptr ? cur_tokens >= cap : cur_tokens + span > cap;
           if (!cur.empty() && (cur_n + nreq > q_tile || cur_tokens + span > hard_cap || (full && cur_n > small_tile) || shared)) close();
           for (int32_t r : s.reqs) taken[r] = 1;
           cur_tokens += span;
           cur_n += nreq;
-          cur.push_back(&s);
+          cur.push_back(i);
         }
         close();
-        kept.insert(kept.end(), tail.begin(), tail.end());
+        for (Bundle b : tail.bundles) {
+          b.begin += kept.order.size();
+          b.end += kept.order.size();
+          kept.bundles.push_back(b);
+        }
+        kept.order.insert(kept.order.end(), tail.order.begin(), tail.order.end());
         return kept;
+      };
+      auto group_chunk = [&](int64_t tokens) { return ceil_div(tokens, tile) * tile; };
+      auto sizes_of = [&](const Packing& packing) {
+        std::vector<Piece> pieces;
+        pieces.reserve(packing.bundles.size());
+        for (const Bundle& b : packing.bundles)
+          pieces.push_back({b.tokens, b.group ? group_chunk(b.tokens) : specs[packing.order[b.begin]].chunk, b.nreq, b.group});
+        return pieces;
       };
       if (direct != nullptr) {
         // Serving path: groups of up to 24 tiles, sized so that the step, the other tasks included, fills a number of rounds of
@@ -432,7 +463,7 @@ int build_plan(const int32_t* parent, const int32_t* seqlen, int32_t n_nodes, co
           const int64_t c = std::min(std::max(ceil_div(ceil_div(cand_tokens, free_tasks), tile) * tile, 4 * tile), hard_cap);
           if (std::find(tried.begin(), tried.end(), c) != tried.end()) continue;
           tried.push_back(c);
-          const std::vector<Piece> pieces = packed(c, hard_cap);
+          const std::vector<Piece> pieces = sizes_of(pack(c, hard_cap));
           if (best_end < 0 && std::none_of(pieces.begin(), pieces.end(), [](const Piece& p) { return p.group; })) {
             cap = c;
             break;
@@ -470,7 +501,7 @@ int build_plan(const int32_t* parent, const int32_t* seqlen, int32_t n_nodes, co
         int64_t first_end = 0, best_end = 0, first_rows = 0;
         for (const int64_t quarters : {4, 2, 3, 6}) {
           const int64_t size = std::max(base * quarters / 4 / tile * tile, 2 * tile), hard = std::max(base_hard, size);
-          std::vector<Piece> pieces = packed(size, hard);
+          std::vector<Piece> pieces = sizes_of(pack(size, hard));
           const bool any = std::any_of(pieces.begin(), pieces.end(), [](const Piece& p) { return p.group; });
           if (quarters == 4 && !any) break;
           split_tail(pieces);
@@ -488,55 +519,30 @@ int build_plan(const int32_t* parent, const int32_t* seqlen, int32_t n_nodes, co
           }
         }
       }
-      std::vector<Spec> kept, tail;
-      std::vector<Spec> cur;
-      std::vector<uint8_t> in_group((size_t)std::max(batch, 1), 0);
-      int64_t cur_tokens = 0, cur_n = 0;
-      auto close = [&]() {
-        for (const Spec& c : cur)
-          for (int32_t r : c.reqs) in_group[r] = 0;
-        if ((int64_t)cur.size() >= m.group_min_members && cur_n > small_tile) {
-          Spec g;
-          int64_t start = 0;
-          for (Spec& c : cur) {
-            g.ranges.insert(g.ranges.end(), c.ranges.begin(), c.ranges.end());
-            g.reqs.insert(g.reqs.end(), c.reqs.begin(), c.reqs.end());
-            g.row_ranges.insert(g.row_ranges.end(), c.reqs.size(), std::make_pair((int32_t)start, (int32_t)(start + c.length)));
-            if (direct != nullptr) g.member_room.push_back(c.room);  // one range per member in the serving path
-            start += c.length + c.room;
-          }
-          g.length = start;
-          g.chunk = ceil_div(start, tile) * tile;
-          tail.push_back(std::move(g));
-          any_groups = true;
-        } else {
-          for (Spec& c : cur) tail.push_back(std::move(c));
+      const Packing packing = pack(cap, hard_cap);
+      std::vector<Spec> result;
+      result.reserve(packing.bundles.size());
+      for (const Bundle& b : packing.bundles) {
+        if (!b.group) {
+          result.push_back(std::move(specs[packing.order[b.begin]]));
+          continue;
         }
-        cur.clear();
-        cur_tokens = cur_n = 0;
-      };
-      for (Spec& s : specs) {
-        const int64_t nreq = (int64_t)s.reqs.size();
-        const int64_t span = s.length + s.room;
-        if (nreq <= small_tile && span <= m.group_member_tokens) {
-          bool shared = false;
-          for (int32_t r : s.reqs) shared = shared || in_group[r] != 0;
-          // (serving path: a group is closed once it has reached the cap, not before it would pass it, so that
-          // the groups number no more than the tasks they were sized for)
-          const bool full = direct != nullptr ? cur_tokens >= cap : cur_tokens + span > cap;
-          if (!cur.empty() && (cur_n + nreq > q_tile || cur_tokens + span > hard_cap || (full && cur_n > small_tile) || shared))
-            close();
-          for (int32_t r : s.reqs) in_group[r] = 1;
-          cur_tokens += span;
-          cur_n += nreq;
-          cur.push_back(std::move(s));
-        } else {
-          kept.push_back(std::move(s));
+        Spec g;
+        int64_t start = 0;
+        for (size_t k = b.begin; k < b.end; ++k) {
+          const Spec& c = specs[packing.order[k]];
+          g.ranges.insert(g.ranges.end(), c.ranges.begin(), c.ranges.end());
+          g.reqs.insert(g.reqs.end(), c.reqs.begin(), c.reqs.end());
+          g.row_ranges.insert(g.row_ranges.end(), c.reqs.size(), std::make_pair((int32_t)start, (int32_t)(start + c.length)));
+          if (direct != nullptr) g.member_room.push_back(c.room);  // one range per member in the serving path
+          start += c.length + c.room;
         }
+        g.length = start;
+        g.chunk = group_chunk(start);
+        result.push_back(std::move(g));
+        any_groups = true;
       }
-      close();
-      specs.swap(kept);
-      for (Spec& t : tail) specs.push_back(std::move(t));
+      specs.swap(result);
     }
 
     if (direct == nullptr) {  // tail split
