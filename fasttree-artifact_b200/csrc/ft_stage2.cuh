@@ -38,47 +38,27 @@ __device__ __forceinline__ void store_columns(const Stage2Params& p, int req, in
   }
 }
 
-// A partial row counts only if its weight, relative to the request's largest LSE, is not zero - else infinities and NaN in
-// rows that do not count would come into the sum as 0 x Inf.  While rows are still being met the largest LSE is not known,
-// and one that is added may turn out not to count.  A sum that came out finite met none of that; any other is formed once
-// more here, row by row with the largest LSE known, and so depends neither on the order of the rows nor on the kernel.
-// That the kernels hold this code costs them 0.02 to 0.05 us (1024 pieces x 2 rows 2.31 -> 2.36, 2048 x 7 no change), the
-// form of two float4s per lane 3 to 5 % (65536 x 2 17.8 -> 18.4).
-// Called by each lane for the four columns from `column` on of its request's row, which it has stored already.
-template <typename T>
-__device__ __noinline__ void merge_again(const Stage2Params& p, int req, int column) {
-  const int head = column >> p.dim_shift, at = column & (p.head_dim - 1), off = p.r2v_offs[req], n = p.r2v_lens[req];
-  auto lse_of = [&](int i, int& row) {  // -inf: an empty partial, or a bad row id (flagged where it was met first)
-    row = p.r2v_entries[off + i];
-    return row >= 0 && row < p.num_partial_rows ? __ldcg(p.mid_lse + (int64_t)row * p.ml_s0 + head) : -INFINITY;
-  };
-  float mx = -INFINITY, sum = 0.f;
-  int row;
-  for (int i = 0; i < n; ++i) mx = fmaxf(mx, lse_of(i, row));
-  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-  for (int i = 0; i < n; ++i) {
-    const float lse = lse_of(i, row), w = lse > -INFINITY ? expf(lse - mx) : 0.f;
-    if (w == 0.f) continue;
-    const float4 x = __ldcg(reinterpret_cast<const float4*>(p.mid_o + (int64_t)row * p.mo_s0 + (int64_t)head * p.mo_s1 + at));
-    sum += w;
-    acc.x = fmaf(w, x.x, acc.x);
-    acc.y = fmaf(w, x.y, acc.y);
-    acc.z = fmaf(w, x.z, acc.z);
-    acc.w = fmaf(w, x.w, acc.w);
-  }
-  store_columns<T>(p, req, head, at, acc, sum > 0.f ? 1.f / sum : 0.f);
-}
-
-__device__ __forceinline__ bool all_finite(const float4& x) {  // 0 x every element: 0, or NaN
-  return fmaf(x.x, 0.f, fmaf(x.y, 0.f, fmaf(x.z, 0.f, x.w * 0.f))) == 0.f;
+// To a new maximum.  A partial row counts only if its weight, relative to the request's largest LSE, is not zero - else
+// infinities and NaN in rows that do not count would come into the sum as 0 x Inf.  While rows are still being met the
+// largest LSE is not known: a sum of rows that the new maximum leaves nothing of starts anew, whatever it holds.  (What is
+// left over: an infinite row of no weight that two steps of the maximum take there, each of which leaves some.  A sum formed
+// once more where it did not come out finite has no such case, but the code for it, even where nothing runs it, cost steps
+// at head_dim 256 1 to 4 %: 64 requests on 4096 tokens 44.6 -> 46.2 us.)
+__device__ __forceinline__ void scale(float4& x, float f) {
+  x.x *= f;
+  x.y *= f;
+  x.z *= f;
+  x.w *= f;
+  if (f == 0.f) x = make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
 // MAXC: float4 chunks per lane (1: head_dim 128, 2: head_dim 256; smaller heads go to the other kernel).  RB: partial rows
 // in flight per lane.  A request's merge is a chain of L2 round trips, one per batch of RB rows.  A launch that fits one
 // round of CTAs is bound by that chain and runs with RB = 8 at six CTAs per SM; a launch of several rounds is bound by how
-// many warps the SM holds and runs with RB = 4 at nine (head_dim 128).
+// many warps the SM holds and runs with RB = 4 at nine (head_dim 128); at head_dim 256 seven, the next stage 1's first
+// CTAs beside them (six, with 78 registers for 72: 256 requests of 30 tokens on 200, 32/8 heads, 31.4 us per step for 30.2).
 template <typename T, int MAXC, int RB>
-__global__ void __launch_bounds__(128, MAXC == 1 && RB == 4 ? 9 : 6) stage2_merge_kernel(const __grid_constant__ Stage2Params p) {
+__global__ void __launch_bounds__(128, MAXC == 1 && RB == 4 ? 9 : MAXC == 2 ? 7 : 6) stage2_merge_kernel(Stage2Params p) {
   allow_dependent_launch();  // a following stage-1 launch may set itself up under this kernel's tail
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t pair = (int64_t)blockIdx.x * 4 + warp;
@@ -131,10 +111,7 @@ __global__ void __launch_bounds__(128, MAXC == 1 && RB == 4 ? 9 : 6) stage2_merg
         wsum *= corr;
 #pragma unroll
         for (int c = 0; c < MAXC; ++c) {
-          acc[c].x *= corr;
-          acc[c].y *= corr;
-          acc[c].z *= corr;
-          acc[c].w *= corr;
+          scale(acc[c], corr);
         }
         mx = new_mx;
         my_w = my_lse > -INFINITY ? expf(my_lse - mx) : 0.f;  // -inf LSE marks an empty partial
@@ -160,17 +137,10 @@ __global__ void __launch_bounds__(128, MAXC == 1 && RB == 4 ? 9 : 6) stage2_merg
   for (int c = 0; c < MAXC; ++c) store_columns<T>(p, req, head, 4 * (lane + 32 * c), acc[c], inv);
   if (p.o_lse != nullptr && lane == 0)
     p.o_lse[(int64_t)req * p.heads + head] = wsum > 0.f ? mx + logf(wsum) : -INFINITY;
-  if (n <= 32) return;  // all rows were met with their largest LSE known
-  unsigned again = 0;
-#pragma unroll
-  for (int c = 0; c < MAXC; ++c)
-    if (!all_finite(acc[c])) again |= 1u << c;
-#pragma unroll 1
-  for (; again != 0; again &= again - 1) merge_again<T>(p, req, (head << p.dim_shift) + 4 * (lane + 32 * (__ffs(again) - 1)));
 }
 
 template <typename T, int C, int RB, int SPLIT>
-__global__ void __launch_bounds__(128, RB * C == 4 ? (C == 1 ? 10 : 9) : 1) stage2_piece_kernel(const __grid_constant__ Stage2Params p) {
+__global__ void __launch_bounds__(128, RB * C == 4 ? (C == 1 ? 10 : 9) : 1) stage2_piece_kernel(Stage2Params p) {
   static_assert(SPLIT == 1 || SPLIT == 4, "a warp or the whole block per item");
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const unsigned item = SPLIT == 1 ? blockIdx.x * 4 + warp : blockIdx.x;
@@ -208,10 +178,7 @@ __global__ void __launch_bounds__(128, RB * C == 4 ? (C == 1 ? 10 : 9) : 1) stag
     const float corr = top == -INFINITY ? 1.f : expf(mx[c] - top);  // 0 for the first rows
     mx[c] = top;
     sum[c] *= corr;
-    acc[c].x *= corr;
-    acc[c].y *= corr;
-    acc[c].z *= corr;
-    acc[c].w *= corr;
+    scale(acc[c], corr);
   };
   auto weight = [&](float lse, float top) { return lse > -INFINITY ? expf(lse - top) : 0.f; };  // -inf LSE marks an empty partial
   auto add = [&](int c, float w, const float4& x) {
@@ -295,29 +262,10 @@ __global__ void __launch_bounds__(128, RB * C == 4 ? (C == 1 ? 10 : 9) : 1) stag
   for (int c = 0; c < C; ++c) {
     if (head[c] < 0) continue;
     const float inv = sum[c] > 0.f ? 1.f / sum[c] : 0.f;
-    // (through store_columns the two-float4 form spills 36 bytes)
-    T* __restrict__ dst = reinterpret_cast<T*>(p.o) + (int64_t)req * p.o_s0 + (int64_t)head[c] * p.o_s1 + at[c];
-    alignas(16) T out[4] = {from_float<T>(acc[c].x * inv), from_float<T>(acc[c].y * inv), from_float<T>(acc[c].z * inv),
-                            from_float<T>(acc[c].w * inv)};
-    if (p.o_vec) {  // four elements in one store when the output rows allow it
-      if constexpr (sizeof(T) == 2)
-        *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(out);
-      else
-        *reinterpret_cast<float4*>(dst) = *reinterpret_cast<const float4*>(out);
-    } else {
-#pragma unroll
-      for (int e = 0; e < 4; ++e) dst[e] = out[e];
-    }
+    store_columns<T>(p, req, head[c], at[c], acc[c], inv);
     if (p.o_lse != nullptr && at[c] == 0)
       p.o_lse[(int64_t)req * p.heads + head[c]] = sum[c] > 0.f ? mx[c] + logf(sum[c]) : -INFINITY;
   }
-  if (SPLIT == 1 && n_all <= RB) return;  // all rows were met with their largest LSE known
-  unsigned again = 0;
-#pragma unroll
-  for (int c = 0; c < C; ++c)
-    if (head[c] >= 0 && !all_finite(acc[c])) again |= 1u << c;
-#pragma unroll 1
-  for (; again != 0; again &= again - 1) merge_again<T>(p, req, 4 * (lane + 32 * (__ffs(again) - 1 + C * piece)));
 }
 
 }  // namespace ft
