@@ -698,6 +698,10 @@ int launch_pieces(ft::Stage2Params p, cudaStream_t st, bool after_stage1) {
 //   fewer rows: weights by every lane              16384 heads of 64 x 3.4 9.0 -> 4.9 (step 37.0 -> 33.1), 8192 x 4 6.1 -> 5.6
 //   very many pieces: two of them per warp         65536 x 2 33.8 -> 21.2, 32768 x 3 20.9 -> 17.0 (one piece 18.7)
 // At head_dim 64 and below one lane per row would leave half of the lanes and more idle: 8192 pieces x 18 rows 19.3 / 13.8.
+// At head_dim 256 a head is two pieces, and weights that every lane computes are computed twice as often as by heads: by pieces
+// only where they are few (by pieces / by heads: 1536 x 2 2.57 / 2.71, 2048 x 2 2.74 / 2.78, 4096 x 4 3.61 / 3.27, 8192 x 3
+// 4.91 / 3.77, 32000 x 3 13.8 / 10.1; 103 requests of 30 tokens on 200, 32/8 heads, 17.2 / 16.2 per step; 233
+// drawn steps of more than 1024 pieces 0.93 to 1.097 of the time by heads, 1.011 in the mean).
 template <typename T>
 int launch_stage2(const ft::Stage2Params& p, int64_t rows, cudaStream_t st, bool after_stage1) {
   const int64_t pieces = (((int64_t)p.batch * p.heads << p.dim_shift) + 127) / 128, heads = (int64_t)p.batch * p.heads;
@@ -708,7 +712,7 @@ int launch_stage2(const ft::Stage2Params& p, int64_t rows, cudaStream_t st, bool
   int dev = 0;
   FT_CUDA_OK(cudaGetDevice(&dev));
   const bool one_round = heads <= 24LL * sm_count(dev);
-  if (p.head_dim >= 128 && ((one_round && rows > 4 * batch) || rows >= 6 * batch)) {
+  if (p.head_dim >= 128 && ((one_round && rows > 4 * batch) || rows >= 6 * batch || (p.head_dim > 128 && pieces > 1024))) {
     auto* kernel = p.head_dim > 128 ? ft::stage2_merge_kernel<T, 2, 4> : one_round ? ft::stage2_merge_kernel<T, 1, 8> : ft::stage2_merge_kernel<T, 1, 4>;
     return launch_merge(kernel, p, (heads + 3) / 4, st, after_stage1);
   }

@@ -23,12 +23,12 @@ def _strided(x, inner):
     (40, 5, 16, 16, torch.bfloat16, 0, True),       # ... on the quarter that the last head leaves, rows in strides
     (9, 3, 256, 26, torch.float16, 1, True),        # four warps, a head in two pieces
     (40, 5, 256, 3, torch.float32, 0, False),       # a warp per piece at head_dim 256
-    (300, 9, 256, 2, torch.bfloat16, 3, True),
+    (50, 9, 256, 2, torch.bfloat16, 3, True),
     (50, 7, 64, 5, torch.float16, 1, True),         # a warp per piece, the last one half full
     (6000, 3, 128, 3, torch.float16, 0, False),     # two float4s per lane, the last piece without its second one
     (6700, 5, 64, 3, torch.bfloat16, 1, True),      # ... the last piece a quarter full
-    (1030, 17, 256, 2, torch.float32, 3, False),
     (60, 6, 128, 14, torch.float16, 3, True),       # a warp per head, scalar stores and strided rows
+    (1030, 17, 256, 2, torch.float32, 3, False),    # ... at head_dim 256
     (70, 6, 256, 12, torch.bfloat16, 1, True),
 ])
 def test_merge_at_ragged_pieces_and_strides(batch, heads, d, most, dtype, spare_o, strided_mid):
