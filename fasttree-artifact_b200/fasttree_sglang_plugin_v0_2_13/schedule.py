@@ -138,10 +138,11 @@ def _upload(md, tabs, last_vnodes, tail_state=None, src_table=None):
     md.phase_node_nums = list(tabs["phase_node_nums"])
     sizes = tabs.get("task_sizes") or _planner.task_sizes(tabs["phase_node_nums"], tabs["vnode_to_kv_lens"],
                                                           tabs["vnode_to_q_lens"], md.kv_group_num)
-    if not md.graph_safe:
-        # The plan's rows, far fewer than the buffers': the merge kernel is chosen by their number (512 requests 13 270 ->
-        # 13 150 us per burst).  A captured step has to fit every later plan and to give what an eager call gives.
-        sizes = (*sizes, int(rows))
+    # The plan's rows, far fewer than the buffers': the merge kernel is chosen by their number (512 requests 13 270 ->
+    # 13 150 us per burst).  A captured step has to fit every later plan and to give what an eager call gives: six rows per
+    # request, which for few requests picks the form that is never far behind (us per step, the buffers' rows / six stated:
+    # 12 requests of 3 rows at 32/8 heads 12.9 / 11.5, 24 of 6 at 28/4 14.7 / 11.4, 12 of 25 at 28/4 14.9 / 15.1).
+    sizes = (*sizes, 6 * int(bsz) if md.graph_safe else int(rows))
     md.vnode_to_kv_lens.task_sizes = sizes
     md.phase_node_offsets = list(tabs["phase_node_offsets"])
     md.req_last_vnodes = [int(v) for v in last_vnodes]

@@ -48,11 +48,11 @@ def test_spare_rows_change_nothing(sizes, lens, hq, hkv, dtype):
 
 @pytest.mark.parametrize("planner,graph_safe", [("b200", False), ("reference", False), ("b200", True)])
 def test_a_serving_plan_states_its_rows(planner, graph_safe):
-    """... but not to a launch that is captured for all plans."""
+    """... and six per request where the launch is captured for all plans, not the buffers' capacity."""
     for name in sorted(plugin_cases.CASES):
         batch, _rows, hq, hkv = plugin_cases.build(name)
         md = metadata.FastTreeMetadata(hq, hkv, 128, "cpu", max_vnodes=4096, max_vnode_to_q_entries=8192, max_batch_size=512,
                                        planner=planner, graph_safe=graph_safe)
         schedule.prepare_for_fasttree_meta(batch, md)
         assert md.num_partial_rows < md.mid_o.shape[0]
-        assert md.vnode_to_kv_lens.task_sizes[4:] == (() if graph_safe else (md.num_partial_rows,))
+        assert md.vnode_to_kv_lens.task_sizes[4:] == ((6 * len(batch.reqs),) if graph_safe else (md.num_partial_rows,))
