@@ -492,28 +492,33 @@ int build_plan(const int32_t* parent, const int32_t* seqlen, int32_t n_nodes, co
           if (fill <= hard_cap) cap = std::max(cap, fill);
         }
         // That size, or a half, three quarters or one and a half times as much where there are groups then too, no more
-        // partial rows for the merge, and a schedule of the step, its tail split included, that ends a twentieth and two and a
-        // half units sooner.  Of 680 drawn trees with groups 122 take another size, 1.12 times as fast together; two steps
-        // of 11.4 us are 4 and 5 % slower though their stage 1 alone is quicker, one of 56 is 3 % slower; of 250 others 38, 1.12
-        // times as fast, none slower.  At the tail split's costs, rows allowed to grow, 264 of the 680 took another size, eighteen
-        // of which were 3 to 24 % slower.
+        // partial rows for the merge, and a schedule of the step, its tail split included, that ends clearly sooner: a
+        // twentieth and two and a half units at the finer costs and, for longer groups, a twentieth at the tail split's too;
+        // for shorter ones that twentieth and a group's tile at the finer costs will do.  Of 780 drawn trees with groups 206
+        // take another size, 1.092 times as fast together; four are 3 to 19 % slower.  (The tail split's costs alone, rows
+        // allowed to grow: 232, 1.086 times, thirteen slower; the finer costs alone: 120, 1.107 times, three slower.)
         const int64_t base = cap, base_hard = hard_cap;
-        int64_t first_end = 0, best_end = 0, first_rows = 0;
+        int64_t first_end = 0, first_fine = 0, best_fine = 0, first_rows = 0;
         for (const int64_t quarters : {4, 2, 3, 6}) {
           const int64_t size = std::max(base * quarters / 4 / tile * tile, 2 * tile), hard = std::max(base_hard, size);
           std::vector<Piece> pieces = sizes_of(pack(size, hard));
           const bool any = std::any_of(pieces.begin(), pieces.end(), [](const Piece& p) { return p.group; });
           if (quarters == 4 && !any) break;
-          split_tail(pieces);
+          const int64_t end = split_tail(pieces);
           std::vector<int64_t> last_end;
           int64_t rows = 0, total = 0;
           for (const Piece& p : pieces) rows += p.nreq * ceil_div(p.length, p.chunk);
-          const int64_t end = simulate(pieces, {{28, 16}, 4, 5, true}, last_end, total);
+          const int64_t fine = simulate(pieces, {{28, 16}, 4, 5, true}, last_end, total);
           if (quarters == 4) {
-            first_end = best_end = end;
+            first_end = end;
+            first_fine = best_fine = fine;
             first_rows = rows;
-          } else if (any && rows <= first_rows && end * 21 <= first_end * 20 && end + 10 <= first_end && end < best_end) {
-            best_end = end;
+            continue;
+          }
+          const bool sooner = end * 20 <= first_end * 19, clearly = fine * 21 <= first_fine * 20 && fine + 10 <= first_fine;
+          if (any && rows <= first_rows && fine < best_fine &&
+              (quarters > 4 ? sooner && clearly : clearly || (sooner && fine + 5 <= first_fine))) {
+            best_fine = fine;
             cap = size;
             hard_cap = hard;
           }

@@ -531,21 +531,27 @@ def b200_sized_groups(vnodes, q_tile, small_tile, m, target_tokens, num_kv_heads
     """:func:`b200_group_short_nodes` at the size it computes, or at a half, three
     quarters or one and a half times as much where there are groups then too, no more
     partial rows for the merge, and a schedule of the step, its tail split included,
-    that ends a twentieth and ten of its units sooner."""
+    that ends clearly sooner: a twentieth and ten units at :data:`GROUP_COST` and, for
+    longer groups, a twentieth at :data:`CUT_COST` too; for shorter ones that twentieth
+    and five units at :data:`GROUP_COST`, a group's tile, will do."""
     slots = max((m.num_sms * m.ctas_per_sm) // max(num_kv_heads, 1), 1)
-    best = best_end = first_end = first_rows = None
+    best = best_fine = first = None
     for quarters in GROUP_CAPS:
         packed = b200_group_short_nodes(vnodes, q_tile, small_tile, m, target_tokens, num_kv_heads=num_kv_heads, quarters=quarters)
         any_group = any(vn.row_ranges is not None for vn in packed)
         if best is None and not any_group:
             return packed
         split = b200_split_tail(packed, q_tile, small_tile, m, num_kv_heads)
-        end = b200_simulated_schedule(split, q_tile, small_tile, m, slots, GROUP_COST)[0]
+        end = b200_simulated_schedule(split, q_tile, small_tile, m, slots)[0]
+        fine = b200_simulated_schedule(split, q_tile, small_tile, m, slots, GROUP_COST)[0]
         rows = sum(len(vn.requests) * -(-sum(e - b for b, e in vn.kv_ranges) // vn.kv_split) for vn in split)
         if best is None:
-            best, best_end, first_end, first_rows = packed, end, end, rows
-        elif any_group and rows <= first_rows and end * 21 <= first_end * 20 and end + 10 <= first_end and end < best_end:
-            best, best_end = packed, end
+            best, best_fine, first = packed, fine, (rows, end, fine)
+            continue
+        sooner, clearly = end * 20 <= first[1] * 19, fine * 21 <= first[2] * 20 and fine + 10 <= first[2]
+        if any_group and rows <= first[0] and fine < best_fine and \
+                (sooner and clearly if quarters > 4 else clearly or (sooner and fine + 5 <= first[2])):
+            best, best_fine = packed, fine
     return best
 
 

@@ -79,7 +79,6 @@ def test_another_group_size_needs_no_more_scratch_than_there_is(monkeypatch, siz
     ([1, 2, 4, 8, 26], [61, 244, 25, 8, 59], 32, 8, 256, 4),          # 1.11
     ([1, 179], [740, 9], 16, 16, 128, 4),                             # 1.11
     ([1, 2, 25], [1218, 63, 9], 64, 8, 128, 4),                       # 1.07: half as many rows again for the merge
-    ([1, 3, 99], [109, 30, 29], 64, 8, 128, 4),                       # 1.05
 ])
 def test_a_group_size_that_runs_slower_is_not_taken(monkeypatch, sizes, lens, hq, hkv, d, quarters):
     nodes = kv_tree_simple.tree_from_rows(tree_generation.generate_tree(sizes, lens))

@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("sizes,lens,hq,hkv,d", [
-    ([1, 235], [2430, 110], 28, 4, 64), ([1, 385], [1908, 44], 32, 8, 64), ([1, 166], [1899, 44], 32, 8, 256),
+    ([1, 235], [2430, 110], 28, 4, 64), ([1, 1, 186, 311], [32, 34, 91, 14], 64, 8, 64), ([1, 166], [1899, 44], 32, 8, 256),
     ([1, 156], [1976, 41], 24, 8, 256),
 ])
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16], ids=["fp16", "bf16"])
